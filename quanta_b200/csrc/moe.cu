@@ -15,7 +15,7 @@
 //   expert e on row x: down_e( silu(gate_e x) * up_e x ), times w, summed over the k slots in slot
 //   order by the next norm kernel (src/quanta/minimax/moe.py:59-88); or, ungated (MODE 3 below),
 //   down_e( relu(up_e x)^2 ).
-#include "common.cuh"
+#include "rows_f32.cuh"
 
 // values of the `renorm` argument of the routing kernels: how the chosen experts are weighted
 #define QB_ROUTE_SIGMOID_RAW 0        // sigmoid scores as they are
@@ -786,15 +786,272 @@ __global__ void moe_grouped_simt_kernel(const X* __restrict__ x, const W* __rest
   }
 }
 
+// What a product leaves behind for one (row, feature): `g` the sum (MODE 1: gate) and `u` the up sum.
+template <int MODE>
+__device__ __forceinline__ float mg_result(float g, float u, float w, int act_kind, float act_limit, float act_alpha) {
+  if (MODE == 2) return w * g;
+  if (MODE == 3) { g = fmaxf(g, 0.f); return g * g; }
+  if (act_kind == 1) {
+    g = fminf(g * w, act_limit);
+    u = fminf(fmaxf(u * w, -act_limit), act_limit);
+    return g / (1.f + expf(-act_alpha * g)) * (u + 1.f);
+  }
+  return g / (1.f + expf(-g)) * u;
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same products in float32 for steps of at most CAP tokens, so at most CAP rows an expert: bound by the bytes of the chosen
+// experts, read once (rows_f32.cuh).  Four tokens, five or six experts of 2,048 x 2,816, both products: 615 us with the kernel
+// above (a block waits for 4 to 8 KB at a time), 75 us with this one (69 us of bytes at 6.0 TB/s).
+// ---------------------------------------------------------------------------------------------
+constexpr int MR_WARPS = 4;
+
+struct MoeRows {
+  const float *x, *weights, *pair_w;
+  float* out;
+  const int* sorted_pair;
+  int top_k, K, N, act_kind;
+  float act_limit, act_alpha;
+};
+
+extern __shared__ __align__(16) float moe_smem[];
+
+template <int MODE, int FW, int U, int R, bool COPIED>
+__device__ __forceinline__ void moe_rows_run(const MoeRows& a, int e, int row0, int rows, int n0, int lane) {
+  constexpr int NF = MODE == 1 ? FW / 2 : FW;              // features a warp; MODE 1 reads a gate and an up row for each
+  constexpr int V = NF * R;
+  const float* wbase = a.weights + (size_t)e * (MODE == 1 ? 2 : 1) * a.N * a.K;
+  const float* wr[FW];
+#pragma unroll
+  for (int f = 0; f < FW; ++f) {
+    const int n = min(n0 + f % NF, a.N - 1);
+    wr[f] = wbase + (size_t)(f < NF ? n : a.N + n) * a.K;
+  }
+  const float* xr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = min(r, rows - 1), p = row0 + i;
+    xr[r] = COPIED ? moe_smem + (size_t)i * a.K : a.x + (size_t)(MODE == 2 ? p : a.sorted_pair[p] / a.top_k) * a.K;
+  }
+  auto x = [&](int r, int k) {
+    return COPIED ? *reinterpret_cast<const float4*>(xr[r] + k) : __ldg(reinterpret_cast<const float4*>(xr[r] + k));
+  };
+  float acc[FW][R];
+  qb_rows_dot<FW, R, U>(wr, x, [] { if (COPIED) qb_rows_ready(); }, a.K, lane, acc);
+  float g[V], u[MODE == 1 ? V : 1];                         // index r * NF + f
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      g[r * NF + f] = acc[f][r];
+      if (MODE == 1) u[r * NF + f] = acc[(MODE == 1 ? NF : 0) + f][r];
+    }
+  const int first = qb_sum_values<V>(g, lane);
+  if (MODE == 1) qb_sum_values<MODE == 1 ? V : 1>(u, lane);
+  if (!qb_sum_stores<V>(lane)) return;
+  constexpr int HELD = V > 32 ? V / 32 : 1;
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) {
+    const int r = (first + i) / NF, n = n0 + (first + i) % NF;
+    if (r >= rows || n >= a.N) continue;
+    const int p = row0 + r, pair = a.sorted_pair[p];
+    const float w = a.pair_w != nullptr ? a.pair_w[pair] : 1.f;
+    a.out[(size_t)(MODE == 2 ? pair : p) * a.N + n] =
+        mg_result<MODE>(g[i], MODE == 1 ? u[MODE == 1 ? i : 0] : 0.f, w, a.act_kind, a.act_limit, a.act_alpha);
+  }
+}
+
+template <int MODE, int FW, int U, int CAP, bool COPIED>
+__global__ void __launch_bounds__(MR_WARPS * 32)
+moe_rows_kernel(MoeRows a, const int* __restrict__ plan, const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, int E,
+                int turn) {
+  const int tile = blockIdx.y;
+  if (tile >= plan[3 * E + 1]) return;
+  const int lane = threadIdx.x & 31;
+  const int n0 = (blockIdx.x * MR_WARPS + (threadIdx.x >> 5)) * (MODE == 1 ? FW / 2 : FW);     // past N: nothing is stored
+  const int e = tile_expert[tile], row0 = tile_row0[tile];
+  const int rows = min(plan[2 * E + e + 1] - row0, MG_BM);
+  for (int g = 0; g < rows; g += turn) {                    // `turn` <= CAP rows at a time: what the shared memory was asked for
+    const int n = min(rows - g, turn);
+    if (COPIED) {
+      if (g) __syncthreads();
+      qb_rows_copy(moe_smem, [&](int r) {
+        const int p = row0 + g + r;
+        return a.x + (size_t)(MODE == 2 ? p : a.sorted_pair[p] / a.top_k) * a.K;
+      }, n, a.K);
+    }
+    if (n <= 1) moe_rows_run<MODE, FW, U, 1, COPIED>(a, e, row0 + g, n, n0, lane);
+    else if (n <= 2) moe_rows_run<MODE, FW, U, 2, COPIED>(a, e, row0 + g, n, n0, lane);
+    else if (CAP <= 4 || n <= 4) moe_rows_run<MODE, FW, U, 4, COPIED>(a, e, row0 + g, n, n0, lane);
+    else if (n <= 8) moe_rows_run<MODE, FW, U, 8, COPIED>(a, e, row0 + g, n, n0, lane);
+    else moe_rows_run<MODE, FW, U, CAP, COPIED>(a, e, row0 + g, n, n0, lane);
+  }
+}
+
+template <int MODE, int FW, int U, int CAP>
+static int moe_rows_launch(const MoeRows& a, const int* plan, const int* tile_expert, const int* tile_row0, int max_tiles, int E,
+                           int max_rows, cudaStream_t stream) {
+  constexpr int PER_BLOCK = MR_WARPS * (MODE == 1 ? FW / 2 : FW);
+  const dim3 grid((a.N + PER_BLOCK - 1) / PER_BLOCK, max_tiles);
+  const int turn = min(max_rows, CAP), smem = qb_rows_smem(turn, a.K);
+  if (smem > 0) {
+    static const cudaError_t once = cudaFuncSetAttribute(moe_rows_kernel<MODE, FW, U, CAP, true>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, QB_ROWS_SMEM);
+    if (once != cudaSuccess) return (int)once;
+    moe_rows_kernel<MODE, FW, U, CAP, true><<<grid, MR_WARPS * 32, smem, stream>>>(a, plan, tile_expert, tile_row0, E, turn);
+  } else {
+    moe_rows_kernel<MODE, FW, U, CAP, false><<<grid, MR_WARPS * 32, 0, stream>>>(a, plan, tile_expert, tile_row0, E, turn);
+  }
+  QB_LAUNCH_CHECK();
+  return 0;
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same products in float32 for more tokens.  A tile is 32 sorted rows x 128 weight rows (MODE 1: 64 gate and 64 up), a thread
+// 4 x 8 sums.  Slices of 16 of the inner dimension arrive by asynchronous copies, three ahead of the one in use, as they lie in
+// memory (80 bytes a row, an odd number of 16-byte units: eight rows' reads meet no bank twice).  Bound by shared memory: twelve
+// 16-byte reads a thread for 128 FMAs.  1,000 tokens, two of eight experts of 2,048 x 2,816: 1,150 + 644 us (40 and 36 TFLOP/s; 8 x 8
+// sums a thread, whose registers leave eight warps an SM, 1,269 + 622 us; packed pairs of sums 1,226 + 688 us; the general kernel
+// above 2,221 + 2,042 us).  Each sum is sequential over the inner dimension, as in the general kernel above.
+// ---------------------------------------------------------------------------------------------
+constexpr int MT_BN = 128, MT_BK = 16, MT_LD = MT_BK + 4, MT_STAGES = 4;
+constexpr int MT_COPIES = (MG_BM + MT_BN) / 32;
+constexpr int MT_STAGE = (MG_BM + MT_BN) * MT_LD;
+constexpr int MT_SMEM = MT_STAGES * MT_STAGE * (int)sizeof(float);
+
+__device__ __forceinline__ void mt_copy16(float* dst, const float* src, bool ok) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  const int n = ok ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(128, 4)
+moe_tile_f32_kernel(MoeRows a, const int* __restrict__ plan, const int* __restrict__ tile_expert, const int* __restrict__ tile_row0,
+                    int E) {
+  extern __shared__ __align__(16) float mt_smem[];
+  const int tile = blockIdx.y;
+  if (tile >= plan[3 * E + 1]) return;
+  constexpr int BF = MODE == 1 ? MT_BN / 2 : MT_BN;         // features a block
+  const int e = tile_expert[tile], row0 = tile_row0[tile], row_end = plan[2 * E + e + 1];
+  const int n0 = blockIdx.x * BF, tid = threadIdx.x, K = a.K, N = a.N;
+  const float* wbase = a.weights + (size_t)e * (MODE == 1 ? 2 : 1) * N * K;
+  // copies: thread (c, q) takes the 16 bytes q of the rows c, c + 32, ...: rows 0 .. 31 are the inputs, then the weights
+  const int c = tid >> 2, q = (tid & 3) * 4;
+  const float* src[MT_COPIES];
+  bool ok[MT_COPIES];
+#pragma unroll
+  for (int i = 0; i < MT_COPIES; ++i) {
+    if (i == 0) {
+      const int p = row0 + c;
+      ok[i] = p < row_end;
+      const int row = MODE == 2 ? p : (ok[i] ? a.sorted_pair[p] / a.top_k : 0);
+      src[i] = a.x + (ok[i] ? (size_t)row * K : 0);
+    } else {
+      const int r = c + 32 * (i - 1), n = n0 + (MODE == 1 ? r % 64 : r);
+      ok[i] = n < N;
+      src[i] = wbase + (ok[i] ? (size_t)(MODE == 1 && r >= 64 ? N + n : n) * K : 0);
+    }
+  }
+  auto fetch = [&](int s) {
+    const int k = s * MT_BK + q;
+    float* st = mt_smem + (s % MT_STAGES) * MT_STAGE;
+#pragma unroll
+    for (int i = 0; i < MT_COPIES; ++i) mt_copy16(st + (c + 32 * i) * MT_LD + q, src[i] + (k < K ? k : 0), ok[i] && k < K);
+  };
+  const int steps = (K + MT_BK - 1) / MT_BK;
+#pragma unroll
+  for (int s = 0; s < MT_STAGES - 1; ++s) {
+    if (s < steps) fetch(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // warps 2 x 2, lanes 4 x 8: thread rows tm + 8 i, weight rows tn + 16 j (MODE 1: j < 4 gate, j >= 4 up of the same features)
+  const int lane = tid & 31, warp = tid >> 5;
+  const int tm = (warp & 1) * 4 + (lane >> 3), tn = (warp >> 1) * 8 + (lane & 7);
+  float acc[4][8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(MT_STAGES - 2) : "memory");
+    __syncthreads();
+    if (s + MT_STAGES - 1 < steps) fetch(s + MT_STAGES - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* xs = mt_smem + (s % MT_STAGES) * MT_STAGE;
+    const float* ws = xs + MG_BM * MT_LD;
+#pragma unroll
+    for (int kk = 0; kk < MT_BK; kk += 4) {
+      float4 xv[4], wv[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) xv[i] = *reinterpret_cast<const float4*>(xs + (tm + 8 * i) * MT_LD + kk);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) wv[j] = *reinterpret_cast<const float4*>(ws + (tn + 16 * j) * MT_LD + kk);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          acc[i][j] = fmaf(xv[i].x, wv[j].x, acc[i][j]);
+          acc[i][j] = fmaf(xv[i].y, wv[j].y, acc[i][j]);
+          acc[i][j] = fmaf(xv[i].z, wv[j].z, acc[i][j]);
+          acc[i][j] = fmaf(xv[i].w, wv[j].w, acc[i][j]);
+        }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int p = row0 + tm + 8 * i;
+    if (p >= row_end) continue;
+    const int pair = a.sorted_pair[p];
+    const float w = a.pair_w != nullptr ? a.pair_w[pair] : 1.f;
+    float* orow = a.out + (size_t)(MODE == 2 ? pair : p) * N;
+#pragma unroll
+    for (int j = 0; j < (MODE == 1 ? 4 : 8); ++j) {
+      const int n = n0 + tn + 16 * j;
+      if (n < N)
+        orow[n] = mg_result<MODE>(acc[i][j], MODE == 1 ? acc[i][MODE == 1 ? j + 4 : j] : 0.f, w, a.act_kind, a.act_limit, a.act_alpha);
+    }
+  }
+}
+
+template <int MODE>
+static int moe_grouped_f32(const MoeRows& a, const int* plan, const int* tile_expert, const int* tile_row0, int max_tiles, int E,
+                           int max_rows, int mean_rows, cudaStream_t stream) {
+  // by rows up to eight an expert on average: 24 tokens, two of eight experts of 2,048 x 2,816 (mean 6) 110 + 74 us by rows, 184 + 115 by
+  // tiles; 64 tokens (mean 16) 201 + 140 by rows, 187 + 118 by tiles
+  if (max_rows <= 4) return moe_rows_launch<MODE, 2, 4, 4>(a, plan, tile_expert, tile_row0, max_tiles, E, max_rows, stream);
+  if (mean_rows <= 8) return moe_rows_launch<MODE, 4, 2, 16>(a, plan, tile_expert, tile_row0, max_tiles, E, max_rows, stream);
+  {
+    static const cudaError_t once = cudaFuncSetAttribute(moe_tile_f32_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM);
+    if (once != cudaSuccess) return (int)once;
+    constexpr int BF = MODE == 1 ? MT_BN / 2 : MT_BN;
+    moe_tile_f32_kernel<MODE><<<dim3((a.N + BF - 1) / BF, max_tiles), 128, MT_SMEM, stream>>>(a, plan, tile_expert, tile_row0, E);
+  }
+  QB_LAUNCH_CHECK();
+  return 0;
+}
+
 // x: [T, H] activations (MODE 1) or [pairs, I] act rows (MODE 2).
 extern "C" int qb_moe_grouped_simt(int mode, const void* x, int x_dtype, const void* weights, int w_dtype,
                                    void* out, int out_dtype, const int* sorted_pair, const float* pair_w,
                                    const int* plan, const int* tile_expert, const int* tile_row0,
-                                   int max_tiles, int E, int top_k, int K, int N, int act_kind, float act_limit,
+                                   int max_tiles, int E, int top_k, int K, int N, int n_pairs, int act_kind, float act_limit,
                                    float act_alpha, cudaStream_t stream) {
   if (max_tiles <= 0) return 0;
   if (act_kind < 0 || act_kind > 1 || (act_kind == 1 && (mode != 1 || pair_w == nullptr))) return QB_ERR_BAD_ARG;
   if (max_tiles > 65535) return QB_ERR_UNSUPPORTED;
+  // all float32 with rows of whole 16-byte pieces: the two kernels above.  A router gives a token an expert once, so an expert has
+  // at most n_pairs / top_k rows (were there more, they would be taken in turns).
+  if (x_dtype == QB_F32 && w_dtype == QB_F32 && out_dtype == QB_F32 && K % 4 == 0 &&
+      ((uintptr_t)x & 15) == 0 && ((uintptr_t)weights & 15) == 0) {
+    const MoeRows a{(const float*)x, (const float*)weights, pair_w, (float*)out, sorted_pair, top_k, K, N,
+                    act_kind, act_limit, act_alpha};
+    const int max_rows = n_pairs / top_k, mean_rows = n_pairs / E;
+    if (mode == 1) return moe_grouped_f32<1>(a, plan, tile_expert, tile_row0, max_tiles, E, max_rows, mean_rows, stream);
+    if (mode == 2) return moe_grouped_f32<2>(a, plan, tile_expert, tile_row0, max_tiles, E, max_rows, mean_rows, stream);
+    if (mode == 3) return moe_grouped_f32<3>(a, plan, tile_expert, tile_row0, max_tiles, E, max_rows, mean_rows, stream);
+    return QB_ERR_BAD_ARG;
+  }
   dim3 grid((N + MG_BN - 1) / MG_BN, max_tiles);
   QB_DISPATCH_DTYPE(x_dtype, X, QB_DISPATCH_DTYPE(w_dtype, W, QB_DISPATCH_DTYPE(out_dtype, O, {
     if (mode == 1)

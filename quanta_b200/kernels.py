@@ -519,6 +519,20 @@ def identity_slots(x, idx, w, y, first_identity: int) -> None:
            "identity_slots")
 
 
+LINEAR_ROWS_MAX = 16
+
+
+def linear_rows(x, w, out) -> None:
+    """``out [n, N] = x [n, K] @ w [N, K].T`` in float32 for at most ``LINEAR_ROWS_MAX`` rows; K a multiple of 4, ``x`` and ``w``
+    on 16 bytes."""
+    for t, name in ((x, "x"), (w, "w"), (out, "out")):
+        _want(t, torch.float32, name)
+    n, K = x.shape
+    if w.shape[1] != K or tuple(out.shape) != (n, w.shape[0]):
+        raise ValueError("linear_rows: shape mismatch")
+    _check(lib().qb_linear_rows(_p(x), _p(w), _p(out), n, K, w.shape[0], _stream()), "linear_rows")
+
+
 EXPERT_ACT_SILU, EXPERT_ACT_CLAMPED = 0, 1
 
 
@@ -537,8 +551,8 @@ def moe_grouped_simt(mode: int, x, weights, out, sorted_pair, pair_w, plan, tile
         raise ValueError(f"moe_grouped: weights {tuple(weights.shape)} do not fit {n_experts} experts of {want}")
     _check(lib().qb_moe_grouped_simt(mode, _p(x), _code(x), _p(weights), _code(weights), _p(out), _code(out),
                                      _p(sorted_pair), _p(pair_w), _p(plan), _p(tile_expert), _p(tile_row0),
-                                     tile_expert.numel(), n_experts, top_k, K, N, int(act[0]), ctypes.c_float(act[1]),
-                                     ctypes.c_float(act[2]), _stream()), "moe_grouped_simt")
+                                     tile_expert.numel(), n_experts, top_k, K, N, sorted_pair.numel(), int(act[0]),
+                                     ctypes.c_float(act[1]), ctypes.c_float(act[2]), _stream()), "moe_grouped_simt")
 
 
 def expert_gemm_tc_supported(x: torch.Tensor, hidden: int, inner: int) -> bool:

@@ -9,6 +9,8 @@ from __future__ import annotations
 
 import torch
 
+from . import kernels
+
 _configured = False
 
 
@@ -44,11 +46,22 @@ def _with_spare_rows(x: torch.Tensor) -> torch.Tensor:
     return x
 
 
+def _few_float32_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether ``kernels.linear_rows`` takes the product: a few float32 rows, bound by the bytes of ``w``."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.is_cuda and x.dim() == 2
+            and 0 < x.shape[0] <= kernels.LINEAR_ROWS_MAX and x.shape[1] % 4 == 0 and x.is_contiguous() and w.is_contiguous()
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
     """``x [T, in] @ w [out, in].T``; accumulation is float32; ``out_dtype`` float32 keeps the
     accumulator's precision for bfloat16 operands.  An ``x`` from ``empty_rows`` is multiplied with its
     spare rows and the result cut back to ``T`` rows."""
     n = x.shape[0]
+    if _few_float32_rows(x, w):
+        out = torch.empty((n, w.shape[0]), dtype=torch.float32, device=x.device)
+        kernels.linear_rows(x, w, out)
+        return out
     xp = _with_spare_rows(x)
     if xp is not x:
         return linear(xp, w, out_dtype)[:n]
