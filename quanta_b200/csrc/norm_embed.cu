@@ -68,6 +68,24 @@ extern "C" int qb_embedding(float* h, const void* table, int table_dtype, const 
 }
 
 // ---------------------------------------------------------------------------------------------
+// Rows of whole 32-byte pieces (H a multiple of 8, at most 8 x 1,024): a thread keeps its 8 elements in registers from the first
+// load to the store, so a row passes memory once and shared memory holds the warps' sums alone; everything a row needs (gains too)
+// is asked for before the first sum, so that a row is one wait for memory and one or two block sums.  Threads: H / 8, whole
+// warps.
+// ---------------------------------------------------------------------------------------------
+static int row_threads(int H) { return (H / 8 + 31) / 32 * 32; }
+static bool row_in_registers(int H, int most) { return H % 8 == 0 && H <= 8 * most; }
+
+// Sum over the block, warps in index order; `scratch` (32 floats) is used by no other sum.
+__device__ __forceinline__ float row_sum(float v, float* scratch) {
+  const int lane = threadIdx.x & 31, n = blockDim.x >> 5;
+  v = qb_warp_sum(v);
+  if (lane == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return qb_warp_sum(lane < n ? scratch[lane] : 0.f);
+}
+
+// ---------------------------------------------------------------------------------------------
 // row r (token rows[r] if rows != null, else r):
 //   x = h[tok,:] + sum_s delta[tok,s,:]          (float32, s ascending)
 //   if store_h: h[tok,:] = x
@@ -145,10 +163,55 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const D* __restrict__ 
   }
 }
 
+// The same for rows in registers.  Measured on a B200 against the kernel above at 12,800 rows of 3,072: bfloat16 delta 128 -> 75 us
+// (470 MB), eight float32 slots (1.7 GB) 262 -> 233 us; one row of eight slots 3.7 -> 3.1 us.
+template <typename D, typename O>
+__global__ void add_rmsnorm_rows_kernel(float* __restrict__ h, const D* __restrict__ delta, int S, const float* __restrict__ w,
+                                        O* __restrict__ out, const int* __restrict__ rows, int H, float eps, int store_h) {
+  __shared__ float scratch[32];
+  const int r = blockIdx.x, tok = rows ? rows[r] : r, i = threadIdx.x * 8;
+  const bool in = i < H;
+  float x[8], g[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] = g[e] = 0.f;
+  if (in) {
+    float* hrow = h + (size_t)tok * H;
+    QbVec8<float>::load(hrow + i, x);
+    if (out != nullptr) QbVec8<float>::load(w + i, g);
+    if (delta != nullptr) {
+      const D* drow = delta + (size_t)tok * S * H + i;
+#pragma unroll 8
+      for (int s = 0; s < S; ++s) {
+        float dv[8];
+        QbVec8<D>::load(drow + (size_t)s * H, dv);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] += dv[e];
+      }
+      if (store_h) QbVec8<float>::store(hrow + i, x);
+    }
+  }
+  if (out == nullptr) return;
+  float ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) ss += x[e] * x[e];
+  const float r_inv = rsqrtf(row_sum(ss, scratch) / (float)H + eps);
+  if (!in) return;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] = g[e] * (x[e] * r_inv);
+  QbVec8<O>::store(out + (size_t)r * H + i, x);
+}
+
 extern "C" int qb_add_rmsnorm(float* h, const void* delta, int delta_dtype, int S, const float* w,
                               void* out, int out_dtype, const int* rows, int n_rows, int H, float eps,
                               int store_h, cudaStream_t stream) {
   if (n_rows <= 0) return 0;
+  if (row_in_registers(H, 1024) && (((uintptr_t)h | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
+    QB_DISPATCH_DTYPE(delta_dtype, D, QB_DISPATCH_DTYPE(out_dtype, O, {
+      add_rmsnorm_rows_kernel<D, O><<<n_rows, row_threads(H), 0, stream>>>(h, (const D*)delta, S, w, (O*)out, rows, H, eps, store_h);
+    }));
+    QB_LAUNCH_CHECK();
+    return 0;
+  }
   const size_t smem = (size_t)(H + 32) * sizeof(float);
   if (smem > 200 * 1024) return QB_ERR_UNSUPPORTED;
   const int threads = H >= 2048 ? 512 : 256;
@@ -222,6 +285,75 @@ __global__ void normed_add_rmsnorm_kernel(float* __restrict__ h, const float* __
   for (int i = threadIdx.x; i < H; i += blockDim.x) orow[i] = qb_from_float<O>(w[i] * (row_buf[i] * r_inv));
 }
 
+// The same for rows in registers.  Measured on a B200 against the kernel above: 4,876 rows of 2,048 with two slots and a second
+// summand (240 MB) 87 -> 46 us, with one slot (160 MB) 56 -> 30 us, 8 rows 4.3 -> 2.9 us.
+template <typename O>
+__global__ void normed_add_rmsnorm_rows_kernel(float* __restrict__ h, const float* __restrict__ y, int S, float y_scale,
+                                               const float* __restrict__ y_bias, const float* __restrict__ y2, float y2_scale,
+                                               const float* __restrict__ y2_bias, const float* __restrict__ g, float eps_y,
+                                               const float* __restrict__ w, O* __restrict__ out, const int* __restrict__ rows,
+                                               int H, float eps, int store_h) {
+  __shared__ float scratch_y[32], scratch[32];
+  const int r = blockIdx.x, tok = rows ? rows[r] : r, i = threadIdx.x * 8;
+  const bool in = i < H;
+  float x[8], v[8], gv[8], wv[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] = v[e] = gv[e] = wv[e] = 0.f;
+  float* hrow = h + (size_t)tok * H + i;
+  if (in) {
+    QbVec8<float>::load(hrow, x);
+    if (w != nullptr && out != nullptr) QbVec8<float>::load(w + i, wv);
+    if (y != nullptr) {
+      QbVec8<float>::load(g + i, gv);
+      const float* yrow = y + (size_t)tok * S * H + i;
+      QbVec8<float>::load(yrow, v);
+#pragma unroll 4
+      for (int s = 1; s < S; ++s) {
+        float t[8];
+        QbVec8<float>::load(yrow + (size_t)s * H, t);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] += t[e];
+      }
+      if (y_bias != nullptr) {
+        float t[8];
+        QbVec8<float>::load(y_bias + i, t);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] += t[e];
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] *= y_scale;
+      if (y2 != nullptr) {
+        float t[8], b[8];
+        QbVec8<float>::load(y2 + (size_t)tok * H + i, t);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) b[e] = 0.f;
+        if (y2_bias != nullptr) QbVec8<float>::load(y2_bias + i, b);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = fmaf(y2_scale, t[e] + b[e], v[e]);
+      }
+    }
+  }
+  if (y != nullptr) {
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
+    const float y_inv = rsqrtf(row_sum(ss, scratch_y) / (float)H + eps_y);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] += gv[e] * (v[e] * y_inv);
+    if (store_h && in) QbVec8<float>::store(hrow, x);
+  }
+  if (out == nullptr) return;
+  if (w != nullptr) {
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += x[e] * x[e];
+    const float r_inv = rsqrtf(row_sum(ss, scratch) / (float)H + eps);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = wv[e] * (x[e] * r_inv);
+  }
+  if (in) QbVec8<O>::store(out + (size_t)r * H + i, x);
+}
+
 extern "C" int qb_normed_add_rmsnorm(float* h, const float* y, int S, float y_scale, const float* y_bias,
                                      const float* y2, float y2_scale, const float* y2_bias, const float* g,
                                      float eps_y, const float* w, void* out,
@@ -229,6 +361,16 @@ extern "C" int qb_normed_add_rmsnorm(float* h, const float* y, int S, float y_sc
                                      cudaStream_t stream) {
   if (n_rows <= 0) return 0;
   if (S < 1 || (y != nullptr && g == nullptr)) return QB_ERR_BAD_ARG;
+  const uintptr_t all = (uintptr_t)h | (uintptr_t)y | (uintptr_t)y_bias | (uintptr_t)y2 | (uintptr_t)y2_bias | (uintptr_t)g |
+                        (uintptr_t)w | (uintptr_t)out;
+  if (row_in_registers(H, 1024) && (all & 15) == 0) {
+    QB_DISPATCH_DTYPE(out_dtype, O, {
+      normed_add_rmsnorm_rows_kernel<O><<<n_rows, row_threads(H), 0, stream>>>(
+          h, y, S, y_scale, y_bias, y2, y2_scale, y2_bias, g, eps_y, w, (O*)out, rows, H, eps, store_h);
+    });
+    QB_LAUNCH_CHECK();
+    return 0;
+  }
   const size_t smem = (size_t)(H + 32) * sizeof(float);
   if (smem > 200 * 1024) return QB_ERR_UNSUPPORTED;
   const int threads = H >= 2048 ? 512 : 256;
@@ -259,8 +401,31 @@ __global__ void silu_mul_kernel(const A* __restrict__ gu, A* __restrict__ out, i
   }
 }
 
+// Rows of whole 16-byte pieces: eight elements a thread, the row is the block's y.  Measured on a B200: 4,876 rows of 5,632 in
+// bfloat16 (165 MB) 87 us with one element a thread and a division to find its row, 29 us with this.
+template <typename A>
+__global__ void silu_mul_rows_kernel(const A* __restrict__ gu, A* __restrict__ out, int n_rows, int I) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (c >= I) return;
+  for (int r = blockIdx.y; r < n_rows; r += gridDim.y) {
+    float g[8], u[8];
+    QbVec8<A>::load(gu + (size_t)r * 2 * I + c, g);
+    QbVec8<A>::load(gu + (size_t)r * 2 * I + I + c, u);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) g[e] = g[e] / (1.f + expf(-g[e])) * u[e];
+    QbVec8<A>::store(out + (size_t)r * I + c, g);
+  }
+}
+
 extern "C" int qb_silu_mul(const void* gu, void* out, int dtype, int n_rows, int I, cudaStream_t stream) {
   if (n_rows <= 0) return 0;
+  if (I % 8 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0) {
+    const int threads = (size_t)n_rows * I >= 1u << 20 ? 256 : 64;        // few rows: more blocks, so more SMs
+    const dim3 grid((I / 8 + threads - 1) / threads, n_rows < 32768 ? n_rows : 32768);
+    QB_DISPATCH_DTYPE(dtype, A, silu_mul_rows_kernel<A><<<grid, threads, 0, stream>>>((const A*)gu, (A*)out, n_rows, I));
+    QB_LAUNCH_CHECK();
+    return 0;
+  }
   const size_t n = (size_t)n_rows * I;
   const int blocks = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
   QB_DISPATCH_DTYPE(dtype, A, silu_mul_kernel<A><<<blocks, 256, 0, stream>>>((const A*)gu, (A*)out, n_rows, I));

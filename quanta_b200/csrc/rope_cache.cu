@@ -217,6 +217,191 @@ __global__ void qknorm_rope_write_kernel(
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same for heads of 128: a warp takes a head, four elements a lane, and keeps its HPW heads of the token in registers from the
+// load to the store (the kernel above passes every row through shared memory four times).  Pairs (j, j + rd/2) meet by a shuffle,
+// neighbours lie in one lane.  One barrier.  Bound by one wait for memory for few tokens and by instructions for many (some 90 a
+// head; blocks that walk tokens with the next row and the gains at hand were slower, 212 us for 12,800 tokens, for the warps
+// they cost).  Measured on a B200 with 48 + 8 + 8 heads in bfloat16 and a norm over all heads: one token 7.7 -> 4.6 us, 64 tokens
+// 7.7 -> 4.7, 536 tokens 13.4 -> 8.9, 12,800 tokens (420 MB) 248 -> 165 us; 16 + 4 heads from float32 with biases, neighbours turned: 16 tokens 4.8 -> 2.9 us,
+// 4,876 tokens 37 -> 16 us.
+// ---------------------------------------------------------------------------------------------
+template <typename T> struct Four;
+template <> struct Four<float> {
+  __device__ static __forceinline__ float4 load(const float* p) { return *reinterpret_cast<const float4*>(p); }
+  __device__ static __forceinline__ void store(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+};
+template <> struct Four<__nv_bfloat16> {
+  __device__ static __forceinline__ float4 load(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+  }
+  __device__ static __forceinline__ void store(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+  }
+};
+
+struct RopeArgs {
+  int row_stride, norm_kind, n_axes, bt_stride, nq, nkv, tied_v, rd, interleaved, temp_every, page_size, page_shift, num_pages;
+  float eps, temp_coef;
+  const float *q_norm_w, *k_norm_w, *inv_freq, *bias, *v_first, *v_lambda, *head_scale;
+  const int *pair_axis, *positions, *tok_pos, *tok_req, *block_table;
+  float* v_export;
+  int* status;
+};
+
+constexpr int ROPE_HD = 128;
+
+template <typename IN, typename A, int HPW>
+__global__ void __launch_bounds__(HPW == 2 ? 1024 : 512, HPW == 2 ? 1 : 2)      // 64 registers: with 85 the 12,800 tokens take 276 us
+qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
+                         const RopeArgs a) {
+  __shared__ __align__(16) float s_cos[ROPE_HD / 2], s_sin[ROPE_HD / 2];
+  __shared__ float s_sum[32 * HPW];
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int nq = a.nq, nk = nq + a.nkv, n = nk + (a.tied_v ? 0 : a.nkv), half = a.rd / 2, d = lane * 4;
+  const bool writes = k_cache != nullptr, normed = a.norm_kind != NORM_NONE, gained = normed && a.q_norm_w != nullptr;
+  const IN* row = qkv + (size_t)t * a.row_stride + d;
+  int pos = 0, page = -1;                // asked for first: a chain of dependent loads
+  if (writes || a.temp_every > 0) pos = a.tok_pos[t];
+  auto gains = [&](int h) {              // of a q or k head
+    const float* g = h < nq ? a.q_norm_w : a.k_norm_w;
+    return Four<float>::load(g + (a.norm_kind == NORM_PER_LAYER ? (h < nq ? h : h - nq) * ROPE_HD : 0) + d);
+  };
+  // few tokens: the gains come from memory that the layer's weights have pushed out of L2 and are asked for now; many: from L1
+  constexpr bool EARLY = HPW == 2;
+  float4 v[HPW], w[EARLY ? HPW : 1];
+#pragma unroll
+  for (int i = 0; i < HPW; ++i) {
+    const int h = warp + i * warps;
+    v[i] = h < n ? Four<IN>::load(row + h * ROPE_HD) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (EARLY && gained && h < nk) w[EARLY ? i : 0] = gains(h);
+  }
+  if (writes) {
+    const int nth = a.page_shift >= 0 ? pos >> a.page_shift : pos / a.page_size;
+    page = a.block_table[(size_t)a.tok_req[t] * a.bt_stride + nth];
+  }
+  for (int j = threadIdx.x; j < half; j += blockDim.x) {
+    const int ax = a.pair_axis ? a.pair_axis[j] : 0;
+    const float ang = (float)a.positions[(size_t)t * a.n_axes + ax] * a.inv_freq[j];
+    sincosf(ang, &s_sin[j], &s_cos[j]);
+  }
+  if (a.bias != nullptr) {
+#pragma unroll
+    for (int i = 0; i < HPW; ++i) {
+      const int h = warp + i * warps;
+      if (h < n) {
+        const float4 b = Four<float>::load(a.bias + h * ROPE_HD + d);
+        v[i] = make_float4(v[i].x + b.x, v[i].y + b.y, v[i].z + b.z, v[i].w + b.w);
+      }
+    }
+  }
+  float ss[HPW];
+  if (normed) {
+#pragma unroll
+    for (int i = 0; i < HPW; ++i) ss[i] = qb_warp_sum(v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w);
+    if (a.norm_kind == NORM_PER_LAYER && lane == 0) {
+#pragma unroll
+      for (int i = 0; i < HPW; ++i) s_sum[warp + i * warps] = ss[i];
+    }
+  }
+  __syncthreads();
+  float rq = 1.f, rk = 1.f;
+  if (a.norm_kind == NORM_PER_LAYER) {
+    float tq = 0.f, tk = 0.f;
+    for (int h = lane; h < nk; h += 32) {
+      const float s = s_sum[h];
+      tq += h < nq ? s : 0.f;
+      tk += h < nq ? 0.f : s;
+    }
+    rq = rsqrtf(qb_warp_sum(tq) / (float)(nq * ROPE_HD) + a.eps);
+    rk = rsqrtf(qb_warp_sum(tk) / (float)max(a.nkv * ROPE_HD, 1) + a.eps);
+  }
+  const float temp = a.temp_every > 0 ? 1.f + a.temp_coef * logf((float)((pos + 1) / a.temp_every) + 1.f) : 1.f;
+  // this lane's pairs: cos and sin of pair j .. j + 3 (halves: the first turns by a c - b s, so its sines change sign), or of j and j + 1
+  // (neighbours)
+  const bool turns = d < a.rd, upper = d >= half;
+  float4 c4 = make_float4(1.f, 1.f, 1.f, 1.f), s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (turns) {
+    if (a.interleaved) {
+      c4.x = s_cos[d / 2]; c4.y = s_cos[d / 2 + 1];
+      s4.x = s_sin[d / 2]; s4.y = s_sin[d / 2 + 1];
+    } else {
+      const int j = upper ? d - half : d;
+      c4 = *reinterpret_cast<const float4*>(&s_cos[j]);
+      s4 = *reinterpret_cast<const float4*>(&s_sin[j]);
+      if (!upper) s4 = make_float4(-s4.x, -s4.y, -s4.z, -s4.w);
+    }
+  }
+  const int partner = turns && !a.interleaved ? (upper ? lane - half / 4 : lane + half / 4) : lane;
+  const bool cache = writes && page >= 0 && page < a.num_pages;
+  const int slot = a.page_shift >= 0 ? pos & (a.page_size - 1) : pos % a.page_size;
+  const size_t at = ((size_t)(cache ? page : 0) * a.nkv * a.page_size + slot) * ROPE_HD + d;      // of kv head 0
+  const int head_step = a.page_size * ROPE_HD;
+  A* q_row = q_out + (size_t)t * nq * ROPE_HD + d;
+#pragma unroll
+  for (int i = 0; i < HPW; ++i) {
+    const int h = warp + i * warps;          // the same for the whole warp
+    if (h >= n) continue;
+    const int hv = h - (a.tied_v ? nq : nk);
+    if (cache && hv >= 0) {                  // values go out as they are (blended with an earlier layer's where asked)
+      float4 x = v[i];
+      const size_t own = ((size_t)t * a.nkv + hv) * ROPE_HD + d;
+      if (a.v_export != nullptr) Four<float>::store(a.v_export + own, x);
+      if (a.v_first != nullptr) {
+        const float lam = a.v_lambda[0];
+        const float4 f = Four<float>::load(a.v_first + own);
+        x = make_float4((1.f - lam) * x.x + lam * f.x, (1.f - lam) * x.y + lam * f.y, (1.f - lam) * x.z + lam * f.z,
+                        (1.f - lam) * x.w + lam * f.w);
+      }
+      Four<A>::store(v_cache + at + hv * head_step, x);
+    }
+    if (h >= nk) continue;
+    float4 x = v[i];
+    if (normed) {
+      const float r = a.norm_kind == NORM_PER_LAYER ? (h < nq ? rq : rk) : rsqrtf(ss[i] / (float)ROPE_HD + a.eps);
+      x = make_float4(x.x * r, x.y * r, x.z * r, x.w * r);
+      if (gained) {
+        const float4 g = EARLY ? w[EARLY ? i : 0] : gains(h);
+        x = make_float4(g.x * x.x, g.y * x.y, g.z * x.z, g.w * x.w);
+      }
+    }
+    if (a.interleaved) {
+      if (turns) x = make_float4(x.x * c4.x - x.y * s4.x, x.y * c4.x + x.x * s4.x, x.z * c4.y - x.w * s4.y, x.w * c4.y + x.z * s4.y);
+    } else if (half > 0) {
+      const float4 o = make_float4(__shfl_sync(0xffffffffu, x.x, partner), __shfl_sync(0xffffffffu, x.y, partner),
+                                   __shfl_sync(0xffffffffu, x.z, partner), __shfl_sync(0xffffffffu, x.w, partner));
+      if (turns) x = make_float4(x.x * c4.x + o.x * s4.x, x.y * c4.y + o.y * s4.y, x.z * c4.z + o.z * s4.z, x.w * c4.w + o.w * s4.w);
+    }
+    if (h < nq) {
+      if (a.temp_every > 0 || a.head_scale != nullptr) {
+        const float m = a.head_scale != nullptr ? temp * a.head_scale[h] : temp;
+        x = make_float4(x.x * m, x.y * m, x.z * m, x.w * m);
+      }
+      Four<A>::store(q_row + h * ROPE_HD, x);
+    } else if (cache) {
+      Four<A>::store(k_cache + at + (h - nq) * head_step, x);
+    }
+  }
+  if (writes && !cache && threadIdx.x == 0) qb_set_status(a.status, QB_STATUS_BAD_PAGE, page, 2);
+}
+
+template <typename IN, typename A>
+static void qknorm_rope_heads(const void* qkv, void* q_out, void* k_cache, void* v_cache, const RopeArgs& a, int T, cudaStream_t stream) {
+  const int heads = a.nq + a.nkv * (a.tied_v ? 1 : 2);
+  // few tokens: two heads a warp, so that a token is one short wait; many: four or eight loads in flight a lane
+  const int hpw = T <= 64 && heads <= 64 ? 2 : heads <= 32 ? 4 : 8;
+  const int threads = (heads + hpw - 1) / hpw * 32;
+#define QB_HEADS(N) \
+  qknorm_rope_heads_kernel<IN, A, N><<<T, threads, 0, stream>>>((const IN*)qkv, (A*)q_out, (A*)k_cache, (A*)v_cache, a)
+  if (hpw == 2) QB_HEADS(2);
+  else if (hpw == 4) QB_HEADS(4);
+  else QB_HEADS(8);
+#undef QB_HEADS
+}
+
 extern "C" int qb_qknorm_rope_write(
     const void* qkv, int in_dtype, int dtype, int row_stride, void* q_out, void* k_cache, void* v_cache, const float* q_norm_w,
     const float* k_norm_w, int norm_kind, float eps, const float* inv_freq, const int* pair_axis,
@@ -238,6 +423,24 @@ extern "C" int qb_qknorm_rope_write(
   if (row_stride < nq * hd + nk * (hd + (tied_v ? 0 : vd))) return QB_ERR_BAD_ARG;
   // rows are moved in 16-byte pieces where every piece starts on such a boundary; else element by element
   const int vec = (hd % 8 == 0 && vd % 8 == 0 && row_stride % 8 == 0 && ((uintptr_t)qkv & 15) == 0) ? 1 : 0;
+  // heads of 128, pairs that fall on whole lanes, every address on a lane's piece; at most 16 warps of eight heads
+  const uintptr_t all = (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)q_norm_w | (uintptr_t)k_norm_w |
+                        (uintptr_t)bias | (uintptr_t)v_first | (uintptr_t)v_export;
+  if (vec && hd == ROPE_HD && vd == ROPE_HD && (interleaved ? rd % 4 : rd % 8) == 0 && (all & 15) == 0 &&
+      nq + nk * (tied_v ? 1 : 2) <= 128) {
+    int shift = -1;
+    for (int i = 0; i < 31; ++i)
+      if (page_size == 1 << i) shift = i;
+    const RopeArgs a{row_stride, norm_kind, n_axes, bt_stride, nq, nk, tied_v, rd, interleaved, temp_every, page_size, shift, num_pages,
+                     eps, temp_coef, q_norm_w, k_norm_w, inv_freq, bias, v_first, v_lambda, head_scale,
+                     pair_axis, positions, tok_pos, tok_req, block_table, v_export, status};
+    if (dtype == QB_F32) qknorm_rope_heads<float, float>(qkv, q_out, k_cache, v_cache, a, T, stream);
+    else if (dtype == QB_BF16 && in_dtype == QB_F32) qknorm_rope_heads<float, __nv_bfloat16>(qkv, q_out, k_cache, v_cache, a, T, stream);
+    else if (dtype == QB_BF16) qknorm_rope_heads<__nv_bfloat16, __nv_bfloat16>(qkv, q_out, k_cache, v_cache, a, T, stream);
+    else return QB_ERR_BAD_ARG;
+    QB_LAUNCH_CHECK();
+    return 0;
+  }
   const size_t smem = (size_t)((nq + nk) * hd + rd + 32 + nq + nk) * sizeof(float);
   if (smem > 200 * 1024) return QB_ERR_UNSUPPORTED;
 #define QB_ROPE_LAUNCH(IN, A)                                                                                   \
