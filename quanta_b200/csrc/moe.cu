@@ -47,8 +47,9 @@ __device__ __forceinline__ void select_topk(const float (&logit)[NPL], const flo
                                             int* __restrict__ idx_row, float* __restrict__ w_row, float* s_score,
                                             int E, int k, int renorm, float scale, int* s_idx = nullptr) {
   const int lane = threadIdx.x & 31;
-  float choice[NPL], score[NPL];
-  unsigned taken = 0u;
+  // a choice as an unsigned number of the same order; 0, below every float, for what is taken or does not exist
+  float score[NPL];
+  unsigned key[NPL];
   float all_max = -INFINITY, all_inv = 0.f;
   if (renorm == QB_ROUTE_SOFTMAX_ALL) {
     // the softmax over all router outputs: maximum, then the sum in lane order, then a butterfly
@@ -66,49 +67,40 @@ __device__ __forceinline__ void select_topk(const float (&logit)[NPL], const flo
   for (int i = 0; i < NPL; ++i) {
     const int e = lane + 32 * i;
     score[i] = 0.f;
+    key[i] = 0u;
     if (e < E) {
       const float x = logit[i];
+      float choice;
       if (renorm == QB_ROUTE_SOFTMAX_CHOSEN) {
-        score[i] = choice[i] = x + bias[i];
+        score[i] = choice = x + bias[i];
       } else if (renorm == QB_ROUTE_SOFTMAX_ALL) {
         score[i] = expf(x - all_max) * all_inv;
-        choice[i] = score[i] + bias[i];
+        choice = score[i] + bias[i];
       } else {
         const float s = 1.f / (1.f + expf(-x));
         score[i] = s;
-        choice[i] = s + bias[i];
+        choice = s + bias[i];
       }
-    } else {
-      choice[i] = -INFINITY;
-      taken |= 1u << i;
+      const unsigned u = __float_as_uint(choice + 0.f);        // one zero
+      key[i] = u & 0x80000000u ? ~u : u | 0x80000000u;
     }
   }
   float sum = 0.f, first = 0.f;
+#pragma unroll 1
   for (int r = 0; r < k; ++r) {
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
+    unsigned top = key[0];
 #pragma unroll
-    for (int i = 0; i < NPL; ++i) {
-      // i ascending is expert index ascending within the lane: the first maximum wins a tie
-      if (!((taken >> i) & 1u) && (bi == 0x7fffffff || choice[i] > bv)) {
-        bv = choice[i];
-        bi = lane + 32 * i;
-      }
-    }
+    for (int i = 1; i < NPL; ++i) top = max(top, key[i]);
+    top = __reduce_max_sync(0xffffffffu, top);
+    unsigned at = 0x7fffffffu;                          // the lowest expert among equals
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      const bool take = (oi != 0x7fffffff) && (bi == 0x7fffffff || ov > bv || (ov == bv && oi < bi));
-      if (take) { bv = ov; bi = oi; }
-    }
+    for (int i = NPL - 1; i >= 0; --i)
+      if (key[i] == top) at = lane + 32 * i;
+    const int bi = (int)__reduce_min_sync(0xffffffffu, at);
     float mine = 0.f;
-    if ((bi & 31) == lane) {
-      taken |= 1u << (bi >> 5);
 #pragma unroll
-      for (int i = 0; i < NPL; ++i)
-        if (i == (bi >> 5)) mine = score[i];
-    }
+    for (int i = 0; i < NPL; ++i)
+      if (bi == lane + 32 * i) { mine = score[i]; key[i] = 0u; }
     float sc = __shfl_sync(0xffffffffu, mine, bi & 31);     // the bias-free score of the chosen expert
     if (renorm == QB_ROUTE_SOFTMAX_CHOSEN) {                // the first chosen value is the largest
       if (r == 0) first = sc;
@@ -400,6 +392,73 @@ __device__ __forceinline__ float4 rs_load4(const __nv_bfloat16* p) {      // a b
                      __uint_as_float(raw.y & 0xffff0000u));
 }
 
+// The end of a router block: its experts' logits from the quarters' sums, and with `select` the selection by the block that finishes a
+// token tile last and the plan by the block that finishes the last tile.
+template <int NPL, int EPB>
+__device__ __forceinline__ void router_finish(const float* s_quarter, PlanShared& sh, float (&s_score)[RS_WARPS][256], int* s_chosen,
+                                              int* s_last, const float* __restrict__ bias, float* logits, int* idx_out,
+                                              float* __restrict__ w_out, int T, int E, int k, int renorm, float scale, int select,
+                                              int* counters, int BM, int* __restrict__ plan, int* __restrict__ sorted_pair,
+                                              int* __restrict__ tile_expert, int* __restrict__ tile_row0, int max_tiles, int* status,
+                                              int tiled) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int t0 = blockIdx.y * RS_TT, nt = min(RS_TT, T - t0);
+  __syncthreads();
+  if (tid < EPB * RS_TT) {
+    const int l2 = tid / RS_TT, t = tid % RS_TT, ee = blockIdx.x * EPB + l2;
+    if (ee < E && t < nt) {
+      float v = s_quarter[(l2 * RS_QUARTERS) * RS_TT + t];
+#pragma unroll
+      for (int q = 1; q < RS_QUARTERS; ++q) v += s_quarter[(l2 * RS_QUARTERS + q) * RS_TT + t];
+      __stcg(logits + (size_t)(t0 + t) * E + ee, v);
+    }
+  }
+  if (!select) return;
+  // the selecting warps will want the bias: fetched now, under the hand-over below
+  float my_bias[NPL];
+  lane_bias<NPL>(bias, E, my_bias);
+  // ---- the last block of this token tile selects ----
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    const int before = atomicAdd(&counters[1 + blockIdx.y], 1);
+    *s_last = before == (int)gridDim.x - 1;
+    if (*s_last) counters[1 + blockIdx.y] = 0;      // every other block of the tile has counted already
+  }
+  __syncthreads();
+  if (!*s_last) return;
+  __threadfence();
+  for (int t = warp; t < nt; t += RS_WARPS) {
+    float logit[NPL];
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) {
+      const int ee = lane + 32 * i;
+      logit[i] = ee < E ? __ldcg(logits + (size_t)(t0 + t) * E + ee) : 0.f;
+    }
+    select_topk<NPL>(logit, my_bias, idx_out + (size_t)(t0 + t) * k, w_out + (size_t)(t0 + t) * k, s_score[warp], E, k,
+                     renorm, scale, (gridDim.y == 1 && k <= 32) ? s_chosen + t * k : nullptr);
+  }
+  // ---- the block that finishes the last tile lays the plan down ----
+  __syncthreads();
+  if (gridDim.y > 1) {
+    if (tid == 0) {
+      __threadfence();
+      const int before = atomicAdd(&counters[0], 1);
+      *s_last = before == (int)gridDim.y - 1;
+      if (*s_last) counters[0] = 0;
+    }
+    __syncthreads();
+    if (!*s_last) return;
+    __threadfence();
+  }
+  if (gridDim.y == 1 && k <= 32)       // the step is this one tile: its choices are still in shared memory
+    plan_small_body<RS_WARPS * 32, true>(s_chosen, T * k, E, BM, plan, sorted_pair, tile_expert, tile_row0, max_tiles,
+                                         status, sh, [] { __syncthreads(); }, tiled);
+  else
+    plan_small_body<RS_WARPS * 32>(idx_out, T * k, E, BM, plan, sorted_pair, tile_expert, tile_row0, max_tiles, status, sh,
+                                   [] { __syncthreads(); }, tiled);
+}
+
 // KW: warps that share an expert (4: a quarter each, two experts a block, for steps of few tokens, whose
 // gate rows then come from many SMs at once; 1: a warp takes the four quarters in turn, eight experts a
 // block, so that a step of many tokens stages its rows in fewer blocks).  The sums are the same in both.
@@ -521,60 +580,88 @@ router_small_kernel(const TX* __restrict__ x, const float* __restrict__ gate, co
       }
     }
   }
-  __syncthreads();
-  if (tid < EPB * RS_TT) {
-    const int l2 = tid / RS_TT, t = tid % RS_TT, ee = blockIdx.x * EPB + l2;
-    if (ee < E && t < nt) {
-      float v = s_quarter[l2 * RS_QUARTERS][t];
+  router_finish<NPL, EPB>(&s_quarter[0][0], sh, s_score, s_chosen, &s_last, bias, logits, idx_out, w_out, T, E, k, renorm, scale, select,
+                          counters, BM, plan, sorted_pair, tile_expert, tile_row0, max_tiles, status, tiled);
+}
+
+// The same for at most RS_FEW tokens, in little code: between two steps of a layer the weights of its experts pass through the
+// caches, so a small launch fetches its instructions from far away, and the kernel above, unrolled over eight tokens and three
+// batches, spent as long on that as on anything else (`no_instruction` its first stall).  A warp's part of the gate row is in registers
+// (rows of up to 4,096; longer ones are read again for every token), tokens go by in pairs.  The same sums in the same order.
+// One token, 256 experts of 3,072: 10.8 -> 7.3 us on its own, 18.0 -> 8.1 us between the launches of a decode step; 16 tokens 15.7 -> 12.4 us.
+constexpr int RS_FEW = 16;
+
+template <typename TX>
+__global__ void __launch_bounds__(RS_WARPS * 32)
+router_few_kernel(const TX* __restrict__ x, const float* __restrict__ gate, const float* __restrict__ bias,
+                  float* logits, int* idx_out, float* __restrict__ w_out, int T, int E, int K, int k, int renorm,
+                  float scale, int select, int* counters, int BM, int* __restrict__ plan,
+                  int* __restrict__ sorted_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
+                  int max_tiles, int* status, int tiled) {
+  constexpr int EPB = RS_WARPS / RS_QUARTERS;
+  extern __shared__ __align__(16) unsigned char rs_smem[];      // [RS_TT][K] of TX: the tile's token rows
+  __shared__ PlanShared sh;
+  __shared__ float s_score[RS_WARPS][256];
+  __shared__ float s_quarter[EPB * RS_QUARTERS][RS_TT];
+  __shared__ int s_chosen[RS_TT * 32];
+  __shared__ int s_last;
+  TX* xs = reinterpret_cast<TX*>(rs_smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int t0 = blockIdx.y * RS_TT, nt = min(RS_TT, T - t0);
+  const int e = blockIdx.x * EPB + warp / RS_QUARTERS, q = warp % RS_QUARTERS;
+  const int units = K / 4, per = (units + RS_QUARTERS - 1) / RS_QUARTERS;
+  const int u0 = q * per, u1 = min(units, u0 + per);
+  const float* grow = gate + (size_t)(e < E ? e : 0) * K;
+  float4 g[RS_BATCH];
+  auto fetch = [&](int f0) {
 #pragma unroll
-      for (int q = 1; q < RS_QUARTERS; ++q) v += s_quarter[l2 * RS_QUARTERS + q][t];
-      __stcg(logits + (size_t)(t0 + t) * E + ee, v);
+    for (int u = 0; u < RS_BATCH; ++u) {
+      const int f = f0 + 32 * u;
+      g[u] = f < u1 ? *reinterpret_cast<const float4*>(grow + (size_t)f * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+  };
+  fetch(u0 + lane);                                        // into flight before anything else
+  {
+    const int n8 = nt * K * (int)sizeof(TX) / 8;
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(x + (size_t)t0 * K);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(xs);
+#pragma unroll 4
+    for (int i = tid; i < n8; i += RS_WARPS * 32)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dst + 8u * (uint32_t)i), "l"(src + 8 * (size_t)i) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
-  if (!select) return;
-  // the selecting warps will want the bias: fetched now, under the hand-over below
-  float my_bias[NPL];
-  lane_bias<NPL>(bias, E, my_bias);
-  // ---- the last block of this token tile selects ----
   __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    const int before = atomicAdd(&counters[1 + blockIdx.y], 1);
-    s_last = before == (int)gridDim.x - 1;
-    if (s_last) counters[1 + blockIdx.y] = 0;      // every other block of the tile has counted already
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (int t = warp; t < nt; t += RS_WARPS) {
-    float logit[NPL];
+  const bool one_batch = per <= 32 * RS_BATCH;
+#pragma unroll 1
+  for (int t = 0; t < nt; t += 2) {
+    const TX* xa = xs + (size_t)t * K;
+    const TX* xb = t + 1 < nt ? xa + K : xa;
+    float a = 0.f, b = 0.f;
+#pragma unroll 1
+    for (int f0 = u0 + lane; f0 < u1; f0 += 32 * RS_BATCH) {
+      if (!one_batch) fetch(f0);
 #pragma unroll
-    for (int i = 0; i < NPL; ++i) {
-      const int ee = lane + 32 * i;
-      logit[i] = ee < E ? __ldcg(logits + (size_t)(t0 + t) * E + ee) : 0.f;
+      for (int u = 0; u < RS_BATCH; ++u) {
+        const int f = f0 + 32 * u;
+        if (f < u1) {
+          const float4 va = rs_load4(xa + (size_t)f * 4), vb = rs_load4(xb + (size_t)f * 4);
+          a = fmaf(va.x, g[u].x, a); b = fmaf(vb.x, g[u].x, b);
+          a = fmaf(va.y, g[u].y, a); b = fmaf(vb.y, g[u].y, b);
+          a = fmaf(va.z, g[u].z, a); b = fmaf(vb.z, g[u].z, b);
+          a = fmaf(va.w, g[u].w, a); b = fmaf(vb.w, g[u].w, b);
+        }
+      }
     }
-    select_topk<NPL>(logit, my_bias, idx_out + (size_t)(t0 + t) * k, w_out + (size_t)(t0 + t) * k, s_score[warp], E, k,
-                     renorm, scale, (gridDim.y == 1 && k <= 32) ? s_chosen + t * k : nullptr);
-  }
-  // ---- the block that finishes the last tile lays the plan down ----
-  __syncthreads();
-  if (gridDim.y > 1) {
-    if (tid == 0) {
-      __threadfence();
-      const int before = atomicAdd(&counters[0], 1);
-      s_last = before == (int)gridDim.y - 1;
-      if (s_last) counters[0] = 0;
+    a = qb_warp_sum(a);
+    b = qb_warp_sum(b);
+    if (lane == 0) {
+      s_quarter[warp][t] = a;
+      if (t + 1 < nt) s_quarter[warp][t + 1] = b;
     }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
   }
-  if (gridDim.y == 1 && k <= 32)       // the step is this one tile: its choices are still in shared memory
-    plan_small_body<RS_WARPS * 32, true>(s_chosen, T * k, E, BM, plan, sorted_pair, tile_expert, tile_row0, max_tiles,
-                                         status, sh, [] { __syncthreads(); }, tiled);
-  else
-    plan_small_body<RS_WARPS * 32>(idx_out, T * k, E, BM, plan, sorted_pair, tile_expert, tile_row0, max_tiles, status, sh,
-                                   [] { __syncthreads(); }, tiled);
+  router_finish<8, EPB>(&s_quarter[0][0], sh, s_score, s_chosen, &s_last, bias, logits, idx_out, w_out, T, E, k, renorm, scale, select,
+                        counters, BM, plan, sorted_pair, tile_expert, tile_row0, max_tiles, status, tiled);
 }
 
 // Token rows of at most this many bytes fit the shared-memory tile.
@@ -600,11 +687,27 @@ extern "C" int qb_router_small(const void* x, int x_dtype, const float* gate, co
   if (smem > RS_MAX_TILE_BYTES) return QB_ERR_UNSUPPORTED;
   const bool vec = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)gate) & 15) == 0;      // rows start on 8 (x) and 16 (gate) bytes
   // few tokens: two experts a block (more SMs pull the gate at once); many: eight (fewer blocks stage the rows)
-  const int kw = T <= 16 ? 4 : 1;
+  const int kw = T <= RS_FEW ? 4 : 1;
   const int epb = RS_WARPS / kw;
   const dim3 grid((E + epb - 1) / epb, (T + RS_TT - 1) / RS_TT);
   if (grid.y > 65535) return QB_ERR_UNSUPPORTED;
   cudaError_t err = cudaSuccess;
+  if (vec && T <= RS_FEW) {
+#define QB_RS_FEW(TX)                                                                                                             \
+  do {                                                                                                                            \
+    err = cudaFuncSetAttribute(router_few_kernel<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                    \
+    if (err != cudaSuccess) return (int)err;                                                                                      \
+    router_few_kernel<TX><<<grid, RS_WARPS * 32, smem, stream>>>((const TX*)x, gate, bias, logits, idx_out, w_out, T, E, K, k,      \
+                                                                 renorm, scale, select, counters, BM, plan, sorted_pair,           \
+                                                                 tile_expert, tile_row0, max_tiles, status, tiled);                \
+  } while (0)
+    if (x_dtype == QB_F32) QB_RS_FEW(float);
+    else if (x_dtype == QB_BF16) QB_RS_FEW(__nv_bfloat16);
+    else return QB_ERR_BAD_ARG;
+#undef QB_RS_FEW
+    QB_LAUNCH_CHECK();
+    return 0;
+  }
 #define QB_RS(TX, N, V, KW_)                                                                                       \
   do {                                                                                                             \
     err = cudaFuncSetAttribute(router_small_kernel<TX, N, V, KW_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -613,9 +716,9 @@ extern "C" int qb_router_small(const void* x, int x_dtype, const float* gate, co
         (const TX*)x, gate, bias, logits, idx_out, w_out, T, E, K, k, renorm, scale, select, counters, BM, plan,  \
         sorted_pair, tile_expert, tile_row0, max_tiles, status, tiled);                                            \
   } while (0)
-#define QB_RS_K(TX, N, V)                                \
-  do {                                                   \
-    if (kw == 4) QB_RS(TX, N, V, 4); else QB_RS(TX, N, V, 1); \
+#define QB_RS_K(TX, N, V)                                                 \
+  do {                                                                    \
+    if (!V && kw == 4) QB_RS(TX, N, false, 4); else QB_RS(TX, N, V, 1);   \
   } while (0)
   // the selecting warp holds eight experts a lane whatever E (at most 256 here): fewer instances to compile
 #define QB_RS_E(TX, V) QB_RS_K(TX, 8, V)
