@@ -167,9 +167,37 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 //   before has finished); otherwise P V (j) needs nothing from the threads but P(j), and the threads
 //   never read O until the end.  Both threads of a row take the maximum over all 128 keys (the same
 //   decision without talking to each other) and the exponentials of their own 64.
+//
+// SPLIT: the probabilities enter P V as the sum of two bfloat16 parts (p = hi + lo: 16 bits of mantissa and not 8), two MMAs a step, for
+// the attentions whose softmax weights stay 32-bit.  The two parts of a thread's 64 keys take the 64 columns of the S buffer that the
+// thread itself has read (hi in the first 32, lo in the others), since TMEM has no room for P buffers of twice the size; the next S of
+// that buffer is issued when the P V that reads it is done, while the softmax of the other buffer runs.
+// CAP: scores pass cap * tanh(score / cap) first.  Both are for attentions over a window or inside chunks of the sequence too.
 // ------------------------------------------------------------------------------------------------
 constexpr int TCS_THREADS = 13 * 32;
 constexpr float TCS_TAU = 8.0f;
+
+// what a query at position p reads: [lo, p]
+struct TcsReach {
+  int window, chunk;
+  __device__ __forceinline__ int lo(int p) const {
+    if (chunk > 0) return p / chunk * chunk;
+    return window > 0 && p - window + 1 > 0 ? p - window + 1 : 0;
+  }
+};
+// cap * tanh(x / cap) as cap - 2 cap / (2^(x * two_over) + 1), two_over = 2 log2(e) / cap, times log2(e)
+__device__ __forceinline__ float tcs_cap(float x, float cap_log2, float two_over) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * two_over));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e + 1.f));
+  return fmaf(-2.f * cap_log2, r, cap_log2);
+}
+__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
 
 struct TcsShared {
   uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], o_full, p_full[2], p_empty[2], fin;
@@ -185,12 +213,13 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 
+template <bool SPLIT, bool CAP>
 __global__ void __launch_bounds__(TCS_THREADS, 1)
 attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                      const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ out,
                      const int* __restrict__ tok_pos, const int* __restrict__ block_table, int bt_stride,
                      const int* __restrict__ tiles, int nq, int nkv, int page_size, int num_pages,
-                     float scale_log2, int window, int* status) {
+                     float scale_log2, float cap, TcsReach reach, int* status) {
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   const uint32_t q_s = smem_u32(base), k_s = q_s + TC_TILE_BYTES, v_s = k_s + 2 * TC_TILE_BYTES;
@@ -212,7 +241,7 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   const int first_tok = tok0 + row0 / G, last_tok = tok0 + (row0 + n_rows - 1) / G;
   const int key_end = tok_pos[last_tok];
   const int p_first = tok_pos[first_tok];
-  const int lo_min = (window > 0 && p_first - window + 1 > 0) ? p_first - window + 1 : 0;   // the lowest key any row reads
+  const int lo_min = reach.lo(p_first);                     // the lowest key any row reads
   const int key_begin = lo_min / TC_BN * TC_BN;
   const int n_blocks = (key_end - key_begin) / TC_BN + 1;
 
@@ -336,16 +365,20 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t vt = v_s + slot * TC_TILE_BYTES;
-        const uint32_t pt = tmem_base + p_col + (uint32_t)(slot * (TC_BN / 2));
+        const uint32_t pt = tmem_base + (SPLIT ? (uint32_t)(slot * TC_BN) : p_col + (uint32_t)(slot * (TC_BN / 2)));
 #pragma unroll
         for (int k16 = 0; k16 < TC_BN / 16; ++k16) {
-          // 16 keys further: 8 columns of P, 16 rows of V
-          umma_bf16_ta(tmem_base + o_col, pt + (uint32_t)(k16 * 8), umma_desc(vt + k16 * 2048, TC_SLAB_BYTES), idesc_pv,
-                       (j | k16) != 0 ? 1u : 0u);
+          // 16 keys further: 8 columns of P, 16 rows of V; with two parts, 64 keys have hi and then lo in 64 columns
+          const uint32_t pa = pt + (uint32_t)(SPLIT ? (k16 >> 2) * 64 + (k16 & 3) * 8 : k16 * 8);
+          umma_bf16_ta(tmem_base + o_col, pa, umma_desc(vt + k16 * 2048, TC_SLAB_BYTES), idesc_pv, (j | k16) != 0 ? 1u : 0u);
+          if (SPLIT) umma_bf16_ta(tmem_base + o_col, pa + 32u, umma_desc(vt + k16 * 2048, TC_SLAB_BYTES), idesc_pv, 1u);
         }
         umma_commit(smem_u32(&sh.v_empty[slot]));
         umma_commit(smem_u32(&sh.p_empty[slot]));
         umma_commit(smem_u32(&sh.o_full));
+        // with two parts the next S of this buffer lies where the P of the product above does
+        if (SPLIT && j + 2 < n_blocks) ok = mbar_wait(smem_u32(&sh.p_empty[slot]), (uint32_t)(j >> 1) & 1u, abort_flag);
+        if (!ok) break;
         if (j + 2 < n_blocks) issue_qk(j + 2);
       }
     }
@@ -356,7 +389,9 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const int R = row0 + r;
     const bool valid = r < n_rows;
     const int pos_r = valid ? tok_pos[tok0 + R / G] : -1;
-    const int lo_r = (window > 0 && pos_r - window + 1 > 0) ? pos_r - window + 1 : 0;
+    const int lo_r = valid ? reach.lo(pos_r) : 0;
+    const float cap_log2 = cap * 1.4426950408889634f, cap_mul = CAP ? scale_log2 * 2.f / cap : 0.f;   // (score / cap) 2 log2(e)
+    const float mul = CAP ? 1.f : scale_log2;                                 // from what the registers hold to log2 of a weight
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
     const uint32_t o_addr = lane_addr + o_col + (uint32_t)(half * 64);       // this thread's 64 columns of O
     const uint32_t p_addr = lane_addr + p_col + (uint32_t)(half * 32);       // its 64 keys: 32 columns of a P buffer
@@ -381,6 +416,13 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         tmem_ld32(mine + 32u, vb);
         tmem_wait_ld();
       }
+      if (CAP) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          va[i] = __float_as_uint(tcs_cap(__uint_as_float(va[i]), cap_log2, cap_mul));
+          vb[i] = __float_as_uint(tcs_cap(__uint_as_float(vb[i]), cap_log2, cap_mul));
+        }
+      }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
       if (all_visible) {
 #pragma unroll
@@ -401,7 +443,7 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       mbar_arrive(smem_u32(&sh.mx_full[quad]));
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.mx_full[quad]), (uint32_t)j & 1u, abort_flag) ? 1 : 0);
       if (!ok) break;
-      const float mx = fmaxf(mx_own, s_mx[j & 1][half ^ 1][r]) * scale_log2;
+      const float mx = fmaxf(mx_own, s_mx[j & 1][half ^ 1][r]) * mul;
       m_true = fmaxf(m_true, mx);
       // raise the reference only when the maximum has grown a lot: O and the sum are rescaled then
       const bool raise = m_true > m_ref + TCS_TAU;          // also true while the reference is -inf and a key is visible
@@ -426,8 +468,8 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       }
       if (raise) m_ref = m_true;
       const float msafe = m_ref == -INFINITY ? 0.f : m_ref;
-      // the P buffer of this block is free once the P V of the block before the last has read it
-      if (j > 1) {
+      // the P buffer of this block is free once the P V of the block before the last has read it (with two parts it is this block's S)
+      if (!SPLIT && j > 1) {
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.p_empty[slot]), (uint32_t)((j >> 1) - 1) & 1u, abort_flag) ? 1 : 0);
         if (!ok) break;
       }
@@ -436,30 +478,37 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       {
         const bool vis = all_visible;
         auto take = [&](const uint32_t (&v)[32], int c) {        // keys kbase + c*32 .. +31
-          uint32_t pk[16];
+          uint32_t pk[16], pl[16];
           if (vis) {
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
-              const float p0 = ex2(__uint_as_float(v[i]) * scale_log2 - msafe);
-              const float p1 = ex2(__uint_as_float(v[i + 1]) * scale_log2 - msafe);
+              const float p0 = ex2(__uint_as_float(v[i]) * mul - msafe);
+              const float p1 = ex2(__uint_as_float(v[i + 1]) * mul - msafe);
               sum2[0] += p0;
               sum2[1] += p1;
-              pk[i >> 1] = pack_bf16(p0, p1);
+              if (SPLIT) split_bf16(p0, p1, pk[i >> 1], pl[i >> 1]);
+              else pk[i >> 1] = pack_bf16(p0, p1);
             }
           } else {
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
               const int key = kbase + c * 32 + i;
-              float p0 = ex2(__uint_as_float(v[i]) * scale_log2 - msafe);
-              float p1 = ex2(__uint_as_float(v[i + 1]) * scale_log2 - msafe);
+              float p0 = ex2(__uint_as_float(v[i]) * mul - msafe);
+              float p1 = ex2(__uint_as_float(v[i + 1]) * mul - msafe);
               if (key < lo_r || key > pos_r) p0 = 0.f;
               if (key + 1 < lo_r || key + 1 > pos_r) p1 = 0.f;
               sum2[0] += p0;
               sum2[1] += p1;
-              pk[i >> 1] = pack_bf16(p0, p1);
+              if (SPLIT) split_bf16(p0, p1, pk[i >> 1], pl[i >> 1]);
+              else pk[i >> 1] = pack_bf16(p0, p1);
             }
           }
-          tmem_st16(p_addr + (uint32_t)(slot * (TC_BN / 2) + c * 16), pk);
+          if (SPLIT) {
+            tmem_st16(s_addr + (uint32_t)(half * 64 + c * 16), pk);
+            tmem_st16(s_addr + (uint32_t)(half * 64 + 32 + c * 16), pl);
+          } else {
+            tmem_st16(p_addr + (uint32_t)(slot * (TC_BN / 2) + c * 16), pk);
+          }
         };
         take(va, 0);
         take(vb, 1);
@@ -553,11 +602,9 @@ extern "C" int qb_attn_span_tc_supported(int nq, int nkv, int hd, int page_size)
 // Query rows per tile of the tcgen05 kernel.
 extern "C" int qb_attn_span_tc_rows(void) { return TC_BM; }
 
-// Same arguments as qb_attn_span; the tile list has qb_attn_span_tc_rows() rows a tile.
-extern "C" int qb_attn_span_tc(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tok_pos,
-                               const int* block_table, int bt_stride, const int* tiles, int n_tiles, int nq, int nkv,
-                               int hd, int page_size, int num_pages, float scale, int window, int* status,
-                               cudaStream_t stream) {
+static int span_tc(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tok_pos,
+                   const int* block_table, int bt_stride, const int* tiles, int n_tiles, int nq, int nkv, int hd, int page_size,
+                   int num_pages, float scale, int window, bool two_part, float cap, int chunk, int* status, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
   if (!qb_attn_span_tc_supported(nq, nkv, hd, page_size)) return QB_ERR_UNSUPPORTED;
   if ((((uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)q | (uintptr_t)out) & 15) != 0) return QB_ERR_UNSUPPORTED;
@@ -571,11 +618,31 @@ extern "C" int qb_attn_span_tc(const void* q, const void* k_cache, const void* v
   if (rc == 0) rc = make_kv_map(&tm_v, v_cache, rows, box_rows);
   if (rc) return rc;
   const size_t smem = 5 * (size_t)TC_TILE_BYTES + 1024;      // Q and two stages each of K and V
-  cudaError_t err = cudaFuncSetAttribute(attn_span_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kern = !two_part ? attn_span_tc_kernel<false, false> : cap > 0.f ? attn_span_tc_kernel<true, true> : attn_span_tc_kernel<true, false>;
+  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return (int)err;
-  attn_span_tc_kernel<<<dim3((unsigned)n_tiles * (unsigned)nkv), TCS_THREADS, smem, stream>>>(
+  kern<<<dim3((unsigned)n_tiles * (unsigned)nkv), TCS_THREADS, smem, stream>>>(
       tm_k, tm_v, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, tok_pos, block_table, bt_stride, tiles, nq, nkv,
-      page_size, num_pages, scale_log2, window, status);
+      page_size, num_pages, scale_log2, cap, TcsReach{window, chunk}, status);
   QB_LAUNCH_CHECK();
   return 0;
+}
+
+// Same arguments as qb_attn_span; the tile list has qb_attn_span_tc_rows() rows a tile.
+extern "C" int qb_attn_span_tc(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tok_pos,
+                               const int* block_table, int bt_stride, const int* tiles, int n_tiles, int nq, int nkv,
+                               int hd, int page_size, int num_pages, float scale, int window, int* status,
+                               cudaStream_t stream) {
+  return span_tc(q, k_cache, v_cache, out, tok_pos, block_table, bt_stride, tiles, n_tiles, nq, nkv, hd, page_size, num_pages, scale,
+                 window, false, 0.f, 0, status, stream);
+}
+
+// The same with probabilities of two bfloat16 parts; cap > 0: score <- cap tanh(score / cap); chunk > 0: a query reads the keys of its own
+// chunk of positions only.
+extern "C" int qb_attn_span_split(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tok_pos,
+                                  const int* block_table, int bt_stride, const int* tiles, int n_tiles, int nq, int nkv,
+                                  int hd, int page_size, int num_pages, float scale, int window, float cap, int chunk, int* status,
+                                  cudaStream_t stream) {
+  return span_tc(q, k_cache, v_cache, out, tok_pos, block_table, bt_stride, tiles, n_tiles, nq, nkv, hd, page_size, num_pages, scale,
+                 window, true, cap, chunk, status, stream);
 }

@@ -371,6 +371,11 @@ def attn_span_tc_supported(nq: int, nkv: int, hd: int, page_size: int) -> bool:
     return bool(lib().qb_attn_span_tc_supported(int(nq), int(nkv), int(hd), int(page_size)))
 
 
+def attn_span_tc_rows() -> int:
+    """Query rows per tile of the tcgen05 kernel."""
+    return int(lib().qb_attn_span_tc_rows())
+
+
 def attn_span(q, k_cache, v_cache, out, tok_pos, block_table, tiles, scale: float, window: int, status) -> None:
     """bfloat16 tensor-core attention for prompt portions.  ``tiles`` int32 [n, 4]: request row, first
     token row of the portion, tokens in the portion, first flattened (token*G + head) row of the tile."""
@@ -382,6 +387,23 @@ def attn_span(q, k_cache, v_cache, out, tok_pos, block_table, tiles, scale: floa
     _check(lib().qb_attn_span(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(tok_pos), _p(block_table),
                               block_table.shape[1], _p(tiles), tiles.shape[0], nq, nkv, hd, page_size, num_pages,
                               ctypes.c_float(scale), int(window), _p(status), _stream()), "attn_span")
+
+
+def attn_span_split(q, k_cache, v_cache, out, tok_pos, block_table, tiles, scale: float, window: int, status, *, softcap: float = 0.0,
+                    chunk: int = 0) -> None:
+    """``attn_span`` on the tcgen05 kernel (shapes of ``attn_span_tc_supported``) whose softmax weights enter the sum in two bfloat16
+    parts, with ``softcap`` and ``chunk`` as in ``window_attention``."""
+    T, nq, hd = q.shape
+    num_pages, nkv, page_size, hd2 = k_cache.shape
+    for t, name in ((q, "q"), (k_cache, "k_cache"), (v_cache, "v_cache"), (out, "out")):
+        _want(t, torch.bfloat16, name)
+    _want(tiles, torch.int32, "tiles")
+    if hd2 != hd or out.shape != q.shape or v_cache.shape != k_cache.shape:
+        raise ValueError("attn_span_split: shape mismatch")
+    _check(lib().qb_attn_span_split(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(tok_pos), _p(block_table),
+                                    block_table.shape[1], _p(tiles), tiles.shape[0], nq, nkv, hd, page_size, num_pages,
+                                    ctypes.c_float(scale), int(window), ctypes.c_float(softcap), int(chunk), _p(status),
+                                    _stream()), "attn_span_split")
 
 
 def attn_decode(q, k_cache, v_cache, out, part_o, part_ml, dec_tok, n_dec: int, tok_pos, tok_req, block_table,

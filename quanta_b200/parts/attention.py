@@ -201,6 +201,11 @@ class GQAttention(Mixer):
         if self.float32_weights:
             # scores and weights in float32 whatever the dtype: portions of shapes the tensor cores take run there
             # with the weights in two bfloat16 parts; single tokens cut their keys into ranges that are joined
+            tiles = split_span_tiles(ctx, q, cache.k, cache.v)
+            if tiles is not None:
+                kernels.attn_span_split(q, cache.k, cache.v, out, ctx.tok_pos, cache.block_table, tiles, self.scale, window,
+                                        ctx.status, chunk=self.chunk or 0)
+                return
             R = int(ctx.req_start.numel()) - 1
             warps = max(1, q.shape[0] * self.nkv)
             # about 2,048 warps in all, at least 32 keys a range (measured on a B200 with 4 kv heads of 128: 8 tokens
@@ -229,17 +234,42 @@ class GQAttention(Mixer):
             kernels.attn_decode(q, cache.k, cache.v, out, part_o, part_ml, dec_tok, n_dec, ctx.tok_pos, ctx.tok_req,
                                 cache.block_table, self.scale, window, n_parts, ctx.status)
         if spans:
-            key = ("span_tiles", G, self.hd, kernels.attn_span_rows(self.hd, self.nq, self.nkv, cache.page_size))
-            if key not in ctx.work:
-                rows = kernels.attn_span_rows(self.hd, self.nq, self.nkv, cache.page_size)
-                tiles = [[r, t0, n, r0] for (r, t0, n) in spans for r0 in range(0, n * G, rows)]
-                # tiles that read the most keys first: the short ones fill the SMs at the end
-                after = ctx.host.get("req_len_after")
-                if after is not None:
-                    tiles.sort(key=lambda t: -(after[t[0]] - t[2] + min(t[2], (t[3] + rows) // G)))
-                ctx.work[key] = torch.tensor(tiles, dtype=torch.int32).to(q.device, non_blocking=True)
-            kernels.attn_span(q, cache.k, cache.v, out, ctx.tok_pos, cache.block_table, ctx.work[key], self.scale,
-                              window, ctx.status)
+            tiles = span_tiles(ctx, spans, G, kernels.attn_span_rows(self.hd, self.nq, self.nkv, cache.page_size), self.hd, q.device)
+            kernels.attn_span(q, cache.k, cache.v, out, ctx.tok_pos, cache.block_table, tiles, self.scale, window, ctx.status)
+
+
+def span_tiles(ctx, spans, G: int, rows: int, hd: int, device):
+    """The list of query tiles of the portions ``spans`` for ``kernels.attn_span`` and ``attn_span_split``: ``rows`` rows (token x q head
+    of the group) each; made once a step."""
+    key = ("span_tiles", G, hd, rows, len(spans))
+    if key not in ctx.work:
+        tiles = [[r, t0, n, r0] for (r, t0, n) in spans for r0 in range(0, n * G, rows)]
+        # tiles that read the most keys first: the short ones fill the SMs at the end
+        after = ctx.host.get("req_len_after")
+        if after is not None:
+            tiles.sort(key=lambda t: -(after[t[0]] - t[2] + min(t[2], (t[3] + rows) // G)))
+        ctx.work[key] = torch.tensor(tiles, dtype=torch.int32).to(device, non_blocking=True)
+    return ctx.work[key]
+
+
+# Steps with at least this many tokens beside one a request take the tcgen05 kernel with probabilities of two parts; below, the keys of
+# each token are cut into ranges on the CUDA cores.  Measured on a B200, 16 + 4 heads of 128, beside the mma.sync kernel (64 rows of the
+# step's token list a block, request after request): 32 tokens alone 13 and 12 us, 32 after 2,000 others with a window of 1,024 82 and 32,
+# 2,048 172 and 57, 24 single tokens of 1,500 keys with a portion of 512 2,738 and 48.
+SPLIT_SPAN_MIN_TOKENS = 32
+
+
+def split_span_tiles(ctx, q, k_cache, v_cache):
+    """The tiles of a step whose attention runs as ``kernels.attn_span_split`` (every request a portion, single tokens too), or None:
+    shapes the kernel does not take, steps of few tokens, or requests' places the host does not know (a captured step)."""
+    T, nq, hd = q.shape
+    nkv, page_size = k_cache.shape[1], k_cache.shape[2]
+    starts = ctx.host.get("req_start")
+    if (q.dtype != torch.bfloat16 or v_cache.shape != k_cache.shape or starts is None
+            or T - (len(starts) - 1) < SPLIT_SPAN_MIN_TOKENS - 1 or not kernels.attn_span_tc_supported(nq, nkv, hd, page_size)):
+        return None
+    spans = [(r, starts[r], starts[r + 1] - starts[r]) for r in range(len(starts) - 1)]
+    return span_tiles(ctx, spans, nq // nkv, kernels.attn_span_tc_rows(), hd, q.device)
 
 
 def step_work(ctx, device):

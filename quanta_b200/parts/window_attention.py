@@ -38,6 +38,7 @@ import torch
 
 from .. import kernels
 from ..matmul import empty_rows, linear
+from .attention import split_span_tiles
 from .base import Addends, CacheSpec, CacheStream, KeepAll, Mixer, TensorSpec, Window, WindowAndOpenBlock, make, register
 
 
@@ -188,9 +189,15 @@ class WindowAttention(Mixer):
         scratch = None
         if self.has_talk:
             scratch = torch.empty((T, self.nq, self.nkv, self.vd), dtype=torch.float32, device=x.device)
-        kernels.window_attention(q, cache.k, cache.v, out, ctx.tok_pos, ctx.tok_req, cache.tables["k"], self.scale,
-                                 self.window, ctx.status, dist_bias=self.dist_table, sink=self.sink,
-                                 softcap=self.softcap, talk=self.talk, scratch=scratch,
-                                 n_requests=int(ctx.req_start.numel()) - 1, **pooled)
+        plain = self.dist_table is None and self.sink is None and not self.has_talk and not self.pool
+        tiles = split_span_tiles(ctx, q, cache.k, cache.v) if plain else None
+        if tiles is not None:
+            kernels.attn_span_split(q, cache.k, cache.v, out, ctx.tok_pos, cache.tables["k"], tiles, self.scale, self.window,
+                                    ctx.status, softcap=self.softcap)
+        else:
+            kernels.window_attention(q, cache.k, cache.v, out, ctx.tok_pos, ctx.tok_req, cache.tables["k"], self.scale,
+                                     self.window, ctx.status, dist_bias=self.dist_table, sink=self.sink,
+                                     softcap=self.softcap, talk=self.talk, scratch=scratch,
+                                     n_requests=int(ctx.req_start.numel()) - 1, **pooled)
         y = linear(out.view(T, self.nq * self.vd), self.w_o, out_dtype=torch.float32)
         return Addends(y, bias=self.b_o) if self.b_o is not None else y
