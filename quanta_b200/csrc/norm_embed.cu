@@ -68,7 +68,7 @@ extern "C" int qb_embedding(float* h, const void* table, int table_dtype, const 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Rows of whole 32-byte pieces (H a multiple of 8, at most 8 x 1,024): a thread keeps its 8 elements in registers from the first
+// Rows of whole 32-byte pieces (H a multiple of 8, at most 8 x 1,024, or 8 x 768 with two norms): a thread keeps its 8 elements in registers from the first
 // load to the store, so a row passes memory once and shared memory holds the warps' sums alone; everything a row needs (gains too)
 // is asked for before the first sum, so that a row is one wait for memory and one or two block sums.  Threads: H / 8, whole
 // warps.
@@ -166,7 +166,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const D* __restrict__ 
 // The same for rows in registers.  Measured on a B200 against the kernel above at 12,800 rows of 3,072: bfloat16 delta 128 -> 75 us
 // (470 MB), eight float32 slots (1.7 GB) 262 -> 233 us; one row of eight slots 3.7 -> 3.1 us.
 template <typename D, typename O>
-__global__ void add_rmsnorm_rows_kernel(float* __restrict__ h, const D* __restrict__ delta, int S, const float* __restrict__ w,
+__global__ void __launch_bounds__(1024) add_rmsnorm_rows_kernel(float* __restrict__ h, const D* __restrict__ delta, int S, const float* __restrict__ w,
                                         O* __restrict__ out, const int* __restrict__ rows, int H, float eps, int store_h) {
   __shared__ float scratch[32];
   const int r = blockIdx.x, tok = rows ? rows[r] : r, i = threadIdx.x * 8;
@@ -288,7 +288,7 @@ __global__ void normed_add_rmsnorm_kernel(float* __restrict__ h, const float* __
 // The same for rows in registers.  Measured on a B200 against the kernel above: 4,876 rows of 2,048 with two slots and a second
 // summand (240 MB) 87 -> 46 us, with one slot (160 MB) 56 -> 30 us, 8 rows 4.3 -> 2.9 us.
 template <typename O>
-__global__ void normed_add_rmsnorm_rows_kernel(float* __restrict__ h, const float* __restrict__ y, int S, float y_scale,
+__global__ void __launch_bounds__(768) normed_add_rmsnorm_rows_kernel(float* __restrict__ h, const float* __restrict__ y, int S, float y_scale,
                                                const float* __restrict__ y_bias, const float* __restrict__ y2, float y2_scale,
                                                const float* __restrict__ y2_bias, const float* __restrict__ g, float eps_y,
                                                const float* __restrict__ w, O* __restrict__ out, const int* __restrict__ rows,
@@ -363,7 +363,7 @@ extern "C" int qb_normed_add_rmsnorm(float* h, const float* y, int S, float y_sc
   if (S < 1 || (y != nullptr && g == nullptr)) return QB_ERR_BAD_ARG;
   const uintptr_t all = (uintptr_t)h | (uintptr_t)y | (uintptr_t)y_bias | (uintptr_t)y2 | (uintptr_t)y2_bias | (uintptr_t)g |
                         (uintptr_t)w | (uintptr_t)out;
-  if (row_in_registers(H, 1024) && (all & 15) == 0) {
+  if (row_in_registers(H, 768) && (all & 15) == 0) {      // 1,024 threads would have 64 registers each, it takes more
     QB_DISPATCH_DTYPE(out_dtype, O, {
       normed_add_rmsnorm_rows_kernel<O><<<n_rows, row_threads(H), 0, stream>>>(
           h, y, S, y_scale, y_bias, y2, y2_scale, y2_bias, g, eps_y, w, (O*)out, rows, H, eps, store_h);

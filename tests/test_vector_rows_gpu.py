@@ -1,0 +1,104 @@
+"""Kernels that read rows in 16-byte pieces, at the sizes where they hand over to those that read a number at a time, against float64.
+Tolerance: a few float32 roundings (2^-24) of the terms, 2^-8 where the result is bfloat16."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def K():
+    from quanta_b200 import kernels
+    return kernels
+
+
+def randn(*shape, seed):
+    return torch.randn(*shape, device=DEV, generator=torch.Generator(device=DEV).manual_seed(seed))
+
+
+def rms(x, gain, eps):
+    return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps) * gain
+
+
+def near(got, want, dtype):
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
+    assert float((got.double() - want).abs().max()) <= tol * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H", [8, 70, 264, 8192, 8200])
+def test_norm_rows(H, dtype):
+    h, delta, w = randn(5, H, seed=1), randn(5, 2, H, seed=2), 1 + 0.1 * randn(H, seed=3)
+    y, y2, g, b = randn(5, H, seed=4), randn(5, H, seed=5), 1 + 0.1 * randn(H, seed=6), randn(H, seed=7)
+    stream, out = h.clone(), torch.empty(5, H, device=DEV, dtype=dtype)
+    K().add_rmsnorm(stream, delta, w, 1e-5, out)
+    want = h.double() + delta.double().sum(1)
+    near(stream, want, torch.float32)
+    near(out, rms(want, w.double(), 1e-5), dtype)
+    stream = h.clone()
+    K().normed_add_rmsnorm(stream, y, g, 1e-6, w, 1e-5, out, y_scale=0.5, y_bias=b, extra=y2, extra_scale=2.0)
+    want = h.double() + rms(0.5 * (y.double() + b.double()) + 2.0 * y2.double(), g.double(), 1e-6)
+    near(stream, want, torch.float32)
+    near(out, rms(want, w.double(), 1e-5), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("inner", [7, 8, 12, 2056])
+def test_silu_mul(inner, dtype):
+    gu = randn(9, 2 * inner, seed=inner).to(dtype)
+    out = torch.empty(9, inner, device=DEV, dtype=dtype)
+    K().silu_mul(gu, out)
+    near(out, torch.nn.functional.silu(gu[:, :inner].double()) * gu[:, inner:].double(), dtype)
+
+
+@pytest.mark.parametrize("gate", ["sigmoid", "silu"])
+@pytest.mark.parametrize("heads,dim,off,shared", [(3, 4, 0, False), (5, 64, 8, True), (33, 8, 4, False), (2, 128, 0, True), (3, 12, 0, False),
+                                                  (3, 64, 3, True), (2, 256, 0, False)])
+def test_head_norm_gate(heads, dim, off, shared, gate):
+    T, P = 7, off + heads * dim + (-(off + heads * dim)) % 4
+    o, proj, gain = randn(T, heads * dim, seed=1), randn(T, P, seed=2), 1 + 0.1 * randn(dim if shared else heads * dim, seed=3)
+    x = o.double().view(T, heads, dim)
+    want = rms(x, gain.double().view(-1, dim), 1e-5)
+    z = proj.double()[:, off:off + heads * dim].view(T, heads, dim)
+    want = want * (torch.sigmoid(z) if gate == "sigmoid" else torch.nn.functional.silu(z))
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.empty(T, heads * dim, device=DEV, dtype=dtype)
+        K().head_norm_gate(o, proj, off, gain, out, heads, dim, 1e-5, gate)
+        near(out, want.reshape(T, -1), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,nkv,hd,vd,window,n_split", [(4, 1, 64, 64, 0, None), (6, 3, 36, 20, 17, 3), (5, 5, 128, 132, 300, None), (8, 1, 256, 4, 0, 5),
+                                                         (4, 2, 50, 64, 90, 2), (4, 2, 64, 66, 0, 1)])
+def test_attention_of_few_tokens(nq, nkv, hd, vd, window, n_split, dtype):
+    """One to several tokens a request, ranges of keys, a bias by distance, a sink, a cap, given-back pages."""
+    kern, page, lens, G = K(), 8, [700, 3, 65], nq // nkv
+    per = -(-max(lens) // page)
+    kc, vc = randn(3 * per, nkv, page, hd, seed=1).to(dtype), randn(3 * per, nkv, page, vd, seed=2).to(dtype)
+    table = torch.randperm(3 * per, generator=torch.Generator().manual_seed(3)).int().view(3, per)
+    req, pos = [0, 0, 1, 2, 2, 2], [698, 699, 2, 62, 63, 64]
+    if window:
+        table[0, : max(0, 699 - window) // page] = -1
+    bias = randn(window, nq, seed=4) if window else None
+    sink, cap, scale = randn(nq, seed=5), 5.0, hd ** -0.5
+    q, st = randn(6, nq, hd, seed=6).to(dtype), kern.new_status(DEV)
+    out = torch.empty(6, nq, vd, device=DEV, dtype=dtype)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    kern.window_attention(q, kc, vc, out, i32(pos), i32(req), table.to(DEV), scale, window, st, dist_bias=bias, sink=sink, softcap=cap,
+                          n_split=n_split, tensor_cores=False)
+    assert st.tolist()[0] == 0
+    for t in range(6):
+        j = torch.arange(max(0, pos[t] - window + 1) if window else 0, pos[t] + 1)
+        rows = table[req[t]].long()[j // page].to(DEV)
+        k, v = kc[rows, :, (j % page).to(DEV)].double(), vc[rows, :, (j % page).to(DEV)].double()
+        s = torch.einsum("hgd,jhd->hgj", q[t].double().view(nkv, G, hd), k).reshape(nq, -1) * scale
+        s = cap * torch.tanh(s / cap)
+        if window:
+            s = s + bias.double()[(pos[t] - j).to(DEV)].T
+        w = torch.softmax(torch.cat([s, sink.double()[:, None]], 1), 1)[:, :-1]
+        want = torch.einsum("hgj,jhd->hgd", w.view(nkv, G, -1), v).reshape(nq, vd)
+        # float32: some 700 terms; the exponents carry a few roundings of scores up to 10
+        tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -17
+        assert float((out[t].double() - want).abs().max()) <= tol * float(v.abs().max())
