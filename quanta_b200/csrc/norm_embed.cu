@@ -662,11 +662,49 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
   }
 }
 
+// Heads of 4, 8, ... 128 numbers in 16-byte pieces: D / 4 lanes a (token, head), the sum a butterfly over them.  2,048 tokens of 32 heads
+// of 64 (42 MB with the bfloat16 result) 24 -> 11.6 us.
+template <typename O>
+__global__ void __launch_bounds__(128)
+head_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_stride, const float* __restrict__ gain,
+                          O* __restrict__ out, int T, int H, int D, float eps, int gain_shared, int gate_kind) {
+  const int lanes = D / 4, per = 128 / lanes;            // (token, head) pairs a block
+  const int h = blockIdx.y * per + threadIdx.x / lanes, i = threadIdx.x % lanes * 4, t = blockIdx.x;
+  const bool in = h < H;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const size_t at = ((size_t)t * H + h) * D + i;
+  const float4 v = in ? *reinterpret_cast<const float4*>(o + at) : zero;
+  const float4 g = in ? *reinterpret_cast<const float4*>(gate + (size_t)t * gate_stride + (size_t)h * D + i) : zero;
+  const float4 w = in ? *reinterpret_cast<const float4*>(gain + (gain_shared ? 0 : h * D) + i) : zero;
+  float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+  for (int s = lanes / 2; s > 0; s >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, s);
+  const float inv = 1.f / sqrtf(ss / (float)D + eps);
+  if (!in) return;
+  auto one = [&](float x, float gx, float wx) {
+    const float sg = 1.f / (1.f + expf(-gx));
+    return x * inv * wx * (gate_kind == 1 ? gx * sg : sg);
+  };
+  struct alignas(4 * sizeof(O)) Four { O v[4]; };
+  Four r;
+  r.v[0] = qb_from_float<O>(one(v.x, g.x, w.x)); r.v[1] = qb_from_float<O>(one(v.y, g.y, w.y));
+  r.v[2] = qb_from_float<O>(one(v.z, g.z, w.z)); r.v[3] = qb_from_float<O>(one(v.w, g.w, w.w));
+  *reinterpret_cast<Four*>(out + at) = r;
+}
+
 extern "C" int qb_head_norm_gate(const float* o, const float* gate, int gate_stride, const float* gain,
                                  void* out, int out_dtype, int T, int H, int D, float eps, int gain_shared,
                                  int gate_kind, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (gate_kind != 0 && gate_kind != 1) return QB_ERR_BAD_ARG;
+  const uintptr_t all = (uintptr_t)o | (uintptr_t)gate | (uintptr_t)gain | (uintptr_t)out;
+  if (D >= 4 && D <= 128 && (D & (D - 1)) == 0 && H <= 65535 && gate_stride % 4 == 0 && (all & 15) == 0) {
+    const int per = 128 / (D / 4);
+    const dim3 grid(T, (H + per - 1) / per);
+    QB_DISPATCH_DTYPE(out_dtype, O, head_norm_gate_vec_kernel<O><<<grid, 128, 0, stream>>>(o, gate, gate_stride, gain, (O*)out, T, H, D,
+                                                                                          eps, gain_shared, gate_kind));
+    QB_LAUNCH_CHECK();
+    return 0;
+  }
   const long warps = (long)T * H;
   const int blocks = (int)((warps + 3) / 4);
   QB_DISPATCH_DTYPE(out_dtype, O, head_norm_gate_kernel<O><<<blocks, 128, 0, stream>>>(
