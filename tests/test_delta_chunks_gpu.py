@@ -67,6 +67,22 @@ def test_chunks(H, D, lens, extra, scale):
         assert float((chain - out[:200]).abs().max()) <= 1e-5 * float(chain.pow(2).mean().sqrt())
 
 
+@pytest.mark.parametrize("R,H,D", [(1, 1, 4), (1, 3, 64), (5, 2, 20), (9, 32, 64), (2, 1, 128), (40, 4, 100), (3, 2, 33)])
+def test_single_tokens(R, H, D):
+    """One launch for steps of single tokens (heads that are multiples of 4), the state carried over three steps."""
+    g = torch.Generator(device=DEV).manual_seed(R + D)
+    S0 = torch.randn(R, H, D, D, device=DEV, generator=g) * 0.3
+    S, HD = S0.clone(), H * D
+    ab, wb = (torch.randn(HD, device=DEV, generator=g) for _ in range(2))
+    steps = [(torch.randn(R, 4 * HD + 3, device=DEV, generator=g), torch.randn(R, HD, device=DEV, generator=g)) for _ in range(3)]
+    outs = [run(proj, wpre, ab, wb, S, [1] * R, H, D, 0.6) for proj, wpre in steps]
+    for r in range(R):
+        want, end = exact(torch.stack([p[r] for p, _ in steps]), torch.stack([w[r] for _, w in steps]), ab, wb, S0[r], H, D, 0.6)
+        got = torch.stack([o[r] for o in outs])
+        for a, b in ((got, want), (S[r], end)):
+            assert float((a.double() - b).abs().max()) <= 1e-5 * float(b.pow(2).mean().sqrt())
+
+
 def test_a_later_infinity_reaches_no_earlier_token():
     H, D, T = 2, 64, 64
     g = torch.Generator(device=DEV).manual_seed(5)
