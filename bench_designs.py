@@ -499,7 +499,8 @@ def plain_attn(tokens_per_req: int, reqs: int, context: int, nq: int, nkv: int, 
     pos = torch.arange(context - tokens_per_req, context, dtype=torch.int32, device=dev).repeat(reqs)
     req = torch.arange(reqs, dtype=torch.int32, device=dev).repeat_interleave(tokens_per_req)
     st = k.new_status(dev)
-    n_split = max(1, min(-(-2048 // (T * nkv)), -(-min(context, chunk or context) // 32), 256))      # as parts/attention.py
+    keys = min(per * page, chunk) if chunk else per * page
+    n_split = max(1, min(-(-keys // 256), 1184 // (T * nkv * max(1, nq // nkv // 4)), 64))      # as kernels.window_attention by itself
 
     def all_layers():
         for kc, vc in caches:

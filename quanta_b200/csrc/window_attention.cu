@@ -17,10 +17,10 @@
 // computed as out_h = sum_g talk[h, g] O[g][kv(h)] with O[g][m] = sum_j w_g(j) v_m(j): every head's weights are
 // applied to the values of ALL kv heads (float32 scratch [T, nq, nkv, vd]) and a second kernel mixes.
 //
-// One warp per (token, q head), or per (token, q head, range of the keys) in steps of few tokens, whose ranges a
-// second kernel joins: lanes own keys for the scores, then own dims for P V.  Long portions in bfloat16 take the
-// tensor-core kernel at the end of this file.
-#include "common.cuh"
+// Without pooled blocks and mixed heads, head sizes that are multiples of 4 run as attention_rows.cuh has it.  Else one warp per (token,
+// q head), or per (token, q head, range of the keys) in steps of few tokens, whose ranges a second kernel joins: lanes own keys for
+// the scores, then own dims for P V.  Long portions in bfloat16 with such extras take the tensor-core kernel at the end of this file.
+#include "attention_rows.cuh"
 
 constexpr int WA_WARPS = 4;
 constexpr int WA_MAX_HD = 256;
@@ -440,7 +440,15 @@ extern "C" int qb_window_attention(const void* q, int dtype, const void* k_cache
   P.vec = (hd % 8 == 0 && ((uintptr_t)k_cache & 15) == 0 && (kp_cache == nullptr || ((uintptr_t)kp_cache & 15) == 0)) ? 1 : 0;
   P.n_split = n_split; P.part = part;
   const int nv = (vd + 31) / 32;
-  if (n_split > 1) {
+  const bool by_rows = talk == nullptr && pool_table == nullptr && rows_attention_takes(nq, nkv, hd, vd, q, k_cache, v_cache, out);
+  if (by_rows) {
+    const RowsAttention R{tok_pos, tok_req, block_table, bt_stride, T, nq, nkv, hd, vd, page_size, num_pages, scale, cap, window, chunk,
+                          dist_bias, sink, n_split, part, status};
+    int rc = 0;
+    QB_DISPATCH_DTYPE(dtype, A, rc = rows_attention<A>((const A*)q, (const A*)k_cache, (const A*)v_cache, (A*)out, R, stream));
+    if (rc != 0 || n_split == 1) return rc;
+  }
+  if (n_split > 1 && !by_rows) {
     const int group = nq / nkv;
     const int gq = group > 4 ? 8 : group > 2 ? 4 : group > 1 ? 2 : 1;
     const int n_chunks = (group + gq - 1) / gq;
@@ -466,6 +474,8 @@ extern "C" int qb_window_attention(const void* q, int dtype, const void* k_cache
 #undef QB_WR_GROUP
 #undef QB_WR_LAUNCH
     QB_LAUNCH_CHECK();
+  }
+  if (n_split > 1) {
     const size_t wsm = (size_t)n_split * sizeof(float);
     if (wsm > 48 * 1024 || (long)T * nq > 0x7fffffffL) return QB_ERR_UNSUPPORTED;
     QB_DISPATCH_DTYPE(dtype, A, wa_merge_kernel<A><<<T * nq, 128, wsm, stream>>>(part, sink, (A*)out, scratch, T, nq, nkv,

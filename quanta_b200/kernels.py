@@ -988,6 +988,11 @@ def window_attention(q, k_cache, v_cache, out, tok_pos, tok_req, block_table, sc
             ctypes.c_float(scale), ctypes.c_float(softcap), int(window), int(pool), int(chunk), _p(dist_bias), _p(sink), _p(status),
             _stream()), "window_attention_mma", 1 + (talk is not None))
         return
+    if n_split is None and talk is None and pool_table is None and hd % 4 == 0 and vd % 4 == 0:
+        # eight warps a (token, kv head, four q heads, range), 64 keys of it a turn of 2.6 us (a look-up and a read of memory): ranges of
+        # 256 keys while that fills the SMs eight warps deep; joining them is a launch of 7 us
+        keys = min(n for n in (window, chunk, block_table.shape[1] * page_size) if n > 0)
+        n_split = max(1, min(-(-keys // 256), 1184 // max(1, T * nkv * max(1, nq // nkv // 4)), 64))
     if n_split is None:
         warps = T * nkv * (nkv if talk is not None else 1)        # of the kernel that shares a key row among q heads
         n_split = 1 if window <= 0 else max(1, min(-(-8192 // warps), -(-window // 32), 64))

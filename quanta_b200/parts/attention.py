@@ -207,12 +207,12 @@ class GQAttention(Mixer):
                                         ctx.status, chunk=self.chunk or 0)
                 return
             R = int(ctx.req_start.numel()) - 1
-            warps = max(1, q.shape[0] * self.nkv)
-            # about 2,048 warps in all, at least 32 keys a range (measured on a B200 with 4 kv heads of 128: 8 tokens
-            # over 2,048 keys 47 us with 64 ranges against 63 with 32; 32 tokens 120 us with 16 against 150 with 64; one
-            # token over 8,192 keys 61 us with 256 against 110 with 64)
-            keys = max(1, min(ctx.max_len_after, self.chunk or self.window or ctx.max_len_after))
-            n_split = max(1, min(-(-2048 // warps), -(-keys // 32), 256))
+            n_split = None
+            if self.hd % 4 or self.vd % 4:
+                # about 2,048 warps in all, at least 32 keys a range
+                warps = max(1, q.shape[0] * self.nkv)
+                keys = max(1, min(ctx.max_len_after, self.chunk or self.window or ctx.max_len_after))
+                n_split = max(1, min(-(-2048 // warps), -(-keys // 32), 256))
             kernels.window_attention(q, cache.k, cache.v, out, ctx.tok_pos, ctx.tok_req, cache.block_table, self.scale,
                                      window, ctx.status, n_split=n_split, n_requests=R, chunk=self.chunk or 0)
             return
