@@ -33,7 +33,7 @@ SRC_DIR = Path(__file__).resolve().parent
 UNITS = {
     "core": ["norm_embed.cu", "grouped_norm.cu", "sampling.cu", "linear_rows.cu"],
     "rope": ["rope_cache.cu"],
-    "attention": ["attention_simt.cu", "attention_mma.cu", "attention_tc.cu"],
+    "attention": ["attention_simt.cu", "attention_mma.cu", "attention_tc.cu", "attention_decode.cu"],
     "experts": ["moe.cu", "router_gemm_mma.cu", "expert_gemm_tc.cu"],
     "short_conv": ["short_conv.cu"],
     "recurrent": ["delta_rule.cu", "gated_delta.cu"],

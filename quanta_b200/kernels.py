@@ -424,6 +424,29 @@ def attn_decode(q, k_cache, v_cache, out, part_o, part_ml, dec_tok, n_dec: int, 
                                 _p(status), _stream()), "attn_decode", 2)
 
 
+def attn_decode_direct_supported(nq: int, nkv: int, hd: int) -> bool:
+    """Whether single tokens of these shapes run as ``attn_decode_direct`` (else as ``attn_decode``)."""
+    return bool(lib().qb_attn_decode_direct_supported(int(nq), int(nkv), int(hd)))
+
+
+def attn_decode_direct(q, k_cache, v_cache, out, dec_tok, n_dec: int, tok_pos, tok_req, block_table, scale: float, window: int,
+                       longest: int, status, *, two_part: bool = False, softcap: float = 0.0, chunk: int = 0) -> None:
+    """bfloat16 attention of the single tokens ``dec_tok`` in one launch, heads of 128 and at most eight q heads a kv head; ``longest``:
+    keys of the longest request (an upper bound is enough).  ``two_part``: the softmax weights enter the sum in two bfloat16 parts;
+    ``softcap``, ``chunk`` as in ``window_attention``."""
+    T, nq, hd = q.shape
+    num_pages, nkv, page_size, hd2 = k_cache.shape
+    for t, name in ((q, "q"), (k_cache, "k_cache"), (v_cache, "v_cache"), (out, "out")):
+        _want(t, torch.bfloat16, name)
+    _want(dec_tok, torch.int32, "dec_tok")
+    if hd2 != hd or out.shape != q.shape or v_cache.shape != k_cache.shape:
+        raise ValueError("attn_decode_direct: shape mismatch")
+    _check(lib().qb_attn_decode_direct(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(dec_tok), int(n_dec), _p(tok_pos), _p(tok_req),
+                                       _p(block_table), block_table.shape[1], nq, nkv, hd, page_size, num_pages,
+                                       ctypes.c_float(scale), int(window), int(longest), int(two_part), ctypes.c_float(softcap), int(chunk),
+                                       _p(status), _stream()), "attn_decode_direct")
+
+
 def split3_bf16(w: torch.Tensor) -> torch.Tensor:
     """A float32 tensor as three bfloat16 tensors ``[3, *w.shape]`` whose sum is ``w`` to float32 accuracy
     (each is the bfloat16 rounding of what the ones before leave over)."""

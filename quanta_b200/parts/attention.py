@@ -206,6 +206,8 @@ class GQAttention(Mixer):
                 kernels.attn_span_split(q, cache.k, cache.v, out, ctx.tok_pos, cache.block_table, tiles, self.scale, window,
                                         ctx.status, chunk=self.chunk or 0)
                 return
+            if split_decode(ctx, q, cache.k, cache.v, out, cache.block_table, self.scale, window, chunk=self.chunk or 0):
+                return
             R = int(ctx.req_start.numel()) - 1
             n_split = None
             if self.hd % 4 or self.vd % 4:
@@ -227,7 +229,10 @@ class GQAttention(Mixer):
             starts = ctx.host.get("req_start") or [0, ctx.n_tokens]
             spans = [(r, starts[r], starts[r + 1] - starts[r]) for r in range(len(starts) - 1)]
             n_dec = 0
-        if n_dec:
+        if n_dec and kernels.attn_decode_direct_supported(self.nq, self.nkv, self.hd):
+            kernels.attn_decode_direct(q, cache.k, cache.v, out, dec_tok, n_dec, ctx.tok_pos, ctx.tok_req, cache.block_table, self.scale,
+                                       window, max(1, ctx.max_len_after), ctx.status)
+        elif n_dec:
             n_parts = kernels.attn_decode_parts(self.nkv, max(1, ctx.max_len_after))
             part_o = torch.empty(n_dec * self.nq * n_parts * self.hd, dtype=torch.float32, device=q.device)
             part_ml = torch.empty(n_dec * self.nq * n_parts * 2, dtype=torch.float32, device=q.device)
@@ -250,6 +255,18 @@ def span_tiles(ctx, spans, G: int, rows: int, hd: int, device):
             tiles.sort(key=lambda t: -(after[t[0]] - t[2] + min(t[2], (t[3] + rows) // G)))
         ctx.work[key] = torch.tensor(tiles, dtype=torch.int32).to(device, non_blocking=True)
     return ctx.work[key]
+
+
+def split_decode(ctx, q, cache_k, cache_v, out, table, scale: float, window: int, *, softcap: float = 0.0, chunk: int = 0) -> bool:
+    """A step of single tokens whose softmax weights stay 32-bit, as ``kernels.attn_decode_direct`` with weights of two parts; False
+    (and nothing done) for other steps and shapes."""
+    T, nq, hd = q.shape
+    if (q.dtype != torch.bfloat16 or cache_v.shape != cache_k.shape or not kernels.attn_decode_direct_supported(nq, cache_k.shape[1], hd)
+            or ctx.dec_tok is None or ctx.n_dec != T):
+        return False
+    kernels.attn_decode_direct(q, cache_k, cache_v, out, ctx.dec_tok, T, ctx.tok_pos, ctx.tok_req, table, scale, window,
+                               max(1, ctx.max_len_after), ctx.status, two_part=True, softcap=softcap, chunk=chunk)
+    return True
 
 
 # Steps with at least this many tokens beside one a request take the tcgen05 kernel with probabilities of two parts; below, the keys of

@@ -38,7 +38,7 @@ import torch
 
 from .. import kernels
 from ..matmul import empty_rows, linear
-from .attention import split_span_tiles
+from .attention import split_decode, split_span_tiles
 from .base import Addends, CacheSpec, CacheStream, KeepAll, Mixer, TensorSpec, Window, WindowAndOpenBlock, make, register
 
 
@@ -194,7 +194,7 @@ class WindowAttention(Mixer):
         if tiles is not None:
             kernels.attn_span_split(q, cache.k, cache.v, out, ctx.tok_pos, cache.tables["k"], tiles, self.scale, self.window,
                                     ctx.status, softcap=self.softcap)
-        else:
+        elif not (plain and split_decode(ctx, q, cache.k, cache.v, out, cache.tables["k"], self.scale, self.window, softcap=self.softcap)):
             kernels.window_attention(q, cache.k, cache.v, out, ctx.tok_pos, ctx.tok_req, cache.tables["k"], self.scale,
                                      self.window, ctx.status, dist_bias=self.dist_table, sink=self.sink,
                                      softcap=self.softcap, talk=self.talk, scratch=scratch,

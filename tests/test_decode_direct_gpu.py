@@ -1,0 +1,95 @@
+"""The attention of single tokens whose operands come straight from the cache rows, against float64: one to eight q heads a kv head, pages of
+any size, contexts at the edges of its rounds of 16 keys, of a block's warps and of the blocks of a cluster, windows.  Tolerance: weights and
+output are rounded to bfloat16 (2^-9 each, relative to the largest value), scores are float32."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def K():
+    from quanta_b200 import kernels
+    return kernels
+
+
+@pytest.mark.parametrize("nq,nkv,page,lens,window", [
+    (48, 8, 16, [1], 0), (48, 8, 16, [2100], 0), (6, 1, 16, [16, 17, 15, 128, 129, 1024, 1025], 0), (8, 1, 5, [333], 0), (2, 2, 64, [40] * 9, 0),
+    (16, 4, 16, [700, 3, 5000], 300), (7, 1, 128, [257], 16), (12, 4, 8, [600 + 7 * i for i in range(40)], 0), (4, 4, 16, [90] * 160, 33),
+    (5, 5, 16, [2000] * 30, 0)])
+def test_decode_direct(nq, nkv, page, lens, window):
+    kern, hd, G = K(), 128, nq // nkv
+    assert kern.attn_decode_direct_supported(nq, nkv, hd)
+    g = torch.Generator(device=DEV).manual_seed(len(lens) + nq)
+    per = [-(-n // page) for n in lens]
+    pages = sum(per) + 1
+    kc = torch.randn(pages, nkv, page, hd, device=DEV, generator=g).bfloat16()
+    vc = torch.randn(pages, nkv, page, hd, device=DEV, generator=g).bfloat16()
+    order = torch.randperm(pages, generator=torch.Generator().manual_seed(2)).int()
+    table = torch.full((len(lens), max(per)), -1, dtype=torch.int32)
+    at = 0
+    for r, n in enumerate(lens):
+        table[r, : per[r]] = order[at: at + per[r]]
+        at += per[r]
+        if window:
+            table[r, : max(0, n - window) // page] = -1            # given back
+    table = table.to(DEV)
+    R = len(lens)
+    q = (torch.randn(R + 2, nq, hd, device=DEV, generator=g) * 1.5).bfloat16()
+    rows = torch.randperm(R + 2, generator=torch.Generator().manual_seed(5))[:R].int()      # single tokens beside others of the step
+    pos, req = torch.zeros(R + 2, dtype=torch.int32), torch.zeros(R + 2, dtype=torch.int32)
+    for r, t in enumerate(rows.tolist()):
+        pos[t], req[t] = lens[r] - 1, r
+    out = torch.full((R + 2, nq, hd), 7.0, device=DEV, dtype=torch.bfloat16)
+    st = kern.new_status(DEV)
+    kern.attn_decode_direct(q, kc, vc, out, rows.to(DEV), R, pos.to(DEV), req.to(DEV), table, hd ** -0.5, window, max(lens) + 100, st)
+    assert st.tolist()[0] == 0
+    for r, t in enumerate(rows.tolist()):
+        j = torch.arange(max(0, lens[r] - window) if window else 0, lens[r], device=DEV)
+        row = table[r].long()[j // page]
+        k, v = kc[row, :, j % page].double(), vc[row, :, j % page].double()
+        s = torch.einsum("hgd,jhd->hgj", q[t].double().view(nkv, G, hd), k) * hd ** -0.5
+        want = torch.einsum("hgj,jhd->hgd", torch.softmax(s, -1), v).reshape(nq, hd)
+        assert float((out[t].double() - want).abs().max()) <= 2.0 ** -8 * float(v.abs().max())
+    others = [t for t in range(R + 2) if t not in rows.tolist()]
+    assert torch.all(out[others] == 7.0)
+    table[0, (lens[0] - 1) // page] = pages                        # a page outside the pool is recorded
+    kern.attn_decode_direct(q, kc, vc, out, rows.to(DEV), R, pos.to(DEV), req.to(DEV), table, hd ** -0.5, window, max(lens), st)
+    assert st.tolist()[0] == 2 and torch.isfinite(out.float()).all()
+
+
+@pytest.mark.parametrize("lens,window,chunk,cap", [([700, 1, 31], 300, 0, 30.0), ([1500] * 16, 1024, 0, 5.0), ([2100], 0, 128, 0.0),
+                                                   ([128, 129, 127, 256], 0, 128, 0.0), ([5000], 0, 0, 0.0), ([90] * 50, 17, 0, 0.0)])
+def test_weights_of_two_parts(lens, window, chunk, cap):
+    """As above with weights that hold 16 bits: 2^-12 of the largest value for them and their scores, and the output's rounding."""
+    kern, hd, nq, nkv, page = K(), 128, 16, 4, 16
+    g = torch.Generator(device=DEV).manual_seed(len(lens))
+    per = [-(-n // page) for n in lens]
+    kc = torch.randn(sum(per), nkv, page, hd, device=DEV, generator=g).bfloat16()
+    vc = torch.randn(sum(per), nkv, page, hd, device=DEV, generator=g).bfloat16()
+    table, at = torch.full((len(lens), max(per)), -1, dtype=torch.int32), 0
+    for r, n in enumerate(lens):
+        table[r, : per[r]] = torch.arange(at, at + per[r], dtype=torch.int32)
+        at += per[r]
+    table = table.to(DEV)
+    R = len(lens)
+    q = (torch.randn(R, nq, hd, device=DEV, generator=g) * 1.5).bfloat16()
+    pos, req = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV), torch.arange(R, dtype=torch.int32, device=DEV)
+    out, st = torch.empty_like(q), kern.new_status(DEV)
+    kern.attn_decode_direct(q, kc, vc, out, req, R, pos, req, table, hd ** -0.5, window, max(lens), st, two_part=True, softcap=cap, chunk=chunk)
+    assert st.tolist()[0] == 0
+    for r, n in enumerate(lens):
+        lo = (n - 1) // chunk * chunk if chunk else max(0, n - window) if window else 0
+        j = torch.arange(lo, n, device=DEV)
+        row = table[r].long()[j // page]
+        k, v = kc[row, :, j % page].double(), vc[row, :, j % page].double()
+        s = torch.einsum("hgd,jhd->hgj", q[r].double().view(nkv, nq // nkv, hd), k) * hd ** -0.5
+        s = cap * torch.tanh(s / cap) if cap else s
+        want = torch.einsum("hgj,jhd->hgd", torch.softmax(s, -1), v).reshape(nq, hd)
+        assert torch.all((out[r].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -12 * float(v.abs().max()))
+
+
+def test_sizes_that_are_not_taken():
+    assert not K().attn_decode_direct_supported(9, 1, 128) and not K().attn_decode_direct_supported(8, 8, 64)
