@@ -65,11 +65,15 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = global_ns();
+  uint64_t t0 = 0;
   for (uint32_t it = 0; it < EG_SPIN_LIMIT; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if ((it & 63u) == 63u && global_ns() - t0 > EG_WAIT_NS) break;      // both an iteration and a time limit
+    if ((it & 63u) == 63u) {      // both an iteration and a time limit
+      if (*abort_flag) return false;
+      const uint64_t now = global_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > EG_WAIT_NS) break;
+    }
   }
   *abort_flag = 1;
   return false;
@@ -92,6 +96,21 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
       " [%0], [%1, {%2, %3}], [%4], %5;"
       ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar), "l"(policy) : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar,
+                                            uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%2, %3, %4}], [%5], %6;"
+      ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint32_t bar,
+                                            uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%2, %3, %4, %5, %6}], [%7], %8;"
+      ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar), "l"(policy) : "memory");
 }
 
 // K-major operand tile in shared memory, rows of 128 bytes, 128-byte swizzle: 8-row groups 1024 bytes apart.
@@ -195,14 +214,19 @@ struct EgShared {
 // takes three quarters of the bytes from L2, and reads two thirds of the bytes from its shared memory, that
 // it would alone.  The first block of the pair issues all MMAs; every copy of either block counts on the
 // first block's barrier; a commit frees the stage in both.
-template <int MODE, int NM, bool PAIR>
+//
+// KS: slabs of 64 k a stage.  Two (launches of so few blocks that each streams its weights at the pace of its producer) come by one copy
+// a matrix: the maps have the slab as a dimension of its own, and with HALF also gate / up and the expert, so that the copy
+// leaves [slab][128 rows][64].
+template <int MODE, int NM, bool PAIR, int KS>
 __device__ __forceinline__ void
 expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
                     void* __restrict__ out, const int* __restrict__ sorted_pair, const float* __restrict__ pair_w,
                     const int* __restrict__ plan, const int* __restrict__ tile_expert,
                     const int* __restrict__ tile_row0, int E, int K, int N_out, int NT, int stages,
                     int tmem_cols, int gather_k, int* status, EgAct act) {
-  constexpr int FEATS = MODE == 1 ? EG_M : NM * EG_M;      // output features a block
+  constexpr bool HALF = MODE == 1 && NM == 1;              // 64 gate and 64 up rows in one weight tile
+  constexpr int FEATS = HALF ? EG_M / 2 : MODE == 1 ? EG_M : NM * EG_M;      // output features a block
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;     // 0: the block that issues the MMAs
   extern __shared__ unsigned char smem_dyn[];
   // stage buffers need 1024-byte alignment for the 128-byte swizzle
@@ -223,10 +247,31 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
   const int n_mma = min(NT, (rows + 15) & ~15);
   // a pair's block holds half of the MMA's token rows: rows [rank * n_mma / 2, +n_mma / 2) of the tile, as
   // the first rows of a box of NT / 2
-  const uint32_t a_bytes = EG_M * EG_BK * 2, b_bytes = (uint32_t)(PAIR ? NT / 2 : NT) * EG_BK * 2;
+  constexpr int BK = KS * EG_BK;
+  constexpr uint32_t A_SLAB = EG_M * EG_BK * 2, a_bytes = KS * A_SLAB;
+  const uint32_t b_slab = (uint32_t)(PAIR ? NT / 2 : NT) * EG_BK * 2, b_bytes = KS * b_slab;
   const uint32_t stage_bytes = NM * a_bytes + b_bytes;
-  const int k_blocks = (K + EG_BK - 1) / EG_BK;
+  const int k_blocks = (K + BK - 1) / BK;
   volatile int* abort_flag = &sh.abort_flag;
+  const int w_row = MODE == 1 ? e * 2 * N_out + j0 : e * N_out + j0;
+
+  // the second weight tile: the up rows of the same features, or the next 128 features (rows past the
+  // expert's last are another expert's and give columns that the epilogue drops)
+  const int w_row2 = w_row + (MODE == 1 ? N_out : EG_M);
+  auto load_weights = [&](int kb, uint32_t st, uint32_t bar, uint64_t pol) {
+    if constexpr (PAIR) {
+      tma_load_2d_pair(st, &tm_w, kb * EG_BK, w_row, bar, pol);
+      if (NM == 2) tma_load_2d_pair(st + a_bytes, &tm_w, kb * EG_BK, w_row2, bar, pol);
+    } else if constexpr (KS == 2 && HALF) {
+      tma_load_5d(st, &tm_w, 0, j0, 0, kb * KS, e, bar, pol);
+    } else if constexpr (KS == 2) {
+      tma_load_3d(st, &tm_w, 0, w_row, kb * KS, bar, pol);
+    } else {
+      tma_load_2d(st, &tm_w, kb * EG_BK, w_row, bar, pol);
+      if (HALF) tma_load_2d(st + a_bytes / 2, &tm_w, kb * EG_BK, w_row2, bar, pol);
+      if (NM == 2) tma_load_2d(st + a_bytes, &tm_w, kb * EG_BK, w_row2, bar, pol);
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -262,7 +307,6 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
   if (warp == 0) {
     // ---------------- TMA producer: lane 0 waits and fetches the boxes; where the token rows are fetched
     // one by one, all lanes take their share of them ----------------
-    const int w_row = MODE == 1 ? e * 2 * N_out + j0 : e * N_out + j0;
     // weights are read once per step by tiles of few rows (evict first); the 256-row tiles of one expert run at
     // about the same time and read the same weights, so those stay (measured: 5 % on a 16,384-token step)
     const uint64_t pol_w = PAIR ? l2_policy_evict_last() : l2_policy_evict_first(), pol_x = l2_policy_evict_last();
@@ -271,43 +315,60 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
     const int r_lo = PAIR ? (int)rank * (n_mma / 2) : 0;
     const int r_hi = PAIR ? min(rows, r_lo + n_mma / 2) : rows;
     int armed = 0;
-    for (int kb = 0; kb < k_blocks; ++kb) {
-      const int s = kb % stages;
-      const uint32_t ph = (uint32_t)(kb / stages) & 1u;
-      int ok = 1;
-      if (lane == 0) ok = mbar_wait(smem_u32(&sh.empty[s]), ph ^ 1u, abort_flag) ? 1 : 0;
-      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-      const uint32_t full = smem_u32(&sh.full[s]);
-      // a pair: every copy of either block counts on the first block's barrier, which expects both blocks'
-      // bytes (the second block's copies may count before the first has said so)
-      const uint32_t bar = PAIR ? mapa_u32(full, 0u) : full;
-      unsigned char* st = tiles + (size_t)s * stage_bytes;
+    // Nothing in this loop waits for memory, and it has to come round faster than the tensor cores use a stage (512 cycles for a pair's
+    // two matrices): stage and parity are counted, addresses step, and lane 0 runs alone unless rows are fetched one by one.  With a
+    // division by the number of stages a turn took 880 cycles, with rows one by one 1,140.
+    const uint32_t x_bytes = by_row ? (uint32_t)rows * BK * 2 : (PAIR ? 2u : 1u) * b_bytes;
+    const uint32_t tx = (PAIR ? 2u : 1u) * NM * a_bytes + x_bytes;
+    const uint32_t full0 = smem_u32(&sh.full[0]), empty0 = smem_u32(&sh.empty[0]), ring = smem_u32(tiles);
+    // a pair: every copy of either block counts on the first block's barrier, which expects both blocks'
+    // bytes (the second block's copies may count before the first has said so)
+    const uint32_t bars = PAIR ? mapa_u32(full0, 0u) : full0;
+    uint32_t st = ring, parity = 1u;
+    int s = 0;
+    auto turn = [&](int kb) {      // lane 0: the boxes of a stage
+      const uint32_t bar = bars + 8u * s;
+      if (rank == 0) mbar_expect_tx(full0 + 8u * s, tx);
+      load_weights(kb, st, bar, pol_w);
+      if (!by_row) {
+        if constexpr (PAIR) tma_load_2d_pair(st + NM * a_bytes, &tm_x, kb * EG_BK, row0 + r_lo, bar, pol_x);
+        else if constexpr (KS == 2) tma_load_3d(st + NM * a_bytes, &tm_x, 0, row0, kb * KS, bar, pol_x);
+        else tma_load_2d(st + NM * a_bytes, &tm_x, kb * EG_BK, row0, bar, pol_x);
+      }
+    };
+    auto next = [&] {
+      st += stage_bytes;
+      if (++s == stages) { s = 0; st = ring; parity ^= 1u; }
+    };
+    if (!by_row) {
       if (lane == 0) {
-        const uint32_t x_bytes = by_row ? (uint32_t)rows * EG_BK * 2 : (PAIR ? 2u : 1u) * b_bytes;
-        if (rank == 0) mbar_expect_tx(full, (PAIR ? 2u : 1u) * NM * a_bytes + x_bytes);
-        // the second weight tile: the up rows of the same features, or the next 128 features (rows past the
-        // expert's last are another expert's and give columns that the epilogue drops)
-        if (PAIR) {
-          tma_load_2d_pair(smem_u32(st), &tm_w, kb * EG_BK, w_row, bar, pol_w);
-          if (NM == 2) tma_load_2d_pair(smem_u32(st + a_bytes), &tm_w, kb * EG_BK, w_row + (MODE == 1 ? N_out : EG_M), bar, pol_w);
-          if (!by_row) tma_load_2d_pair(smem_u32(st + NM * a_bytes), &tm_x, kb * EG_BK, row0 + r_lo, bar, pol_x);
-        } else {
-          tma_load_2d(smem_u32(st), &tm_w, kb * EG_BK, w_row, bar, pol_w);
-          if (NM == 2) tma_load_2d(smem_u32(st + a_bytes), &tm_w, kb * EG_BK, w_row + (MODE == 1 ? N_out : EG_M), bar, pol_w);
-          if (!by_row) tma_load_2d(smem_u32(st + NM * a_bytes), &tm_x, kb * EG_BK, row0, bar, pol_x);
+#pragma unroll 1
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!mbar_wait(empty0 + 8u * s, parity, abort_flag)) break;
+          turn(kb);
+          armed = kb + 1;
+          next();
         }
       }
-      if (by_row) {
+    } else {
+#pragma unroll 1
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        int ok = 1;
+        if (lane == 0) ok = mbar_wait(empty0 + 8u * s, parity, abort_flag) ? 1 : 0;
+        if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+        if (lane == 0) turn(kb);
         // boxes of one row: the swizzle follows the shared-memory address, so a row lands where a box of
         // many rows would have put it; the rows past the expert's last keep what the stage held before, and
         // their columns of the product are never read
         for (int i = r_lo + lane; i < r_hi; i += 32) {
-          const uint32_t dst = smem_u32(st + NM * a_bytes + (i - r_lo) * (EG_BK * 2));
-          if (PAIR) tma_load_2d_pair(dst, &tm_x, kb * EG_BK, s_pair[i], bar, pol_x);
-          else tma_load_2d(dst, &tm_x, kb * EG_BK, s_pair[i], bar, pol_x);
+          const uint32_t dst = st + NM * a_bytes + (i - r_lo) * (EG_BK * 2);
+          if (PAIR) tma_load_2d_pair(dst, &tm_x, kb * BK, s_pair[i], bars + 8u * s, pol_x);
+          else tma_load_2d(dst, &tm_x, kb * BK, s_pair[i], bars + 8u * s, pol_x);
+          if (KS == 2) tma_load_2d(dst + b_slab, &tm_x, kb * BK + EG_BK, s_pair[i], bars + 8u * s, pol_x);      // zeros past the last slab
         }
+        armed = kb + 1;
+        next();
       }
-      armed = kb + 1;
     }
     if (lane == 0) {
       if (*abort_flag && PAIR && rank != 0) {
@@ -330,30 +391,34 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
     if (lane == 0 && rank == 0) {
       const uint32_t idesc = umma_idesc(PAIR ? 2 * EG_M : EG_M, n_mma);
       bool ok = true;
-      for (int kb = 0; kb < k_blocks && ok; ++kb) {
-        const int s = kb % stages;
-        const uint32_t ph = (uint32_t)(kb / stages) & 1u;
-        ok = mbar_wait(smem_u32(&sh.full[s]), ph, abort_flag);
+      const uint32_t full0 = smem_u32(&sh.full[0]), empty0 = smem_u32(&sh.empty[0]);
+      // the descriptors of the first stage's tiles; the address field counts 16 bytes
+      const uint64_t a_first = umma_desc_sw128(smem_u32(tiles)), b_first = umma_desc_sw128(smem_u32(tiles) + NM * a_bytes);
+      uint64_t at = 0;
+      uint32_t parity = 0u, acc = 0u;
+      int s = 0;
+#pragma unroll 1
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        ok = mbar_wait(full0 + 8u * s, parity, abort_flag);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = smem_u32(tiles + (size_t)s * stage_bytes);
-        const uint64_t b_desc = umma_desc_sw128(st + NM * a_bytes);
 #pragma unroll
         for (int m = 0; m < NM; ++m) {
-          const uint64_t a_desc = umma_desc_sw128(st + m * a_bytes);
 #pragma unroll
-          for (int k16 = 0; k16 < EG_BK / 16; ++k16) {
+          for (int k16 = 0; k16 < BK / 16; ++k16) {
             // 16 k elements = 32 bytes further along the swizzled row: +2 in the 16-byte address field
-            if (PAIR)
-              umma_bf16_pair(tmem_base + (uint32_t)(m * NT), a_desc + (uint64_t)(k16 * 2), b_desc + (uint64_t)(k16 * 2),
-                             idesc, (kb | k16) != 0 ? 1u : 0u);
-            else
-              umma_bf16(tmem_base + (uint32_t)(m * NT), a_desc + (uint64_t)(k16 * 2), b_desc + (uint64_t)(k16 * 2), idesc,
-                        (kb | k16) != 0 ? 1u : 0u);
+            const int slab = k16 / (EG_BK / 16), in = k16 % (EG_BK / 16) * 2;
+            const uint64_t a_desc = a_first + at + (uint64_t)((m * (int)a_bytes + slab * (int)A_SLAB) / 16 + in);
+            const uint64_t b_desc = b_first + at + (uint64_t)(slab * (int)(b_slab >> 4) + in);
+            if (PAIR) umma_bf16_pair(tmem_base + (uint32_t)(m * NT), a_desc, b_desc, idesc, k16 != 0 ? 1u : acc);
+            else umma_bf16(tmem_base + (uint32_t)(m * NT), a_desc, b_desc, idesc, k16 != 0 ? 1u : acc);
           }
         }
         // the stage is free once these MMAs have read it
-        if (PAIR) umma_commit_pair(smem_u32(&sh.empty[s])); else umma_commit(smem_u32(&sh.empty[s]));
+        if (PAIR) umma_commit_pair(empty0 + 8u * s); else umma_commit(empty0 + 8u * s);
+        acc = 1u;
+        at += stage_bytes >> 4;
+        if (++s == stages) { s = 0; at = 0; parity ^= 1u; }
       }
       if (ok) {
         if (PAIR) umma_commit_pair(smem_u32(&sh.tmem_full)); else umma_commit(smem_u32(&sh.tmem_full));
@@ -365,6 +430,7 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
     constexpr int SPLIT = PAIR ? 2 : 1;
     constexpr int EPI_THREADS = SPLIT * 128;
     const int quad = warp & 3, sub = (warp - 2) >> 2;
+    float* ups = reinterpret_cast<float*>(tiles);      // HALF: [NT][64], over the ring when all products are done
     const int feat = j0 + quad * 32 + lane;
     if (MODE == 2 || (MODE == 1 && act.kind == 1)) {
       // where each row goes and its routing weight: fetched here, under the main loop, by the warps that
@@ -383,6 +449,19 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
     if (acc_ready) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
+      if (HALF && quad >= 2) {
+        for (int c0 = 0; c0 < rows; c0 += 16) {
+          uint32_t v[16];
+          tmem_ld16(lane_addr + (uint32_t)c0, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 16; ++i) ups[(c0 + i) * (EG_M / 2) + (quad - 2) * 32 + lane] = __uint_as_float(v[i]);
+        }
+      }
+    }
+    if (HALF) asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
+    if (acc_ready && !(HALF && quad >= 2)) {
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
       for (int c0 = 16 * sub; c0 < rows; c0 += 16 * SPLIT) {
         uint32_t v0[16], v1[16];
         tmem_ld16(lane_addr + (uint32_t)c0, v0);
@@ -394,7 +473,7 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
           __nv_bfloat16 r[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const float g = __uint_as_float(v0[i]), u = __uint_as_float(v1[i]);
+            const float g = __uint_as_float(v0[i]), u = HALF ? ups[(c0 + i) * (EG_M / 2) + quad * 32 + lane] : __uint_as_float(v1[i]);
             r[i] = __float2bfloat16_rn(act.kind == 1 ? clamped_glu(g, u, s_w[c0 + i], act) : silu_mul(g, u));
           }
           if (feat < N_out) {
@@ -452,13 +531,13 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
       int stages, int tmem_cols, int gather_k, int* status, EgAct act
 #define QB_EG_ARGS tm_w, tm_x, out, sorted_pair, pair_w, plan, tile_expert, tile_row0, E, K, N_out, NT, stages, tmem_cols, gather_k, status, act
 
-template <int MODE, int NM>
+template <int MODE, int NM, int KS>
 __global__ void __launch_bounds__(EG_THREADS, 2) expert_gemm_tc_kernel(QB_EG_PARAMS) {
-  expert_gemm_tc_body<MODE, NM, false>(QB_EG_ARGS);
+  expert_gemm_tc_body<MODE, NM, false, KS>(QB_EG_ARGS);
 }
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EG_PAIR_THREADS, 1) expert_gemm_tc_pair_kernel(QB_EG_PARAMS) {
-  expert_gemm_tc_body<MODE, 2, true>(QB_EG_ARGS);
+  expert_gemm_tc_body<MODE, 2, true, 1>(QB_EG_ARGS);
 }
 
 // out[p, :] = x[sorted_pair[p] / top_k, :]   (rows of 16-byte chunks)
@@ -487,18 +566,33 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// 2-D bfloat16 tensor [rows, K] row-major, boxes of [box_rows, 64] with the 128-byte swizzle
-int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
+// bfloat16, boxes with the 128-byte swizzle; dims and boxes innermost first, strides in bytes of all but the innermost
+int make_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return QB_ERR_UNSUPPORTED;
-  const cuuint64_t dims[2] = {K, rows};
-  const cuuint64_t strides[1] = {K * 2};
-  const cuuint32_t box[2] = {EG_BK, box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : QB_ERR_BAD_ARG;
+}
+// [rows, K] row-major, boxes of [box_rows, 64]
+int map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
+  const cuuint64_t dims[2] = {K, rows}, strides[1] = {K * 2};
+  const cuuint32_t box[2] = {EG_BK, box_rows};
+  return make_map(map, base, 2, dims, strides, box);
+}
+// [rows, K / 64, 64], boxes of two slabs: [2][box_rows][64] in shared memory (zeros past the last slab)
+int map_slabs(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
+  const cuuint64_t dims[3] = {EG_BK, rows, K / EG_BK}, strides[2] = {K * 2, EG_BK * 2};
+  const cuuint32_t box[3] = {EG_BK, box_rows, 2};
+  return make_map(map, base, 3, dims, strides, box);
+}
+// [experts, gate / up, I, K / 64, 64], boxes [2 slabs][gate, up][64 features][64]
+int map_gate_up(CUtensorMap* map, const void* base, uint64_t experts, uint64_t I, uint64_t K) {
+  const cuuint64_t dims[5] = {EG_BK, I, 2, K / EG_BK, experts}, strides[4] = {K * 2, I * K * 2, EG_BK * 2, 2 * I * K * 2};
+  const cuuint32_t box[5] = {EG_BK, EG_M / 2, 2, 2, 1};
+  return make_map(map, base, 5, dims, strides, box);
 }
 
 }  // namespace
@@ -533,43 +627,54 @@ extern "C" int qb_expert_gemm_tc(int mode, const void* x_rows, const void* weigh
   if (mode != 1 && mode != 2 && mode != 3) return QB_ERR_BAD_ARG;
   // weight tiles a block: gate and up (mode 1); two blocks of 128 features for the down product of 256-row
   // token tiles (see the kernel)
-  const int nm = (mode == 1 || NT >= 128) ? 2 : 1;
-  const int feats = mode == 1 ? EG_M : nm * EG_M;
-  // tiles of 256 token rows (steps bound by the tensor cores) are taken by pairs of blocks, see the kernel
-  const bool pair = NT == 256;
-  if (((uintptr_t)x_rows | (uintptr_t)weights) & 15) return QB_ERR_BAD_ARG;
-  CUtensorMap tm_w, tm_x;
-  int rc = make_map(&tm_w, weights, (uint64_t)weight_experts * (mode == 1 ? 2 : 1) * N_out, (uint64_t)K, EG_M);
-  if (rc) return rc;
-  if (gather_k < 0 || (gather_k > 0 && (mode == 2 || n_rows <= 0))) return QB_ERR_BAD_ARG;
-  rc = gather_k > 0 ? make_map(&tm_x, x_rows, (uint64_t)n_rows, (uint64_t)K, 1u)
-                    : make_map(&tm_x, x_rows, (uint64_t)n_pairs, (uint64_t)K, (uint32_t)(pair ? NT / 2 : NT));
-  if (rc) return rc;
-  const size_t stage_bytes = (size_t)nm * EG_M * EG_BK * 2 + (size_t)(pair ? NT / 2 : NT) * EG_BK * 2;
-  // Two blocks share an SM (shared memory is the limit), so that one block's prologue and epilogue run
-  // under the other's main loop; each gets a ring of about 105 KB.
-  // a tile of 256 token rows has a block to itself on its SM (its two accumulators fill the TMEM)
-  // and so has every block of a launch of no more blocks than there are SMs (a single token's step)
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       sms = 1;
   }
+  // the gated first product of so few tiles that blocks of 128 features would leave SMs idle: blocks of 64, gate and up in one weight tile
+  // (one token, 8 of 256 experts of 3,072 x 1,536: 96 blocks 33.0 us with one slab a stage, 192 blocks of half the size 28.4)
+  const bool half = mode == 1 && NT <= 32 && (size_t)((N_out + EG_M - 1) / EG_M) * (size_t)max_tiles <= (size_t)sms;
+  const int nm = half ? 1 : (mode == 1 || NT >= 128) ? 2 : 1;
+  const int feats = half ? EG_M / 2 : mode == 1 ? EG_M : nm * EG_M;
+  // tiles of 256 token rows (steps bound by the tensor cores) are taken by pairs of blocks, see the kernel
+  const bool pair = NT == 256;
+  if (((uintptr_t)x_rows | (uintptr_t)weights) & 15) return QB_ERR_BAD_ARG;
+  // Two blocks share an SM (shared memory is the limit), so that one block's prologue and epilogue run
+  // under the other's main loop; each gets a ring of about 105 KB.
+  // a tile of 256 token rows has a block to itself on its SM (its two accumulators fill the TMEM)
+  // and so has every block of a launch of no more blocks than there are SMs (a single token's step)
   int grid_x = (N_out + feats - 1) / feats;
   if (pair) grid_x = (grid_x + 1) & ~1;      // a pair's second block may lie past the last feature: it drops its columns
   const size_t blocks = (size_t)grid_x * (size_t)max_tiles;
   const bool alone = NT > 128 || blocks <= (size_t)sms;
+  // Launches of at most two blocks an SM are bound by how fast a block's producer and issuer go round: stages of two slabs (one token of
+  // an 8-expert layer 2,048 x 2,112, 18 MB: 16.1 + 12.6 us for its two products with one slab a stage, 10.9 + 10.7 with two).
+  const int ks = nm == 1 && NT <= 32 && K % EG_BK == 0 && blocks <= 2 * (size_t)sms ? 2 : 1;
+  const uint64_t w_experts = (uint64_t)weight_experts, rows_x = (uint64_t)(gather_k > 0 ? n_rows : n_pairs);
+  if (gather_k < 0 || (gather_k > 0 && (mode == 2 || n_rows <= 0))) return QB_ERR_BAD_ARG;
+  CUtensorMap tm_w, tm_x;
+  int rc;
+  if (ks == 2 && half) rc = map_gate_up(&tm_w, weights, w_experts, (uint64_t)N_out, (uint64_t)K);
+  else if (ks == 2) rc = map_slabs(&tm_w, weights, w_experts * N_out, (uint64_t)K, EG_M);
+  else rc = map_2d(&tm_w, weights, w_experts * (mode == 1 ? 2 : 1) * N_out, (uint64_t)K, half ? EG_M / 2 : EG_M);
+  if (rc) return rc;
+  if (gather_k > 0) rc = map_2d(&tm_x, x_rows, rows_x, (uint64_t)K, 1u);
+  else if (ks == 2) rc = map_slabs(&tm_x, x_rows, rows_x, (uint64_t)K, (uint32_t)NT);
+  else rc = map_2d(&tm_x, x_rows, rows_x, (uint64_t)K, (uint32_t)(pair ? NT / 2 : NT));
+  if (rc) return rc;
+  const size_t stage_bytes = (size_t)ks * EG_BK * 2 * ((size_t)nm * EG_M + (size_t)(pair ? NT / 2 : NT));
   // Token tiles of at most 32 rows (decode steps of a few tokens: short blocks, one expert's 128 features
   // each): three blocks an SM with rings of about 70 KB hide a block's prologue and epilogue better than
   // two with 105 KB (measured at 8 tokens: 154 + 80 us against 161 + 86 us for the two products of a layer).
-  int stages = (int)((size_t)(alone ? 200 * 1024 : 105 * 1024) / stage_bytes);
-  if (!alone && NT <= 32 && 72000 / stage_bytes >= 2) stages = (int)(72000 / stage_bytes);    // three blocks an SM
+  int stages = (int)((size_t)(alone ? 200 * 1024 : ks == 2 ? 109 * 1024 : 105 * 1024) / stage_bytes);
+  if (blocks > 2 * (size_t)sms && NT <= 32 && 72000 / stage_bytes >= 2) stages = (int)(72000 / stage_bytes);    // three blocks an SM
   // the down product of 64-row tiles (steps of 33 to 64 tokens): four blocks an SM with two stages each
   // (measured at 64 tokens: 308 us against 330 us)
   if (!alone && mode == 2 && NT == 64 && 50000 / stage_bytes >= 2) stages = (int)(50000 / stage_bytes);
   if (stages > 8) stages = 8;
-  const int k_blocks = (K + EG_BK - 1) / EG_BK;
+  const int k_blocks = (K + ks * EG_BK - 1) / (ks * EG_BK);
   if (stages > k_blocks) stages = k_blocks;
   if (stages < 2 && k_blocks >= 2) return QB_ERR_UNSUPPORTED;
   const size_t smem = stage_bytes * stages + 1024;
@@ -587,11 +692,15 @@ extern "C" int qb_expert_gemm_tc(int mode, const void* x_rows, const void* weigh
   if (pair && mode == 1) QB_EG(expert_gemm_tc_pair_kernel<1>, gather_k, EG_PAIR_THREADS);
   else if (pair && mode == 3) QB_EG(expert_gemm_tc_pair_kernel<3>, gather_k, EG_PAIR_THREADS);
   else if (pair) QB_EG(expert_gemm_tc_pair_kernel<2>, 0, EG_PAIR_THREADS);
-  else if (mode == 1) QB_EG((expert_gemm_tc_kernel<1, 2>), gather_k, EG_THREADS);
-  else if (mode == 3 && nm == 2) QB_EG((expert_gemm_tc_kernel<3, 2>), gather_k, EG_THREADS);
-  else if (mode == 3) QB_EG((expert_gemm_tc_kernel<3, 1>), gather_k, EG_THREADS);
-  else if (nm == 2) QB_EG((expert_gemm_tc_kernel<2, 2>), 0, EG_THREADS);
-  else QB_EG((expert_gemm_tc_kernel<2, 1>), 0, EG_THREADS);
+  else if (ks == 2 && mode == 1) QB_EG((expert_gemm_tc_kernel<1, 1, 2>), gather_k, EG_THREADS);
+  else if (ks == 2 && mode == 3) QB_EG((expert_gemm_tc_kernel<3, 1, 2>), gather_k, EG_THREADS);
+  else if (ks == 2) QB_EG((expert_gemm_tc_kernel<2, 1, 2>), 0, EG_THREADS);
+  else if (half) QB_EG((expert_gemm_tc_kernel<1, 1, 1>), gather_k, EG_THREADS);
+  else if (mode == 1) QB_EG((expert_gemm_tc_kernel<1, 2, 1>), gather_k, EG_THREADS);
+  else if (mode == 3 && nm == 2) QB_EG((expert_gemm_tc_kernel<3, 2, 1>), gather_k, EG_THREADS);
+  else if (mode == 3) QB_EG((expert_gemm_tc_kernel<3, 1, 1>), gather_k, EG_THREADS);
+  else if (nm == 2) QB_EG((expert_gemm_tc_kernel<2, 2, 1>), 0, EG_THREADS);
+  else QB_EG((expert_gemm_tc_kernel<2, 1, 1>), 0, EG_THREADS);
 #undef QB_EG
   QB_LAUNCH_CHECK();
   return 0;
