@@ -67,6 +67,7 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(DD_MAX_WARPS * 32)
 attn_decode_direct_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
                           const __nv_bfloat16* __restrict__ v_cache, __nv_bfloat16* __restrict__ out, const DecodeArgs P) {
+  qb_follow();
   extern __shared__ __align__(128) unsigned char dd_smem[];
   // rings first; then a warp's sums, a head's 128 numbers in the order 8 e + g | 64 + 8 e + g
   __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(dd_smem);
@@ -321,12 +322,14 @@ extern "C" int qb_attn_decode_direct(const void* q, const void* k_cache, const v
   auto kern = two_part ? attn_decode_direct_kernel<true> : attn_decode_direct_kernel<false>;
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DD_MAX_WARPS * DD_STAGES * DD_ROUND * 2);
   if (err != cudaSuccess) return (int)err;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)S;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see qb_follow
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)S;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = S > 1 ? 1 : 0;
+  cfg.numAttrs = S > 1 ? 2 : 1;
   err = cudaLaunchKernelEx(&cfg, kern, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache,
                                              (const __nv_bfloat16*)v_cache, (__nv_bfloat16*)out, P);
   if (err != cudaSuccess) return (int)err;

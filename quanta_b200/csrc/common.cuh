@@ -33,6 +33,30 @@
     if (e__ != cudaSuccess) return (int)e__;     \
   } while (0)
 
+// A kernel launched with qb_launch may have its blocks placed while the launch before it on the stream still runs.  Its first statement,
+// qb_follow(), waits until that launch has ended and its writes are seen, and only then lets the launch after it be placed; so whatever
+// was enqueued two launches before has ended too, and the order on the stream is what it was.  What it saves is the gap between
+// two launches (a step of one token has 42, a step of 8 tokens of the model with a delta rule 68).  All threads of all blocks call it, whatever they do next.
+__device__ __forceinline__ void qb_follow() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t qb_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ void qb_set_status(int* status, int code, int detail, int kernel_id) {
   if (status != nullptr && atomicCAS(status, 0, code) == 0) {
     status[1] = detail;

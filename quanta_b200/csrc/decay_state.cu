@@ -141,6 +141,7 @@ __global__ void memory_gates_single_kernel(const float* __restrict__ proj, int s
                                            float* __restrict__ m_state, float* __restrict__ log_decay,
                                            float* __restrict__ weight, float* __restrict__ floor_out,
                                            const int* __restrict__ req_slot, int R, int H) {
+  qb_follow();
   const int at = blockIdx.x * blockDim.x + threadIdx.x;        // token r of request r
   if (at >= R * H) return;
   const int r = at / H, h = at % H;
@@ -162,7 +163,7 @@ extern "C" int qb_memory_gates(const float* proj, int stride, int i_off, int f_o
   if (T <= 0 || R <= 0) return 0;
   if (H <= 0 || H > 65535 || !(cap > 0.f)) return QB_ERR_BAD_ARG;
   if (T == R) {                                     // every request of a step brings at least one token
-    memory_gates_single_kernel<<<(R * H + 63) / 64, 64, 0, stream>>>(proj, stride, i_off, f_off, i_bias, f_bias, cap, m_state,
+    qb_launch(memory_gates_single_kernel, (R * H + 63) / 64, 64, 0, stream, proj, stride, i_off, f_off, i_bias, f_bias, cap, m_state,
                                                                      log_decay, weight, floor_out, req_slot, R, H);
     QB_LAUNCH_CHECK();
     return 0;
@@ -193,6 +194,7 @@ ds_chain_kernel(const U* __restrict__ q, const U* __restrict__ k, const U* __res
                 float* __restrict__ state, float* __restrict__ n_state, const float* __restrict__ floor_in,
                 float* __restrict__ den, float* __restrict__ out, const int* __restrict__ req_start,
                 const int* __restrict__ req_slot, float q_scale, int silu, int cols, int max_tokens) {
+  qb_follow();
   extern __shared__ __align__(16) float ds_sm[];
   const int D = sh.D, E = sh.E, H = sh.H;
   float* s_k = ds_sm;                          // [TB][D]
@@ -361,7 +363,7 @@ extern "C" int qb_decay_chain(const void* q, const void* k, const void* v, int i
 #define DS_CHAIN(VEC, NR)                                                                                          \
   if (single) DS_CHAIN_TURN(VEC, NR, 1); else DS_CHAIN_TURN(VEC, NR, DS_TURN)
 #define DS_CHAIN_TURN(VEC, NR, TB_)                                                                                \
-  ds_chain_kernel<U, VEC, NR, TB_><<<grid, DS_CHAIN_THREADS, smem, stream>>>(                                           \
+  qb_launch(ds_chain_kernel<U, VEC, NR, TB_>, grid, DS_CHAIN_THREADS, smem, stream,                                            \
       (const U*)q, (const U*)k, (const U*)v, sh, gates, state, n_state, floor_in, den, out, req_start, req_slot,   \
       q_scale, silu, cols, max_tokens)
   QB_DISPATCH_DTYPE(in_dtype, U, {
@@ -927,6 +929,7 @@ extern "C" int qb_decay_chunks(const void* q, const void* k, const void* v, long
 template <typename O>
 __global__ void rows_act_kernel(const float* __restrict__ x, long long stride, O* __restrict__ out, int T, int n, int silu,
                                 int vec) {
+  qb_follow();
   if (vec) {
     const int n8 = n / 8;
     const size_t total = (size_t)T * n8;
@@ -956,7 +959,7 @@ extern "C" int qb_rows_act(const float* x, long long stride, void* out, int out_
   const int vec = n % 8 == 0 && stride % 4 == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0;
   const size_t items = (size_t)T * n / (vec ? 8 : 1);
   const int blocks = (int)((items + 255) / 256 < 8192 ? (items + 255) / 256 : 8192);
-  QB_DISPATCH_DTYPE(out_dtype, O, rows_act_kernel<O><<<blocks, 256, 0, stream>>>(x, stride, (O*)out, T, n, silu, vec));
+  QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(rows_act_kernel<O>, blocks, 256, 0, stream, x, stride, (O*)out, T, n, silu, vec));
   QB_LAUNCH_CHECK();
   return 0;
 }
@@ -977,6 +980,7 @@ decay_out_kernel(const float* __restrict__ o, const float* __restrict__ den, con
                  const float* __restrict__ skip, const float* __restrict__ gate, long long gate_stride,
                  const float* __restrict__ gain, O* __restrict__ out, int T, int H, int E, int parts, float eps,
                  int gate_first) {
+  qb_follow();
   extern __shared__ __align__(16) float s_part[];
   __shared__ float s_sum[32];
   const int HE = H * E, n = HE / parts;
@@ -1093,7 +1097,7 @@ extern "C" int qb_decay_out(const float* o, const float* den, const void* x, lon
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);              \
       if (e != cudaSuccess) return (int)e;                                                                            \
     }                                                                                                                 \
-    kern<<<(unsigned)blocks, WARPS == 1 ? 128 : 256, smem, stream>>>(o, den, (const O*)x, x_stride, skip, gate,        \
+    qb_launch(kern, (unsigned)blocks, WARPS == 1 ? 128 : 256, smem, stream, o, den, (const O*)x, x_stride, skip, gate,  \
                                                                      gate_stride, gain, (O*)out, T, H, E, parts, eps, \
                                                                      gate_first);                                     \
   } while (0)

@@ -163,6 +163,7 @@ delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, 
                     const float* __restrict__ wpre, const float* __restrict__ a_bias, const float* __restrict__ w_bias,
                     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ req_start,
                     const int* __restrict__ req_slot, int H, int D, int c4, float decay_scale, float unit_eps) {
+  qb_follow();
   __shared__ float s_u[DS_MAX_DIM], s_w[DS_MAX_DIM], s_au[DS_MAX_DIM], s_k[DS_MAX_DIM], s_r[DS_MAX_DIM], s_ss[8];
   __shared__ __align__(16) float4 s_dot[8][16], s_out[8][16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, r = blockIdx.z;
@@ -701,7 +702,7 @@ extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int 
     const int c4 = CB / 4, rows = (D * c4 + DS_THREADS - 1) / DS_THREADS;
     const dim3 single((D + CB - 1) / CB, H, R);
 #define DS_SINGLE(N)                                                                                                             \
-  delta_single_kernel<N><<<single, DS_THREADS, 0, stream>>>(proj, proj_stride, r_off, k_off, v_off, a_off, wpre, a_bias, w_bias,  \
+  qb_launch(delta_single_kernel<N>, single, DS_THREADS, 0, stream, proj, proj_stride, r_off, k_off, v_off, a_off, wpre, a_bias, w_bias,  \
                                                             state, out, req_start, req_slot, H, D, c4, decay_scale, unit_eps)
     if (rows <= 2) DS_SINGLE(2);
     else if (rows <= 4) DS_SINGLE(4);
@@ -755,6 +756,7 @@ extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int 
 template <typename O>
 __global__ void tanh_cols_kernel(const float* __restrict__ x, int x_stride, int off, O* __restrict__ out,
                                  int T, int n) {
+  qb_follow();
   const size_t total = (size_t)T * n;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t t = i / n, c = i % n;
@@ -767,7 +769,7 @@ extern "C" int qb_tanh_cols(const float* x, int x_stride, int off, void* out, in
   if (T <= 0 || n <= 0) return 0;
   const size_t total = (size_t)T * n;
   const int blocks = (int)((total + 255) / 256 < 2048 ? (total + 255) / 256 : 2048);
-  QB_DISPATCH_DTYPE(out_dtype, O, tanh_cols_kernel<O><<<blocks, 256, 0, stream>>>(x, x_stride, off, (O*)out, T, n));
+  QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(tanh_cols_kernel<O>, blocks, 256, 0, stream, x, x_stride, off, (O*)out, T, n));
   QB_LAUNCH_CHECK();
   return 0;
 }

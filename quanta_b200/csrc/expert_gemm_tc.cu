@@ -224,7 +224,8 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
                     void* __restrict__ out, const int* __restrict__ sorted_pair, const float* __restrict__ pair_w,
                     const int* __restrict__ plan, const int* __restrict__ tile_expert,
                     const int* __restrict__ tile_row0, int E, int K, int N_out, int NT, int stages,
-                    int tmem_cols, int gather_k, int* status, EgAct act) {
+                    int tmem_cols, int gather_k, int* status, EgAct act, int early) {
+  if (!early) qb_follow();
   constexpr bool HALF = MODE == 1 && NM == 1;              // 64 gate and 64 up rows in one weight tile
   constexpr int FEATS = HALF ? EG_M / 2 : MODE == 1 ? EG_M : NM * EG_M;      // output features a block
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;     // 0: the block that issues the MMAs
@@ -235,11 +236,15 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
   __shared__ int s_pair[256];
   __shared__ float s_w[256];
 
-  const int num_tiles = plan[3 * E + 1];
+  // (from L2: an early block has not waited yet)
+  const int num_tiles = __ldcg(plan + 3 * E + 1);
   const int tile = blockIdx.y;
-  if (tile >= num_tiles) return;
-  const int e = tile_expert[tile], row0 = tile_row0[tile];
-  const int rows = min(NT, plan[2 * E + e + 1] - row0);          // valid token rows of this tile
+  if (tile >= num_tiles) {
+    if (early) qb_follow();
+    return;
+  }
+  const int e = __ldcg(tile_expert + tile), row0 = __ldcg(tile_row0 + tile);
+  const int rows = min(NT, __ldcg(plan + 2 * E + e + 1) - row0);          // valid token rows of this tile
   const int j0 = blockIdx.x * FEATS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the MMA's N is what this tile holds, in steps of 16: an expert's last tile of a few rows costs the
@@ -254,6 +259,7 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
   const int k_blocks = (K + BK - 1) / BK;
   volatile int* abort_flag = &sh.abort_flag;
   const int w_row = MODE == 1 ? e * 2 * N_out + j0 : e * N_out + j0;
+  const int ahead = MODE == 2 && !PAIR && early ? min(stages, k_blocks) : 0;      // k blocks whose weights are fetched before the wait
 
   // the second weight tile: the up rows of the same features, or the next 128 features (rows past the
   // expert's last are another expert's and give columns that the epilogue drops)
@@ -281,7 +287,15 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
     mbar_init(smem_u32(&sh.tmem_full), 1);
     sh.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // an early block's first weights are on their way while the launch before it ends
+    for (int kb = 0; kb < ahead; ++kb) {
+      const uint32_t full = smem_u32(&sh.full[kb]);
+      mbar_expect_tx(full, NM * a_bytes + b_bytes);
+      load_weights(kb, smem_u32(tiles) + (uint32_t)kb * stage_bytes, full, l2_policy_evict_first());
+    }
   }
+  // TMEM only now: the blocks that an early one waits for may still have to allocate theirs
+  if (early) qb_follow();
   if (warp == 1) {      // one warp allocates the accumulator columns (in a pair: the same warp of both blocks)
     if (PAIR) {
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -326,10 +340,12 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
     const uint32_t bars = PAIR ? mapa_u32(full0, 0u) : full0;
     uint32_t st = ring, parity = 1u;
     int s = 0;
-    auto turn = [&](int kb) {      // lane 0: the boxes of a stage
+    auto turn = [&](int kb, bool weights) {      // lane 0: the boxes of a stage
       const uint32_t bar = bars + 8u * s;
-      if (rank == 0) mbar_expect_tx(full0 + 8u * s, tx);
-      load_weights(kb, st, bar, pol_w);
+      if (weights) {
+        if (rank == 0) mbar_expect_tx(full0 + 8u * s, tx);
+        load_weights(kb, st, bar, pol_w);
+      }
       if (!by_row) {
         if constexpr (PAIR) tma_load_2d_pair(st + NM * a_bytes, &tm_x, kb * EG_BK, row0 + r_lo, bar, pol_x);
         else if constexpr (KS == 2) tma_load_3d(st + NM * a_bytes, &tm_x, 0, row0, kb * KS, bar, pol_x);
@@ -345,7 +361,7 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
 #pragma unroll 1
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait(empty0 + 8u * s, parity, abort_flag)) break;
-          turn(kb);
+          turn(kb, kb >= ahead);      // an early block's first weights are on their way
           armed = kb + 1;
           next();
         }
@@ -356,7 +372,7 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
         int ok = 1;
         if (lane == 0) ok = mbar_wait(empty0 + 8u * s, parity, abort_flag) ? 1 : 0;
         if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-        if (lane == 0) turn(kb);
+        if (lane == 0) turn(kb, true);
         // boxes of one row: the swizzle follows the shared-memory address, so a row lands where a box of
         // many rows would have put it; the rows past the expert's last keep what the stage held before, and
         // their columns of the product are never read
@@ -528,8 +544,8 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
   const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, void* __restrict__ out,     \
       const int* __restrict__ sorted_pair, const float* __restrict__ pair_w, const int* __restrict__ plan,        \
       const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, int E, int K, int N_out, int NT,    \
-      int stages, int tmem_cols, int gather_k, int* status, EgAct act
-#define QB_EG_ARGS tm_w, tm_x, out, sorted_pair, pair_w, plan, tile_expert, tile_row0, E, K, N_out, NT, stages, tmem_cols, gather_k, status, act
+      int stages, int tmem_cols, int gather_k, int* status, EgAct act, int early
+#define QB_EG_ARGS tm_w, tm_x, out, sorted_pair, pair_w, plan, tile_expert, tile_row0, E, K, N_out, NT, stages, tmem_cols, gather_k, status, act, early
 
 template <int MODE, int NM, int KS>
 __global__ void __launch_bounds__(EG_THREADS, 2) expert_gemm_tc_kernel(QB_EG_PARAMS) {
@@ -618,7 +634,7 @@ extern "C" int qb_expert_gemm_tc(int mode, const void* x_rows, const void* weigh
                                  const float* pair_w, const int* plan, const int* tile_expert, const int* tile_row0,
                                  int max_tiles, int n_pairs, int E, int K, int N_out, int NT, int gather_k, int n_rows,
                                  int* status, int weight_experts, int act_kind, float act_limit, float act_alpha,
-                                 cudaStream_t stream) {
+                                 int after_first, cudaStream_t stream) {
   if (max_tiles <= 0 || n_pairs <= 0) return 0;
   if (act_kind < 0 || act_kind > 1 || (act_kind == 1 && (mode != 1 || pair_w == nullptr))) return QB_ERR_BAD_ARG;
   const EgAct act{act_kind, act_limit, act_alpha};
@@ -681,13 +697,14 @@ extern "C" int qb_expert_gemm_tc(int mode, const void* x_rows, const void* weigh
   int tmem_cols = 32;
   while (tmem_cols < nm * NT) tmem_cols *= 2;
   dim3 grid(grid_x, max_tiles);
+  const int early = mode == 2 && !pair && after_first ? 1 : 0;
   cudaError_t err;
 #define QB_EG(KERNEL_, GK, THREADS_)                                                                                       \
   do {                                                                                                             \
     err = cudaFuncSetAttribute(KERNEL_, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                  \
     if (err != cudaSuccess) return (int)err;                                                                       \
-    KERNEL_<<<grid, THREADS_, smem, stream>>>(tm_w, tm_x, out, sorted_pair, pair_w, plan, tile_expert, tile_row0, E, K, \
-                                               N_out, NT, stages, tmem_cols, GK, status, act);                     \
+    qb_launch(KERNEL_, grid, THREADS_, smem, stream, tm_w, tm_x, out, sorted_pair, pair_w, plan, tile_expert, tile_row0, E, K, \
+              N_out, NT, stages, tmem_cols, GK, status, act, early);                                               \
   } while (0)
   if (pair && mode == 1) QB_EG(expert_gemm_tc_pair_kernel<1>, gather_k, EG_PAIR_THREADS);
   else if (pair && mode == 3) QB_EG(expert_gemm_tc_pair_kernel<3>, gather_k, EG_PAIR_THREADS);

@@ -42,6 +42,7 @@ __global__ void latent_write_kernel(const float* __restrict__ dkv, const float* 
                                     const int* __restrict__ tok_pos, const int* __restrict__ tok_req,
                                     const int* __restrict__ block_table, int bt_stride, int T, int C, int R,
                                     int rd, int interleaved, int page_size, int num_pages, float eps, int* status) {
+  qb_follow();
   __shared__ float scratch[32];
   const int t = blockIdx.x;
   if (t >= T) return;
@@ -90,7 +91,7 @@ extern "C" int qb_latent_write(const float* dkv, int dkv_stride, const float* ga
   if (rd % 2 || rd < 0 || rd > R || C <= 0 || page_size <= 0) return QB_ERR_BAD_ARG;
   if (dq != nullptr && (q_gain == nullptr || cq == nullptr || q_rank <= 0)) return QB_ERR_BAD_ARG;
   const dim3 grid(T, dq != nullptr && dkv != nullptr ? 2 : 1);
-  QB_DISPATCH_DTYPE(dtype, A, latent_write_kernel<A><<<grid, 128, 0, stream>>>(
+  QB_DISPATCH_DTYPE(dtype, A, qb_launch(latent_write_kernel<A>, grid, 128, 0, stream,
       dkv, gain, inv_freq, (A*)cache, dq, q_gain, (A*)cq, q_rank, dkv_stride, dq_stride, tok_pos, tok_req, block_table,
       bt_stride, T, C, R, rd, interleaved, page_size, num_pages, eps, status));
   QB_LAUNCH_CHECK();
@@ -103,6 +104,7 @@ __global__ void latent_query_kernel(const float* __restrict__ q, const float* __
                                     A* __restrict__ q_plain, float* __restrict__ q_rot,
                                     const int* __restrict__ tok_pos, int T, int H, int D, int R, int rd,
                                     int interleaved) {
+  qb_follow();
   const int t = blockIdx.x, h = blockIdx.y;
   const float* row = q + ((size_t)t * H + h) * (D + R);
   A* qp = q_plain + ((size_t)h * T + t) * D;
@@ -127,7 +129,7 @@ extern "C" int qb_latent_query(const float* q, const float* inv_freq, void* q_pl
   if (T <= 0) return 0;
   if (rd % 2 || rd < 0 || rd > R) return QB_ERR_BAD_ARG;
   dim3 grid(T, H);
-  QB_DISPATCH_DTYPE(dtype, A, latent_query_kernel<A><<<grid, 64, 0, stream>>>(
+  QB_DISPATCH_DTYPE(dtype, A, qb_launch(latent_query_kernel<A>, grid, 64, 0, stream,
       q, inv_freq, (A*)q_plain, q_rot, tok_pos, T, H, D, R, rd, interleaved));
   QB_LAUNCH_CHECK();
   return 0;
@@ -271,6 +273,7 @@ template <typename A>
 __global__ void latent_merge_kernel(const float* __restrict__ part, const float* __restrict__ sink,
                                     const float* __restrict__ gate, int gate_stride, A* __restrict__ out, int T, int H,
                                     int C, int n_ranges) {
+  qb_follow();
   __shared__ float s_w[LA_MAX_RANGES];
   __shared__ float s_inv;
   const int t = blockIdx.x / H, h = blockIdx.x % H;
@@ -313,7 +316,7 @@ extern "C" int qb_latent_merge(const float* part, const float* sink, const float
   if (T <= 0) return 0;
   if (n_ranges < 1 || n_ranges > LA_MAX_RANGES) return QB_ERR_UNSUPPORTED;
   const int threads = C >= 256 ? 256 : C >= 128 ? 128 : 64;
-  QB_DISPATCH_DTYPE(dtype, A, latent_merge_kernel<A><<<T * H, threads, 0, stream>>>(part, sink, gate, gate_stride,
+  QB_DISPATCH_DTYPE(dtype, A, qb_launch(latent_merge_kernel<A>, T * H, threads, 0, stream, part, sink, gate, gate_stride,
                                                                                  (A*)out, T, H, C, n_ranges));
   QB_LAUNCH_CHECK();
   return 0;
@@ -369,6 +372,7 @@ latent_attend_mma_kernel(const float* __restrict__ q_lat, const float* __restric
                          int page_size, int num_pages, int n_ranges, int window, float scale,
                          const float* __restrict__ sink, const float* __restrict__ gate, int gate_stride,
                          __nv_bfloat16* __restrict__ out, int* status) {
+  qb_follow();
   constexpr int CP = 32 * NT;
   extern __shared__ __align__(16) unsigned char lm_smem[];
   const int W = C + R, WP = W + 8;
@@ -691,7 +695,7 @@ extern "C" int qb_latent_attend_mma(const float* q_lat, const float* q_rot, cons
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
       if (e != cudaSuccess) return (int)e;                                                                  \
     }                                                                                                       \
-    kern<<<grid, 128 * LM_RG, smem, stream>>>(q_lat, q_rot, (const __nv_bfloat16*)cache, part, tok_pos,    \
+    qb_launch(kern, grid, 128 * LM_RG, smem, stream, q_lat, q_rot, (const __nv_bfloat16*)cache, part, tok_pos, \
                                               req_start, block_table, bt_stride, n_req, T, H, C, R,         \
                                               page_size, num_pages, n_ranges, window, scale, sink, gate,    \
                                               gate_stride, (__nv_bfloat16*)out, status);                    \

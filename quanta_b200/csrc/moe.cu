@@ -362,6 +362,7 @@ __global__ void __launch_bounds__(1024)
 moe_plan_small_kernel(const int* __restrict__ idx, int n_pairs, int E, int BM, int* __restrict__ plan,
                       int* __restrict__ sorted_pair, int* __restrict__ tile_expert,
                       int* __restrict__ tile_row0, int max_tiles, int* status, int tiled) {
+  qb_follow();
   __shared__ PlanShared sh;
   plan_small_body<1024>(idx, n_pairs, E, BM, plan, sorted_pair, tile_expert, tile_row0, max_tiles, status, sh,
                         [] { __syncthreads(); }, tiled);
@@ -598,6 +599,7 @@ router_few_kernel(const TX* __restrict__ x, const float* __restrict__ gate, cons
                   float scale, int select, int* counters, int BM, int* __restrict__ plan,
                   int* __restrict__ sorted_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                   int max_tiles, int* status, int tiled) {
+  qb_follow();
   constexpr int EPB = RS_WARPS / RS_QUARTERS;
   extern __shared__ __align__(16) unsigned char rs_smem[];      // [RS_TT][K] of TX: the tile's token rows
   __shared__ PlanShared sh;
@@ -697,7 +699,7 @@ extern "C" int qb_router_small(const void* x, int x_dtype, const float* gate, co
   do {                                                                                                                            \
     err = cudaFuncSetAttribute(router_few_kernel<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                    \
     if (err != cudaSuccess) return (int)err;                                                                                      \
-    router_few_kernel<TX><<<grid, RS_WARPS * 32, smem, stream>>>((const TX*)x, gate, bias, logits, idx_out, w_out, T, E, K, k,      \
+    qb_launch(router_few_kernel<TX>, grid, RS_WARPS * 32, smem, stream, (const TX*)x, gate, bias, logits, idx_out, w_out, T, E, K, k,      \
                                                                  renorm, scale, select, counters, BM, plan, sorted_pair,           \
                                                                  tile_expert, tile_row0, max_tiles, status, tiled);                \
   } while (0)
@@ -739,7 +741,7 @@ extern "C" int qb_moe_plan(const int* idx, int n_pairs, int E, int BM, int* plan
   if (E > 1024) return QB_ERR_UNSUPPORTED;
   if (tiled <= 0 || tiled > E) tiled = E;
   if (n_pairs <= 4096) {
-    moe_plan_small_kernel<<<1, 1024, 0, stream>>>(idx, n_pairs, E, BM, plan, sorted_pair, tile_expert, tile_row0,
+    qb_launch(moe_plan_small_kernel, 1, 1024, 0, stream, idx, n_pairs, E, BM, plan, sorted_pair, tile_expert, tile_row0,
                                                   max_tiles, status, tiled);
     QB_LAUNCH_CHECK();
     return 0;

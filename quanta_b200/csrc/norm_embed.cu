@@ -16,6 +16,7 @@ __global__ void embedding_kernel(float* __restrict__ h, const W* __restrict__ ta
                                  const int* __restrict__ ids, int T, int H, int V, float scale,
                                  const W* __restrict__ pos_table, const int* __restrict__ tok_pos, int n_pos,
                                  int copies, int* status) {
+  qb_follow();
   const int t = blockIdx.x;
   if (t >= T) return;
   const int id = ids[t];
@@ -61,7 +62,7 @@ extern "C" int qb_embedding(float* h, const void* table, int table_dtype, const 
   if (T <= 0) return 0;
   if (copies < 1 || (pos_table != nullptr && (tok_pos == nullptr || n_pos <= 0))) return QB_ERR_BAD_ARG;
   QB_DISPATCH_DTYPE(table_dtype, W,
-                    embedding_kernel<W><<<T, 256, 0, stream>>>(h, (const W*)table, ids, T, H, V, scale,
+                    qb_launch(embedding_kernel<W>, T, 256, 0, stream, h, (const W*)table, ids, T, H, V, scale,
                                                                (const W*)pos_table, tok_pos, n_pos, copies, status));
   QB_LAUNCH_CHECK();
   return 0;
@@ -168,6 +169,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const D* __restrict__ 
 template <typename D, typename O>
 __global__ void __launch_bounds__(1024) add_rmsnorm_rows_kernel(float* __restrict__ h, const D* __restrict__ delta, int S, const float* __restrict__ w,
                                         O* __restrict__ out, const int* __restrict__ rows, int H, float eps, int store_h) {
+  qb_follow();
   __shared__ float scratch[32];
   const int r = blockIdx.x, tok = rows ? rows[r] : r, i = threadIdx.x * 8;
   const bool in = i < H;
@@ -207,7 +209,7 @@ extern "C" int qb_add_rmsnorm(float* h, const void* delta, int delta_dtype, int 
   if (n_rows <= 0) return 0;
   if (row_in_registers(H, 1024) && (((uintptr_t)h | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
     QB_DISPATCH_DTYPE(delta_dtype, D, QB_DISPATCH_DTYPE(out_dtype, O, {
-      add_rmsnorm_rows_kernel<D, O><<<n_rows, row_threads(H), 0, stream>>>(h, (const D*)delta, S, w, (O*)out, rows, H, eps, store_h);
+      qb_launch(add_rmsnorm_rows_kernel<D, O>, n_rows, row_threads(H), 0, stream, h, (const D*)delta, S, w, (O*)out, rows, H, eps, store_h);
     }));
     QB_LAUNCH_CHECK();
     return 0;
@@ -293,6 +295,7 @@ __global__ void __launch_bounds__(768) normed_add_rmsnorm_rows_kernel(float* __r
                                                const float* __restrict__ y2_bias, const float* __restrict__ g, float eps_y,
                                                const float* __restrict__ w, O* __restrict__ out, const int* __restrict__ rows,
                                                int H, float eps, int store_h) {
+  qb_follow();
   __shared__ float scratch_y[32], scratch[32];
   const int r = blockIdx.x, tok = rows ? rows[r] : r, i = threadIdx.x * 8;
   const bool in = i < H;
@@ -365,7 +368,7 @@ extern "C" int qb_normed_add_rmsnorm(float* h, const float* y, int S, float y_sc
                         (uintptr_t)w | (uintptr_t)out;
   if (row_in_registers(H, 768) && (all & 15) == 0) {      // 1,024 threads would have 64 registers each, it takes more
     QB_DISPATCH_DTYPE(out_dtype, O, {
-      normed_add_rmsnorm_rows_kernel<O><<<n_rows, row_threads(H), 0, stream>>>(
+      qb_launch(normed_add_rmsnorm_rows_kernel<O>, n_rows, row_threads(H), 0, stream,
           h, y, S, y_scale, y_bias, y2, y2_scale, y2_bias, g, eps_y, w, (O*)out, rows, H, eps, store_h);
     });
     QB_LAUNCH_CHECK();
@@ -405,6 +408,7 @@ __global__ void silu_mul_kernel(const A* __restrict__ gu, A* __restrict__ out, i
 // bfloat16 (165 MB) 87 us with one element a thread and a division to find its row, 29 us with this.
 template <typename A>
 __global__ void silu_mul_rows_kernel(const A* __restrict__ gu, A* __restrict__ out, int n_rows, int I) {
+  qb_follow();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (c >= I) return;
   for (int r = blockIdx.y; r < n_rows; r += gridDim.y) {
@@ -422,7 +426,7 @@ extern "C" int qb_silu_mul(const void* gu, void* out, int dtype, int n_rows, int
   if (I % 8 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0) {
     const int threads = (size_t)n_rows * I >= 1u << 20 ? 256 : 64;        // few rows: more blocks, so more SMs
     const dim3 grid((I / 8 + threads - 1) / threads, n_rows < 32768 ? n_rows : 32768);
-    QB_DISPATCH_DTYPE(dtype, A, silu_mul_rows_kernel<A><<<grid, threads, 0, stream>>>((const A*)gu, (A*)out, n_rows, I));
+    QB_DISPATCH_DTYPE(dtype, A, qb_launch(silu_mul_rows_kernel<A>, grid, threads, 0, stream, (const A*)gu, (A*)out, n_rows, I));
     QB_LAUNCH_CHECK();
     return 0;
   }
@@ -592,6 +596,7 @@ extern "C" int qb_streams_mix_rmsnorm(float* x, int S, const void* delta, int de
 // ---------------------------------------------------------------------------------------------
 template <typename A>
 __global__ void relu_squared_kernel(const A* __restrict__ x, A* __restrict__ out, size_t n) {
+  qb_follow();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const float v = fmaxf(qb_to_float<A>(x[i]), 0.f);
     out[i] = qb_from_float<A>(v * v);
@@ -601,7 +606,7 @@ __global__ void relu_squared_kernel(const A* __restrict__ x, A* __restrict__ out
 extern "C" int qb_relu_squared(const void* x, void* out, int dtype, long long n, cudaStream_t stream) {
   if (n <= 0) return 0;
   const int blocks = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
-  QB_DISPATCH_DTYPE(dtype, A, relu_squared_kernel<A><<<blocks, 256, 0, stream>>>((const A*)x, (A*)out, (size_t)n));
+  QB_DISPATCH_DTYPE(dtype, A, qb_launch(relu_squared_kernel<A>, blocks, 256, 0, stream, (const A*)x, (A*)out, (size_t)n));
   QB_LAUNCH_CHECK();
   return 0;
 }
@@ -668,6 +673,7 @@ template <typename O>
 __global__ void __launch_bounds__(128)
 head_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_stride, const float* __restrict__ gain,
                           O* __restrict__ out, int T, int H, int D, float eps, int gain_shared, int gate_kind) {
+  qb_follow();
   const int lanes = D / 4, per = 128 / lanes;            // (token, head) pairs a block
   const int h = blockIdx.y * per + threadIdx.x / lanes, i = threadIdx.x % lanes * 4, t = blockIdx.x;
   const bool in = h < H;
@@ -700,7 +706,7 @@ extern "C" int qb_head_norm_gate(const float* o, const float* gate, int gate_str
   if (D >= 4 && D <= 128 && (D & (D - 1)) == 0 && H <= 65535 && gate_stride % 4 == 0 && (all & 15) == 0) {
     const int per = 128 / (D / 4);
     const dim3 grid(T, (H + per - 1) / per);
-    QB_DISPATCH_DTYPE(out_dtype, O, head_norm_gate_vec_kernel<O><<<grid, 128, 0, stream>>>(o, gate, gate_stride, gain, (O*)out, T, H, D,
+    QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(head_norm_gate_vec_kernel<O>, grid, 128, 0, stream, o, gate, gate_stride, gain, (O*)out, T, H, D,
                                                                                           eps, gain_shared, gate_kind));
     QB_LAUNCH_CHECK();
     return 0;

@@ -258,6 +258,7 @@ template <typename IN, typename A, int HPW>
 __global__ void __launch_bounds__(HPW == 2 ? 1024 : 512, HPW == 2 ? 1 : 2)      // 64 registers: with 85 the 12,800 tokens take 276 us
 qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
                          const RopeArgs a) {
+  qb_follow();
   __shared__ __align__(16) float s_cos[ROPE_HD / 2], s_sin[ROPE_HD / 2];
   __shared__ float s_sum[32 * HPW];
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -395,7 +396,7 @@ static void qknorm_rope_heads(const void* qkv, void* q_out, void* k_cache, void*
   const int hpw = T <= 64 && heads <= 64 ? 2 : heads <= 32 ? 4 : 8;
   const int threads = (heads + hpw - 1) / hpw * 32;
 #define QB_HEADS(N) \
-  qknorm_rope_heads_kernel<IN, A, N><<<T, threads, 0, stream>>>((const IN*)qkv, (A*)q_out, (A*)k_cache, (A*)v_cache, a)
+  qb_launch(qknorm_rope_heads_kernel<IN, A, N>, T, threads, 0, stream, (const IN*)qkv, (A*)q_out, (A*)k_cache, (A*)v_cache, a)
   if (hpw == 2) QB_HEADS(2);
   else if (hpw == 4) QB_HEADS(4);
   else QB_HEADS(8);

@@ -304,6 +304,7 @@ extern "C" int qb_apply_penalties(float* logits, int n, int V, const int* prev, 
 __global__ void slots_advance_kernel(int* __restrict__ slots, int n_slots, const int* __restrict__ req_slot,
                                      const int* __restrict__ req_start, const int* __restrict__ req_len_after, int R,
                                      int* status) {
+  qb_follow();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
     const int slot = req_slot[r];
     if (slot < 0 || slot >= n_slots) { qb_set_status(status, QB_STATUS_SLOT_MISMATCH, slot, 8); continue; }
@@ -318,7 +319,7 @@ extern "C" int qb_slots_advance(int* slots, int n_slots, const int* req_slot, co
                                 const int* req_len_after, int R, int* status, cudaStream_t stream) {
   if (R <= 0) return 0;
   if (n_slots <= 0) return QB_ERR_BAD_ARG;
-  slots_advance_kernel<<<(R + 127) / 128, 128, 0, stream>>>(slots, n_slots, req_slot, req_start, req_len_after, R, status);
+  qb_launch(slots_advance_kernel, (R + 127) / 128, 128, 0, stream, slots, n_slots, req_slot, req_start, req_len_after, R, status);
   QB_LAUNCH_CHECK();
   return 0;
 }

@@ -141,6 +141,7 @@ __global__ void short_conv_step_kernel(const float* __restrict__ x, const float*
                                        O* __restrict__ out, const int* __restrict__ req_start,
                                        const int* __restrict__ req_slot, int R, int C, int taps, int x_stride,
                                        const float* __restrict__ bias, int act) {
+  qb_follow();
   const int r = blockIdx.x;
   if (r >= R) return;
   const int first = req_start[r], n = req_start[r + 1] - first;
@@ -186,7 +187,7 @@ extern "C" int qb_short_conv(const float* x, const float* w, float* state, void*
   if (taps < 1 || C <= 0 || x_stride < C || act < 0 || act > 2) return QB_ERR_BAD_ARG;
   const int threads = C >= 1024 ? 256 : 128;
   if (qb_short_conv_one_launch(T, R)) {
-    QB_DISPATCH_DTYPE(out_dtype, O, short_conv_step_kernel<O><<<dim3(R, min(64, (C + threads - 1) / threads)), threads, 0, stream>>>(
+    QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(short_conv_step_kernel<O>, dim3(R, min(64, (C + threads - 1) / threads)), threads, 0, stream, 
         x, w, state, (O*)out, req_start, req_slot, R, C, taps, x_stride, bias, act));
     QB_LAUNCH_CHECK();
     return 0;

@@ -633,7 +633,7 @@ def gather_rows(x, out, sorted_pair, top_k: int) -> None:
 
 def expert_gemm_tc(mode: int, x_rows, weights, out, sorted_pair, pair_w, plan, tile_expert, tile_row0,
                    n_experts: int, tile_rows: int, status, gather_top_k: int = 0, weight_experts: int = 0,
-                   act: tuple = (0, 0.0, 1.0)) -> None:
+                   act: tuple = (0, 0.0, 1.0), after_first: bool = False) -> None:
     """Expert products on tcgen05/TMEM fed by TMA.  ``x_rows`` bf16 [pairs, K] in expert order; mode 1:
     ``out[p, :I] = silu(gate) * up`` (bf16), mode 2: ``out[pair(p)] = w[pair(p)] * down`` (float32), mode 3:
     ``out[p] = relu(up)^2`` (bf16; ungated experts, weights ``[E, I, K]``).  The plan's
@@ -641,7 +641,8 @@ def expert_gemm_tc(mode: int, x_rows, weights, out, sorted_pair, pair_w, plan, t
     step's activations [T, K] and the kernel fetches the row of token ``pair // gather_top_k`` itself, one
     TMA box a row (for steps of few tokens: it saves the gathered copy and its launch).  ``weight_experts`` > 0: the
     plan counts ``n_experts`` experts of which only the first so many have weights (and tiles).  ``act`` and a
-    ``pair_w`` of None in mode 2 as in ``moe_grouped_simt``."""
+    ``pair_w`` of None in mode 2 as in ``moe_grouped_simt``.  ``after_first``: the launch before this one on the stream is
+    the same plan's first product, so weights and plan may be read while it ends."""
     n_x, K = x_rows.shape
     n_pairs = sorted_pair.numel()
     N = out.shape[1]
@@ -656,7 +657,7 @@ def expert_gemm_tc(mode: int, x_rows, weights, out, sorted_pair, pair_w, plan, t
     _check(lib().qb_expert_gemm_tc(mode, _p(x_rows), _p(weights), _p(out), _p(sorted_pair), _p(pair_w), _p(plan),
                                    _p(tile_expert), _p(tile_row0), tile_expert.numel(), n_pairs, n_experts, K, N,
                                    int(tile_rows), int(gather_top_k), n_x, _p(status), int(weight_experts), int(act[0]),
-                                   ctypes.c_float(act[1]), ctypes.c_float(act[2]), _stream()),
+                                   ctypes.c_float(act[1]), ctypes.c_float(act[2]), int(after_first), _stream()),
            "expert_gemm_tc")
 
 

@@ -183,7 +183,7 @@ class SigmoidTopKExperts(FeedForward):
                 kernels.expert_gemm_tc(self.first_product_mode, xg, self.w13, act, sorted_pair, w.view(-1), plan,
                                        tile_expert, tile_row0, self.E, bm, ctx.status, weight_experts=self.E_w, act=ea)
             kernels.expert_gemm_tc(2, act, self.w2, y.view(n_pairs, self.H), sorted_pair, w_down, plan,
-                                   tile_expert, tile_row0, self.E, bm, ctx.status, weight_experts=self.E_w)
+                                   tile_expert, tile_row0, self.E, bm, ctx.status, weight_experts=self.E_w, after_first=True)
         else:
             kernels.moe_grouped_simt(self.first_product_mode, x, self.w13, act, sorted_pair, w.view(-1), plan, tile_expert,
                                      tile_row0, self.E, self.k, act=ea)

@@ -30,11 +30,11 @@ def test_two_products(T, E, top, H, I, gated, clamped, with_weights):
     act, limits = torch.zeros(n, I, dtype=torch.bfloat16, device=DEV), (k.EXPERT_ACT_CLAMPED, 1.5, 1.7) if clamped else (0, 0.0, 1.0)
     mode, w_down = 1 if gated else 3, None if clamped else w
     results = []
-    for gather in (top, 0):
+    for gather, behind in ((top, True), (0, False)):
         rows = x if gather else x[(pairs.long() // top)].contiguous()
         y = torch.zeros(n, H, device=DEV)
         k.expert_gemm_tc(mode, rows, w13, act, pairs, w, plan, te, tr, E, bm, st, gather_top_k=gather, weight_experts=with_weights, act=limits)
-        k.expert_gemm_tc(2, act, w2, y, pairs, w_down, plan, te, tr, E, bm, st, weight_experts=with_weights)
+        k.expert_gemm_tc(2, act, w2, y, pairs, w_down, plan, te, tr, E, bm, st, weight_experts=with_weights, after_first=behind)
         results.append(y)
     assert st.tolist()[0] == 0 and torch.equal(*results)
     for p, e in enumerate(idx.view(-1).tolist()):
