@@ -226,9 +226,22 @@ __device__ __forceinline__ void attend_block(const __nv_bfloat16* qs, const __nv
       s[i][e] = p;
       l[e >> 1] += p;
     }
-  // O += P V
+  // O += P V.  Rows of V that no row of the warp reads meet weights of zero, and 0 x NaN is NaN: a page comes whole, with what its last
+  // holder left behind the request's end.  Such rows are zeros here (a fragment is two keys, 2 q and 2 q + 1 of eight, of one dim).
+  int lo_all = 0, hi_all = 0;
+  if (!all_visible) {
+    lo_all = __reduce_min_sync(0xffffffffu, min(row_hi[0] < 0 ? 0x7fffffff : row_lo[0], row_hi[1] < 0 ? 0x7fffffff : row_lo[1]));
+    hi_all = __reduce_max_sync(0xffffffffu, max(row_hi[0], row_hi[1]));
+  }
+  auto read = [&](int key) { return key >= lo_all && key <= hi_all; };
 #pragma unroll
   for (int j = 0; j < NK / 16; ++j) {
+    const int key = key0 + j * 16 + 2 * q;
+    uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;
+    if (!all_visible) {
+      keep0 = (read(key) ? 0xffffu : 0u) | (read(key + 1) ? 0xffff0000u : 0u);
+      keep1 = (read(key + 8) ? 0xffffu : 0u) | (read(key + 9) ? 0xffff0000u : 0u);
+    }
     uint32_t a[4];
     a[0] = pack_bf16(s[2 * j][0], s[2 * j][1]);
     a[1] = pack_bf16(s[2 * j][2], s[2 * j][3]);
@@ -238,6 +251,7 @@ __device__ __forceinline__ void attend_block(const __nv_bfloat16* qs, const __nv
     for (int dt = 0; dt < HDP / 16; ++dt) {
       uint32_t b[4];
       ldmatrix_x4_trans(b, kv.at(vs, koff + j * 16 + (lane & 7) + 8 * ((lane >> 3) & 1), dt * 16 + 8 * (lane >> 4)));
+      if (!all_visible) { b[0] &= keep0; b[1] &= keep1; b[2] &= keep0; b[3] &= keep1; }
       mma16816(o[2 * dt], a, b[0], b[1]);
       mma16816(o[2 * dt + 1], a, b[2], b[3]);
     }
@@ -416,8 +430,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     s_pos[z] = tok_pos[t];
     s_req[z] = tok_req[t];
   }
-  // The rings start as zeros: padding columns and Q rows past the group are never copied into, and a
-  // tile's unused key rows only ever hold older (finite) keys or zeros.
+  // The rings start as zeros: padding columns and Q rows past the group are never copied into (a tile's unused key rows
+  // may hold anything: attend_block masks their scores and their rows of V).
   {
     const size_t n16 = ((size_t)stages * 2 * tile_elems + ((size_t)q_slots * q_rows + 8) * LD) / 8;
     for (size_t i = tid; i < n16; i += blockDim.x) reinterpret_cast<uint4*>(ring)[i] = make_uint4(0, 0, 0, 0);
@@ -556,7 +570,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           __nv_bfloat16* vs = ks + tile_elems;
           // boxes of the TMA path: rows of one page (or 64 rows of a larger page) x 64 dims
           const int n_boxes = (n_keys + box_rows - 1) >> box_shift;       // pages of the tile that hold visible keys
-          // keys before the window are not fetched (their rows keep older, finite values and are masked)
+          // keys before the window are not fetched (their rows keep older values and are masked, those of V too)
           const int key_skip = d.lo > d.key0 ? d.lo - d.key0 : 0;
           const int box_first = TMA ? key_skip >> box_shift : 0;
           const bool new_q = which == 0 && (d.flags & AD_FIRST) != 0;
@@ -715,8 +729,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         // With at most 8 q heads a kv head the four warps' rows fit the K half of the tile ([4][8][HDP] floats):
         // what they leave there can only reach scores that the mask replaces, so the tile need not be wiped,
         // and each warp gives the tile back when it has read what it merges.  With more heads the parts
-        // fill K and V ([4][16][HDP]) and the tile goes back as zeros (V rows that a later, shorter copy does
-        // not cover must stay finite).
+        // fill K and V ([4][16][HDP]) and the tile goes back as zeros (its padded dims must be).
         const bool compact = RB == 1 && G <= 8 && hd == HDP;      // no padded dims: every K element of a row is copied over
         const int sc_rows = compact ? 8 : 16;
         if (!cons_sync()) break;                         // every warp has read the tile

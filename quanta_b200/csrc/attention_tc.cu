@@ -514,6 +514,19 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         take(vb, 1);
       }
       l += sum2[0] + sum2[1];
+      // Rows of V that no row of the tile reads meet weights of zero, and 0 x NaN is NaN: a page comes whole, with what its last holder
+      // left behind this request's end or with the request's own keys before the window, and the stage keeps rows of two blocks
+      // before.  A thread wipes its 64 dims of the row of its number, in the first and the last block only.
+      if (key0 < lo_min || key0 + TC_BN - 1 > key_end) {
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.v_full[slot]), (uint32_t)(j >> 1) & 1u, abort_flag) ? 1 : 0);
+        if (!ok) break;
+        if (key0 + r < lo_min || key0 + r > key_end) {
+          uint4* row = reinterpret_cast<uint4*>(base + 3 * TC_TILE_BYTES + slot * TC_TILE_BYTES + half * TC_SLAB_BYTES + r * 128);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) row[(i + r) & 7] = make_uint4(0, 0, 0, 0);      // (+ r: eight rows' stores meet no bank twice)
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the zeros, before the MMA reads them
+      }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");      // P, before the MMA reads it
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(smem_u32(&sh.p_full[slot]));
