@@ -120,9 +120,10 @@ paged_attention_rows_kernel(const A* __restrict__ q, const A* __restrict__ k_cac
     float top = mine;
 #pragma unroll
     for (int o = 4; o <= 16; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-    const float m_new = fmaxf(m, top);
-    const float p = seen ? expf(mine - m_new) : 0.f;
-    const float corr = m_new > -INFINITY ? expf(m - m_new) : 1.f;
+    // keys may have scores of minus infinity (a bias that masks them): while nothing else has been seen, exponents are taken against 0
+    const float m_new = fmaxf(m, top), ref = m_new > -INFINITY ? m_new : 0.f;
+    const float p = seen ? expf(mine - ref) : 0.f;
+    const float corr = expf(m - ref);
     float sum = p;
 #pragma unroll
     for (int o = 4; o <= 16; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
