@@ -267,7 +267,7 @@ attn_decode_direct_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
       sum = s_pl[h];
     }
     const int dim = (d & 64) + (d & 7) * 8 + ((d & 63) >> 3);
-    out[((size_t)tok * P.nq + kvh * G + h) * DD_HD + dim] = __float2bfloat16_rn(sum > 0.f ? x / sum : 0.f);
+    out[((size_t)tok * P.nq + kvh * G + h) * DD_HD + dim] = __float2bfloat16_rn(sum == 0.f ? 0.f : x / sum);     // no key read: 0; a sum that is no number stays none
   }
   if (P.S > 1) dd_cluster_sync();                    // nobody leaves while its sums are read
 }

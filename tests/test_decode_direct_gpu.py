@@ -91,5 +91,46 @@ def test_weights_of_two_parts(lens, window, chunk, cap):
         assert torch.all((out[r].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -12 * float(v.abs().max()))
 
 
+@pytest.mark.parametrize("two_part", [False, True])
+@pytest.mark.parametrize("lens", [[40, 2100], [300] * 40])
+def test_what_is_no_number_stays_none(two_part, lens):
+    """A query, a key or a value that holds NaN gives NaN to the heads (and dims) that meet it and to no other."""
+    kern, hd, nq, nkv, page = K(), 128, 8, 2, 16
+    g = torch.Generator(device=DEV).manual_seed(1)
+    per = [-(-n // page) for n in lens]
+    kc = torch.randn(sum(per), nkv, page, hd, device=DEV, generator=g).bfloat16()
+    vc = torch.randn(sum(per), nkv, page, hd, device=DEV, generator=g).bfloat16()
+    table, at = torch.full((len(lens), max(per)), -1, dtype=torch.int32), 0
+    for r, n in enumerate(per):
+        table[r, :n] = torch.arange(at, at + n, dtype=torch.int32)
+        at += n
+    R = len(lens)
+    q = torch.randn(R, nq, hd, device=DEV, generator=g).bfloat16()
+    pos, req = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV), torch.arange(R, dtype=torch.int32, device=DEV)
+
+    def run(q_, k_, v_):
+        out, st = torch.empty_like(q), kern.new_status(DEV)
+        kern.attn_decode_direct(q_, k_, v_, out, req, R, pos, req, table.to(DEV), hd ** -0.5, 0, max(lens), st, two_part=two_part)
+        assert st.tolist()[0] == 0
+        return out
+
+    clean = run(q, kc, vc)
+    where = (torch.tensor(per[:1]).sum().item(), 1, 5)                # token 1's key 5, kv head 1: its q heads 4 .. 7
+    for name in ("q", "k", "v"):
+        qq, kk, vv = q.clone(), kc.clone(), vc.clone()
+        hit = torch.zeros(R, nq, hd, dtype=torch.bool, device=DEV)
+        if name == "q":
+            qq[1, 6, 17] = float("nan")
+            hit[1, 6] = True
+        elif name == "k":
+            kk[where][3] = float("nan")
+            hit[1, 4:] = True
+        else:
+            vv[where][100] = float("nan")
+            hit[1, 4:, 100] = True
+        out = run(qq, kk, vv)
+        assert torch.isnan(out[hit].float()).all() and torch.equal(out[~hit], clean[~hit])
+
+
 def test_sizes_that_are_not_taken():
     assert not K().attn_decode_direct_supported(9, 1, 128) and not K().attn_decode_direct_supported(8, 8, 64)
