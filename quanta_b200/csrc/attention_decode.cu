@@ -1,8 +1,9 @@
 // Attention of single tokens over the paged cache for heads of 128 and at most eight q heads a kv head (bfloat16, mma.sync).
 //
 //   out[t, h] = softmax_j(q[t, h] . k_j * scale) v_j       over the keys [lo, pos] of the token's request
-//   (src/quanta/minimax/attention.py:194-203; float32 scores and sums, weights rounded to bfloat16 before P V, or with SPLIT as two
-//   bfloat16 parts, two products a tile; a cap on the scores and a chunk of the sequence besides the window)
+//   (src/quanta/minimax/attention.py:194-203; float32 scores and sums, weights rounded to bfloat16 before P V, or with SPLIT as they
+//   are: three bfloat16 parts hold a float32's 24 bits, three products a tile; a cap on the scores and a chunk of the sequence
+//   besides the window)
 //
 // A warp works by itself, 16 keys at a time, until the end: its keys and values come by asynchronous copies of its own into a ring of
 // three rounds, so it waits for no other warp, and the tensor cores take their operands as the rows lie.
@@ -175,10 +176,14 @@ attn_decode_direct_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
     l = l * corr + sum;
     const float c0 = __shfl_sync(0xffffffffu, corr, 8 * t), c1 = __shfl_sync(0xffffffffu, corr, 8 * t + 4);
     const uint32_t b0 = dd_pack(s[0][0], s[0][1]), b1 = dd_pack(s[1][0], s[1][1]);
-    uint32_t r0 = 0u, r1 = 0u;                       // what the rounding left
+    uint32_t mid0 = 0u, mid1 = 0u, low0 = 0u, low1 = 0u;        // what the rounding left, and what is left of that: exact
     if (SPLIT) {
-      r0 = dd_pack(s[0][0] - __uint_as_float(b0 << 16), s[0][1] - __uint_as_float(b0 & 0xffff0000u));
-      r1 = dd_pack(s[1][0] - __uint_as_float(b1 << 16), s[1][1] - __uint_as_float(b1 & 0xffff0000u));
+      auto left = [](float x, uint32_t part, int e) { return x - __uint_as_float(e ? part & 0xffff0000u : part << 16); };
+      float r[4] = {left(s[0][0], b0, 0), left(s[0][1], b0, 1), left(s[1][0], b1, 0), left(s[1][1], b1, 1)};
+      mid0 = dd_pack(r[0], r[1]);
+      mid1 = dd_pack(r[2], r[3]);
+      low0 = dd_pack(left(r[0], mid0, 0), left(r[1], mid0, 1));
+      low1 = dd_pack(left(r[2], mid1, 0), left(r[3], mid1, 1));
     }
     if (__any_sync(0xffffffffu, corr != 1.f)) {      // a maximum has grown
 #pragma unroll
@@ -191,7 +196,10 @@ attn_decode_direct_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
       const uint32_t a0 = __byte_perm(word(x.v[0][0]), word(x.v[1][0]), sel), a1 = __byte_perm(word(x.v[0][1]), word(x.v[1][1]), sel);
       const uint32_t a2 = __byte_perm(word(x.v[2][0]), word(x.v[3][0]), sel), a3 = __byte_perm(word(x.v[2][1]), word(x.v[3][1]), sel);
       dd_mma(o[e], a0, a1, a2, a3, b0, b1);
-      if (SPLIT) dd_mma(o[e], a0, a1, a2, a3, r0, r1);
+      if (SPLIT) {
+        dd_mma(o[e], a0, a1, a2, a3, mid0, mid1);
+        dd_mma(o[e], a0, a1, a2, a3, low0, low1);
+      }
     }
   };
 
@@ -297,7 +305,7 @@ extern "C" int qb_attn_decode_direct(const void* q, const void* k_cache, const v
   // more units than SMs blocks of four warps, two to an SM, a unit two of them where that leaves eight rounds a warp.  This kernel and the
   // persistent one with its merge launch, 48 + 8 heads: one token of 60 keys 5.5 and 10.8 us, of 2,100 10.0 and 15.8, of 24,000 33 and
   // 35; 2 of 24,000 and 18,000 42 and 48 (four blocks a unit 53), 4 of 4,000 19 and 29, 8 of 2,100 to 1,050 18 and 26, 16 of 2,000 27 and 40,
-  // 64 of 500 33 and 49, of 2,100 to 1,050 91 to 95 and 100.
+  // 64 of 500 33 and 49, of 2,100 to 1,050 91 to 95 and 100.  `two_part`: weights in parts (SPLIT).
   int keys = window > 0 && window < longest ? window : longest;
   if (chunk > 0 && chunk < keys) keys = chunk;
   const int rounds = (keys + DD_KEYS - 1) / DD_KEYS;

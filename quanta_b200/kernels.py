@@ -432,8 +432,8 @@ def attn_decode_direct_supported(nq: int, nkv: int, hd: int) -> bool:
 def attn_decode_direct(q, k_cache, v_cache, out, dec_tok, n_dec: int, tok_pos, tok_req, block_table, scale: float, window: int,
                        longest: int, status, *, two_part: bool = False, softcap: float = 0.0, chunk: int = 0) -> None:
     """bfloat16 attention of the single tokens ``dec_tok`` in one launch, heads of 128 and at most eight q heads a kv head; ``longest``:
-    keys of the longest request (an upper bound is enough).  ``two_part``: the softmax weights enter the sum in two bfloat16 parts;
-    ``softcap``, ``chunk`` as in ``window_attention``."""
+    keys of the longest request (an upper bound is enough).  ``two_part``: the softmax weights enter the sum unrounded, as the three
+    bfloat16 parts of a float32 (two in ``attn_span_split``); ``softcap``, ``chunk`` as in ``window_attention``."""
     T, nq, hd = q.shape
     num_pages, nkv, page_size, hd2 = k_cache.shape
     for t, name in ((q, "q"), (k_cache, "k_cache"), (v_cache, "v_cache"), (out, "out")):

@@ -132,5 +132,29 @@ def test_what_is_no_number_stays_none(two_part, lens):
         assert torch.isnan(out[hit].float()).all() and torch.equal(out[~hit], clean[~hit])
 
 
+@pytest.mark.parametrize("R,n,window,cap", [(16, 1500, 1024, 30.0), (32, 700, 0, 0.0), (4, 9000, 0, 5.0)])
+def test_weights_hold_24_bits(R, n, window, cap):
+    """The share of outputs that are not the bfloat16 nearest to the exact value.  Queries are short, so that the weights are near one
+    another and all of them count: an error of e in each weight, independent of the others, moves an output by some e / 2 of its
+    size, and a bfloat16 boundary lies within that of it for e / 2^-8 of the outputs.  Weights of 16 bits (e = 2^-17) put 2e-3 of them
+    on the wrong side (measured 1.4e-3 to 3.1e-3), float32 arithmetic throughout 1e-4 to 7e-4 (scores of 128 products)."""
+    kern, hd, nq, nkv, page = K(), 128, 16, 4, 16
+    g = torch.Generator(device=DEV).manual_seed(n)
+    per = -(-n // page)
+    kc = torch.randn(R * per, nkv, page, hd, device=DEV, generator=g).bfloat16()
+    vc = torch.randn(R * per, nkv, page, hd, device=DEV, generator=g).bfloat16()
+    table = torch.arange(R * per, dtype=torch.int32, device=DEV).view(R, per)
+    q = (torch.randn(R, nq, hd, device=DEV, generator=g) * 0.3).bfloat16()
+    pos, req = torch.full((R,), n - 1, dtype=torch.int32, device=DEV), torch.arange(R, dtype=torch.int32, device=DEV)
+    lo = max(0, n - window) if window else 0
+    k, v = (c.view(R, per, nkv, page, hd).transpose(1, 2).reshape(R, nkv, per * page, hd)[:, :, lo:n].double() for c in (kc, vc))
+    s = torch.einsum("rmgd,rmjd->rmgj", q.double().view(R, nkv, nq // nkv, hd), k) * hd ** -0.5
+    s = cap * torch.tanh(s / cap) if cap else s
+    want = torch.einsum("rmgj,rmjd->rmgd", torch.softmax(s, -1), v).reshape(R, nq, hd).bfloat16()
+    out, st = torch.empty_like(q), kern.new_status(DEV)
+    kern.attn_decode_direct(q, kc, vc, out, req, R, pos, req, table, hd ** -0.5, window, n, st, two_part=True, softcap=cap)
+    assert st.tolist()[0] == 0 and float((out != want).float().mean()) <= 9e-4
+
+
 def test_sizes_that_are_not_taken():
     assert not K().attn_decode_direct_supported(9, 1, 128) and not K().attn_decode_direct_supported(8, 8, 64)
