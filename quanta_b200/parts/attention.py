@@ -17,8 +17,8 @@ causal convolution over time on every channel of the projected q, k and v, befor
 projected rows of a request are per-request state, so a portion that starts anywhere sees what the whole prompt
 sees); a learned number per q head that multiplies the head's scores (tensor ``names["head_temperature"]``
 ``[heads]``, float32; folded into the normed, rotated query); softmax weights that stay 32-bit on the tensor
-cores too (``float32_weights``: the kernels that feed ``P V`` with the weights in two bfloat16 parts, and float32
-arithmetic for single tokens, instead of the kernels that round the weights to bfloat16); values that are the projected
+cores too (``float32_weights``: the kernels that feed ``P V`` with the weights in two bfloat16 parts for long portions
+and with all 24 bits otherwise, instead of the kernels that round the weights to bfloat16); values that are the projected
 keys themselves, before norm and rotation (``values_from_keys``: no ``v`` tensor); keys of the token's own chunk of the
 sequence only (``chunk``: position i sees j <= i with ``i // chunk == j // chunk``; with ``float32_weights``); the
 projection's float32 accumulators kept up to norm and rotation (``float32_projection``).
@@ -199,8 +199,9 @@ class GQAttention(Mixer):
         token-by-head rows)."""
         window = self.window or 0
         if self.float32_weights:
-            # scores and weights in float32 whatever the dtype: portions of shapes the tensor cores take run there
-            # with the weights in two bfloat16 parts; single tokens cut their keys into ranges that are joined
+            # scores and weights in float32 whatever the dtype: long portions of shapes the tensor cores take run there
+            # with the weights in two bfloat16 parts, single tokens with all 24 bits (in three parts on the tensor cores, or on
+            # the CUDA cores with their keys cut into ranges that are joined)
             tiles = split_span_tiles(ctx, q, cache.k, cache.v)
             if tiles is not None:
                 kernels.attn_span_split(q, cache.k, cache.v, out, ctx.tok_pos, cache.block_table, tiles, self.scale, window,
@@ -258,7 +259,7 @@ def span_tiles(ctx, spans, G: int, rows: int, hd: int, device):
 
 
 def split_decode(ctx, q, cache_k, cache_v, out, table, scale: float, window: int, *, softcap: float = 0.0, chunk: int = 0) -> bool:
-    """A step of single tokens whose softmax weights stay 32-bit, as ``kernels.attn_decode_direct`` with weights of two parts; False
+    """A step of single tokens whose softmax weights stay 32-bit, as ``kernels.attn_decode_direct`` with weights in parts; False
     (and nothing done) for other steps and shapes."""
     T, nq, hd = q.shape
     if (q.dtype != torch.bfloat16 or cache_v.shape != cache_k.shape or not kernels.attn_decode_direct_supported(nq, cache_k.shape[1], hd)
@@ -269,21 +270,23 @@ def split_decode(ctx, q, cache_k, cache_v, out, table, scale: float, window: int
     return True
 
 
-# Steps with at least this many tokens beside one a request take the tcgen05 kernel with probabilities of two parts; below, the keys of
-# each token are cut into ranges on the CUDA cores.  Measured on a B200, 16 + 4 heads of 128, beside the mma.sync kernel (64 rows of the
-# step's token list a block, request after request): 32 tokens alone 13 and 12 us, 32 after 2,000 others with a window of 1,024 82 and 32,
-# 2,048 172 and 57, 24 single tokens of 1,500 keys with a portion of 512 2,738 and 48.
-SPLIT_SPAN_MIN_TOKENS = 32
+# Portions of at least this many tokens, and this many a request on average, take the tcgen05 kernel with softmax weights of two
+# bfloat16 parts (16 bits), the steps that ``kernels.window_attention`` gives to its own two-part kernel; in all others weights stay
+# float32.  Measured on a B200, 16 + 4 heads of 128, beside the mma.sync kernel (64 rows of the step's token list a block, request
+# after request): 32 tokens alone 13 and 12 us, 32 after 2,000 others with a window of 1,024 82 and 32, 2,048 172 and 57, 24 single
+# tokens of 1,500 keys with a portion of 512 2,738 and 48.
+SPLIT_SPAN_MIN_TOKENS, SPLIT_SPAN_MIN_MEAN = 32, 8
 
 
 def split_span_tiles(ctx, q, k_cache, v_cache):
     """The tiles of a step whose attention runs as ``kernels.attn_span_split`` (every request a portion, single tokens too), or None:
-    shapes the kernel does not take, steps of few tokens, or requests' places the host does not know (a captured step)."""
+    shapes the kernel does not take, steps of few tokens, in all or a request, or requests' places the host does not know (a captured
+    step)."""
     T, nq, hd = q.shape
     nkv, page_size = k_cache.shape[1], k_cache.shape[2]
     starts = ctx.host.get("req_start")
     if (q.dtype != torch.bfloat16 or v_cache.shape != k_cache.shape or starts is None
-            or T - (len(starts) - 1) < SPLIT_SPAN_MIN_TOKENS - 1 or not kernels.attn_span_tc_supported(nq, nkv, hd, page_size)):
+            or T < max(SPLIT_SPAN_MIN_TOKENS, SPLIT_SPAN_MIN_MEAN * (len(starts) - 1)) or not kernels.attn_span_tc_supported(nq, nkv, hd, page_size)):
         return None
     spans = [(r, starts[r], starts[r + 1] - starts[r]) for r in range(len(starts) - 1)]
     return span_tiles(ctx, spans, nq // nkv, kernels.attn_span_tc_rows(), hd, q.device)

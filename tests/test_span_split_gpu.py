@@ -59,3 +59,16 @@ def test_split_spans(nq, nkv, page, lens, cached, window, chunk, cap):
             tol = 2.0 ** -8 * want.abs() + 2.0 ** -12 * float(v.abs().max())
             assert torch.all((out[t0: t0 + n, h].double() - want).abs() <= tol)
         t0 += n
+
+
+def test_which_steps_have_weights_of_16_bits():
+    """The steps that kernels.window_attention gives to the tensor cores: at least 32 tokens and eight a request; no others."""
+    from types import SimpleNamespace
+    from quanta_b200.parts.attention import split_span_tiles
+    cache = torch.zeros(4, 2, 16, 128, device=DEV, dtype=torch.bfloat16)
+    for lens, taken in (([32], True), ([31], False), ([1, 40], True), ([1] * 24 + [32], False), ([1] * 24 + [176], True), ([1] * 24 + [175], False),
+                        ([1] * 64, False), ([8] * 9, True), ([7] * 9, False)):
+        T, starts = sum(lens), [0, *torch.tensor(lens).cumsum(0).tolist()]
+        ctx = SimpleNamespace(host={"req_start": starts}, work={})
+        tiles = split_span_tiles(ctx, torch.zeros(T, 8, 128, device=DEV, dtype=torch.bfloat16), cache, cache)
+        assert (tiles is not None) == taken, lens
