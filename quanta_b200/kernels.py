@@ -760,12 +760,11 @@ DELTA_RULE_MAX_DIM = 256
 
 
 def delta_rule(proj, offsets, wpre, a_bias, w_bias, state, out, req_start, req_slot, n_heads: int, dim: int,
-               decay_scale: float, unit_eps: float, longest: int | None = None) -> None:
+               decay_scale: float, unit_eps: float) -> None:
     """The recurrence ``S <- diag(w) S - (a u)(u^T S) + k v^T``, ``o = S^T r`` per (request, head) over the
     step's tokens, from and into ``state`` ``[slots, heads, dim, dim]`` float32.  ``proj`` float32 ``[T, P]``
     holds r, k, v and the pre-activation of a at the column ``offsets`` (r, k, v, a), heads x dim each;
-    ``wpre`` float32 ``[T, heads*dim]`` the pre-activation of the decay; ``out`` float32 ``[T, heads, dim]``.  ``longest``: tokens
-    of the longest request's portion, which chooses between two forms of the same recurrence (None or 0: not known, the most it can be)."""
+    ``wpre`` float32 ``[T, heads*dim]`` the pre-activation of the decay; ``out`` float32 ``[T, heads, dim]``."""
     for t, n in ((proj, "proj"), (wpre, "wpre"), (a_bias, "a_bias"), (w_bias, "w_bias"), (state, "state"), (out, "out")):
         _want(t, torch.float32, n)
     T = proj.shape[0]
@@ -777,13 +776,12 @@ def delta_rule(proj, offsets, wpre, a_bias, w_bias, state, out, req_start, req_s
         raise ValueError("delta_rule: proj rows must be dense")
     r_off, k_off, v_off, a_off = (int(o) for o in offsets)
     R = req_slot.numel()
-    longest = int(longest or T - R + 1)
     words = lib().qb_delta_rule_scratch
     words.restype = ctypes.c_longlong
-    scratch = torch.empty(words(R, T, n_heads, dim, longest, ctypes.c_float(decay_scale)), dtype=torch.float32, device=proj.device)
+    scratch = torch.empty(words(T, n_heads, dim), dtype=torch.float32, device=proj.device)
     _check(lib().qb_delta_rule(ctypes.c_void_p(proj.data_ptr()), int(proj.stride(0)), r_off, k_off, v_off, a_off,
                                _p(wpre), _p(a_bias), _p(w_bias), _p(state), _p(out), _p(scratch), _p(req_start),
-                               _p(req_slot), R, T, n_heads, dim, longest, ctypes.c_float(decay_scale),
+                               _p(req_slot), R, T, n_heads, dim, ctypes.c_float(decay_scale),
                                ctypes.c_float(unit_eps), _stream()), "delta_rule", 1 if T == R and dim % 4 == 0 and dim <= 128 else 2)
 
 

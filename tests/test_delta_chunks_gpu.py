@@ -1,7 +1,7 @@
-"""The delta rule in chunks of 16 tokens against the same recurrence in float64 and against its token-by-token form, at the edges of
-chunks, heads that are no multiple of 4, several requests, strided rows.  Both forms are float32 throughout; a position's output is a sum of D
+"""The delta rule over portions and single tokens against the same recurrence in float64, at the edges of the chunks in which tokens come
+into shared memory, heads that are no multiple of 4, several requests, strided rows.  Everything is float32; a position's output is a sum of D
 products whose factors carry some tens of roundings, so 1e-5 of the outputs' root mean square is far above float32 and far below any
-error of indexing."""
+error of indexing.  How a request is cut and what shares its steps changes no bit."""
 from __future__ import annotations
 
 import math
@@ -43,7 +43,6 @@ def exact(proj, wpre, ab, wb, S, H, D, scale):
 def test_chunks(H, D, lens, extra, scale):
     g = torch.Generator(device=DEV).manual_seed(H * 100 + D)
     T, HD = sum(lens), H * D
-    assert T - len(lens) + 1 >= max(32, 6 * len(lens))  # these steps run in chunks
     proj = torch.randn(T, 4 * HD + extra, device=DEV, generator=g)
     wpre, ab, wb = (torch.randn(n, device=DEV, generator=g) for n in ((T, HD), (HD,), (HD,)))
     wpre[::7] = -40.0                                   # hardly any decay, and the strongest one
@@ -57,7 +56,7 @@ def test_chunks(H, D, lens, extra, scale):
         for got, ref in ((out[at: at + n], want), (S[i], end)):
             assert float((got.double() - ref).abs().max()) <= 1e-5 * float(ref.pow(2).mean().sqrt())
         at += n
-    # the same tokens a few at a time run token by token
+    # the same tokens a few at a time
     if lens == [200, 15, 16, 17]:
         S1, parts = S0[:1].clone(), []
         for lo in range(0, 200, 16):
@@ -81,6 +80,37 @@ def test_single_tokens(R, H, D):
         got = torch.stack([o[r] for o in outs])
         for a, b in ((got, want), (S[r], end)):
             assert float((a.double() - b).abs().max()) <= 1e-5 * float(b.pow(2).mean().sqrt())
+
+
+@pytest.mark.parametrize("H,D,T", [(32, 64, 100), (3, 33, 70), (2, 128, 50), (1, 256, 20), (4, 20, 40), (2, 3, 35)])
+def test_cut_and_batch_change_no_bit(H, D, T):
+    """One request whole, in portions, one token at a time, as the last of many requests (so that a block has other columns) and beside
+    single tokens: the same outputs and the same state, bit by bit."""
+    g = torch.Generator(device=DEV).manual_seed(D)
+    HD, others = H * D, 7
+    proj, wpre = torch.randn(T, 4 * HD, device=DEV, generator=g), torch.randn(T, HD, device=DEV, generator=g)
+    ab, wb = (torch.randn(HD, device=DEV, generator=g) for _ in range(2))
+    S0 = torch.randn(1, H, D, D, device=DEV, generator=g) * 0.3
+    whole = S0.clone()
+    out = run(proj, wpre, ab, wb, whole, [T], H, D, 0.6)
+    for sizes in ([1] * T, [5, 1, 17] * T, [33] * T):
+        S, at, parts = S0.clone(), 0, []
+        for n in sizes:
+            if at < T:
+                parts.append(run(proj[at: at + n].contiguous(), wpre[at: at + n].contiguous(), ab, wb, S, [min(n, T - at)], H, D, 0.6))
+                at += n
+        assert torch.equal(torch.cat(parts), out) and torch.equal(S, whole)
+    for beside in ([1] * others, [T] * 40):
+        n = sum(beside)
+        more = torch.randn(n, 4 * HD, device=DEV, generator=g), torch.randn(n, HD, device=DEV, generator=g)
+        S = torch.cat([torch.randn(len(beside), H, D, D, device=DEV, generator=g), S0])
+        got = run(torch.cat([more[0], proj]), torch.cat([more[1], wpre]), ab, wb, S, [*beside, T], H, D, 0.6)
+        assert torch.equal(got[n:], out) and torch.equal(S[-1:], whole)
+        if beside[0] == 1:      # a step of single tokens in its own kernel
+            S, S1 = torch.cat([S[:-1], S0]), S0.clone()
+            got = run(torch.cat([more[0], proj[:1]]), torch.cat([more[1], wpre[:1]]), ab, wb, S, [1] * (others + 1), H, D, 0.6)
+            alone = run(torch.cat([proj[:1]]), wpre[:1].contiguous(), ab, wb, S1, [1], H, D, 0.6)
+            assert torch.equal(got[-1:], out[:1]) and torch.equal(alone, out[:1]) and torch.equal(S[-1:], S1)
 
 
 def test_a_later_infinity_reaches_no_earlier_token():
