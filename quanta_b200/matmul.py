@@ -8,6 +8,8 @@ process-wide when the first engine is built.
 from __future__ import annotations
 
 import torch
+import torch.autograd.forward_ad as forward_ad
+from torch.utils._python_dispatch import _get_current_dispatch_mode
 
 from . import kernels
 
@@ -46,11 +48,23 @@ def _with_spare_rows(x: torch.Tensor) -> torch.Tensor:
     return x
 
 
-def _few_float32_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether ``kernels.linear_rows`` takes the product: a few float32 rows, bound by the bytes of ``w``."""
-    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.is_cuda and x.dim() == 2
-            and 0 < x.shape[0] <= kernels.LINEAR_ROWS_MAX and x.shape[1] % 4 == 0 and x.is_contiguous() and w.is_contiguous()
-            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+def _few_float32_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None) -> bool:
+    """Whether ``kernels.linear_rows`` takes the product: a few float32 rows, bound by the bytes of ``w``, on the current device.  What
+    torch does with its own product besides computing it (gradients, forward mode, vmap, autocast, tracing, the errors of operands that
+    do not fit) stays with torch."""
+    if x.dtype != torch.float32 or w.dtype != torch.float32 or out_dtype not in (None, torch.float32):
+        return False
+    if type(x) is not torch.Tensor or type(w) not in (torch.Tensor, torch.nn.Parameter) or _get_current_dispatch_mode() is not None:
+        return False
+    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch.is_autocast_enabled("cuda") or forward_ad._current_level >= 0:
+        return False
+    if any(torch._C._functorch.is_functorch_wrapped_tensor(t) for t in (x, w)):
+        return False
+    if torch.is_grad_enabled() and (x.requires_grad or w.requires_grad):
+        return False
+    return (x.is_cuda and w.device == x.device and x.device.index == torch.cuda.current_device() and x.dim() == 2 and w.dim() == 2
+            and 0 < x.shape[0] <= kernels.LINEAR_ROWS_MAX and x.shape[1] == w.shape[1] and x.shape[1] > 0 and x.shape[1] % 4 == 0
+            and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
@@ -58,7 +72,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     accumulator's precision for bfloat16 operands.  An ``x`` from ``empty_rows`` is multiplied with its
     spare rows and the result cut back to ``T`` rows."""
     n = x.shape[0]
-    if _few_float32_rows(x, w):
+    if _few_float32_rows(x, w, out_dtype):
         out = torch.empty((n, w.shape[0]), dtype=torch.float32, device=x.device)
         kernels.linear_rows(x, w, out)
         return out

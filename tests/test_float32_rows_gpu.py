@@ -45,6 +45,37 @@ def test_linear_takes_the_library_where_rows_do_not_fit():
         assert torch.all((linear(x, ww).double() - want).abs() <= 2 * x.shape[1] * U * (x.double().abs() @ ww.double().abs().T))
 
 
+def test_linear_leaves_to_torch_what_is_torchs():
+    """Gradients, forward mode, vmap, autocast, another result type, an empty inner dimension and operands that do not fit: as torch.mm."""
+    import torch.autograd.forward_ad as forward_ad
+    from torch.func import vmap
+    from quanta_b200.matmul import linear
+    g = torch.Generator(device=DEV).manual_seed(2)
+    x, w = torch.randn(3, 64, device=DEV, generator=g), torch.randn(8, 64, device=DEV, generator=g)
+    xg, wg = x.clone().requires_grad_(), torch.nn.Parameter(w.clone())
+    linear(xg, wg).sum().backward()
+    assert torch.allclose(xg.grad, w.sum(0).expand(3, 64), rtol=1e-4, atol=1e-4) and torch.allclose(wg.grad, x.sum(0).expand(8, 64), rtol=1e-4, atol=1e-4)
+    with torch.no_grad():
+        assert torch.allclose(linear(xg, wg), x @ w.T, rtol=1e-4, atol=1e-4)
+    with forward_ad.dual_level():
+        out = linear(forward_ad.make_dual(x, torch.ones_like(x)), w)
+        assert torch.allclose(forward_ad.unpack_dual(out).tangent, w.sum(1).expand(3, 8), rtol=1e-4, atol=1e-4)
+    many = torch.randn(5, 40, 64, device=DEV, generator=g)
+    assert torch.allclose(vmap(lambda t: linear(t, w))(many), many @ w.T, rtol=1e-4, atol=1e-4)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert linear(x, w).dtype == torch.mm(x, w.T).dtype
+    for op in (lambda f: f(x, w, torch.bfloat16), lambda f: f(x, w[:, :60].contiguous()), lambda f: f(x, w[0]), lambda f: f(x, w.cpu()),
+               lambda f: f(x, w.bfloat16())):
+        got = []
+        for f in (linear, lambda a, b, dt=None: torch.mm(a, b.t(), out_dtype=dt) if dt else torch.mm(a, b.t())):
+            try:
+                got.append(op(f).dtype)
+            except Exception as e:
+                got.append(type(e))
+        assert got[0] == got[1], got
+    assert torch.equal(linear(x[:, :0], w[:, :0]), torch.zeros(3, 8, device=DEV))
+
+
 @pytest.mark.parametrize("T,H,I,E,k,mode,kind", [
     (1, 8, 4, 4, 2, 1, 0), (3, 132, 36, 5, 2, 1, 1), (4, 2048, 68, 3, 3, 3, 0), (4, 8192, 20, 4, 1, 1, 0), (7, 64, 100, 6, 4, 1, 0),
     (16, 260, 130, 2, 1, 3, 0), (40, 64, 36, 16, 2, 1, 1), (60, 132, 70, 4, 1, 1, 0), (100, 36, 260, 2, 2, 3, 0)])
