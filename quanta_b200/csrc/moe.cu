@@ -15,7 +15,7 @@
 //   expert e on row x: down_e( silu(gate_e x) * up_e x ), times w, summed over the k slots in slot
 //   order by the next norm kernel (src/quanta/minimax/moe.py:59-88); or, ungated (MODE 3 below),
 //   down_e( relu(up_e x)^2 ).
-#include "rows_f32.cuh"
+#include "common.cuh"
 
 // values of the `renorm` argument of the routing kernels: how the chosen experts are weighted
 #define QB_ROUTE_SIGMOID_RAW 0        // sigmoid scores as they are
@@ -905,11 +905,17 @@ __device__ __forceinline__ float mg_result(float g, float u, float w, int act_ki
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same products in float32 for steps of at most CAP tokens, so at most CAP rows an expert: bound by the bytes of the chosen
-// experts, read once (rows_f32.cuh).  Four tokens, five or six experts of 2,048 x 2,816, both products: 615 us with the kernel
-// above (a block waits for 4 to 8 KB at a time), 75 us with this one (69 us of bytes at 6.0 TB/s).
+// The same products in float32 for few rows an expert: bound by the bytes of the chosen experts, read once.  A block is a warp and takes 32
+// rows of weights (MODE 1: 16 gate and 16 up) and up to MF_ROWS rows of inputs; a thread owns a row of weights and adds its products with
+// all the inputs in the order of the inner dimension, as the kernel above does.  Slices of 64 of the inner dimension arrive by
+// asynchronous copies, two ahead of the one in use, as they lie in memory (272 bytes a row, an odd number of 16-byte units: eight
+// rows' reads meet no bank twice; an input's 16 bytes are the same for all threads).  One to four tokens are bound by the chain of additions
+// (a slice 256 cycles and its copies).  Measured on a B200, 4 tokens, seven of eight experts of 2,048 x 2,816, both products (74 us of
+// bytes): 615 us with the kernel above, 90 us with this one (84 with sums over lanes that read a row together, whose bits
+// are others than those of the kernels for more rows); 16 tokens 112 us, 24 189.
 // ---------------------------------------------------------------------------------------------
-constexpr int MR_WARPS = 4;
+constexpr int MF_THREADS = 32, MF_ROWS = 16, MF_BK = 64, MF_LD = MF_BK + 4, MF_STAGES = 3;
+constexpr int MF_PIECES = MF_BK / 4, MF_AT_ONCE = MF_THREADS / MF_PIECES;      // 16-byte pieces a row, rows a pass of the copies
 
 struct MoeRows {
   const float *x, *weights, *pair_w;
@@ -919,96 +925,114 @@ struct MoeRows {
   float act_limit, act_alpha;
 };
 
-extern __shared__ __align__(16) float moe_smem[];
+__device__ __forceinline__ void moe_copy16(float* dst, const float* src, bool ok) {      // zeros where it is not
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  const int n = ok ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
 
-template <int MODE, int FW, int U, int R, bool COPIED>
-__device__ __forceinline__ void moe_rows_run(const MoeRows& a, int e, int row0, int rows, int n0, int lane) {
-  constexpr int NF = MODE == 1 ? FW / 2 : FW;              // features a warp; MODE 1 reads a gate and an up row for each
-  constexpr int V = NF * R;
-  const float* wbase = a.weights + (size_t)e * (MODE == 1 ? 2 : 1) * a.N * a.K;
-  const float* wr[FW];
+template <int MODE, int R>                // R: rows of inputs, `rows` of them there
+__device__ __forceinline__ void moe_few_run(const MoeRows& a, float* smem, int e, int row0, int rows, int n0) {
+  constexpr int NF = MODE == 1 ? MF_THREADS / 2 : MF_THREADS;                // features a block
+  constexpr int STAGE = (MF_THREADS + R) * MF_LD, PASSES = MF_THREADS / MF_AT_ONCE, X_PASSES = (R + MF_AT_ONCE - 1) / MF_AT_ONCE;
+  const int tid = threadIdx.x, K = a.K, N = a.N;
+  const float* wbase = a.weights + (size_t)e * (MODE == 1 ? 2 : 1) * N * K;
+  // copies: thread (c, q) takes the 16 bytes q of the rows c, c + MF_AT_ONCE, ...: the weights, then the inputs
+  const int c = tid / MF_PIECES, q = tid % MF_PIECES * 4;
+  const float *src[PASSES], *x_src[X_PASSES];
 #pragma unroll
-  for (int f = 0; f < FW; ++f) {
-    const int n = min(n0 + f % NF, a.N - 1);
-    wr[f] = wbase + (size_t)(f < NF ? n : a.N + n) * a.K;
+  for (int i = 0; i < PASSES; ++i) {
+    const int r = c + MF_AT_ONCE * i, n = n0 + r % NF;
+    src[i] = n < N ? wbase + (size_t)(r < NF ? n : N + n) * K : nullptr;
   }
-  const float* xr[R];
+#pragma unroll
+  for (int i = 0; i < X_PASSES; ++i) {
+    const int r = c + MF_AT_ONCE * i, p = row0 + r;
+    x_src[i] = r < rows ? a.x + (size_t)(MODE == 2 ? p : a.sorted_pair[p] / a.top_k) * K : nullptr;
+  }
+  auto fetch = [&](int s) {
+    const int k = s * MF_BK + q;
+    float* st = smem + (s % MF_STAGES) * STAGE;
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+      const bool ok = src[i] != nullptr && k < K;
+      moe_copy16(st + (c + MF_AT_ONCE * i) * MF_LD + q, ok ? src[i] + k : a.weights, ok);
+    }
+#pragma unroll
+    for (int i = 0; i < X_PASSES; ++i) {
+      const bool ok = x_src[i] != nullptr && k < K;
+      if (c + MF_AT_ONCE * i < R) moe_copy16(st + (MF_THREADS + c + MF_AT_ONCE * i) * MF_LD + q, ok ? x_src[i] + k : a.x, ok);
+    }
+  };
+  const int steps = (K + MF_BK - 1) / MF_BK;
+#pragma unroll
+  for (int s = 0; s < MF_STAGES - 1; ++s) {
+    if (s < steps) fetch(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float acc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r] = 0.f;
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(MF_STAGES - 2) : "memory");
+    __syncthreads();
+    if (s + MF_STAGES - 1 < steps) fetch(s + MF_STAGES - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* w = smem + (s % MF_STAGES) * STAGE + tid * MF_LD;
+    const float* x = smem + (s % MF_STAGES) * STAGE + MF_THREADS * MF_LD;
+#pragma unroll
+    for (int k = 0; k < MF_BK; k += 4) {      // past K: zeros
+      const float4 v = *reinterpret_cast<const float4*>(w + k);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float4 u = *reinterpret_cast<const float4*>(x + r * MF_LD + k);
+        acc[r] = fmaf(u.x, v.x, acc[r]);
+        acc[r] = fmaf(u.y, v.y, acc[r]);
+        acc[r] = fmaf(u.z, v.z, acc[r]);
+        acc[r] = fmaf(u.w, v.w, acc[r]);
+      }
+    }
+  }
+  if (MODE == 1) {                            // the up sums to the threads of their gates
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (tid >= NF) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) smem[r * NF + tid - NF] = acc[r];
+    }
+    __syncthreads();
+  }
+  const int n = n0 + tid;
+  if (tid >= NF || n >= N) return;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int i = min(r, rows - 1), p = row0 + i;
-    xr[r] = COPIED ? moe_smem + (size_t)i * a.K : a.x + (size_t)(MODE == 2 ? p : a.sorted_pair[p] / a.top_k) * a.K;
-  }
-  auto x = [&](int r, int k) {
-    return COPIED ? *reinterpret_cast<const float4*>(xr[r] + k) : __ldg(reinterpret_cast<const float4*>(xr[r] + k));
-  };
-  float acc[FW][R];
-  qb_rows_dot<FW, R, U>(wr, x, [] { if (COPIED) qb_rows_ready(); }, a.K, lane, acc);
-  float g[V], u[MODE == 1 ? V : 1];                         // index r * NF + f
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-      g[r * NF + f] = acc[f][r];
-      if (MODE == 1) u[r * NF + f] = acc[(MODE == 1 ? NF : 0) + f][r];
-    }
-  const int first = qb_sum_values<V>(g, lane);
-  if (MODE == 1) qb_sum_values<MODE == 1 ? V : 1>(u, lane);
-  if (!qb_sum_stores<V>(lane)) return;
-  constexpr int HELD = V > 32 ? V / 32 : 1;
-#pragma unroll
-  for (int i = 0; i < HELD; ++i) {
-    const int r = (first + i) / NF, n = n0 + (first + i) % NF;
-    if (r >= rows || n >= a.N) continue;
+    if (r >= rows) break;
     const int p = row0 + r, pair = a.sorted_pair[p];
-    const float w = a.pair_w != nullptr ? a.pair_w[pair] : 1.f;
-    a.out[(size_t)(MODE == 2 ? pair : p) * a.N + n] =
-        mg_result<MODE>(g[i], MODE == 1 ? u[MODE == 1 ? i : 0] : 0.f, w, a.act_kind, a.act_limit, a.act_alpha);
+    a.out[(size_t)(MODE == 2 ? pair : p) * N + n] =
+        mg_result<MODE>(acc[r], MODE == 1 ? smem[r * NF + tid] : 0.f, a.pair_w != nullptr ? a.pair_w[pair] : 1.f, a.act_kind, a.act_limit,
+                        a.act_alpha);
   }
 }
 
-template <int MODE, int FW, int U, int CAP, bool COPIED>
-__global__ void __launch_bounds__(MR_WARPS * 32)
-moe_rows_kernel(MoeRows a, const int* __restrict__ plan, const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, int E,
-                int turn) {
+template <int MODE>
+__global__ void __launch_bounds__(MF_THREADS)
+moe_few_f32_kernel(MoeRows a, const int* __restrict__ plan, const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, int E,
+                   int turn) {
+  extern __shared__ __align__(16) float mt_smem[];
   const int tile = blockIdx.y;
   if (tile >= plan[3 * E + 1]) return;
-  const int lane = threadIdx.x & 31;
-  const int n0 = (blockIdx.x * MR_WARPS + (threadIdx.x >> 5)) * (MODE == 1 ? FW / 2 : FW);     // past N: nothing is stored
+  const int n0 = blockIdx.x * (MODE == 1 ? MF_THREADS / 2 : MF_THREADS);
   const int e = tile_expert[tile], row0 = tile_row0[tile];
   const int rows = min(plan[2 * E + e + 1] - row0, MG_BM);
-  for (int g = 0; g < rows; g += turn) {                    // `turn` <= CAP rows at a time: what the shared memory was asked for
+  for (int g = 0; g < rows; g += turn) {                    // `turn` rows at a time: what the shared memory was asked for
     const int n = min(rows - g, turn);
-    if (COPIED) {
-      if (g) __syncthreads();
-      qb_rows_copy(moe_smem, [&](int r) {
-        const int p = row0 + g + r;
-        return a.x + (size_t)(MODE == 2 ? p : a.sorted_pair[p] / a.top_k) * a.K;
-      }, n, a.K);
-    }
-    if (n <= 1) moe_rows_run<MODE, FW, U, 1, COPIED>(a, e, row0 + g, n, n0, lane);
-    else if (n <= 2) moe_rows_run<MODE, FW, U, 2, COPIED>(a, e, row0 + g, n, n0, lane);
-    else if (CAP <= 4 || n <= 4) moe_rows_run<MODE, FW, U, 4, COPIED>(a, e, row0 + g, n, n0, lane);
-    else if (n <= 8) moe_rows_run<MODE, FW, U, 8, COPIED>(a, e, row0 + g, n, n0, lane);
-    else moe_rows_run<MODE, FW, U, CAP, COPIED>(a, e, row0 + g, n, n0, lane);
+    if (g) __syncthreads();
+    if (n <= 1) moe_few_run<MODE, 1>(a, mt_smem, e, row0 + g, n, n0);
+    else if (n <= 2) moe_few_run<MODE, 2>(a, mt_smem, e, row0 + g, n, n0);
+    else if (n <= 4) moe_few_run<MODE, 4>(a, mt_smem, e, row0 + g, n, n0);
+    else if (n <= 8) moe_few_run<MODE, 8>(a, mt_smem, e, row0 + g, n, n0);
+    else moe_few_run<MODE, 16>(a, mt_smem, e, row0 + g, n, n0);
   }
-}
-
-template <int MODE, int FW, int U, int CAP>
-static int moe_rows_launch(const MoeRows& a, const int* plan, const int* tile_expert, const int* tile_row0, int max_tiles, int E,
-                           int max_rows, cudaStream_t stream) {
-  constexpr int PER_BLOCK = MR_WARPS * (MODE == 1 ? FW / 2 : FW);
-  const dim3 grid((a.N + PER_BLOCK - 1) / PER_BLOCK, max_tiles);
-  const int turn = min(max_rows, CAP), smem = qb_rows_smem(turn, a.K);
-  if (smem > 0) {
-    static const cudaError_t once = cudaFuncSetAttribute(moe_rows_kernel<MODE, FW, U, CAP, true>,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, QB_ROWS_SMEM);
-    if (once != cudaSuccess) return (int)once;
-    moe_rows_kernel<MODE, FW, U, CAP, true><<<grid, MR_WARPS * 32, smem, stream>>>(a, plan, tile_expert, tile_row0, E, turn);
-  } else {
-    moe_rows_kernel<MODE, FW, U, CAP, false><<<grid, MR_WARPS * 32, 0, stream>>>(a, plan, tile_expert, tile_row0, E, turn);
-  }
-  QB_LAUNCH_CHECK();
-  return 0;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1023,12 +1047,6 @@ constexpr int MT_BN = 128, MT_BK = 16, MT_LD = MT_BK + 4, MT_STAGES = 4;
 constexpr int MT_COPIES = (MG_BM + MT_BN) / 32;
 constexpr int MT_STAGE = (MG_BM + MT_BN) * MT_LD;
 constexpr int MT_SMEM = MT_STAGES * MT_STAGE * (int)sizeof(float);
-
-__device__ __forceinline__ void mt_copy16(float* dst, const float* src, bool ok) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  const int n = ok ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
 
 template <int MODE>
 __global__ void __launch_bounds__(128, 4)
@@ -1062,7 +1080,7 @@ moe_tile_f32_kernel(MoeRows a, const int* __restrict__ plan, const int* __restri
     const int k = s * MT_BK + q;
     float* st = mt_smem + (s % MT_STAGES) * MT_STAGE;
 #pragma unroll
-    for (int i = 0; i < MT_COPIES; ++i) mt_copy16(st + (c + 32 * i) * MT_LD + q, src[i] + (k < K ? k : 0), ok[i] && k < K);
+    for (int i = 0; i < MT_COPIES; ++i) moe_copy16(st + (c + 32 * i) * MT_LD + q, src[i] + (k < K ? k : 0), ok[i] && k < K);
   };
   const int steps = (K + MT_BK - 1) / MT_BK;
 #pragma unroll
@@ -1119,19 +1137,21 @@ moe_tile_f32_kernel(MoeRows a, const int* __restrict__ plan, const int* __restri
   }
 }
 
+// All float32 with rows of whole 16-byte pieces.  Both kernels give the bits of the general one.  Few rows an expert: up to eleven on
+// average (40 tokens, two of eight experts, mean 10: 124 + 87 us by rows, 184 + 116 by tiles; 64, mean 16: 201 + 114 and 186 + 117).
 template <int MODE>
 static int moe_grouped_f32(const MoeRows& a, const int* plan, const int* tile_expert, const int* tile_row0, int max_tiles, int E,
                            int max_rows, int mean_rows, cudaStream_t stream) {
-  // by rows up to eight an expert on average: 24 tokens, two of eight experts of 2,048 x 2,816 (mean 6) 110 + 74 us by rows, 184 + 115 by
-  // tiles; 64 tokens (mean 16) 201 + 140 by rows, 187 + 118 by tiles
-  if (max_rows <= 4) return moe_rows_launch<MODE, 2, 4, 4>(a, plan, tile_expert, tile_row0, max_tiles, E, max_rows, stream);
-  if (mean_rows <= 8) return moe_rows_launch<MODE, 4, 2, 16>(a, plan, tile_expert, tile_row0, max_tiles, E, max_rows, stream);
-  {
-    static const cudaError_t once = cudaFuncSetAttribute(moe_tile_f32_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM);
-    if (once != cudaSuccess) return (int)once;
-    constexpr int BF = MODE == 1 ? MT_BN / 2 : MT_BN;
-    moe_tile_f32_kernel<MODE><<<dim3((a.N + BF - 1) / BF, max_tiles), 128, MT_SMEM, stream>>>(a, plan, tile_expert, tile_row0, E);
-  }
+  const bool few = mean_rows < 12;
+  const int turn = max_rows <= 1 ? 1 : max_rows <= 2 ? 2 : max_rows <= 4 ? 4 : max_rows <= 8 ? 8 : MF_ROWS;
+  const int bf = few ? (MODE == 1 ? MF_THREADS / 2 : MF_THREADS) : MODE == 1 ? MT_BN / 2 : MT_BN;
+  const int smem = few ? MF_STAGES * (MF_THREADS + turn) * MF_LD * (int)sizeof(float) : MT_SMEM;
+  const dim3 grid((a.N + bf - 1) / bf, max_tiles);
+  const cudaError_t err = few ? cudaFuncSetAttribute(moe_few_f32_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
+                              : cudaFuncSetAttribute(moe_tile_f32_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) return (int)err;
+  if (few) moe_few_f32_kernel<MODE><<<grid, MF_THREADS, smem, stream>>>(a, plan, tile_expert, tile_row0, E, turn);
+  else moe_tile_f32_kernel<MODE><<<grid, 128, smem, stream>>>(a, plan, tile_expert, tile_row0, E);
   QB_LAUNCH_CHECK();
   return 0;
 }
@@ -1145,8 +1165,7 @@ extern "C" int qb_moe_grouped_simt(int mode, const void* x, int x_dtype, const v
   if (max_tiles <= 0) return 0;
   if (act_kind < 0 || act_kind > 1 || (act_kind == 1 && (mode != 1 || pair_w == nullptr))) return QB_ERR_BAD_ARG;
   if (max_tiles > 65535) return QB_ERR_UNSUPPORTED;
-  // all float32 with rows of whole 16-byte pieces: the two kernels above.  A router gives a token an expert once, so an expert has
-  // at most n_pairs / top_k rows (were there more, they would be taken in turns).
+  // A router gives a token an expert once, so an expert has at most n_pairs / top_k rows (were there more, they would be taken in turns).
   if (x_dtype == QB_F32 && w_dtype == QB_F32 && out_dtype == QB_F32 && K % 4 == 0 &&
       ((uintptr_t)x & 15) == 0 && ((uintptr_t)weights & 15) == 0) {
     const MoeRows a{(const float*)x, (const float*)weights, pair_w, (float*)out, sorted_pair, top_k, K, N,

@@ -124,6 +124,38 @@ def test_expert_products_float32(T, H, I, E, k, mode, kind):
     assert st.tolist()[0] == 0
 
 
+@pytest.mark.parametrize("H,I,E,k,mode,kind", [(132, 36, 4, 2, 1, 0), (64, 100, 6, 4, 1, 1), (260, 70, 3, 1, 3, 0), (2048, 68, 8, 2, 1, 0), (36, 260, 2, 2, 3, 0)])
+def test_expert_products_do_not_depend_on_the_step(H, I, E, k, mode, kind):
+    """A token alone, in a step of few rows an expert (in turns of 16 too), of many, and through the kernel that reads number by number
+    (rows that do not start on 16 bytes): the same bits."""
+    kern = K()
+    T = 130
+    g = torch.Generator(device=DEV).manual_seed(H)
+    x = torch.randn(T, H, device=DEV, generator=g)
+    w1 = torch.randn(E, (2 if mode == 1 else 1) * I, H, device=DEV, generator=g) / math.sqrt(H)
+    w2 = torch.randn(E, H, I, device=DEV, generator=g) / math.sqrt(I)
+    idx = torch.stack([torch.randperm(E, device=DEV, generator=g)[:k] for _ in range(T)]).int()
+    pw = torch.rand(T, k, device=DEV, generator=g) + 0.2
+
+    def run(lo, hi, by=1):
+        n, m = (hi - lo) * k, hi - lo
+        words, tiles = kern.moe_plan_sizes(n, E, kern.MOE_SIMT_BM)
+        plan, sp, te, tr = (torch.empty(c, device=DEV, dtype=torch.int32) for c in (words, n, tiles, tiles))
+        st = kern.new_status(DEV)
+        kern.moe_plan(idx[lo:hi].contiguous(), E, kern.MOE_SIMT_BM, plan, sp, te, tr, st)
+        at = lambda t: t.contiguous() if by else torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)      # off 16 bytes
+        act, y = torch.empty(n * I + 1, device=DEV)[1 - by: n * I + 1 - by].view(n, I), torch.empty(n, H, device=DEV)
+        kern.moe_grouped_simt(mode, at(x[lo:hi]), w1, act, sp, pw[lo:hi].contiguous(), plan, te, tr, E, k, act=(kind, 1.5, 1.7))
+        kern.moe_grouped_simt(2, act, w2, y, sp, None if kind else pw[lo:hi].contiguous().view(-1), plan, te, tr, E, k)
+        assert st.tolist()[0] == 0
+        return y.view(m, k, H)
+
+    whole = run(0, T)
+    assert torch.equal(run(0, T, by=0), whole)
+    for lo, hi in ((0, 1), (5, 7), (9, 12), (20, 27), (40, 53), (60, 90), (0, 64)):
+        assert torch.equal(run(lo, hi), whole[lo:hi]), (lo, hi)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("nq,nkv,hd,vd,page,window,lens", [
     (4, 1, 4, 4, 4, 0, [1, 9]), (6, 3, 64, 64, 8, 0, [70, 3]), (5, 5, 132, 20, 16, 0, [33]), (8, 1, 128, 128, 16, 40, [130, 7, 8]),
