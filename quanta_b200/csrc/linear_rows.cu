@@ -57,9 +57,9 @@ template <int FW, int U, int CAP>
 static int linear_rows_launch(const LinearRows& a, cudaStream_t stream) {
   const int grid = (a.N + FW * LR_WARPS - 1) / (FW * LR_WARPS), smem = qb_rows_smem(a.rows, a.K);
   if (smem > 0) {
-    static const cudaError_t once = cudaFuncSetAttribute(linear_rows_kernel<FW, U, CAP, true>,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, QB_ROWS_SMEM);
-    if (once != cudaSuccess) return (int)once;
+    const cudaError_t err = cudaFuncSetAttribute(linear_rows_kernel<FW, U, CAP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 QB_ROWS_SMEM);
+    if (err != cudaSuccess) return (int)err;
     linear_rows_kernel<FW, U, CAP, true><<<grid, LR_WARPS * 32, smem, stream>>>(a);
   } else {
     linear_rows_kernel<FW, U, CAP, false><<<grid, LR_WARPS * 32, 0, stream>>>(a);
