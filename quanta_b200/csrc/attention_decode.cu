@@ -20,7 +20,9 @@
 // shared memory in a fixed order: one launch, no scratch in memory.
 //
 // Bound by the bytes of keys and values for many keys and by three memory latencies for few.  Measured on a B200, 48 + 8 heads, beside the
-// persistent kernel of attention_mma.cu with its merge launch: see the rule in qb_attn_decode_direct.
+// persistent kernel of attention_mma.cu with its merge launch: see the rule in qb_attn_decode_direct_wins.
+#include <math.h>
+
 #include "common.cuh"
 
 namespace {
@@ -287,6 +289,55 @@ extern "C" int qb_attn_decode_direct_supported(int nq, int nkv, int hd) {
   return hd == DD_HD && nkv > 0 && nq % nkv == 0 && nq / nkv <= 8 ? 1 : 0;
 }
 
+// Warps a block and blocks a unit (a (token, kv head)).  Eight warps a block and as many blocks a unit, up to eight, as fill the SMs once,
+// but no more than the keys give rounds for; with more units than SMs blocks of four warps, two to an SM, a unit two of them where that
+// leaves eight rounds a warp.
+static void dd_shape(long units, int keys, int& warps, int& S) {
+  const int rounds = (keys + DD_KEYS - 1) / DD_KEYS;
+  warps = 8;
+  S = 1;
+  if (units >= 148) {
+    warps = 4;
+    S = units < 592 && rounds >= 64 ? 2 : 1;
+  } else {
+    // clusters fill a GPC of 16 to 20 SMs in part only: what does not fit waits for a second wave (48 units of 3 blocks: 32 us for 6 tokens
+    // of 3,000 keys, 2 blocks 22)
+    while (S < 6 && units * (S + 1) <= (S < 2 ? 148 : S < 4 ? 128 : 120)) ++S;
+    if (units <= 12) S = 8;
+  }
+  while (S > 1 && (S - 1) * warps >= rounds) --S;
+}
+static int dd_keys(int longest, int window, int chunk) {
+  const int keys = window > 0 && window < longest ? window : longest;
+  return chunk > 0 && chunk < keys ? chunk : keys;
+}
+
+// Whether these single tokens, with `longest` and `total` keys, are faster here than in the kernel that takes all other shapes: the persistent
+// one with its merge, whose blocks share the keys of all tokens alike, or for weights that stay 32-bit the one of attention_rows.cuh.  Here a
+// unit's keys are walked by its own S blocks, so one long request among short ones, or few units, which eight blocks each do not make
+// fill the SMs, cost what that walk costs: 8.0 us for 1,000 keys a block of eight warps.  The others' times are lines through what they
+// measure; over 370 mixes of lengths the choice is 0.3 % off the better kernel on average, 17 % at most.  Measured on a B200, here / persistent, 48 + 8 heads: 16 tokens, one of 131,072 keys and the others of 500, 1,029 / 164 us, one of 8,000 69
+// / 33, one of 2,000 23 / 25, all of 8,000 87 / 116; one of 131,072 140 / 119, of 24,000 33 / 37; 6 + 1 heads, one token of 131,072 141 / 62, of
+// 24,000 31 / 52.
+extern "C" int qb_attn_decode_direct_wins(int n_dec, int nq, int nkv, int hd, int longest, long long total, int window, int chunk,
+                                          int two_part) {
+  if (n_dec <= 0 || longest <= 0 || !qb_attn_decode_direct_supported(nq, nkv, hd)) return 0;
+  const long units = (long)n_dec * nkv;
+  const int keys = dd_keys(longest, window, chunk), G = nq / nkv;
+  int warps, S;
+  dd_shape(units, keys, warps, S);
+  const double all = (double)(total < (long long)n_dec * keys ? (total > keys ? total : keys) : (long long)n_dec * keys) * nkv;
+  const double here = (5.5 + 0.0080 * keys / S * 8 / warps) * (two_part ? 1.12 : 1.08);      // 1.08: the other kernel where they are close
+  if (two_part) {
+    const int groups = G % 4 == 0 ? G / 4 : G % 2 == 0 ? G / 2 : G;      // q heads of a kv head a block: 4, 2 or 1
+    double ranges = 1184.0 / (units * (G / 4 > 1 ? G / 4 : 1));
+    ranges = fmin(fmin(ranges, 64.0), (keys + 255) / 256);
+    return here <= 12.0 + 2.8 / 64 * fmax(all * groups / 148, keys / fmax(ranges, 1.0)) ? 1 : 0;
+  }
+  const double segments = fmin(148.0 * keys / all, (keys + 63) / 64);     // that the longest pair is cut into: the merge adds them one by one
+  return here <= 13.0 + all * (4 * DD_HD) / 5.0e6 + 0.2 * segments ? 1 : 0;
+}
+
 // dec_tok: the token rows of the n_dec single tokens; longest: keys of the longest request (an upper bound is enough).
 extern "C" int qb_attn_decode_direct(const void* q, const void* k_cache, const void* v_cache, void* out, const int* dec_tok, int n_dec,
                                      const int* tok_pos, const int* tok_req, const int* block_table, int bt_stride, int nq, int nkv,
@@ -301,25 +352,11 @@ extern "C" int qb_attn_decode_direct(const void* q, const void* k_cache, const v
     if (page_size == 1 << i) shift = i;
   const long units = (long)n_dec * nkv;
   if (units * 8 > 0x7fffffffL || (long)num_pages * nkv * page_size > 0x7fffffffL) return QB_ERR_UNSUPPORTED;
-  // Eight warps a block and as many blocks a unit, up to eight, as fill the SMs once, but no more than the keys give rounds for; with
-  // more units than SMs blocks of four warps, two to an SM, a unit two of them where that leaves eight rounds a warp.  This kernel and the
-  // persistent one with its merge launch, 48 + 8 heads: one token of 60 keys 5.5 and 10.8 us, of 2,100 10.0 and 15.8, of 24,000 33 and
-  // 35; 2 of 24,000 and 18,000 42 and 48 (four blocks a unit 53), 4 of 4,000 19 and 29, 8 of 2,100 to 1,050 18 and 26, 16 of 2,000 27 and 40,
-  // 64 of 500 33 and 49, of 2,100 to 1,050 91 to 95 and 100.  `two_part`: weights in parts (SPLIT).
-  int keys = window > 0 && window < longest ? window : longest;
-  if (chunk > 0 && chunk < keys) keys = chunk;
-  const int rounds = (keys + DD_KEYS - 1) / DD_KEYS;
-  int warps = 8, S = 1;
-  if (units >= 148) {
-    warps = 4;
-    S = units < 592 && rounds >= 64 ? 2 : 1;
-  } else {
-    // clusters fill a GPC of 16 to 20 SMs in part only: what does not fit waits for a second wave (48 units of 3 blocks: 32 us for 6 tokens
-    // of 3,000 keys, 2 blocks 22)
-    while (S < 6 && units * (S + 1) <= (S < 2 ? 148 : S < 4 ? 128 : 120)) ++S;
-    if (units <= 12) S = 8;
-  }
-  while (S > 1 && (S - 1) * warps >= rounds) --S;
+  // This kernel and the persistent one with its merge launch, contexts of like length, 48 + 8 heads: one token of 60 keys 5.5 and 10.8 us, of
+  // 2,100 10.0 and 15.8; 2 of 24,000 and 18,000 42 and 48 (four blocks a unit 53), 4 of 4,000 19 and 29, 8 of 2,100 to 1,050 18 and 26,
+  // 16 of 2,000 27 and 40, 64 of 500 33 and 49, of 2,100 to 1,050 91 to 95 and 100.  `two_part`: weights in parts (SPLIT).
+  int warps, S;
+  dd_shape(units, dd_keys(longest, window, chunk), warps, S);
   const DecodeArgs P{dec_tok, tok_pos, tok_req, block_table, bt_stride, nq, nkv, page_size, shift, num_pages, window, chunk, S,
                      scale, cap, status};
   cudaLaunchConfig_t cfg = {};

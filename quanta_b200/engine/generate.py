@@ -103,7 +103,7 @@ class LLM:
         if not ahead:
             return None
         wants = {r.rid: mgr.length(r.rid) + 1 for r in ahead}
-        if not mgr.can_reserve(wants) or not eng.decode_graph_ready(len(ahead), max(wants.values())):
+        if not mgr.can_reserve(wants) or not eng.decode_graph_ready(len(ahead), 0, lens=list(wants.values())):
             return None
         return ahead
 

@@ -8,8 +8,8 @@ into one pinned buffer, copies it once, runs the model on exactly these tokens, 
 logits at the wanted places.  Nothing inside synchronises with the host.
 
 Steps in which every request brings exactly one token (decoding) are launch-bound when run kernel
-by kernel, so they are captured once per (batch size, context bucket) in a CUDA graph and replayed:
-the graph reads its integers from a fixed device buffer that each step overwrites.  At most
+by kernel, so they are captured once per (batch size, context bucket; above 2,048 keys also lengths
+alike or not) in a CUDA graph and replayed: the graph reads its integers from a fixed device buffer that each step overwrites.  At most
 ``max_graphs`` captured steps are kept; the one used longest ago goes when another is captured.
 
 Every live request has a state slot: a row of each mixer's fixed-size state and one record of the
@@ -41,7 +41,7 @@ class StepEntry:
 
 
 class _DecodeGraph:
-    """A captured decode step for one (batch size, context bucket)."""
+    """A captured decode step for one key of ``Engine._graph_key``."""
 
     def __init__(self):
         self.graph = None
@@ -240,7 +240,7 @@ class Engine:
         return pieces, info
 
     def _context(self, dev: torch.Tensor, sizes: list[int], R: int, T: int, max_pages: int, info: dict,
-                 max_len_after: int, max_new: int, with_host: bool):
+                 max_len_after: int, max_new: int, with_host: bool, even: bool = True):
         out, off = [], 0
         for n in sizes:
             out.append(dev[off: off + n])
@@ -251,7 +251,7 @@ class Engine:
         ctx = StepContext(
             n_tokens=T, positions=d_positions.view(T, self.n_axes), tok_pos=d_pos, tok_req=d_req, req_slot=d_slot,
             req_start=d_start, req_len_after=d_len, status=self.status, dtype=self.model.dtype,
-            max_new_tokens_per_req=max_new, max_len_after=max_len_after,
+            max_new_tokens_per_req=max_new, max_len_after=max_len_after, even=even,
             host={k: info[k] for k in ("req_start", "req_len_after", "req_slot")} if with_host else {},
             dec_tok=d_dec if info["n_dec"] else None, n_dec=info["n_dec"], spans=info["spans"])
         caches = []
@@ -293,22 +293,30 @@ class Engine:
             bucket *= 2
         return bucket
 
-    def decode_graph_ready(self, batch: int, max_len_after: int, entries=None) -> bool:
-        """Whether a decode step of ``batch`` requests, the longest ``max_len_after`` tokens afterwards,
+    @classmethod
+    def _graph_key(cls, lens: list[int], batch: int | None = None) -> tuple:
+        """The captured step for requests of these lengths: (batch, bucket), and a word more where long contexts are of unlike length,
+        since kernels that suit like lengths then leave most of the device waiting for the longest request."""
+        batch, longest = batch or len(lens), max(lens)
+        bucket = cls._bucket(longest)
+        even = bucket <= 2048 or len(lens) < batch or sum(lens) >= 0.6 * batch * longest
+        return (batch, bucket) if even else (batch, bucket, "uneven")
+
+    def decode_graph_ready(self, batch: int, max_len_after: int, entries=None, lens: list[int] | None = None) -> bool:
+        """Whether a decode step of ``batch`` requests, the longest ``max_len_after`` tokens afterwards (``lens``: each of them),
         replays a captured graph (else it runs eagerly and is captured at its second use)."""
         if not self.use_graphs:
             return False
         if entries is not None:
-            max_len_after = max(self.manager.length(e.rid) + 1 for e in entries if self.manager.has(e.rid))
-        g = self._graphs.get((batch, self._bucket(max_len_after)))
+            lens = [self.manager.length(e.rid) + 1 for e in entries if self.manager.has(e.rid)]
+        g = self._graphs.get(self._graph_key(lens or [max_len_after], batch))
         return g is not None and g.graph is not None
 
     def _run_decode(self, entries: list[StepEntry]) -> torch.Tensor | None:
         mgr, ps = self.manager, self.page_size
         B = len(entries)
-        max_len_after = max(mgr.length(e.rid) + 1 for e in entries)
-        bucket = self._bucket(max_len_after)
-        key = (B, bucket)
+        key = self._graph_key([mgr.length(e.rid) + 1 for e in entries])
+        bucket = key[1]
         g = self._graphs.setdefault(key, _DecodeGraph())
         if g.graph is None and (g.seen < 1 or g.failed >= 2):
             g.seen += 1
@@ -333,7 +341,8 @@ class Engine:
             # ids sampled by the step before, still on the device, in the requests' records
             g.dev[:B].copy_(torch.index_select(self.slots[:, kernels.SLOT_LAST], 0, row_slots))
         if g.graph is None:
-            d_ids, d_want, ctx, caches = self._context(g.dev, sizes, B, B, max_pages, info, bucket, 1, with_host=False)
+            d_ids, d_want, ctx, caches = self._context(g.dev, sizes, B, B, max_pages, info, bucket, 1, with_host=False,
+                                                       even=len(key) == 2)
             torch.cuda.synchronize()
             before = kernels.LAUNCHES
             graph = torch.cuda.CUDAGraph()

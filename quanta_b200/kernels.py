@@ -425,8 +425,16 @@ def attn_decode(q, k_cache, v_cache, out, part_o, part_ml, dec_tok, n_dec: int, 
 
 
 def attn_decode_direct_supported(nq: int, nkv: int, hd: int) -> bool:
-    """Whether single tokens of these shapes run as ``attn_decode_direct`` (else as ``attn_decode``)."""
+    """Whether ``attn_decode_direct`` takes these shapes."""
     return bool(lib().qb_attn_decode_direct_supported(int(nq), int(nkv), int(hd)))
+
+
+def attn_decode_direct_wins(n_dec: int, nq: int, nkv: int, hd: int, longest: int, total: int, window: int, *, chunk: int = 0,
+                            two_part: bool = False) -> bool:
+    """Whether ``attn_decode_direct`` takes these shapes and is the faster kernel for ``n_dec`` single tokens whose requests have
+    ``total`` keys, the longest ``longest`` (else ``attn_decode``; with ``two_part`` ``window_attention``)."""
+    return bool(lib().qb_attn_decode_direct_wins(int(n_dec), int(nq), int(nkv), int(hd), int(longest), ctypes.c_longlong(int(total)),
+                                                 int(window), int(chunk), int(two_part)))
 
 
 def attn_decode_direct(q, k_cache, v_cache, out, dec_tok, n_dec: int, tok_pos, tok_req, block_table, scale: float, window: int,
@@ -1013,7 +1021,7 @@ def window_attention(q, k_cache, v_cache, out, tok_pos, tok_req, block_table, sc
     if n_split is None and talk is None and pool_table is None and hd % 4 == 0 and vd % 4 == 0:
         # eight warps a (token, kv head, four q heads, range), 64 keys of it a turn of 2.6 us (a look-up and a read of memory): ranges of
         # 256 keys while that fills the SMs eight warps deep; joining them is a launch of 7 us
-        keys = min(n for n in (window, chunk, block_table.shape[1] * page_size) if n > 0)
+        keys = min((n for n in (window, chunk, block_table.shape[1] * page_size) if n > 0), default=1)
         n_split = max(1, min(-(-keys // 256), 1184 // max(1, T * nkv * max(1, nq // nkv // 4)), 64))
     if n_split is None:
         warps = T * nkv * (nkv if talk is not None else 1)        # of the kernel that shares a key row among q heads

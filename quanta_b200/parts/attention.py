@@ -230,9 +230,10 @@ class GQAttention(Mixer):
             starts = ctx.host.get("req_start") or [0, ctx.n_tokens]
             spans = [(r, starts[r], starts[r + 1] - starts[r]) for r in range(len(starts) - 1)]
             n_dec = 0
-        if n_dec and kernels.attn_decode_direct_supported(self.nq, self.nkv, self.hd):
+        longest, total = single_keys(ctx, n_dec)
+        if n_dec and kernels.attn_decode_direct_wins(n_dec, self.nq, self.nkv, self.hd, longest, total, window):
             kernels.attn_decode_direct(q, cache.k, cache.v, out, dec_tok, n_dec, ctx.tok_pos, ctx.tok_req, cache.block_table, self.scale,
-                                       window, max(1, ctx.max_len_after), ctx.status)
+                                       window, longest, ctx.status)
         elif n_dec:
             n_parts = kernels.attn_decode_parts(self.nkv, max(1, ctx.max_len_after))
             part_o = torch.empty(n_dec * self.nq * n_parts * self.hd, dtype=torch.float32, device=q.device)
@@ -258,15 +259,29 @@ def span_tiles(ctx, spans, G: int, rows: int, hd: int, device):
     return ctx.work[key]
 
 
+def single_keys(ctx, n_dec: int) -> tuple[int, int]:
+    """Keys of the longest request that brings one token to the step, and of all of them: exact where the host knows them, in a captured
+    step what its class of steps (``StepContext.even``) has at most and on average."""
+    key = ("single_keys", n_dec)
+    if key not in ctx.work:
+        starts, after = ctx.host.get("req_start"), ctx.host.get("req_len_after")
+        lens = [n for n, lo, hi in zip(after, starts, starts[1:]) if hi - lo == 1] if starts and after else []
+        longest = max(lens, default=max(1, ctx.max_len_after))
+        ctx.work[key] = longest, sum(lens) or int(longest * max(1.0, (0.8 if ctx.even else 0.35) * n_dec))
+    return ctx.work[key]
+
+
 def split_decode(ctx, q, cache_k, cache_v, out, table, scale: float, window: int, *, softcap: float = 0.0, chunk: int = 0) -> bool:
     """A step of single tokens whose softmax weights stay 32-bit, as ``kernels.attn_decode_direct`` with weights in parts; False
-    (and nothing done) for other steps and shapes."""
+    (and nothing done) for other steps and shapes, and where the CUDA cores are faster."""
     T, nq, hd = q.shape
-    if (q.dtype != torch.bfloat16 or cache_v.shape != cache_k.shape or not kernels.attn_decode_direct_supported(nq, cache_k.shape[1], hd)
-            or ctx.dec_tok is None or ctx.n_dec != T):
+    if q.dtype != torch.bfloat16 or cache_v.shape != cache_k.shape or ctx.dec_tok is None or ctx.n_dec != T:
         return False
-    kernels.attn_decode_direct(q, cache_k, cache_v, out, ctx.dec_tok, T, ctx.tok_pos, ctx.tok_req, table, scale, window,
-                               max(1, ctx.max_len_after), ctx.status, two_part=True, softcap=softcap, chunk=chunk)
+    longest, total = single_keys(ctx, T)
+    if not kernels.attn_decode_direct_wins(T, nq, cache_k.shape[1], hd, longest, total, window, chunk=chunk, two_part=True):
+        return False
+    kernels.attn_decode_direct(q, cache_k, cache_v, out, ctx.dec_tok, T, ctx.tok_pos, ctx.tok_req, table, scale, window, longest, ctx.status,
+                               two_part=True, softcap=softcap, chunk=chunk)
     return True
 
 

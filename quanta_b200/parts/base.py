@@ -192,6 +192,7 @@ class StepContext:
     dtype: torch.dtype                 # activation dtype
     max_new_tokens_per_req: int = 0    # largest portion in the step
     max_len_after: int = 0             # largest req_len_after (host copy, for launch sizing)
+    even: bool = True                  # a captured step: whether its requests' lengths are alike (for launch sizing too)
     host: dict = field(default_factory=dict)   # host copies of the small arrays, for parts that need them
     # how the step's tokens fall into requests, for mixers that treat single tokens and portions
     # differently: rows of requests that bring exactly one token, and (request row, first token row,
