@@ -70,18 +70,22 @@ def attn_decode(batch: int, context: int, nq: int, nkv: int, hd: int, page: int)
     tok_req = torch.arange(batch, dtype=torch.int32, device=DEV)
     dec = torch.arange(batch, dtype=torch.int32, device=DEV)
     st = k.new_status(DEV)
+    direct = k.attn_decode_direct_wins(batch, nq, nkv, hd, context, batch * context, 0)      # as parts/attention.py chooses
     n_parts = k.attn_decode_parts(nkv, context)
-    po = torch.empty(batch * nq * n_parts * hd, device=DEV)
-    pml = torch.empty(batch * nq * n_parts * 2, device=DEV)
+    po = torch.empty(0 if direct else batch * nq * n_parts * hd, device=DEV)
+    pml = torch.empty(0 if direct else batch * nq * n_parts * 2, device=DEV)
 
     def step():
         for kc, vc in caches:
-            k.attn_decode(q, kc, vc, out, po, pml, dec, batch, tok_pos, tok_req, table, hd ** -0.5, 0, n_parts, st)
+            if direct:
+                k.attn_decode_direct(q, kc, vc, out, dec, batch, tok_pos, tok_req, table, hd ** -0.5, 0, context, st)
+            else:
+                k.attn_decode(q, kc, vc, out, po, pml, dec, batch, tok_pos, tok_req, table, hd ** -0.5, 0, n_parts, st)
 
     ms = timed_graph(step, reps=2) / layers
     k.raise_on_status(st.cpu())
     gb = batch * context * nkv * hd * 2 * 2 / 1e9
-    return {"kernel": "attn_decode", "batch": batch, "context": context, "q_heads": nq, "kv_heads": nkv,
+    return {"kernel": "attn_decode_direct" if direct else "attn_decode", "batch": batch, "context": context, "q_heads": nq, "kv_heads": nkv,
             "head_dim": hd, "page": page, "layers": layers, "us": round(ms * 1e3, 1), "kv_gb": round(gb, 3),
             "GB/s": round(gb / ms * 1e3, 1)}
 

@@ -156,5 +156,41 @@ def test_weights_hold_24_bits(R, n, window, cap):
     assert st.tolist()[0] == 0 and float((out != want).float().mean()) <= 9e-4
 
 
+@pytest.mark.parametrize("two_part", [False, True])
+@pytest.mark.parametrize("batch,length,page,nq,nkv,window", [(1, 131072, 16, 6, 1, 0), (4, 131072, 16, 6, 1, 0), (2, 9100, 4, 4, 2, 0), (40, 20000, 64, 16, 4, 0),
+                                                           (3, 131072, 16, 8, 1, 70000)])
+def test_long_contexts(batch, length, page, nq, nkv, window, two_part):
+    """Many rounds of the ring, clusters of eight blocks at full length, tables of more than 2,048 pages; one far key carries a row."""
+    kern, hd = K(), 128
+    g = torch.Generator(device=DEV).manual_seed(batch + page)
+    per = -(-length // page)
+    kc = torch.empty(batch * per, nkv, page, hd, device=DEV, dtype=torch.bfloat16).normal_(generator=g)
+    vc = torch.empty(batch * per, nkv, page, hd, device=DEV, dtype=torch.bfloat16).normal_(generator=g)
+    table = torch.randperm(batch * per, generator=torch.Generator().manual_seed(4)).int().view(batch, per)
+    lens = [max(1, length - 37 * r * r) for r in range(batch)]
+    q = torch.randn(batch, nq, hd, device=DEV, generator=g).bfloat16()
+    far = max(0, lens[0] - window) if window else 1
+    page_of, slot = int(table[0, far // page]), far % page
+    kc[page_of, :, slot] = 0
+    kc[page_of, :, slot, 0] = 30.0
+    q[0, : nq // 2, 0] = 8.0
+    pos, req = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV), torch.arange(batch, dtype=torch.int32, device=DEV)
+    table = table.to(DEV)
+    out, st = torch.full_like(q, float("nan")), kern.new_status(DEV)
+    kern.attn_decode_direct(q, kc, vc, out, req, batch, pos, req, table, hd ** -0.5, window, length, st, two_part=two_part)
+    assert st.tolist()[0] == 0
+    for r in {0, batch // 2, batch - 1}:
+        j = torch.arange(max(0, lens[r] - window) if window else 0, lens[r], device=DEV)
+        rows = table[r].long()[j // page]
+        for m in range(nkv):
+            k, v = kc[rows, m, j % page].double(), vc[rows, m, j % page].double()
+            G = nq // nkv
+            w = torch.softmax(q[r, m * G: (m + 1) * G].double() @ k.T * hd ** -0.5, -1)
+            # rounded weights: 2^-9 each, of random sign; their sum in float32
+            tol = 2.0 ** -8 * (w @ v).abs() + (2.0 ** -20 if two_part else 2.0 ** -8 * float(w.pow(2).sum(-1).max().sqrt())) * float(v.abs().max())
+            assert torch.all((out[r, m * G: (m + 1) * G].double() - w @ v).abs() <= tol)
+    assert torch.allclose(out[0, 0].float(), vc[page_of, 0, slot].float(), atol=0.05)
+
+
 def test_sizes_that_are_not_taken():
     assert not K().attn_decode_direct_supported(9, 1, 128) and not K().attn_decode_direct_supported(8, 8, 64)

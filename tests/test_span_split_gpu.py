@@ -72,3 +72,10 @@ def test_which_steps_have_weights_of_16_bits():
         ctx = SimpleNamespace(host={"req_start": starts}, work={})
         tiles = split_span_tiles(ctx, torch.zeros(T, 8, 128, device=DEV, dtype=torch.bfloat16), cache, cache)
         assert (tiles is not None) == taken, lens
+
+
+@pytest.mark.parametrize("page", [4, 16])
+def test_single_tokens_of_long_requests_beside_a_portion(page):
+    """Every single token of a mixed step is a portion of one: contexts of up to 9,300 keys (more than 2,048 pages of 4)."""
+    test_split_spans(16, 4, page, [1, 40, 1, 1, 1], [9299, 3, 127, 4096, 8191], 0, 0, 0.0)
+    test_split_spans(16, 4, page, [1, 40, 1], [9299, 3, 5000], 1000, 0, 30.0)

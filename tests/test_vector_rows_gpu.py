@@ -45,6 +45,37 @@ def test_norm_rows(H, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H", [6136, 6144, 6152, 7176, 8184])
+def test_normed_rows_at_the_end_of_their_registers(H, dtype):
+    """768 threads hold rows of up to 6,144 numbers; longer ones pass through shared memory.  Every summand alone and all together."""
+    h, y, y2 = randn(3, H, seed=1), randn(3, 2, H, seed=2), randn(3, H, seed=3)
+    g, w, b, b2 = 1 + 0.1 * randn(H, seed=4), 1 + 0.1 * randn(H, seed=5), randn(H, seed=6), randn(H, seed=7)
+    for bias, extra, extra_bias in ((None, None, None), (b, None, None), (None, y2, None), (b, y2, b2)):
+        stream, out = h.clone(), torch.empty(3, H, device=DEV, dtype=dtype)
+        K().normed_add_rmsnorm(stream, y, g, 1e-6, w, 1e-5, out, y_scale=0.5, y_bias=bias, extra=extra, extra_scale=2.0, extra_bias=extra_bias)
+        v = y.double().sum(1) + (bias.double() if bias is not None else 0)
+        v = 0.5 * v + (2.0 * (extra.double() + (extra_bias.double() if extra_bias is not None else 0)) if extra is not None else 0)
+        want = h.double() + rms(v, g.double(), 1e-6)
+        near(stream, want, torch.float32)
+        near(out, rms(want, w.double(), 1e-5), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("E,width", [(8, 64), (33, 516), (256, 3072), (5, 4100), (7, 6144), (9, 130)])
+def test_router_logits_depend_on_the_width_alone(E, width, dtype):
+    """Steps of up to 16 tokens and of more run in two kernels with the same additions: a token's logits have the same bits in both."""
+    x, gate = randn(40, width, seed=E).to(dtype), randn(E, width, seed=width)
+    whole = torch.empty(40, E, device=DEV)
+    K().router_small(x, gate, None, whole)
+    want = x.double() @ gate.double().T
+    assert float((whole.double() - want).abs().max()) <= 2.0 ** -20 * float((x.double().abs() @ gate.double().abs().T).max())
+    for lo, hi in ((0, 1), (3, 5), (7, 16), (9, 25), (20, 37)):
+        some = torch.empty(hi - lo, E, device=DEV)      # (a copy: rows that start on 16 bytes, as the whole does)
+        K().router_small(x[lo:hi].clone(), gate, None, some)
+        assert torch.equal(some, whole[lo:hi])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("inner", [7, 8, 12, 2056])
 def test_silu_mul(inner, dtype):
     gu = randn(9, 2 * inner, seed=inner).to(dtype)
