@@ -84,6 +84,15 @@ def test_silu_mul(inner, dtype):
     near(out, torch.nn.functional.silu(gu[:, :inner].double()) * gu[:, inner:].double(), dtype)
 
 
+@pytest.mark.parametrize("rows,inner", [(1, 8), (65, 8), (70000, 16), (8193, 64), (300, 504), (2100, 512), (513, 2048), (3, 2064)])
+def test_silu_mul_of_many_short_rows(rows, inner):
+    """Short rows lie several to a block, on both sides of a million numbers and past the grid's 32,768 rows of blocks."""
+    gu = randn(rows, 2 * inner, seed=inner)
+    out = torch.full((rows, inner), float("nan"), device=DEV)
+    K().silu_mul(gu, out)
+    near(out, torch.nn.functional.silu(gu[:, :inner].double()) * gu[:, inner:].double(), torch.float32)
+
+
 @pytest.mark.parametrize("gate", ["sigmoid", "silu"])
 @pytest.mark.parametrize("heads,dim,off,shared", [(3, 4, 0, False), (5, 64, 8, True), (33, 8, 4, False), (2, 128, 0, True), (3, 12, 0, False),
                                                   (3, 64, 3, True), (2, 256, 0, False)])
@@ -133,3 +142,4 @@ def test_attention_of_few_tokens(nq, nkv, hd, vd, window, n_split, dtype):
         # float32: some 700 terms; the exponents carry a few roundings of scores up to 10
         tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -17
         assert float((out[t].double() - want).abs().max()) <= tol * float(v.abs().max())
+
