@@ -2,7 +2,8 @@
 //
 // Bound by the bytes of W.  Measured on a B200 (weights from HBM) beside the library's float32 product of as many rows: 4 rows of
 // 2,048 x 3,072 8.4 us against 39 (52 with the spare rows of a bfloat16 step), x 32,000 53 against 79 (4.9 TB/s), 16 rows of 3,072 x 8,192
-// 61 against 78; above 16 rows the products of one input no longer fit a warp's registers and the library's tiles win.
+// 61 against 78; above 16 rows the products of one input no longer fit a warp's registers and the library's tiles win, and above eight of
+// more than 8,192 numbers, which are not copied to shared memory (16 rows of 16,384 x 512: 110 us, the library 97).
 #include "rows_f32.cuh"
 
 constexpr int LR_WARPS = 4;

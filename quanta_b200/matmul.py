@@ -63,7 +63,7 @@ def _few_float32_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype |
     if torch.is_grad_enabled() and (x.requires_grad or w.requires_grad):
         return False
     return (x.is_cuda and w.device == x.device and x.device.index == torch.cuda.current_device() and x.dim() == 2 and w.dim() == 2
-            and 0 < x.shape[0] <= kernels.LINEAR_ROWS_MAX and x.shape[1] == w.shape[1] and x.shape[1] > 0 and x.shape[1] % 4 == 0
+            and 0 < x.shape[0] <= (kernels.LINEAR_ROWS_MAX if x.shape[1] <= 8192 else 8) and x.shape[1] == w.shape[1] and x.shape[1] > 0 and x.shape[1] % 4 == 0
             and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 

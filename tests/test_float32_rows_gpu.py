@@ -40,7 +40,7 @@ def test_linear_takes_the_library_where_rows_do_not_fit():
     w = torch.randn(9, 150, device=DEV)
     flat = torch.randn(4 * 128 + 1, device=DEV)
     for x, ww in ((wide[:, :150], w), (wide[:, :148], w[:, :148]), (flat[1:].view(4, 128), torch.randn(5, 128, device=DEV)),
-                  (torch.randn(17, 64, device=DEV), torch.randn(5, 64, device=DEV))):
+                  (torch.randn(17, 64, device=DEV), torch.randn(5, 64, device=DEV)), (torch.randn(9, 8196, device=DEV), torch.randn(5, 8196, device=DEV))):
         want = x.double() @ ww.double().T
         assert torch.all((linear(x, ww).double() - want).abs() <= 2 * x.shape[1] * U * (x.double().abs() @ ww.double().abs().T))
 
