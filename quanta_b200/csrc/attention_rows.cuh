@@ -200,9 +200,28 @@ static bool rows_attention_takes(int nq, int nkv, int hd, int vd, const void* q,
          (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) == 0;
 }
 
+// q heads a block of the kernel.
+static int rows_attention_heads(int nq, int nkv) {
+  const int per_kv = nq / nkv;
+  return per_kv % 4 == 0 ? 4 : per_kv % 2 == 0 ? 2 : 1;
+}
+
+// Whether the kernel is faster than the one that gives a range of a token's keys to a warp for all q heads of a kv head.  A turn of 64 keys takes
+// a block 2.6 us whatever the head size and the number of its q heads, so few blocks are always faster here, many where the rows are
+// long and shared.  Measured on a B200 (ranges of the keys / here, us): 16 + 4 heads of 128, bfloat16, windows of 512, 16 tokens 25 / 17, 1,000 406 / 282;
+// 8 + 8 of 64, 16 tokens 20 / 19, 1,000 301 / 459; 6 + 2 of 128, 64 tokens 1.4 times slower here; 16 + 4 of 16, float32, 1,000 tokens 154 / 303;
+// 12 + 2 of 256, 64 tokens 142 / 249; 8 + 2 of 80, float32, 64 tokens 1.4 times slower, bfloat16 0.8.
+static bool rows_attention_wins(bool f32, int T, int nq, int nkv, int hd) {
+  const int GH = rows_attention_heads(nq, nkv);
+  const long blocks = (long)T * nq / GH;
+  if (blocks <= 64) return true;
+  if (f32) return (GH == 4 && hd >= 64 && hd < 80 && blocks <= 1024) || (hd >= 112 && (GH > 1 || nq == nkv) && (hd <= 128 || GH == 4));
+  return GH == 4 && (hd >= 80 || (hd >= 64 && blocks <= 256));
+}
+
 template <typename A>
 static int rows_attention(const A* q, const A* k, const A* v, A* out, const RowsAttention& P, cudaStream_t stream) {
-  const int per_kv = P.nq / P.nkv, GH = per_kv % 4 == 0 ? 4 : per_kv % 2 == 0 ? 2 : 1, NV = P.hd > 128 || P.vd > 128 ? 2 : 1;
+  const int GH = rows_attention_heads(P.nq, P.nkv), NV = P.hd > 128 || P.vd > 128 ? 2 : 1;
   const long blocks = (long)P.T * P.nq / GH * P.n_split;
   if (blocks > 0x7fffffffL) return QB_ERR_UNSUPPORTED;
   const size_t smem = (size_t)ATS_WARPS * GH * P.vd * sizeof(float);            // at most 32 KB

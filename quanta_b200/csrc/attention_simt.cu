@@ -11,7 +11,8 @@
 // Keys (and queries) have `hd` elements a head, values and outputs `vd`; any positive sizes up to 256 (rows
 // whose size is no multiple of the 16-byte vector are read element by element).
 //
-// Two kernels.  Head sizes that are multiples of 4: attention_rows.cuh.  Other sizes: one warp per (token, q head): lanes own keys for the scores, then own dims for P V.
+// Two kernels.  Head sizes that are multiples of 4: attention_rows.cuh (but see the launch).  Others: one warp per (token, q head): lanes
+// own keys for the scores, then own dims for P V.
 #include "attention_rows.cuh"
 
 template <typename A> struct Vec16;
@@ -128,7 +129,11 @@ extern "C" int qb_paged_attention_simt(const void* q, int dtype, const void* k_c
                                        cudaStream_t stream) {
   if (T <= 0) return 0;
   if (hd <= 0 || vd <= 0 || hd > ATT_MAX_HD || vd > ATT_MAX_HD || nq % nkv || page_size <= 0) return QB_ERR_UNSUPPORTED;
-  if (rows_attention_takes(nq, nkv, hd, vd, q, k_cache, v_cache, out)) {
+  // the kernel below where it fills the SMs and the other's lanes are idle or its rows long: bfloat16, 1,000 tokens, 8 + 8 heads of 64 with a
+  // window of 512 405 us and 460 by rows (without one 652 and 613), 5 + 5 of 36 216 and 262, 12 + 2 of 256 1,432 and 1,578
+  const int heads = rows_attention_heads(nq, nkv);
+  const bool below = dtype == QB_BF16 && (long)T * nq >= 4096 && ((heads == 1 && hd <= 64 && window > 0) || (heads < 4 && hd > 128));
+  if (!below && rows_attention_takes(nq, nkv, hd, vd, q, k_cache, v_cache, out)) {
     const RowsAttention P{tok_pos, tok_req, block_table, bt_stride, T, nq, nkv, hd, vd, page_size, num_pages, scale, 0.f, window, 0,
                           nullptr, nullptr, 1, nullptr, status};
     QB_DISPATCH_DTYPE(dtype, A, return rows_attention<A>((const A*)q, (const A*)k_cache, (const A*)v_cache, (A*)out, P, stream));

@@ -418,13 +418,19 @@ talk_mix_kernel(const float* __restrict__ scratch, const float* __restrict__ tal
   }
 }
 
+// Whether a step's attention without pooled blocks and mixed heads runs as attention_rows.cuh has it, rather than in ranges of keys a warp.
+extern "C" int qb_window_attention_by_rows(int dtype, int T, int nq, int nkv, int hd, int vd) {
+  return nkv > 0 && nq % nkv == 0 && hd % 4 == 0 && vd % 4 == 0 && rows_attention_wins(dtype == QB_F32, T, nq, nkv, hd > vd ? hd : vd) ? 1 : 0;
+}
+
+// rows: 0 keeps attention_rows.cuh out.
 extern "C" int qb_window_attention(const void* q, int dtype, const void* k_cache, const void* v_cache,
                                    const void* kp_cache, const void* vp_cache, void* out, float* scratch,
                                    const float* talk, const int* tok_pos, const int* tok_req, const int* block_table,
                                    int bt_stride, const int* pool_table, int pool_stride, int T, int nq, int nkv,
                                    int hd, int vd, int page_size, int num_pages, int num_pool_pages, float scale,
                                    float cap, int window, int pool, int chunk, const float* dist_bias, const float* sink,
-                                   float* part, int n_split, int* status, cudaStream_t stream) {
+                                   float* part, int n_split, int rows, int* status, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (n_split < 1 || (n_split > 1 && part == nullptr)) return QB_ERR_BAD_ARG;
   if (hd <= 0 || vd <= 0 || hd > WA_MAX_HD || vd > WA_MAX_HD || nq % nkv || page_size <= 0) return QB_ERR_UNSUPPORTED;
@@ -440,7 +446,7 @@ extern "C" int qb_window_attention(const void* q, int dtype, const void* k_cache
   P.vec = (hd % 8 == 0 && ((uintptr_t)k_cache & 15) == 0 && (kp_cache == nullptr || ((uintptr_t)kp_cache & 15) == 0)) ? 1 : 0;
   P.n_split = n_split; P.part = part;
   const int nv = (vd + 31) / 32;
-  const bool by_rows = talk == nullptr && pool_table == nullptr && rows_attention_takes(nq, nkv, hd, vd, q, k_cache, v_cache, out);
+  const bool by_rows = rows && talk == nullptr && pool_table == nullptr && rows_attention_takes(nq, nkv, hd, vd, q, k_cache, v_cache, out);
   if (by_rows) {
     const RowsAttention R{tok_pos, tok_req, block_table, bt_stride, T, nq, nkv, hd, vd, page_size, num_pages, scale, cap, window, chunk,
                           dist_bias, sink, n_split, part, status};

@@ -966,10 +966,16 @@ def window_attention_uses_tensor_cores(dtype, hd: int, vd: int) -> bool:
     return dtype == torch.bfloat16 and bool(lib().qb_window_attention_mma_supported(BF16, int(hd), int(vd)))
 
 
+def window_attention_by_rows(dtype, T: int, nq: int, nkv: int, hd: int, vd: int) -> bool:
+    """Whether ``window_attention`` without pooled blocks and mixed heads is faster with a block a (token, up to four q heads of a kv head)
+    than with a warp a range of a token's keys."""
+    return bool(lib().qb_window_attention_by_rows(F32 if dtype == torch.float32 else BF16, int(T), int(nq), int(nkv), int(hd), int(vd)))
+
+
 def window_attention(q, k_cache, v_cache, out, tok_pos, tok_req, block_table, scale: float, window: int, status, *,
                      dist_bias=None, sink=None, softcap: float = 0.0, pool: int = 0, pooled_k=None, pooled_v=None,
                      pool_table=None, talk=None, scratch=None, n_split: int | None = None, n_requests: int | None = None,
-                     tensor_cores: bool | None = None, chunk: int = 0) -> None:
+                     tensor_cores: bool | None = None, chunk: int = 0, by_rows: bool | None = None) -> None:
     """Softmax attention of every token over the last ``window`` keys of its request (0: all of them); ``chunk`` C > 0:
     over the keys of its own chunk of C positions (counted from the request's first) only.  Options:
     ``dist_bias`` float32 ``[window, heads]`` added to the score by distance; ``sink`` float32 ``[heads]``, a term
@@ -978,7 +984,8 @@ def window_attention(q, k_cache, v_cache, out, tok_pos, tok_req, block_table, sc
     ``talk`` float32 ``[heads, heads]``: the heads' softmax weights are mixed, ``w'_h = sum_g talk[h, g] w_g``
     (``scratch`` float32 ``[T, heads, kv heads, vd]``).  float32 arithmetic; q, caches and out in one dtype.
     A step of few tokens (single tokens of a few requests) cuts every token's keys into ``n_split`` ranges that
-    run as warps of their own and are joined by a second launch (None: chosen from the step's size).
+    run as warps of their own and are joined by a second launch (None: chosen from the step's size).  ``by_rows``: as in
+    ``window_attention_by_rows`` (None: chosen too).
     A step with long portions (``n_requests`` given, at least 32 tokens and 8 a request on average) of shapes that
     ``window_attention_uses_tensor_cores`` takes runs scores and sums on the tensor cores; ``tensor_cores`` True
     forces that path (and raises where it cannot run), False keeps the CUDA cores."""
@@ -1018,7 +1025,11 @@ def window_attention(q, k_cache, v_cache, out, tok_pos, tok_req, block_table, sc
             ctypes.c_float(scale), ctypes.c_float(softcap), int(window), int(pool), int(chunk), _p(dist_bias), _p(sink), _p(status),
             _stream()), "window_attention_mma", 1 + (talk is not None))
         return
-    if n_split is None and talk is None and pool_table is None and hd % 4 == 0 and vd % 4 == 0:
+    if by_rows is None:
+        # without a window the other kernel is one that does not cut the keys
+        by_rows = talk is None and pool_table is None and hd % 4 == 0 and vd % 4 == 0 and (
+            n_split is not None or window <= 0 or window_attention_by_rows(q.dtype, T, nq, nkv, hd, vd))
+    if n_split is None and by_rows:
         # eight warps a (token, kv head, four q heads, range), 64 keys of it a turn of 2.6 us (a look-up and a read of memory): ranges of
         # 256 keys while that fills the SMs eight warps deep; joining them is a launch of 7 us
         keys = min((n for n in (window, chunk, block_table.shape[1] * page_size) if n > 0), default=1)
@@ -1035,7 +1046,7 @@ def window_attention(q, k_cache, v_cache, out, tok_pos, tok_req, block_table, sc
         _p(tok_pos), _p(tok_req), _p(block_table), block_table.shape[1], _p(pool_table),
         pool_table.shape[1] if pool_table is not None else 0, T, nq, nkv, hd, vd, page_size, num_pages, n_pool_pages,
         ctypes.c_float(scale), ctypes.c_float(softcap), int(window), int(pool), int(chunk), _p(dist_bias), _p(sink), _p(part),
-        int(n_split), _p(status), _stream()), "window_attention", 1 + (talk is not None) + (n_split > 1))
+        int(n_split), int(by_rows), _p(status), _stream()), "window_attention", 1 + (talk is not None) + (n_split > 1))
 
 
 def pool_blocks(k_cache, v_cache, pooled_k, pooled_v, tok_pos, tok_req, block_table, pool_table, pool: int, status) -> None:

@@ -210,14 +210,14 @@ class GQAttention(Mixer):
             if split_decode(ctx, q, cache.k, cache.v, out, cache.block_table, self.scale, window, chunk=self.chunk or 0):
                 return
             R = int(ctx.req_start.numel()) - 1
-            n_split = None
-            if self.hd % 4 or self.vd % 4:
+            n_split, by_rows = None, kernels.window_attention_by_rows(q.dtype, q.shape[0], self.nq, self.nkv, self.hd, self.vd)
+            if not by_rows:
                 # about 2,048 warps in all, at least 32 keys a range
                 warps = max(1, q.shape[0] * self.nkv)
                 keys = max(1, min(ctx.max_len_after, self.chunk or self.window or ctx.max_len_after))
                 n_split = max(1, min(-(-2048 // warps), -(-keys // 32), 256))
             kernels.window_attention(q, cache.k, cache.v, out, ctx.tok_pos, ctx.tok_req, cache.block_table, self.scale,
-                                     window, ctx.status, n_split=n_split, n_requests=R, chunk=self.chunk or 0)
+                                     window, ctx.status, n_split=n_split, n_requests=R, chunk=self.chunk or 0, by_rows=by_rows)
             return
         if q.dtype != torch.bfloat16 or not self.mma_shapes:
             kernels.paged_attention_simt(q, cache.k, cache.v, out, ctx.tok_pos, ctx.tok_req, cache.block_table,

@@ -3,6 +3,7 @@ shared by all blocks in the other, so the mix of lengths decides.  Rules of size
 from __future__ import annotations
 
 import pytest
+import torch
 
 from quanta_b200 import kernels as k
 from quanta_b200.engine.step import Engine
@@ -38,3 +39,14 @@ def test_captured_steps():
     assert key([5000] * 4) == (4, 8192) and key([5000, 4000, 2000, 1500]) == (4, 8192)
     assert key([5000, 300, 300, 300]) == (4, 8192, "uneven") and key([9000, 100]) == (2, 16384, "uneven")
     assert key([9000], 4) == (4, 16384)                                    # lengths that are not known
+
+
+def test_a_block_or_a_warp_a_range_of_keys():
+    rows = lambda dtype, T, nq, nkv, hd, vd=None: k.window_attention_by_rows(dtype, T, nq, nkv, hd, vd or hd)
+    for dtype in (torch.float32, torch.bfloat16):
+        for nq, nkv, hd in ((16, 4, 128), (8, 8, 64), (6, 2, 128), (5, 5, 36), (12, 2, 256), (16, 4, 16)):
+            assert rows(dtype, 1, nq, nkv, hd)                             # few blocks
+        assert rows(dtype, 4096, 16, 4, 128) and rows(dtype, 64, 16, 4, 64)
+        for nq, nkv, hd in ((5, 5, 36), (12, 2, 256), (16, 4, 16), (16, 4, 32), (6, 2, 128), (8, 8, 64), (6, 1, 64)):
+            assert not rows(dtype, 1000, nq, nkv, hd)
+        assert not rows(dtype, 1, 4, 2, 50) and not rows(dtype, 1, 4, 2, 64, 66) and not rows(dtype, 1, 5, 2, 64)

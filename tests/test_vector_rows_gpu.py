@@ -143,3 +143,24 @@ def test_attention_of_few_tokens(nq, nkv, hd, vd, window, n_split, dtype):
         tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -17
         assert float((out[t].double() - want).abs().max()) <= tol * float(v.abs().max())
 
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,nkv,hd,T,window,chunk", [(8, 8, 64, 40, 100, 0), (6, 2, 128, 70, 0, 96), (16, 4, 16, 33, 50, 0), (12, 2, 256, 24, 300, 0)])
+def test_a_block_or_a_warp_a_range(nq, nkv, hd, T, window, chunk, dtype):
+    """Steps that either kernel may take (the choice is by speed): both within float32 sums of one another, each range cut or not."""
+    kern, page = K(), 16
+    per = -(-400 // page)
+    kc, vc = randn(T * per, nkv, page, hd, seed=1).to(dtype), randn(T * per, nkv, page, hd, seed=2).to(dtype)
+    table = torch.arange(T * per, dtype=torch.int32, device=DEV).view(T, per)
+    pos = torch.arange(400 - T, 400, dtype=torch.int32, device=DEV)
+    req = torch.arange(T, dtype=torch.int32, device=DEV)
+    q, outs = randn(T, nq, hd, seed=3).to(dtype), []
+    for by_rows, n_split in ((True, None), (True, 3), (False, None), (False, 5)):
+        out, st = torch.full_like(q, float("nan")), kern.new_status(DEV)
+        kern.window_attention(q, kc, vc, out, pos, req, table, hd ** -0.5, window, st, chunk=chunk, n_split=n_split, by_rows=by_rows,
+                              tensor_cores=False)
+        assert st.tolist()[0] == 0
+        outs.append(out.double())
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -18
+    for out in outs[1:]:
+        assert float((out - outs[0]).abs().max()) <= tol * float(vc.double().abs().max())
