@@ -185,13 +185,6 @@ struct TcsReach {
     return window > 0 && p - window + 1 > 0 ? p - window + 1 : 0;
   }
 };
-// cap * tanh(x / cap) as cap - 2 cap / (2^(x * two_over) + 1), two_over = 2 log2(e) / cap, times log2(e)
-__device__ __forceinline__ float tcs_cap(float x, float cap_log2, float two_over) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * two_over));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e + 1.f));
-  return fmaf(-2.f * cap_log2, r, cap_log2);
-}
 __device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
   const __nv_bfloat162 l = __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
@@ -390,7 +383,8 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const bool valid = r < n_rows;
     const int pos_r = valid ? tok_pos[tok0 + R / G] : -1;
     const int lo_r = valid ? reach.lo(pos_r) : 0;
-    const float cap_log2 = cap * 1.4426950408889634f, cap_mul = CAP ? scale_log2 * 2.f / cap : 0.f;   // (score / cap) 2 log2(e)
+    // tanhf, which keeps the relative accuracy of a score near zero; 1 - 2 / (e^2x + 1) loses it to the difference, more the larger the cap
+    const float cap_log2 = cap * 1.4426950408889634f, over_cap = CAP ? scale_log2 * 0.6931471805599453f / cap : 0.f;
     const float mul = CAP ? 1.f : scale_log2;                                 // from what the registers hold to log2 of a weight
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
     const uint32_t o_addr = lane_addr + o_col + (uint32_t)(half * 64);       // this thread's 64 columns of O
@@ -419,8 +413,8 @@ attn_span_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       if (CAP) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          va[i] = __float_as_uint(tcs_cap(__uint_as_float(va[i]), cap_log2, cap_mul));
-          vb[i] = __float_as_uint(tcs_cap(__uint_as_float(vb[i]), cap_log2, cap_mul));
+          va[i] = __float_as_uint(cap_log2 * tanhf(__uint_as_float(va[i]) * over_cap));
+          vb[i] = __float_as_uint(cap_log2 * tanhf(__uint_as_float(vb[i]) * over_cap));
         }
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};

@@ -61,6 +61,28 @@ def test_split_spans(nq, nkv, page, lens, cached, window, chunk, cap):
         t0 += n
 
 
+@pytest.mark.parametrize("cap", [5.0, 50.0, 1000.0])
+def test_capped_scores_keep_their_accuracy(cap):
+    """A cap of any size costs the weights nothing: an output (of unit values' averages) is off by less than the bits of its weights, so few
+    come out as another bfloat16 than the one nearest the exact value.  A relative error e of an output moves a share of about e / 2^-8 of
+    roundings: 2^-16 of weights and scores together 0.4 %, scores off by some 2e-4 (a difference that cancels, at a cap of 1,000) 3 %."""
+    from quanta_b200 import kernels
+    T, nq, nkv, hd, page, scale = 256, 4, 2, 128, 16, 128 ** -0.5
+    g = torch.Generator(device=DEV).manual_seed(11)
+    q = torch.randn(T, nq, hd, device=DEV, generator=g).bfloat16()
+    kc, vc = (torch.randn(T // page, nkv, page, hd, device=DEV, generator=g).bfloat16() for _ in range(2))
+    table = torch.arange(T // page, device=DEV, dtype=torch.int32)[None]
+    tiles = torch.tensor([[0, 0, T, r] for r in range(0, T * nq // nkv, kernels.attn_span_tc_rows())], dtype=torch.int32, device=DEV)
+    out, st = torch.empty_like(q), kernels.new_status(DEV)
+    kernels.attn_span_split(q, kc, vc, out, torch.arange(T, device=DEV, dtype=torch.int32), table, tiles, scale, 0, st, softcap=cap)
+    assert st.tolist()[0] == 0
+    k, v = (t.transpose(1, 2).reshape(T, nkv, hd).repeat_interleave(nq // nkv, 1).double() for t in (kc, vc))
+    s = cap * torch.tanh(torch.einsum("thd,jhd->htj", q.double(), k) * scale / cap)
+    s = s.masked_fill(torch.ones(T, T, device=DEV, dtype=torch.bool).triu(1), float("-inf"))
+    want = torch.einsum("htj,jhd->thd", torch.softmax(s, -1), v).bfloat16()
+    assert float((out != want).float().mean()) < 0.008
+
+
 def test_which_steps_have_weights_of_16_bits():
     """The steps that kernels.window_attention gives to the tensor cores: at least 32 tokens and eight a request; no others."""
     from types import SimpleNamespace
