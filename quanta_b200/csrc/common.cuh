@@ -36,7 +36,7 @@
 // A kernel launched with qb_launch may have its blocks placed while the launch before it on the stream still runs.  Its first statement,
 // qb_follow(), waits until that launch has ended and its writes are seen, and only then lets the launch after it be placed; so whatever
 // was enqueued two launches before has ended too, and the order on the stream is what it was.  What it saves is the gap between
-// two launches (a step of one token has 42, a step of 8 tokens of the model with a delta rule 68).  All threads of all blocks call it, whatever they do next.
+// two launches, which a step of few tokens has after each of its launches.  All threads of all blocks call it, whatever they do next.
 __device__ __forceinline__ void qb_follow() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -23,7 +23,7 @@ __host__ __device__ __forceinline__ int qb_rows_smem(int rows, int K) {       //
   return n <= QB_ROWS_SMEM ? (int)n : 0;
 }
 
-// Starts the copy of `rows` rows (row r at src(r)) by all threads of the block; QbRowsReady waits for it.
+// Starts the copy of `rows` rows (row r at src(r)) by all threads of the block; qb_rows_ready waits for it.
 template <typename Src>
 __device__ __forceinline__ void qb_rows_copy(float* dst, Src src, int rows, int K) {
   const int pieces = K >> 2;
