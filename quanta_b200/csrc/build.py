@@ -31,7 +31,7 @@ from pathlib import Path
 SRC_DIR = Path(__file__).resolve().parent
 # unit -> its sources.  A file that calls into another one is in the same unit.
 UNITS = {
-    "core": ["norm_embed.cu", "grouped_norm.cu", "sampling.cu", "linear_rows.cu"],
+    "core": ["norm_embed.cu", "grouped_norm.cu", "sampling.cu", "linear_rows.cu", "linear_few.cu"],
     "rope": ["rope_cache.cu"],
     "attention": ["attention_simt.cu", "attention_mma.cu", "attention_tc.cu", "attention_decode.cu"],
     "experts": ["moe.cu", "router_gemm_mma.cu", "expert_gemm_tc.cu"],

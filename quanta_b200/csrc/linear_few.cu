@@ -1,0 +1,153 @@
+// out[r] = x[r] W^T for a few bfloat16 rows: the projections, dense feed-forwards and output matrices of a step that decodes.
+//
+// Bound by the bytes of W.  A block takes 16 rows of W, its eight warps 64 numbers of the inner dimension in turn.  A lane loads the 16
+// numbers of a row's 128 bytes that it then multiplies (the order of the inner dimension inside an mma is free as long as both operands
+// have it), 32 bytes a load, so that weights go from memory to registers without shared memory or a barrier: up to 128 KB on
+// their way an SM, of which 45 keep the memory busy.  Between the launches of a step the library's kernels wait for the launch before
+// them and then for their first weights; here the first pieces are asked for before that wait (`early`), and the products
+// follow the arrival of x.  x is read by every block, out of L1 after the SM's first.  A row's sums are taken in an order that depends on K alone.
+//
+// Measured on a B200, one product after another in a graph, weights from memory, microseconds (library: at 32 rows, its fastest kernel):
+//   [N, K]            bytes at 6.5 TB/s   library   8 rows   16 rows   32 rows
+//   8,192 x 3,072            7.7            11.4      9.1      10.8      14.6
+//   3,072 x 6,144            5.8            11.2      7.7       8.8      13.0
+//   32,000 x 2,048          20.0            27.0     21.3      24.7      36.1
+//   2,048 x 5,632            3.5             9.9      6.2       7.5       8.2
+//   2,048 x 2,048            1.3             5.5      2.2       2.8       3.6
+//   3,072 x 768              0.7             4.2      1.8       2.0       2.6
+// Above 16 rows the reads of x outweigh those of W where several blocks follow one another on an SM: there the kernel takes matrices
+// of one block an SM at most (four pieces ahead) and small ones, the library the others; above 32 rows, the library all of them.
+#include "common.cuh"
+
+constexpr int LF_WARPS = 8;
+constexpr int LF_KB = 64;                // numbers of the inner dimension a warp takes at a time: 128 bytes of each row of W
+
+struct LinearFew {
+  const __nv_bfloat16 *x, *w;
+  void* out;
+  int rows, K, N;
+};
+
+struct alignas(32) LfPiece {
+  uint32_t u[8];
+};
+
+__device__ __forceinline__ LfPiece lf_stream(const __nv_bfloat16* p) {       // read once: not kept in L1
+  LfPiece v;
+  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v.u[0]), "=r"(v.u[1]), "=r"(v.u[2]), "=r"(v.u[3]), "=r"(v.u[4]), "=r"(v.u[5]), "=r"(v.u[6]), "=r"(v.u[7])
+               : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ LfPiece lf_load(const __nv_bfloat16* p) {
+  LfPiece v;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v.u[0]), "=r"(v.u[1]), "=r"(v.u[2]), "=r"(v.u[3]), "=r"(v.u[4]), "=r"(v.u[5]), "=r"(v.u[6]), "=r"(v.u[7])
+               : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ void lf_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// NT: tiles of 8 input rows.  D, XD: pieces of W and of x a warp holds ahead.
+template <int NT, int D, int XD, int MINB, typename O>
+__global__ void __launch_bounds__(LF_WARPS * 32, MINB) linear_few_kernel(LinearFew a, int early) {
+  static_assert(D % XD == 0, "the ring of x divides the ring of W");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * 16;
+  const int kbs = (a.K + LF_KB - 1) / LF_KB;
+  const __nv_bfloat16* wr[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) wr[h] = a.w + (size_t)min(n0 + h * 8 + g, a.N - 1) * a.K + t * 16;
+  const __nv_bfloat16* xr[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) xr[n] = a.x + (size_t)min(n * 8 + g, a.rows - 1) * a.K + t * 16;
+  const LfPiece none = {};
+  LfPiece wb[D][2], xb[XD][NT];
+  auto fetch_w = [&](int kb, LfPiece (&b)[2]) {
+    const bool in = kb < kbs && kb * LF_KB + t * 16 < a.K;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) b[h] = in ? lf_stream(wr[h] + kb * LF_KB) : none;
+  };
+  auto fetch_x = [&](int kb, LfPiece (&b)[NT]) {
+    const bool in = kb < kbs && kb * LF_KB + t * 16 < a.K;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) b[n] = in ? lf_load(xr[n] + kb * LF_KB) : none;
+  };
+  if (!early) qb_follow();
+#pragma unroll
+  for (int d = 0; d < D; ++d) fetch_w(warp + d * LF_WARPS, wb[d]);
+  if (early) qb_follow();
+#pragma unroll
+  for (int d = 0; d < XD; ++d) fetch_x(warp + d * LF_WARPS, xb[d]);
+  float acc[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+  for (int k0 = warp; k0 < kbs; k0 += D * LF_WARPS) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const int kb = k0 + d * LF_WARPS;
+      if (kb >= kbs) break;
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+          lf_mma(acc[n], wb[d][0].u[2 * s], wb[d][1].u[2 * s], wb[d][0].u[2 * s + 1], wb[d][1].u[2 * s + 1],
+                 xb[d % XD][n].u[2 * s], xb[d % XD][n].u[2 * s + 1]);
+      fetch_w(kb + D * LF_WARPS, wb[d]);
+      fetch_x(kb + XD * LF_WARPS, xb[d % XD]);
+    }
+  }
+  // the warps' parts, added in the order of the warps
+  constexpr int ROWS = 16, PAD = ROWS + 4, TOK = NT * 8;
+  __shared__ float part[LF_WARPS][TOK][PAD];
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) part[warp][n * 8 + 2 * t + (i & 1)][g + 8 * (i >> 1)] = acc[n][i];
+  __syncthreads();
+  for (int v = threadIdx.x; v < TOK * ROWS; v += LF_WARPS * 32) {
+    const int tok = v / ROWS, row = v % ROWS;
+    if (tok >= a.rows || n0 + row >= a.N) continue;
+    float s = part[0][tok][row];
+#pragma unroll
+    for (int w = 1; w < LF_WARPS; ++w) s += part[w][tok][row];
+    reinterpret_cast<O*>(a.out)[(size_t)tok * a.N + n0 + row] = qb_from_float<O>(s);
+  }
+}
+
+template <int NT, int D, int XD, int MINB>
+static int linear_few_launch(const LinearFew& a, int out_dtype, int early, cudaStream_t stream) {
+  const int grid = (a.N + 15) / 16;
+  QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(linear_few_kernel<NT, D, XD, MINB, O>, grid, LF_WARPS * 32, 0, stream, a, early));
+  QB_LAUNCH_CHECK();
+  return 0;
+}
+
+// Whether the kernel is the faster way for `rows` rows of [N, K]: the rule of qb_linear_few.
+static bool linear_few_small(int K, int N) { return (N + 15) / 16 <= 148 || (long long)K * N <= 4 << 20; }
+
+extern "C" int qb_linear_few_takes(int rows, int K, int N) {
+  return rows > 0 && rows <= 32 && K >= LF_KB && K % 16 == 0 && N > 0 && (rows <= 16 || linear_few_small(K, N));
+}
+
+// K a multiple of 16; x and w on 32 bytes.  early: W was written two launches before this one at the latest (or by the host), so that
+// its first pieces are read before the launch before this one has ended.
+extern "C" int qb_linear_few(const void* x, const void* w, void* out, int out_dtype, int rows, int K, int N, int early,
+                             cudaStream_t stream) {
+  if (rows <= 0 || N <= 0) return 0;
+  if (K <= 0 || K % 16 || ((uintptr_t)x & 31) || ((uintptr_t)w & 31)) return QB_ERR_BAD_ARG;
+  if (rows > 32) return QB_ERR_UNSUPPORTED;
+  const LinearFew a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, rows, K, N};
+  if (rows <= 8) return linear_few_launch<1, 4, 4, 2>(a, out_dtype, early, stream);
+  if (rows <= 16) return linear_few_launch<2, 4, 2, 2>(a, out_dtype, early, stream);
+  if ((N + 15) / 16 <= 148) return linear_few_launch<4, 4, 2, 1>(a, out_dtype, early, stream);
+  return linear_few_launch<4, 2, 1, 2>(a, out_dtype, early, stream);
+}

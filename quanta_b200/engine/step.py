@@ -253,7 +253,7 @@ class Engine:
             req_start=d_start, req_len_after=d_len, status=self.status, dtype=self.model.dtype,
             max_new_tokens_per_req=max_new, max_len_after=max_len_after, even=even,
             host={k: info[k] for k in ("req_start", "req_len_after", "req_slot")} if with_host else {},
-            dec_tok=d_dec if info["n_dec"] else None, n_dec=info["n_dec"], spans=info["spans"])
+            dec_tok=d_dec if info["n_dec"] else None, n_dec=info["n_dec"], spans=info["spans"], settled=True)
         caches = []
         for pos, entry in enumerate(self.model.schedule):
             src = pos if entry.read_cache_of is None else entry.read_cache_of

@@ -48,12 +48,9 @@ def _with_spare_rows(x: torch.Tensor) -> torch.Tensor:
     return x
 
 
-def _few_float32_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None) -> bool:
-    """Whether ``kernels.linear_rows`` takes the product: a few float32 rows, bound by the bytes of ``w``, on the current device.  What
-    torch does with its own product besides computing it (gradients, forward mode, vmap, autocast, tracing, the errors of operands that
-    do not fit) stays with torch."""
-    if x.dtype != torch.float32 or w.dtype != torch.float32 or out_dtype not in (None, torch.float32):
-        return False
+def _plain(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether nothing hangs on the product besides its numbers, on the current device.  What torch does with its own product besides
+    computing it (gradients, forward mode, vmap, autocast, tracing, the errors of operands that do not fit) stays with torch."""
     if type(x) is not torch.Tensor or type(w) not in (torch.Tensor, torch.nn.Parameter) or _get_current_dispatch_mode() is not None:
         return False
     if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch.is_autocast_enabled("cuda") or forward_ad._current_level >= 0:
@@ -63,22 +60,42 @@ def _few_float32_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype |
     if torch.is_grad_enabled() and (x.requires_grad or w.requires_grad):
         return False
     return (x.is_cuda and w.device == x.device and x.device.index == torch.cuda.current_device() and x.dim() == 2 and w.dim() == 2
-            and 0 < x.shape[0] <= (kernels.LINEAR_ROWS_MAX if x.shape[1] <= 8192 else 8) and x.shape[1] == w.shape[1] and x.shape[1] > 0 and x.shape[1] % 4 == 0
-            and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+            and x.shape[1] == w.shape[1] and x.is_contiguous() and w.is_contiguous())
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
+def _few_float32_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None) -> bool:
+    """Whether ``kernels.linear_rows`` takes the product: a few float32 rows, bound by the bytes of ``w``."""
+    if x.dtype != torch.float32 or w.dtype != torch.float32 or out_dtype not in (None, torch.float32) or not _plain(x, w):
+        return False
+    return (0 < x.shape[0] <= (kernels.LINEAR_ROWS_MAX if x.shape[1] <= 8192 else 8) and x.shape[1] > 0 and x.shape[1] % 4 == 0
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def _few_bfloat16_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None) -> bool:
+    """Whether ``kernels.linear_few`` takes the product: a few bfloat16 rows, bound by the bytes of ``w``."""
+    if (x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or out_dtype not in (None, torch.bfloat16, torch.float32)
+            or x.dim() != 2 or x.shape[0] > kernels.LINEAR_FEW_MAX or not _plain(x, w)):
+        return False
+    return x.data_ptr() % 32 == 0 and w.data_ptr() % 32 == 0 and kernels.linear_few_takes(x.shape[0], x.shape[1], w.shape[0])
+
+
+def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None, ctx=None) -> torch.Tensor:
     """``x [T, in] @ w [out, in].T``; accumulation is float32; ``out_dtype`` float32 keeps the
     accumulator's precision for bfloat16 operands.  An ``x`` from ``empty_rows`` is multiplied with its
-    spare rows and the result cut back to ``T`` rows."""
+    spare rows and the result cut back to ``T`` rows.  ``ctx``: the step's context; where it says that the weights
+    are settled (``StepContext.settled``), the kernel for few rows starts to read them before the launch before it has ended."""
     n = x.shape[0]
+    if _few_bfloat16_rows(x, w, out_dtype):
+        out = torch.empty((n, w.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
+        kernels.linear_few(x, w, out, early=getattr(ctx, "settled", False))
+        return out
     if _few_float32_rows(x, w, out_dtype):
         out = torch.empty((n, w.shape[0]), dtype=torch.float32, device=x.device)
         kernels.linear_rows(x, w, out)
         return out
     xp = _with_spare_rows(x)
     if xp is not x:
-        return linear(xp, w, out_dtype)[:n]
+        return linear(xp, w, out_dtype, ctx)[:n]
     if out_dtype is not None and out_dtype != x.dtype:
         return torch.mm(x, w.t(), out_dtype=out_dtype)
     return torch.mm(x, w.t())

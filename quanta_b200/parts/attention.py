@@ -154,14 +154,14 @@ class GQAttention(Mixer):
         T = x.shape[0]
         if self.taps:
             # the projection's float32 accumulators pass the convolution and reach norm and rotation unrounded
-            proj = linear(x, self.w_qkv, out_dtype=torch.float32)
+            proj = linear(x, self.w_qkv, out_dtype=torch.float32, ctx=ctx)
             C = self.conv_channels
             qkv = torch.empty((T, C), dtype=torch.float32, device=x.device)
             hist = state[self.conv_state_name] if self.taps > 1 else \
                 torch.empty((0, 0, C), dtype=torch.float32, device=x.device)
             kernels.short_conv(proj[:, :C], self.conv_w, hist, qkv, ctx.tok_req, ctx.req_start, ctx.req_slot, plain=True)
         else:
-            qkv = linear(x, self.w_qkv, out_dtype=torch.float32 if self.float32_projection else None)
+            qkv = linear(x, self.w_qkv, out_dtype=torch.float32 if self.float32_projection else None, ctx=ctx)
         q = torch.empty((T, self.nq, self.hd), dtype=x.dtype, device=x.device)
         tables = self.position.rotary_tables(x.device)
         if tables is None:
@@ -190,7 +190,7 @@ class GQAttention(Mixer):
         if self.gated:
             kernels.head_sigmoid_gate(out, qkv[:, self.gate_off: self.gate_off + self.nq], self.nq, self.vd)
         return linear(out.view(T, self.nq * self.vd), self.w_o,
-                      out_dtype=torch.float32 if self.float32_output else None)
+                      out_dtype=torch.float32 if self.float32_output else None, ctx=ctx)
 
     def attend(self, q, cache, out, ctx):
         """float32 (and head sizes the tensor-core kernels do not take: keys and values of different sizes, or

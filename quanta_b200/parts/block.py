@@ -367,7 +367,7 @@ class LinearHead(Head):
         n = rows.numel()
         x = empty_rows(n, self.H, dtype=ctx.dtype, device=h.device)
         self.norm.forward(h, pending, x, rows=rows, store_h=False)
-        logits = linear(x, self.weight, out_dtype=torch.float32)
+        logits = linear(x, self.weight, out_dtype=torch.float32, ctx=ctx)
         if self.logit_scale != 1.0:
             logits.mul_(self.logit_scale)       # on the float32 products: one rounding, as the formula has it
         if self.softcap > 0.0:

@@ -118,7 +118,7 @@ class MatrixMemory(_DecayState):
 
     def forward(self, x, ctx, cache, state):
         T = x.shape[0]
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, ctx=ctx)
         log_decay, weight, floor = kernels.memory_gates(proj, self.i_off, self.i_off + self.H, self.b_i, self.b_f, self.cap,
                                                         state[self.state_name + "_max"], ctx.req_start, ctx.req_slot, self.H)
         den = torch.empty((T, self.H), dtype=torch.float32, device=x.device)
@@ -126,7 +126,7 @@ class MatrixMemory(_DecayState):
                                   q_scale=self.q_scale, n_state=state[self.state_name + "_norm"], floor=floor, den=den)
         y = empty_rows(T, self.H * self.E, dtype=x.dtype, device=x.device)
         kernels.decay_out(o, proj[:, self.g_off: self.i_off], self.gain, y, self.H, self.E, self.H, self.eps, den=den)
-        return linear(y, self.w_o, out_dtype=torch.float32)
+        return linear(y, self.w_o, out_dtype=torch.float32, ctx=ctx)
 
 
 @register("mixer", "state_space_dual")
@@ -167,7 +167,7 @@ class StateSpaceDual(_DecayState):
 
     def forward(self, x, ctx, cache, state):
         T, I, C, GD = x.shape[0], self.inner, self.n_conv, self.G * self.D
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, ctx=ctx)
         u = torch.empty((T, C), dtype=x.dtype, device=x.device)
         hist = state[self.conv_state_name] if self.taps > 1 else torch.empty((0, 0, C), dtype=torch.float32, device=x.device)
         kernels.short_conv(proj[:, I: I + C], self.conv_w, hist, u, ctx.tok_req, ctx.req_start, ctx.req_slot, bias=self.conv_b,
@@ -183,7 +183,7 @@ class StateSpaceDual(_DecayState):
         y = empty_rows(T, I, dtype=x.dtype, device=x.device)
         kernels.decay_out(o, proj[:, :I], self.gain, y, self.H, self.E, self.parts, self.eps, x=values, skip=self.skip,
                           gate_first=True)
-        return linear(y, self.w_o, out_dtype=torch.float32)
+        return linear(y, self.w_o, out_dtype=torch.float32, ctx=ctx)
 
 
 @register("mixer", "constant_decay_attention")
@@ -213,8 +213,8 @@ class ConstantDecayAttention(_DecayState):
 
     def forward(self, x, ctx, cache, state):
         T = x.shape[0]
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, ctx=ctx)
         o = self._from_projection(proj, ctx, x.dtype, self.gates, state, True)
         y = empty_rows(T, self.H * self.E, dtype=x.dtype, device=x.device)
         kernels.decay_out(o, proj[:, self.g_off: self.g_off + self.H * self.E], self.gain, y, self.H, self.E, 1, self.eps)
-        return linear(y, self.w_o, out_dtype=torch.float32)
+        return linear(y, self.w_o, out_dtype=torch.float32, ctx=ctx)

@@ -63,13 +63,13 @@ class DeltaRule(Mixer):
 
     def forward(self, x, ctx, cache, state):
         T, HD = x.shape[0], self.H * self.D
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, ctx=ctx)
         inner = empty_rows(T, self.L, dtype=x.dtype, device=x.device)
         kernels.tanh_cols(proj, 5 * HD, self.L, inner)
-        wpre = linear(inner, self.w_decay, out_dtype=torch.float32)
+        wpre = linear(inner, self.w_decay, out_dtype=torch.float32, ctx=ctx)
         o = torch.empty((T, self.H, self.D), dtype=torch.float32, device=x.device)
         kernels.delta_rule(proj, (0, HD, 2 * HD, 4 * HD), wpre, self.a_bias, self.w_bias, state[self.state_name], o,
                            ctx.req_start, ctx.req_slot, self.H, self.D, self.decay_scale, self.unit_eps)
         y = empty_rows(T, HD, dtype=x.dtype, device=x.device)
         kernels.head_norm_gate(o, proj, 3 * HD, self.gain, y, self.H, self.D, self.norm_eps)
-        return linear(y, self.w_o, out_dtype=torch.float32)
+        return linear(y, self.w_o, out_dtype=torch.float32, ctx=ctx)

@@ -55,14 +55,14 @@ class GatedDense(FeedForward):
 
     def forward(self, x, ctx):
         T = x.shape[0]
-        gate_up = linear(x, self.w_gate_up)
+        gate_up = linear(x, self.w_gate_up, ctx=ctx)
         act = empty_rows(T, self.inner, dtype=x.dtype, device=x.device)
         if self.activation == "silu" and not self.biases:
             kernels.silu_mul(gate_up, act)
         else:
             kernels.glu_act(gate_up, act, bias=self.b_gate_up, limit=self.limit, alpha=self.alpha,
                             kind=self.KINDS[self.activation])
-        y = linear(act, self.w_down, out_dtype=torch.float32)
+        y = linear(act, self.w_down, out_dtype=torch.float32, ctx=ctx)
         return Addends(y, bias=self.b_down) if self.biases else y
 
 
@@ -87,7 +87,7 @@ class UngatedDense(FeedForward):
 
     def forward(self, x, ctx):
         T = x.shape[0]
-        up = linear(x, self.w_up)
+        up = linear(x, self.w_up, ctx=ctx)
         act = empty_rows(T, self.inner, dtype=x.dtype, device=x.device)
         kernels.relu_squared(up, act)
-        return linear(act, self.w_down, out_dtype=torch.float32)
+        return linear(act, self.w_down, out_dtype=torch.float32, ctx=ctx)

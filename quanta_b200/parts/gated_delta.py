@@ -129,7 +129,7 @@ class GatedDeltaRule(Mixer):
 
     def forward(self, x, ctx, cache, state):
         T, C = x.shape[0], self.n_conv
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, ctx=ctx)
         qkv = torch.empty((T, C), dtype=torch.float32, device=x.device)
         hist = state[self.conv_state_name] if self.taps > 1 else \
             torch.empty((0, 0, C), dtype=torch.float32, device=x.device)
@@ -146,4 +146,4 @@ class GatedDeltaRule(Mixer):
             gate, gate_off = self.w_gate(proj[:, self.gate_off: self.gate_off + self.gate_rank]), 0
         y = empty_rows(T, self.H * self.DV, dtype=x.dtype, device=x.device)
         kernels.head_norm_gate(o, gate, gate_off, self.gain, y, self.H, self.DV, self.norm_eps, gate=self.gate_activation)
-        return linear(y, self.w_o, out_dtype=torch.float32)
+        return linear(y, self.w_o, out_dtype=torch.float32, ctx=ctx)

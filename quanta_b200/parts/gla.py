@@ -64,10 +64,10 @@ class GatedLinearAttention(Mixer):
 
     def forward(self, x, ctx, cache, state):
         T, HD, HE = x.shape[0], self.H * self.D, self.H * self.E
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, ctx=ctx)
         o = torch.empty((T, self.H, self.E), dtype=torch.float32, device=x.device)
         kernels.gla(proj, (0, HD, 2 * HD), 2 * HD + 2 * HE, self.L, self.w_decay, self.decay_bias,
                     state[self.state_name], o, ctx.req_start, ctx.req_slot, self.H, self.D, self.E, self.tau, self.q_scale)
         y = empty_rows(T, HE, dtype=x.dtype, device=x.device)
         kernels.head_norm_gate(o, proj, 2 * HD + HE, self.gain, y, self.H, self.E, self.norm_eps, gate="silu")
-        return linear(y, self.w_o, out_dtype=torch.float32)
+        return linear(y, self.w_o, out_dtype=torch.float32, ctx=ctx)

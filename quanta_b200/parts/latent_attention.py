@@ -112,7 +112,7 @@ class LatentAttention(Mixer):
                 raise ValueError("latent_attention: position encodings with several axes are not built")
         interleaved = bool(getattr(self.position, "interleaved", False))
         # the queries' latent, this step's latent rows and rotated key parts (which go into the pages), the gates
-        down = linear(x, self.w_in, out_dtype=f32)
+        down = linear(x, self.w_in, out_dtype=f32, ctx=ctx)
         cq = empty_rows(T, self.q_rank, dtype=x.dtype, device=dev)
         pages = cache.streams[STREAM]
         kernels.latent_write(down[:, self.dkv_off: self.gate_off] if cache.write else None, self.dkv_gain, inv_freq, pages,
@@ -120,7 +120,7 @@ class LatentAttention(Mixer):
                              ctx.status, interleaved=interleaved, q_down=down[:, : self.q_rank], q_gain=self.dq_gain,
                              q_out=cq)
         gate = down[:, self.gate_off: self.gate_off + self.H] if self.gated else None
-        q = linear(cq, self.w_uq, out_dtype=f32)
+        q = linear(cq, self.w_uq, out_dtype=f32, ctx=ctx)
         q_plain = torch.empty((H, T, self.D), dtype=x.dtype, device=dev)
         q_rot = torch.empty((T, H, self.R), dtype=f32, device=dev)
         kernels.latent_query(q, inv_freq, q_plain, q_rot, ctx.tok_pos, H, self.D, self.R, rd, interleaved)
@@ -132,4 +132,4 @@ class LatentAttention(Mixer):
                               window=self.window or 0, gate=gate, float32_weights=self.float32_weights)
         o = empty_rows(T, H * self.V, dtype=x.dtype, device=dev)
         torch.bmm(o_lat, self.w_uv_t, out=o.view(T, H, self.V).transpose(0, 1))
-        return linear(o, self.w_o, out_dtype=f32)
+        return linear(o, self.w_o, out_dtype=f32, ctx=ctx)

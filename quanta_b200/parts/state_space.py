@@ -71,16 +71,16 @@ class SelectiveScan(Mixer):
 
     def forward(self, x, ctx, cache, state):
         T, C = x.shape[0], self.inner
-        uz = linear(x, self.w_in, out_dtype=torch.float32)
+        uz = linear(x, self.w_in, out_dtype=torch.float32, ctx=ctx)
         u = empty_rows(T, C, dtype=x.dtype, device=x.device)
         kernels.short_conv(uz[:, :C], self.conv_w, state[self.conv_state_name], u, ctx.tok_req, ctx.req_start,
                            ctx.req_slot, bias=self.conv_b, silu=True)
-        proj = linear(u, self.w_x, out_dtype=torch.float32)
+        proj = linear(u, self.w_x, out_dtype=torch.float32, ctx=ctx)
         y = empty_rows(T, C, dtype=x.dtype, device=x.device)
-        dt_pre = linear(proj[:, : self.R], self.w_dt)          # float32 operands: a true float32 product
+        dt_pre = linear(proj[:, : self.R], self.w_dt, ctx=ctx)          # float32 operands: a true float32 product
         kernels.selective_scan(u, proj, uz[:, C:], dt_pre, self.dt_b, self.A, self.D, state[self.state_name], y,
                                ctx.req_start, ctx.req_slot, self.R, self.N)
-        return linear(y, self.w_o, out_dtype=torch.float32)
+        return linear(y, self.w_o, out_dtype=torch.float32, ctx=ctx)
 
 
 @register("mixer", "parallel_mixers")

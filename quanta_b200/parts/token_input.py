@@ -45,6 +45,6 @@ class GatedTokenRow(TokenInput):
     def forward(self, x, ctx):
         T = x.shape[0]
         g = empty_rows(T, self.dim, dtype=x.dtype, device=x.device)
-        gate = None if T <= kernels.TOKEN_INPUT_SMALL else linear(x, self.w_gate, out_dtype=torch.float32)
+        gate = None if T <= kernels.TOKEN_INPUT_SMALL else linear(x, self.w_gate, out_dtype=torch.float32, ctx=ctx)
         kernels.token_input(x, self.w_gate, self.table, self.index * self.dim, ctx.token_ids, g, ctx.status, gate=gate)
-        return NormedPending(linear(g, self.w_proj, out_dtype=torch.float32), self.norm)
+        return NormedPending(linear(g, self.w_proj, out_dtype=torch.float32, ctx=ctx), self.norm)

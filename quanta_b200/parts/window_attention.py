@@ -159,7 +159,7 @@ class WindowAttention(Mixer):
         T = x.shape[0]
         if cache is None or not cache.write:
             raise ValueError("window_attention fills a cache of its own")
-        qkv = linear(x, self.w_qkv, out_dtype=torch.float32)
+        qkv = linear(x, self.w_qkv, out_dtype=torch.float32, ctx=ctx)
         q = torch.empty((T, self.nq, self.hd), dtype=x.dtype, device=x.device)
         tables = self.position.rotary_tables(x.device)
         if tables is None:
@@ -199,5 +199,5 @@ class WindowAttention(Mixer):
                                      self.window, ctx.status, dist_bias=self.dist_table, sink=self.sink,
                                      softcap=self.softcap, talk=self.talk, scratch=scratch,
                                      n_requests=int(ctx.req_start.numel()) - 1, **pooled)
-        y = linear(out.view(T, self.nq * self.vd), self.w_o, out_dtype=torch.float32)
+        y = linear(out.view(T, self.nq * self.vd), self.w_o, out_dtype=torch.float32, ctx=ctx)
         return Addends(y, bias=self.b_o) if self.b_o is not None else y
