@@ -586,6 +586,25 @@ def linear_rows(x, w, out) -> None:
     _check(lib().qb_linear_rows(_p(x), _p(w), _p(out), n, K, w.shape[0], _stream()), "linear_rows")
 
 
+LINEAR_FEW_MAX = 32
+
+
+def linear_few_takes(rows: int, K: int, N: int) -> bool:
+    """Whether ``linear_few`` is the faster way for ``rows`` bfloat16 rows and a ``[N, K]`` matrix."""
+    return 0 < rows <= LINEAR_FEW_MAX and bool(lib().qb_linear_few_takes(rows, K, N))
+
+
+def linear_few(x, w, out, early: bool = False) -> None:
+    """``out [n, N] = x [n, K] @ w [N, K].T`` for at most ``LINEAR_FEW_MAX`` bfloat16 rows, summed in float32; K a multiple of 16,
+    ``x`` and ``w`` on 32 bytes.  ``early``: nothing the two launches before this one do writes ``w`` (the kernel starts to read it
+    before the launch before it has ended)."""
+    _want(x, torch.bfloat16, "x"); _want(w, torch.bfloat16, "w")
+    n, K = x.shape
+    if w.shape[1] != K or tuple(out.shape) != (n, w.shape[0]):
+        raise ValueError("linear_few: shape mismatch")
+    _check(lib().qb_linear_few(_p(x), _p(w), _p(out), _code(out), n, K, w.shape[0], int(early), _stream()), "linear_few")
+
+
 EXPERT_ACT_SILU, EXPERT_ACT_CLAMPED = 0, 1
 
 
