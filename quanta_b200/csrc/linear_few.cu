@@ -4,8 +4,11 @@
 // numbers of a row's 128 bytes that it then multiplies (the order of the inner dimension inside an mma is free as long as both operands
 // have it), 32 bytes a load, so that weights go from memory to registers without shared memory or a barrier: up to 128 KB on
 // their way an SM, of which 45 keep the memory busy.  Between the launches of a step the library's kernels wait for the launch before
-// them and then for their first weights; here the first pieces are asked for before that wait (`early`), and the products
-// follow the arrival of x.  x is read by every block, out of L1 after the SM's first.  A row's sums are taken in an order that depends on K alone.
+// them and then for their first weights; here, where the caller allows it (`early`), blocks are placed while the launch before runs and ask
+// for their first pieces before they wait for it, and the products follow the arrival of x.  That pays behind launches that are one
+// short chain of reads (8 requests, a delta rule's model: 637 us for two steps without, 603 with it), not behind those that
+// use the memory or fill the SMs themselves (an attention, the norm over eight experts' slots: the blocks slow them and fall unevenly
+// on the SMs that are left; 8 requests of the M2-family sizes 2,518 us with, 2,474 without).  x is read by every block, out of L1 after the SM's first.  A row's sums are taken in an order that depends on K alone.
 //
 // Measured on a B200, one product after another in a graph, weights from memory, microseconds (library: at 32 rows, its fastest kernel):
 //   [N, K]            bytes at 6.5 TB/s   library   8 rows   16 rows   32 rows
@@ -79,10 +82,9 @@ __global__ void __launch_bounds__(LF_WARPS * 32, MINB) linear_few_kernel(LinearF
 #pragma unroll
     for (int n = 0; n < NT; ++n) b[n] = in ? lf_load(xr[n] + kb * LF_KB) : none;
   };
-  if (!early) qb_follow();
 #pragma unroll
   for (int d = 0; d < D; ++d) fetch_w(warp + d * LF_WARPS, wb[d]);
-  if (early) qb_follow();
+  if (early) qb_follow();         // (a launch that is not early starts behind the one before it)
 #pragma unroll
   for (int d = 0; d < XD; ++d) fetch_x(warp + d * LF_WARPS, xb[d]);
   float acc[NT][4];
@@ -126,7 +128,8 @@ __global__ void __launch_bounds__(LF_WARPS * 32, MINB) linear_few_kernel(LinearF
 template <int NT, int D, int XD, int MINB>
 static int linear_few_launch(const LinearFew& a, int out_dtype, int early, cudaStream_t stream) {
   const int grid = (a.N + 15) / 16;
-  QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(linear_few_kernel<NT, D, XD, MINB, O>, grid, LF_WARPS * 32, 0, stream, a, early));
+  if (early) QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(linear_few_kernel<NT, D, XD, MINB, O>, grid, LF_WARPS * 32, 0, stream, a, 1));
+  else QB_DISPATCH_DTYPE(out_dtype, O, (linear_few_kernel<NT, D, XD, MINB, O><<<grid, LF_WARPS * 32, 0, stream>>>(a, 0)));
   QB_LAUNCH_CHECK();
   return 0;
 }

@@ -82,8 +82,9 @@ def _few_bfloat16_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None, ctx=None) -> torch.Tensor:
     """``x [T, in] @ w [out, in].T``; accumulation is float32; ``out_dtype`` float32 keeps the
     accumulator's precision for bfloat16 operands.  An ``x`` from ``empty_rows`` is multiplied with its
-    spare rows and the result cut back to ``T`` rows.  ``ctx``: the step's context; where it says that the weights
-    are settled (``StepContext.settled``), the kernel for few rows starts to read them before the launch before it has ended."""
+    spare rows and the result cut back to ``T`` rows.  ``ctx``: the step's context, given where the launch before is
+    short and leaves the memory idle; where it says that the weights are settled (``StepContext.settled``), the kernel for few rows
+    starts to read them before that launch has ended."""
     n = x.shape[0]
     if _few_bfloat16_rows(x, w, out_dtype):
         out = torch.empty((n, w.shape[0]), dtype=out_dtype or x.dtype, device=x.device)

@@ -161,7 +161,7 @@ class GQAttention(Mixer):
                 torch.empty((0, 0, C), dtype=torch.float32, device=x.device)
             kernels.short_conv(proj[:, :C], self.conv_w, hist, qkv, ctx.tok_req, ctx.req_start, ctx.req_slot, plain=True)
         else:
-            qkv = linear(x, self.w_qkv, out_dtype=torch.float32 if self.float32_projection else None, ctx=ctx)
+            qkv = linear(x, self.w_qkv, out_dtype=torch.float32 if self.float32_projection else None)
         q = torch.empty((T, self.nq, self.hd), dtype=x.dtype, device=x.device)
         tables = self.position.rotary_tables(x.device)
         if tables is None:
@@ -190,7 +190,7 @@ class GQAttention(Mixer):
         if self.gated:
             kernels.head_sigmoid_gate(out, qkv[:, self.gate_off: self.gate_off + self.nq], self.nq, self.vd)
         return linear(out.view(T, self.nq * self.vd), self.w_o,
-                      out_dtype=torch.float32 if self.float32_output else None, ctx=ctx)
+                      out_dtype=torch.float32 if self.float32_output else None)
 
     def attend(self, q, cache, out, ctx):
         """float32 (and head sizes the tensor-core kernels do not take: keys and values of different sizes, or

@@ -199,5 +199,5 @@ class WindowAttention(Mixer):
                                      self.window, ctx.status, dist_bias=self.dist_table, sink=self.sink,
                                      softcap=self.softcap, talk=self.talk, scratch=scratch,
                                      n_requests=int(ctx.req_start.numel()) - 1, **pooled)
-        y = linear(out.view(T, self.nq * self.vd), self.w_o, out_dtype=torch.float32, ctx=ctx)
+        y = linear(out.view(T, self.nq * self.vd), self.w_o, out_dtype=torch.float32)
         return Addends(y, bias=self.b_o) if self.b_o is not None else y
