@@ -7,21 +7,40 @@
 //   S_t = diag(w) S_{t-1} - (a * u) (u^T S_{t-1}) + k v^T     (both terms read the old state)
 //   o_t = S_t^T r
 //
-// A column j of S never meets another column.  Eight lanes share one: lane p has its rows p, p + 8, ..., adds its part of u^T S (and of
-// the output) in the order of the rows, and the eight parts meet two by two (lanes 1, 2, 4 apart).  Both kernels below do exactly these
-// operations, so a position's numbers depend neither on the cut nor on the batch, not even by rounding.  (Portions once ran in
-// chunks of 16 tokens as products, 240 us for the prompt below, whose outputs were 1.7e-7 off float64 against 1.1e-7 here and depended
-// on what shared the step.)
+// A column j of S never meets another column.  Sixteen lanes share one: lane p has its rows p + 16 n.  Its part of u^T S (and of the output)
+// is two sums, over the rows of even and of odd n in the order of n, added up; the sixteen parts meet two by two (lanes 1, 2, 4, 8 apart).
+// Both kernels below do exactly these operations, so a position's numbers depend neither on the cut nor on the batch, not even by rounding.
+// (Portions once ran in chunks of 16 tokens as products, 240 us for the prompt below, whose outputs were 1.7e-7 off float64 against 0.9e-7 here
+// and depended on what shared the step.)
 //
 // The per-head RMS norm with gain and gate that follows is a kernel of the common unit (norm_embed.cu).
 #include "common.cuh"
 
-constexpr int DR_LANES = 8;   // lanes that share a column
+constexpr int DR_LANES = 16;  // lanes that share a column
 constexpr int DR_ARRAYS = 5;  // of a (token, head): u, w, a*u, k, r
 
-// What a token does to one row of a column, and to the column's output.
-__device__ __forceinline__ float dr_row(float w, float s, float au, float dot, float k, float v) {
-  return fmaf(k, v, fmaf(w, s, -(au * dot)));
+// Two float32 numbers in one 64-bit register: the halves of a packed operation round as the operations of one number do.
+typedef unsigned long long dr_pair;
+__device__ __forceinline__ dr_pair dr_pack(float a, float b) {
+  dr_pair v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+__device__ __forceinline__ void dr_unpack(dr_pair v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ dr_pair dr_fma(dr_pair a, dr_pair b, dr_pair c) {
+  dr_pair v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+__device__ __forceinline__ dr_pair dr_mul(dr_pair a, dr_pair b) {
+  dr_pair v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+
+// What a token does to two rows of a column: k v + (w s + a u (-dot)).
+__device__ __forceinline__ dr_pair dr_rows2(dr_pair w, dr_pair s, dr_pair au, dr_pair minus_dot, dr_pair k, dr_pair v) {
+  return dr_fma(k, v, dr_fma(w, s, dr_mul(au, minus_dot)));
 }
 __device__ __forceinline__ float dr_decay(float x, float scale) { return expf(-scale * (1.f / (1.f + expf(-x)))); }
 __device__ __forceinline__ float dr_rate(float x) { return 1.f / (1.f + expf(-x)); }
@@ -33,169 +52,293 @@ __device__ __forceinline__ float dr_unit(const float* __restrict__ k, int D, int
 }
 
 // ---------------------------------------------------------------------------------------------
-// Portions.  A first kernel turns the projections of every (token, head) into the five arrays of [8 RPT] floats in the order in which the
-// lanes read them: row i = p + 8 (4 q + e) is number (8 q + p) 4 + e, zeros past D; so lane p's rows are 16-byte pieces, and the
-// pieces of the eight lanes lie side by side.  One warp a (token, head).
+// Portions.  A first kernel turns the projections of every (head, token) into arrays of DP floats: u, w, a*u, k, r in the order in which the
+// lanes read them (row i = p + 16 (4 q + e) is number (16 q + p) 4 + e, zeros past D, so that a lane's rows are 16-byte pieces and the pieces of
+// the sixteen lanes lie side by side).  A head's tokens follow one another: a chunk of them is one run of memory.
 //
-// The recurrence is a chain in time.  A lane group owns one or two columns in registers for the whole portion, a block some columns of one
-// (request, head).  Chunks of tokens come into shared memory by asynchronous copies while the chunk before is walked without any barrier.
-// One portion alone is bound by the chain of a token (345 cycles: eight multiply-adds, three exchanges, three more, 100 instructions a
-// warp): one column a lane, few columns a block.  Enough portions to fill the SMs are bound by the reads of the five arrays from
-// shared memory, which two columns a lane halve.  Measured on a B200, token by token with four-byte reads / with this: one portion of
-// 2,048 tokens, 32 heads of 64, 618 / 406 us, 8 of 512 615 / 362 (one column a lane 546), 16 heads of 128 962 / 616.
+// The recurrence is a chain in time.  A lane group owns two columns in registers for the whole portion, a block some columns of one
+// (request, head).  Chunks of 16 tokens come into shared memory by copies of a warp of their own, three ahead.  One portion alone is bound by the
+// chain of a token: two packed multiply-adds, four exchanges (29 cycles each), three more packed operations; the rows of the next token are
+// read meanwhile, and the sixteen tokens' outputs are summed over the lanes together (16 exchanges a column instead of 64).  Eight lanes
+// a column have one exchange less but twice the reads of shared memory, behind which the exchanges queue (281 us for the prompt below, 240 with
+// sixteen; with a branch a token around the step 338).  Measured on a B200, one portion of 2,048 tokens, 32 heads of 64: 331 + 42 us with eight
+// lanes a column, 264 + 30 with this; the same in a step (the chain and the preparation).
 // ---------------------------------------------------------------------------------------------
-__global__ void delta_prep_kernel(const float* __restrict__ proj, int proj_stride, int r_off, int k_off, int a_off,
-                                  const float* __restrict__ wpre, const float* __restrict__ a_bias, const float* __restrict__ w_bias,
-                                  float* __restrict__ scratch, int T, int H, int D, int DP, float decay_scale, float unit_eps) {
+constexpr int DR_MAX_COLS = 32, DR_CHUNK_FLOATS = 16 * DR_ARRAYS * 64, DR_STAGE_FLOATS = DR_CHUNK_FLOATS + 16 * DR_MAX_COLS, DR_STAGES = 4;
+
+template <int RPT>
+__global__ void __launch_bounds__(128)
+delta_prep_kernel(const float* __restrict__ proj, int proj_stride, int r_off, int k_off, int a_off, const float* __restrict__ wpre,
+                  const float* __restrict__ a_bias, const float* __restrict__ w_bias, float* __restrict__ scratch, int T, int H, int D,
+                  float decay_scale, float unit_eps) {
+  constexpr int DP = DR_LANES * RPT, N = DP / 32;
   const int lane = threadIdx.x & 31;
   const long wid = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (wid >= (long)T * H) return;
   const int t = (int)(wid / H), h = (int)(wid % H);
   const float* row = proj + (size_t)t * proj_stride + (size_t)h * D;
+  float k[N], a[N], w[N], r[N], ab[N], wb[N];              // all reads before the first use
+#pragma unroll
+  for (int x = 0; x < N; ++x) {
+    const int at = lane + 32 * x, i = ((at >> 2) & 15) + DR_LANES * ((at & 3) + 4 * (at >> 6));
+    const bool in = i < D;
+    k[x] = in ? row[k_off + i] : 0.f;
+    a[x] = in ? row[a_off + i] : 0.f;
+    w[x] = in ? wpre[(size_t)wid * D + i] : 0.f;
+    r[x] = in ? row[r_off + i] : 0.f;
+    ab[x] = in ? a_bias[h * D + i] : 0.f;
+    wb[x] = in ? w_bias[h * D + i] : 0.f;
+  }
   const float inv = dr_unit(row + k_off, D, lane, unit_eps);
-  float* to = scratch + (size_t)wid * DR_ARRAYS * DP;
-  for (int i = lane; i < DP; i += 32) {
-    float u = 0.f, w = 0.f, au = 0.f, k = 0.f, r = 0.f;
-    if (i < D) {
-      k = row[k_off + i];
-      u = k * inv;
-      au = dr_rate(row[a_off + i] + a_bias[h * D + i]) * u;
-      w = dr_decay(wpre[(size_t)wid * D + i] + w_bias[h * D + i], decay_scale);
-      r = row[r_off + i];
-    }
-    const int p = i & 7, n = i >> 3, at = ((n >> 2) * 8 + p) * 4 + (n & 3);
-    to[at] = u; to[DP + at] = w; to[2 * DP + at] = au; to[3 * DP + at] = k; to[4 * DP + at] = r;
+  float* to = scratch + ((size_t)h * T + t) * DR_ARRAYS * DP;
+#pragma unroll
+  for (int x = 0; x < N; ++x) {
+    const int at = lane + 32 * x, i = ((at >> 2) & 15) + DR_LANES * ((at & 3) + 4 * (at >> 6));
+    const bool in = i < D;
+    const float u = k[x] * inv;
+    to[at] = u;                                              // (past D: k is zero)
+    to[DP + at] = in ? dr_decay(w[x] + wb[x], decay_scale) : 0.f;
+    to[2 * DP + at] = in ? dr_rate(a[x] + ab[x]) * u : 0.f;
+    to[3 * DP + at] = k[x];
+    to[4 * DP + at] = r[x];
   }
 }
 
-template <int BYTES>
-__device__ __forceinline__ void dr_copy(float* dst_smem, const float* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+// The sums over the sixteen lanes of N values each, N at most 16: lane p then holds the value dr_first<N>(p) (lanes that differ in the bits
+// beyond N's hold the same).
+template <int N>
+__device__ __forceinline__ void dr_sum_lanes(float (&x)[N], int p) {
+  int n = N;
+#pragma unroll
+  for (int d = 1; d < DR_LANES; d <<= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool upper = p & d;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i) {
+        if (i >= n) break;
+        const float give = upper ? x[i] : x[i + n], keep = upper ? x[i + n] : x[i];
+        x[i] = keep + __shfl_xor_sync(0xffffffffu, give, d);
+      }
+    } else {
+      x[0] += __shfl_xor_sync(0xffffffffu, x[0], d);
+    }
+  }
+}
+template <int N>
+__device__ __forceinline__ int dr_first(int p) {
+  int first = 0, n = N;
+#pragma unroll
+  for (int d = 1; d < N; d <<= 1) {
+    n >>= 1;
+    first += p & d ? n : 0;
+  }
+  return first;
 }
 
-template <int RPT, int C>            // rows of a column a lane holds (D <= DR_LANES * RPT), columns a lane
-__global__ void __launch_bounds__(C == 1 ? 128 : 256, 1)
-delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, const float* __restrict__ scratch,
-                  float* __restrict__ state, float* __restrict__ out, const int* __restrict__ req_start,
-                  const int* __restrict__ req_slot, int H, int D, int cols, int chunk) {
+__device__ __forceinline__ unsigned dr_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+// Bounded wait: false when the limit (iterations and 0.2 s) is reached or another warp gave up.
+__device__ __forceinline__ bool dr_wait(unsigned bar, unsigned parity, volatile int* abort_flag) {
+  unsigned long long t0 = 0;
+  for (unsigned it = 0; it < 4000000u; ++it) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((it & 63u) == 63u) {
+      if (*abort_flag) return false;
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > 200000000ull) break;
+    }
+  }
+  *abort_flag = 1;
+  return false;
+}
+
+// RPT: rows of a column a lane holds (D <= 16 RPT); U: tokens whose outputs are summed together; W: warps that walk the tokens, one more
+// brings them
+template <int RPT, int U, int W>
+__global__ void __launch_bounds__(32 * W + 32, W == 8 ? 2 : 1)
+delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, const float* __restrict__ scratch, float* __restrict__ state,
+                  float* __restrict__ out, const int* __restrict__ req_start, const int* __restrict__ req_slot, int T, int H, int D, int* status) {
   extern __shared__ __align__(16) float sm[];
-  constexpr int DP = DR_LANES * RPT, PER = DR_ARRAYS * DP;      // floats of a token's five arrays
+  __shared__ __align__(8) unsigned long long s_full[DR_STAGES], s_empty[DR_STAGES];
+  __shared__ int s_abort;
+  constexpr int DP = DR_LANES * RPT, PER = DR_ARRAYS * DP, P = RPT / 2, C = 2;
+  constexpr int CHUNK = DR_CHUNK_FLOATS / PER, COLS = 4 * W;    // 16 tokens of heads up to 64, fewer of larger ones
   const int r = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-  const int p = tid % DR_LANES, c = tid / DR_LANES * C, col0 = blockIdx.z * cols, j = col0 + c;
+  const int p = tid % DR_LANES, col0 = blockIdx.z * COLS, jj = tid / DR_LANES * C, j = col0 + jj;
   const int t0 = req_start[r], t1 = req_start[r + 1];
   if (t0 >= t1) return;
+  const unsigned sm0 = dr_smem(sm);
+  const int n_all = t1 - t0, chunks = (n_all + CHUNK - 1) / CHUNK;
+  volatile int* abort_flag = &s_abort;
+  if (tid == 0) {
+    for (int b = 0; b < DR_STAGES; ++b) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 33;" ::"r"(dr_smem(&s_full[b])));       // the run of scratch, and each lane's copies
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(dr_smem(&s_empty[b])), "r"(W));
+    }
+    s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (tid >= 32 * W) {
+    // ---- the warp that brings the tokens.  A stage: [CHUNK][PER] in one copy, then v [CHUNK][COLS], 4 bytes a copy (columns start
+    // anywhere; past D zeros)
+    const int lane = tid & 31;
+    const float* from = scratch + ((size_t)h * T + t0) * PER;
+    const float* v_from = proj + (size_t)t0 * proj_stride + v_off + (size_t)h * D + col0;
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c % DR_STAGES, n = min(CHUNK, n_all - c * CHUNK);
+      if (c >= DR_STAGES && !__all_sync(0xffffffffu, dr_wait(dr_smem(&s_empty[b]), (unsigned)(c / DR_STAGES - 1) & 1u, abort_flag))) break;
+      const unsigned to = sm0 + 4 * b * DR_STAGE_FLOATS, bar = dr_smem(&s_full[b]);
+      if (lane == 0) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(4 * n * PER) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(to), "l"(from + (size_t)c * DR_CHUNK_FLOATS), "r"(4 * n * PER), "r"(bar) : "memory");
+      }
+#pragma unroll 4
+      for (int i = lane; i < n * COLS; i += 32) {
+        const int tt = i / COLS, x = i % COLS;
+        const bool in = col0 + x < D;
+        const float* v = in ? v_from + (size_t)(c * CHUNK + tt) * proj_stride + x : proj;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + 4 * (CHUNK * PER + i)), "l"(v), "r"(in ? 4 : 0) : "memory");
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    // the copies in flight land before the block leaves: the walking warps wait for every chunk, unless one gave up
+    if (*abort_flag) {
+      if (lane == 0 && status != nullptr) qb_set_status(status, QB_STATUS_WAIT_TIMEOUT, r, 9);
+      __nanosleep(100000);
+    }
+    return;
+  }
   float* S = state + ((size_t)req_slot[r] * H + h) * D * D + j;
-  float col[RPT][C];
+  auto held = [&](int n, int e) { return j + e < D && p + DR_LANES * n < D; };
+  auto cell = [&](int n, int e) { return held(n, e) ? S[(size_t)(p + DR_LANES * n) * D + e] : 0.f; };
+  dr_pair col[C][P];
 #pragma unroll
-  for (int n = 0; n < RPT; ++n)
+  for (int e = 0; e < C; ++e)
 #pragma unroll
-    for (int e = 0; e < C; ++e) col[n][e] = (j + e < D && p + DR_LANES * n < D) ? S[(size_t)(p + DR_LANES * n) * D + e] : 0.f;
-  const int buffer = chunk * (PER + cols);             // [chunk][PER], then v [chunk][cols]
-  auto fetch = [&](int c0, int buf) {
-    const int n = min(chunk, t1 - c0);
-    float* b = sm + (size_t)buf * buffer;
-    for (int i = tid; i < n * (PER / 4); i += blockDim.x) {
-      const int tt = i / (PER / 4), piece = i % (PER / 4);
-      dr_copy<16>(b + 4 * i, scratch + ((size_t)(c0 + tt) * H + h) * PER + 4 * piece);
-    }
-    for (int i = tid; i < n * cols; i += blockDim.x) {
-      const int tt = i / cols, cc = i % cols;
-      if (col0 + cc < D) dr_copy<4>(b + chunk * PER + i, proj + (size_t)(c0 + tt) * proj_stride + v_off + (size_t)h * D + col0 + cc);
-      else b[chunk * PER + i] = 0.f;
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int i = 0; i < P; ++i) col[e][i] = dr_pack(cell(2 * i, e), cell(2 * i + 1, e));
+  struct Token {
+    dr_pair u[P], w[P], au[P], k[P], r[P];
+    float v[C];
   };
-  auto rows = [&](const float* from, float (&x)[RPT]) {      // this lane's rows of one array
+  // shared-memory reads that stay where they are written, before the exchanges of the token in work (the compiler put them behind: 368 us)
+  auto rows = [&](unsigned a, dr_pair (&x)[P]) {               // this lane's rows of one array
 #pragma unroll
-    for (int q = 0; q < RPT / 4; ++q) {
-      const float4 v = *reinterpret_cast<const float4*>(from + (q * 8 + p) * 4);
-      x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
+    for (int q = 0; q < P / 2; ++q)
+      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x[2 * q]), "=l"(x[2 * q + 1]) : "r"(a + 16 * (q * DR_LANES)));
+  };
+  auto read = [&](unsigned a, unsigned v, Token& t) {
+    rows(a, t.u); rows(a + 8 * DP, t.au); rows(a + 4 * DP, t.w); rows(a + 12 * DP, t.k); rows(a + 16 * DP, t.r);
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t.v[0]), "=f"(t.v[1]) : "r"(v));
+  };
+  auto step = [&](const Token& t, float (&o)[C]) {             // this lane's part of the output
+    float dot[C];
+#pragma unroll
+    for (int e = 0; e < C; ++e) {
+      dr_pair sum = 0;
+#pragma unroll
+      for (int i = 0; i < P; ++i) sum = dr_fma(t.u[i], col[e][i], sum);
+      float a, b;
+      dr_unpack(sum, a, b);
+      dot[e] = a + b;
+    }
+#pragma unroll
+    for (int d = 1; d < DR_LANES; d <<= 1)
+#pragma unroll
+      for (int e = 0; e < C; ++e) dot[e] += __shfl_xor_sync(0xffffffffu, dot[e], d);
+#pragma unroll
+    for (int e = 0; e < C; ++e) {
+      const dr_pair minus = dr_pack(-dot[e], -dot[e]), v = dr_pack(t.v[e], t.v[e]);
+      dr_pair sum = 0;
+#pragma unroll
+      for (int i = 0; i < P; ++i) col[e][i] = dr_rows2(t.w[i], col[e][i], t.au[i], minus, t.k[i], v);
+#pragma unroll
+      for (int i = 0; i < P; ++i) sum = dr_fma(t.r[i], col[e][i], sum);
+      float a, b;
+      dr_unpack(sum, a, b);
+      o[e] = a + b;
     }
   };
-  auto over_lanes = [&](float (&x)[C], float (&y)[C]) {
+  float* to = out + ((size_t)t0 * H + h) * D + j;
+  const size_t next = (size_t)H * D;
+  for (int c = 0; c < chunks; ++c) {
+    const int b = c % DR_STAGES;
+    if (!__all_sync(0xffffffffu, dr_wait(dr_smem(&s_full[b]), (unsigned)(c / DR_STAGES) & 1u, abort_flag))) return;
+    unsigned a = sm0 + 4 * b * DR_STAGE_FLOATS, v = a + 4 * (CHUNK * PER + jj);
+    a += 16 * p;
+    const int n = min(CHUNK, n_all - c * CHUNK);
+    Token now;
+    read(a, v, now);
+    int tt = 0;
+#pragma unroll 1
+    for (; tt + U <= n; tt += U) {          // no branch inside: the next token's rows are read during this one's exchanges
+      float o[C][U];
 #pragma unroll
-    for (int o = 1; o < DR_LANES; o <<= 1) {
+      for (int x = 0; x < U; ++x) {
+        Token ahead;
+        read(a + 4 * (x + 1) * PER, v + 4 * (x + 1) * COLS, ahead);      // behind the last token: whatever lies there, not used
+        float part[C];
+        step(now, part);
 #pragma unroll
-      for (int e = 0; e < C; ++e) x[e] += __shfl_xor_sync(0xffffffffu, x[e], o);
-#pragma unroll
-      for (int e = 0; e < C; ++e) y[e] += __shfl_xor_sync(0xffffffffu, y[e], o);
-    }
-  };
-  // u of a token and r of the token before meet the same state, so both sums are worked out together
-  float u[RPT], r_before[RPT], dot[C], o_before[C];
-  auto sums = [&] {
-#pragma unroll
-    for (int e = 0; e < C; ++e) dot[e] = o_before[e] = 0.f;
-#pragma unroll
-    for (int n = 0; n < RPT; ++n)
+        for (int e = 0; e < C; ++e) o[e][x] = part[e];
+        now = ahead;
+      }
+      a += 4 * U * PER;
+      v += 4 * U * COLS;
+      const int first = dr_first<U>(p);
 #pragma unroll
       for (int e = 0; e < C; ++e) {
-        dot[e] = fmaf(u[n], col[n][e], dot[e]);
-        o_before[e] = fmaf(r_before[n], col[n][e], o_before[e]);
+        dr_sum_lanes<U>(o[e], p);
+        if ((U == DR_LANES || p < U) && j + e < D) to[(size_t)first * next + e] = o[e][0];
       }
-    over_lanes(dot, o_before);
-  };
-  float* to = out + ((size_t)t0 * H + h) * D + j;      // of the token before
-  auto store = [&] {
-#pragma unroll
-    for (int e = 0; e < C; ++e)
-      if (p == 0 && j + e < D) to[e] = o_before[e];
-    to += (size_t)H * D;
-  };
-  fetch(t0, 0);
-#pragma unroll
-  for (int n = 0; n < RPT; ++n) r_before[n] = 0.f;
-  bool first = true;
-  int buf = 0;
-  for (int c0 = t0; c0 < t1; c0 += chunk, buf ^= 1) {
-    const int n_tokens = min(chunk, t1 - c0);
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                        // this chunk has landed, and everyone is done with the other buffer
-    if (c0 + chunk < t1) fetch(c0 + chunk, buf ^ 1);
-    const float* at = sm + (size_t)buf * buffer;
-    const float* v = at + chunk * PER + c;
-    rows(at, u);
-    constexpr int UNROLL = C == 1 && RPT <= 16 ? 4 : 1;
-#pragma unroll UNROLL
-    for (int tt = 0; tt < n_tokens; ++tt, at += PER, v += cols) {
-      float w[RPT], au[RPT], k[RPT], vj[C];
-      rows(at + DP, w);
-      rows(at + 2 * DP, au);
-      rows(at + 3 * DP, k);
-#pragma unroll
-      for (int e = 0; e < C; ++e) vj[e] = v[e];
-      sums();
-      if (!first) store();
-      first = false;
-      rows(at + 4 * DP, r_before);
-      rows(at + PER, u);                    // behind the last token: whatever lies there, not used
-#pragma unroll
-      for (int n = 0; n < RPT; ++n)
-#pragma unroll
-        for (int e = 0; e < C; ++e) col[n][e] = dr_row(w[n], col[n][e], au[n], dot[e], k[n], vj[e]);
+      to += U * next;
     }
+#pragma unroll 1
+    for (; tt < n; ++tt) {                  // the portion's last tokens
+      float o[C];
+      read(a, v, now);
+      a += 4 * PER;
+      v += 4 * COLS;
+      step(now, o);
+#pragma unroll
+      for (int e = 0; e < C; ++e) {
+        float one[1] = {o[e]};
+        dr_sum_lanes<1>(one, p);
+        if (p == 0 && j + e < D) to[e] = one[0];
+      }
+      to += next;
+    }
+    __syncwarp();
+    if ((tid & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dr_smem(&s_empty[b])) : "memory");
   }
-  sums();
-  store();
 #pragma unroll
-  for (int n = 0; n < RPT; ++n)
+  for (int e = 0; e < C; ++e)
 #pragma unroll
-    for (int e = 0; e < C; ++e)
-      if (j + e < D && p + DR_LANES * n < D) S[(size_t)(p + DR_LANES * n) * D + e] = col[n][e];
+    for (int i = 0; i < P; ++i) {
+      float x, y;
+      dr_unpack(col[e][i], x, y);
+      if (held(2 * i, e)) S[(size_t)(p + DR_LANES * 2 * i) * D + e] = x;
+      if (held(2 * i + 1, e)) S[(size_t)(p + DR_LANES * (2 * i + 1)) * D + e] = y;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
 // Steps in which every request brings one token: preparation and recurrence in one launch.  A thread takes four columns of its rows, so
-// that S is read and written in 16-byte pieces that are asked for before anything else; a warp takes 16 columns, a block 16 to 64 of one
+// that S is read and written in 16-byte pieces that are asked for before anything else; a warp takes 8 columns, a block 16 to 64 of one
 // (request, head).  Bound by the chain of the unit key's sum and two column sums.  8 tokens, 32 heads of 64 (8.4 MB of state): 10.4 us
 // as two launches with the columns of S read a float at a time, 4.5 us with this; 64 tokens 51 and 19.
 // ---------------------------------------------------------------------------------------------
 constexpr int DS_MAX_DIM = 128;
 
 template <int RPT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, int k_off, int v_off, int a_off,
                     const float* __restrict__ wpre, const float* __restrict__ a_bias, const float* __restrict__ w_bias,
                     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ req_start,
@@ -204,26 +347,29 @@ delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, 
   constexpr int DP = DR_LANES * RPT;
   __shared__ float s_u[DP], s_w[DP], s_au[DP], s_k[DP], s_r[DP];
   const int tid = threadIdx.x, lane = tid & 31, h = blockIdx.y, r = blockIdx.z;
-  const int p = lane >> 2, c = (tid >> 5) * 16 + (lane & 3) * 4, j = blockIdx.x * cols + c;
+  const int p = lane >> 1, c = (tid >> 5) * 8 + (lane & 1) * 4, j = blockIdx.x * cols + c;
   const int t0 = req_start[r], t1 = req_start[r + 1];
   if (t0 >= t1) return;
   float* S = state + ((size_t)req_slot[r] * H + h) * D * D + j;
-  const bool owns = c < cols && j < D;      // other warps help with the preparation
+  const bool owns = j < D;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 st[RPT];
+  // four columns, the rows in pairs as in the kernel for portions
+  constexpr int P = RPT / 2;
+  dr_pair st[4][P];
 #pragma unroll
-  for (int n = 0; n < RPT; ++n) {
-    const int i = p + DR_LANES * n;
-    st[n] = i < D && owns ? *reinterpret_cast<const float4*>(S + (size_t)i * D) : zero;
+  for (int i = 0; i < P; ++i) {
+    const int x = p + DR_LANES * 2 * i, y = x + DR_LANES;
+    const float4 a = x < D && owns ? *reinterpret_cast<const float4*>(S + (size_t)x * D) : zero;
+    const float4 b = y < D && owns ? *reinterpret_cast<const float4*>(S + (size_t)y * D) : zero;
+    st[0][i] = dr_pack(a.x, b.x); st[1][i] = dr_pack(a.y, b.y); st[2][i] = dr_pack(a.z, b.z); st[3][i] = dr_pack(a.w, b.w);
   }
-  auto over_lanes = [&](float4 x) {
+  auto over_lanes = [&](float (&x)[4]) {
 #pragma unroll
-    for (int o = 4; o < 32; o <<= 1) {
-      x.x += __shfl_xor_sync(0xffffffffu, x.x, o); x.y += __shfl_xor_sync(0xffffffffu, x.y, o);
-      x.z += __shfl_xor_sync(0xffffffffu, x.z, o); x.w += __shfl_xor_sync(0xffffffffu, x.w, o);
-    }
-    return x;
+    for (int o = 2; o < 32; o <<= 1)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] += __shfl_xor_sync(0xffffffffu, x[e], o);
   };
+  auto two = [&](const float* a, int i) { return dr_pack(a[p + DR_LANES * 2 * i], a[p + DR_LANES * (2 * i + 1)]); };
   for (int t = t0; t < t1; ++t) {
     const float* row = proj + (size_t)t * proj_stride + (size_t)h * D;
     float4 v = zero;
@@ -242,34 +388,54 @@ delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, 
       s_au[i] *= u;
     }
     __syncthreads();
-    float4 dot = zero;
+    const float ve[4] = {v.x, v.y, v.z, v.w};
+    dr_pair sum[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int n = 0; n < RPT; ++n) {
-      const float u = s_u[p + DR_LANES * n];
-      dot = make_float4(fmaf(u, st[n].x, dot.x), fmaf(u, st[n].y, dot.y), fmaf(u, st[n].z, dot.z), fmaf(u, st[n].w, dot.w));
-    }
-    dot = over_lanes(dot);
-    float4 o = zero;
+    for (int i = 0; i < P; ++i) {
+      const dr_pair u = two(s_u, i);
 #pragma unroll
-    for (int n = 0; n < RPT; ++n) {
-      const int i = p + DR_LANES * n;
-      const float w = s_w[i], au = s_au[i], k = s_k[i], rr = s_r[i];
-      st[n] = make_float4(dr_row(w, st[n].x, au, dot.x, k, v.x), dr_row(w, st[n].y, au, dot.y, k, v.y),
-                          dr_row(w, st[n].z, au, dot.z, k, v.z), dr_row(w, st[n].w, au, dot.w, k, v.w));
-      o = make_float4(fmaf(rr, st[n].x, o.x), fmaf(rr, st[n].y, o.y), fmaf(rr, st[n].z, o.z), fmaf(rr, st[n].w, o.w));
+      for (int e = 0; e < 4; ++e) sum[e] = dr_fma(u, st[e][i], sum[e]);
     }
-    o = over_lanes(o);
-    if (p == 0 && owns) *reinterpret_cast<float4*>(out + ((size_t)t * H + h) * D + j) = o;
+    float dot[4], o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float x, y;
+      dr_unpack(sum[e], x, y);
+      dot[e] = x + y;
+      sum[e] = 0;
+    }
+    over_lanes(dot);
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const dr_pair w = two(s_w, i), au = two(s_au, i), k = two(s_k, i), rr = two(s_r, i);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        st[e][i] = dr_rows2(w, st[e][i], au, dr_pack(-dot[e], -dot[e]), k, dr_pack(ve[e], ve[e]));
+        sum[e] = dr_fma(rr, st[e][i], sum[e]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float x, y;
+      dr_unpack(sum[e], x, y);
+      o[e] = x + y;
+    }
+    over_lanes(o);
+    if (p == 0 && owns) *reinterpret_cast<float4*>(out + ((size_t)t * H + h) * D + j) = make_float4(o[0], o[1], o[2], o[3]);
     if (t + 1 < t1) __syncthreads();
   }
 #pragma unroll
-  for (int n = 0; n < RPT; ++n) {
-    const int i = p + DR_LANES * n;
-    if (i < D && owns) *reinterpret_cast<float4*>(S + (size_t)i * D) = st[n];
+  for (int i = 0; i < P; ++i) {
+    float a[4], b[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dr_unpack(st[e][i], a[e], b[e]);
+    const int x = p + DR_LANES * 2 * i, y = x + DR_LANES;
+    if (x < D && owns) *reinterpret_cast<float4*>(S + (size_t)x * D) = make_float4(a[0], a[1], a[2], a[3]);
+    if (y < D && owns) *reinterpret_cast<float4*>(S + (size_t)y * D) = make_float4(b[0], b[1], b[2], b[3]);
   }
 }
 
-static int dr_rows(int D) { return D <= 32 ? 4 : D <= 64 ? 8 : D <= 128 ? 16 : 32; }
+static int dr_rows(int D) { return D <= 64 ? 4 : D <= 128 ? 8 : 16; }
 
 // Floats of scratch that a step wants.
 extern "C" long long qb_delta_rule_scratch(int T, int H, int D) {
@@ -280,7 +446,7 @@ extern "C" long long qb_delta_rule_scratch(int T, int H, int D) {
 extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int k_off, int v_off, int a_off,
                              const float* wpre, const float* a_bias, const float* w_bias, float* state,
                              float* out, float* scratch, const int* req_start, const int* req_slot, int R,
-                             int T, int H, int D, float decay_scale, float unit_eps, cudaStream_t stream) {
+                             int T, int H, int D, float decay_scale, float unit_eps, int* status, cudaStream_t stream) {
   if (R <= 0 || T <= 0) return 0;
   if (D <= 0 || D > 256 || H <= 0) return QB_ERR_UNSUPPORTED;
   const int rpt = dr_rows(D), dp = rpt * DR_LANES;
@@ -289,50 +455,40 @@ extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int 
     int CB = 64;
     while (CB > 16 && (CB / 2 >= D || (long)R * H * ((D + CB - 1) / CB) < 132)) CB /= 2;
     const dim3 single((D + CB - 1) / CB, H, R);
-#define DS_SINGLE(N)                                                                                                             \
-  qb_launch(delta_single_kernel<N>, single, 128, 0, stream, proj, proj_stride, r_off, k_off, v_off, a_off, wpre, a_bias, w_bias, \
+#define DS_SINGLE(N)                                                                                                                \
+  qb_launch(delta_single_kernel<N>, single, CB * 4, 0, stream, proj, proj_stride, r_off, k_off, v_off, a_off, wpre, a_bias, w_bias, \
             state, out, req_start, req_slot, H, D, CB, decay_scale, unit_eps)
     if (rpt == 4) DS_SINGLE(4);
-    else if (rpt == 8) DS_SINGLE(8);
-    else DS_SINGLE(16);
+    else DS_SINGLE(8);
 #undef DS_SINGLE
     QB_LAUNCH_CHECK();
     return 0;
   }
   if (((uintptr_t)scratch & 15) != 0) return QB_ERR_BAD_ARG;
   const long warps = (long)T * H;
-  delta_prep_kernel<<<(int)((warps + 3) / 4), 128, 0, stream>>>(proj, proj_stride, r_off, k_off, a_off, wpre, a_bias, w_bias, scratch,
-                                                              T, H, D, dp, decay_scale, unit_eps);
+#define DR_PREP(N)                                                                                                              \
+  delta_prep_kernel<N><<<(int)((warps + 3) / 4), 128, 0, stream>>>(proj, proj_stride, r_off, k_off, a_off, wpre, a_bias, w_bias, \
+                                                                   scratch, T, H, D, decay_scale, unit_eps)
+  if (rpt == 4) DR_PREP(4);
+  else if (rpt == 8) DR_PREP(8);
+  else DR_PREP(16);
+#undef DR_PREP
   QB_LAUNCH_CHECK();
-  // columns a block: all of them (at most 64, or what the registers allow) unless that leaves most SMs idle; then fewer, down to 16
-  // where requests bring portions (the block's threads also fetch the chunks) and down to 4 where every request
-  // brings one token (the state's bytes are what counts, spread over all SMs); whole warps
-  const int min_cols = T > R ? 16 : 4, max_cols = rpt == 32 ? 16 : 64;
-  int splits = (D + max_cols - 1) / max_cols;
-  while ((long)R * H * splits < 132 && (D + 2 * splits - 1) / (2 * splits) >= min_cols) splits *= 2;
-  int cols = (D + splits - 1) / splits;
-  const int C = cols > 16 ? 2 : 1;
-  cols = (cols + 4 * C - 1) / (4 * C) * (4 * C);
-  splits = (D + cols - 1) / cols;
-  const int chunk = rpt <= 8 ? 32 : rpt == 16 ? 16 : 8;
-  const size_t smem = ((size_t)2 * chunk * (DR_ARRAYS * dp + cols) + DR_ARRAYS * dp) * sizeof(float);      // (reads of u go a token past the end)
-  dim3 grid(R, H, splits);
-#define DR_LAUNCH(N, C_)                                                                                   \
-  do {                                                                                                     \
-    auto kern = delta_rule_kernel<N, C_>;                                                                  \
-    if (smem > 48 * 1024) {                                                                                \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-      if (e != cudaSuccess) return (int)e;                                                                 \
-    }                                                                                                      \
-    kern<<<grid, cols / C * DR_LANES, smem, stream>>>(proj, proj_stride, v_off, scratch, state, out, req_start, req_slot, H, D, cols, chunk); \
+  // columns a block: 32 (16 of heads above 64, for their registers), or 16 where that leaves SMs idle
+  const int cols = rpt == 4 && D > 16 && (long)R * H * ((D + 31) / 32) >= 132 ? 32 : 16;
+  const size_t smem = ((size_t)DR_STAGES * DR_STAGE_FLOATS + DR_ARRAYS * dp) * sizeof(float);      // (reads go a token past the end)
+  dim3 grid(R, H, (D + cols - 1) / cols);
+#define DR_LAUNCH(N, U, W)                                                                                                     \
+  do {                                                                                                                         \
+    auto kern = delta_rule_kernel<N, U, W>;                                                                                    \
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                  \
+    if (e != cudaSuccess) return (int)e;                                                                                       \
+    kern<<<grid, 32 * W + 32, smem, stream>>>(proj, proj_stride, v_off, scratch, state, out, req_start, req_slot, T, H, D, status); \
   } while (0)
-  if (rpt == 4 && C == 1) DR_LAUNCH(4, 1);
-  else if (rpt == 4) DR_LAUNCH(4, 2);
-  else if (rpt == 8 && C == 1) DR_LAUNCH(8, 1);
-  else if (rpt == 8) DR_LAUNCH(8, 2);
-  else if (rpt == 16 && C == 1) DR_LAUNCH(16, 1);
-  else if (rpt == 16) DR_LAUNCH(16, 2);
-  else DR_LAUNCH(32, 1);
+  if (rpt == 4 && cols == 32) DR_LAUNCH(4, 8, 8);
+  else if (rpt == 4) DR_LAUNCH(4, 16, 4);
+  else if (rpt == 8) DR_LAUNCH(8, 8, 4);
+  else DR_LAUNCH(16, 4, 4);
 #undef DR_LAUNCH
   QB_LAUNCH_CHECK();
   return 0;

@@ -787,7 +787,7 @@ DELTA_RULE_MAX_DIM = 256
 
 
 def delta_rule(proj, offsets, wpre, a_bias, w_bias, state, out, req_start, req_slot, n_heads: int, dim: int,
-               decay_scale: float, unit_eps: float) -> None:
+               decay_scale: float, unit_eps: float, status=None) -> None:
     """The recurrence ``S <- diag(w) S - (a u)(u^T S) + k v^T``, ``o = S^T r`` per (request, head) over the
     step's tokens, from and into ``state`` ``[slots, heads, dim, dim]`` float32.  ``proj`` float32 ``[T, P]``
     holds r, k, v and the pre-activation of a at the column ``offsets`` (r, k, v, a), heads x dim each;
@@ -809,7 +809,7 @@ def delta_rule(proj, offsets, wpre, a_bias, w_bias, state, out, req_start, req_s
     _check(lib().qb_delta_rule(ctypes.c_void_p(proj.data_ptr()), int(proj.stride(0)), r_off, k_off, v_off, a_off,
                                _p(wpre), _p(a_bias), _p(w_bias), _p(state), _p(out), _p(scratch), _p(req_start),
                                _p(req_slot), R, T, n_heads, dim, ctypes.c_float(decay_scale),
-                               ctypes.c_float(unit_eps), _stream()), "delta_rule", 1 if T == R and dim % 4 == 0 and dim <= 128 else 2)
+                               ctypes.c_float(unit_eps), _p(status), _stream()), "delta_rule", 1 if T == R and dim % 4 == 0 and dim <= 128 else 2)
 
 
 def head_norm_gate(o, proj, gate_off: int, gain, out, n_heads: int, dim: int, eps: float, gate: str = "sigmoid") -> None:
