@@ -8,7 +8,7 @@
 //   o_t = S_t^T r
 //
 // A column j of S never meets another column.  Sixteen lanes share one: lane p has its rows p + 16 n.  Its part of u^T S (and of the output)
-// is two sums, over the rows of even and of odd n in the order of n, added up; the sixteen parts meet two by two (lanes 1, 2, 4, 8 apart).
+// is two sums, over the rows of even and of odd n in the order of n, added up; the sixteen parts meet two by two (lanes 8, 4, 2, 1 apart).
 // Both kernels below do exactly these operations, so a position's numbers depend neither on the cut nor on the batch, not even by rounding.
 // (Portions once ran in chunks of 16 tokens as products, 240 us for the prompt below, whose outputs were 1.7e-7 off float64 against 0.9e-7 here
 // and depended on what shared the step.)
@@ -61,8 +61,10 @@ __device__ __forceinline__ float dr_unit(const float* __restrict__ k, int D, int
 // chain of a token: two packed multiply-adds, four exchanges (29 cycles each), three more packed operations; the rows of the next token are
 // read meanwhile, and the sixteen tokens' outputs are summed over the lanes together (16 exchanges a column instead of 64).  Eight lanes
 // a column have one exchange less but twice the reads of shared memory, behind which the exchanges queue (281 us for the prompt below, 240 with
-// sixteen; with a branch a token around the step 338).  Measured on a B200, one portion of 2,048 tokens, 32 heads of 64: 331 + 42 us with eight
-// lanes a column, 264 + 30 with this; the same in a step (the chain and the preparation).
+// sixteen; with a branch a token around the step 338).  Enough portions to fill the SMs are bound by the reads of the five arrays, which
+// four columns a lane halve.  Measured on a B200, chain and preparation, with eight lanes a column / with this: one portion of 2,048 tokens, 32
+// heads of 64, 378 / 298 us, 8 of 512 355 / 329, 16 heads of 128 588 / 410 and 574 / 502, 8 heads of 256, 300 tokens, 172 / 114, 23 single
+// tokens beside 512 236 / 160.
 // ---------------------------------------------------------------------------------------------
 constexpr int DR_MAX_COLS = 32, DR_CHUNK_FLOATS = 16 * DR_ARRAYS * 64, DR_STAGE_FLOATS = DR_CHUNK_FLOATS + 16 * DR_MAX_COLS, DR_STAGES = 4;
 
@@ -104,13 +106,13 @@ delta_prep_kernel(const float* __restrict__ proj, int proj_stride, int r_off, in
   }
 }
 
-// The sums over the sixteen lanes of N values each, N at most 16: lane p then holds the value dr_first<N>(p) (lanes that differ in the bits
-// beyond N's hold the same).
+// The sums over the sixteen lanes of N values each, N at most 16: lane p then holds the value dr_first<N>(p) (lanes that differ in their lower
+// bits only, those that N does not use, hold the same).
 template <int N>
 __device__ __forceinline__ void dr_sum_lanes(float (&x)[N], int p) {
   int n = N;
 #pragma unroll
-  for (int d = 1; d < DR_LANES; d <<= 1) {
+  for (int d = DR_LANES / 2; d > 0; d >>= 1) {
     if (n > 1) {
       n >>= 1;
       const bool upper = p & d;
@@ -129,7 +131,7 @@ template <int N>
 __device__ __forceinline__ int dr_first(int p) {
   int first = 0, n = N;
 #pragma unroll
-  for (int d = 1; d < N; d <<= 1) {
+  for (int d = DR_LANES / 2; n > 1; d >>= 1) {
     n >>= 1;
     first += p & d ? n : 0;
   }
@@ -157,17 +159,17 @@ __device__ __forceinline__ bool dr_wait(unsigned bar, unsigned parity, volatile 
   return false;
 }
 
-// RPT: rows of a column a lane holds (D <= 16 RPT); U: tokens whose outputs are summed together; W: warps that walk the tokens, one more
-// brings them
-template <int RPT, int U, int W>
-__global__ void __launch_bounds__(32 * W + 32, W == 8 ? 2 : 1)
+// RPT: rows of a column a lane holds (D <= 16 RPT); C: columns a lane; U: tokens whose outputs are summed together.  Four warps walk the
+// tokens, one more brings them.
+template <int RPT, int C, int U>
+__global__ void __launch_bounds__(160, C == 4 ? 2 : 1)
 delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, const float* __restrict__ scratch, float* __restrict__ state,
                   float* __restrict__ out, const int* __restrict__ req_start, const int* __restrict__ req_slot, int T, int H, int D, int* status) {
   extern __shared__ __align__(16) float sm[];
   __shared__ __align__(8) unsigned long long s_full[DR_STAGES], s_empty[DR_STAGES];
   __shared__ int s_abort;
-  constexpr int DP = DR_LANES * RPT, PER = DR_ARRAYS * DP, P = RPT / 2, C = 2;
-  constexpr int CHUNK = DR_CHUNK_FLOATS / PER, COLS = 4 * W;    // 16 tokens of heads up to 64, fewer of larger ones
+  constexpr int DP = DR_LANES * RPT, PER = DR_ARRAYS * DP, P = RPT / 2, W = 4;
+  constexpr int CHUNK = DR_CHUNK_FLOATS / PER, COLS = 2 * W * C;    // 16 tokens of heads up to 64, fewer of larger ones
   const int r = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int p = tid % DR_LANES, col0 = blockIdx.z * COLS, jj = tid / DR_LANES * C, j = col0 + jj;
   const int t0 = req_start[r], t1 = req_start[r + 1];
@@ -236,7 +238,8 @@ delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, co
   };
   auto read = [&](unsigned a, unsigned v, Token& t) {
     rows(a, t.u); rows(a + 8 * DP, t.au); rows(a + 4 * DP, t.w); rows(a + 12 * DP, t.k); rows(a + 16 * DP, t.r);
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t.v[0]), "=f"(t.v[1]) : "r"(v));
+    if constexpr (C == 2) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t.v[0]), "=f"(t.v[1]) : "r"(v));
+    else asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.v[0]), "=f"(t.v[1]), "=f"(t.v[2]), "=f"(t.v[3]) : "r"(v));
   };
   auto step = [&](const Token& t, float (&o)[C]) {             // this lane's part of the output
     float dot[C];
@@ -250,7 +253,7 @@ delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, co
       dot[e] = a + b;
     }
 #pragma unroll
-    for (int d = 1; d < DR_LANES; d <<= 1)
+    for (int d = DR_LANES / 2; d > 0; d >>= 1)
 #pragma unroll
       for (int e = 0; e < C; ++e) dot[e] += __shfl_xor_sync(0xffffffffu, dot[e], d);
 #pragma unroll
@@ -296,7 +299,7 @@ delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, co
 #pragma unroll
       for (int e = 0; e < C; ++e) {
         dr_sum_lanes<U>(o[e], p);
-        if ((U == DR_LANES || p < U) && j + e < D) to[(size_t)first * next + e] = o[e][0];
+        if (p % (DR_LANES / U) == 0 && j + e < D) to[(size_t)first * next + e] = o[e][0];
       }
       to += U * next;
     }
@@ -331,14 +334,14 @@ delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, co
 
 // ---------------------------------------------------------------------------------------------
 // Steps in which every request brings one token: preparation and recurrence in one launch.  A thread takes four columns of its rows, so
-// that S is read and written in 16-byte pieces that are asked for before anything else; a warp takes 8 columns, a block 16 to 64 of one
+// that S is read and written in 16-byte pieces that are asked for before anything else; a warp takes 16 columns, a block 16 to 64 of one
 // (request, head).  Bound by the chain of the unit key's sum and two column sums.  8 tokens, 32 heads of 64 (8.4 MB of state): 10.4 us
 // as two launches with the columns of S read a float at a time, 4.5 us with this; 64 tokens 51 and 19.
 // ---------------------------------------------------------------------------------------------
 constexpr int DS_MAX_DIM = 128;
 
 template <int RPT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128, RPT == 4 ? 6 : 3)
 delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, int k_off, int v_off, int a_off,
                     const float* __restrict__ wpre, const float* __restrict__ a_bias, const float* __restrict__ w_bias,
                     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ req_start,
@@ -347,29 +350,38 @@ delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, 
   constexpr int DP = DR_LANES * RPT;
   __shared__ float s_u[DP], s_w[DP], s_au[DP], s_k[DP], s_r[DP];
   const int tid = threadIdx.x, lane = tid & 31, h = blockIdx.y, r = blockIdx.z;
-  const int p = lane >> 1, c = (tid >> 5) * 8 + (lane & 1) * 4, j = blockIdx.x * cols + c;
+  const int p = lane >> 2, c = (tid >> 5) * 16 + (lane & 3) * 4, j = blockIdx.x * cols + c;
   const int t0 = req_start[r], t1 = req_start[r + 1];
   if (t0 >= t1) return;
   float* S = state + ((size_t)req_slot[r] * H + h) * D * D + j;
-  const bool owns = j < D;
+  const bool owns = c < cols && j < D;      // other warps help with the preparation
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  // four columns, the rows in pairs as in the kernel for portions
+  // four columns; a lane stands for the lanes p (v = 0) and p + 8 (v = 1) of the kernel for portions, whose parts meet first
   constexpr int P = RPT / 2;
-  dr_pair st[4][P];
+  dr_pair st[4][2][P];
 #pragma unroll
-  for (int i = 0; i < P; ++i) {
-    const int x = p + DR_LANES * 2 * i, y = x + DR_LANES;
-    const float4 a = x < D && owns ? *reinterpret_cast<const float4*>(S + (size_t)x * D) : zero;
-    const float4 b = y < D && owns ? *reinterpret_cast<const float4*>(S + (size_t)y * D) : zero;
-    st[0][i] = dr_pack(a.x, b.x); st[1][i] = dr_pack(a.y, b.y); st[2][i] = dr_pack(a.z, b.z); st[3][i] = dr_pack(a.w, b.w);
-  }
-  auto over_lanes = [&](float (&x)[4]) {
+  for (int v = 0; v < 2; ++v)
 #pragma unroll
-    for (int o = 2; o < 32; o <<= 1)
+    for (int i = 0; i < P; ++i) {
+      const int x = p + 8 * v + DR_LANES * 2 * i, y = x + DR_LANES;
+      const float4 a = x < D && owns ? *reinterpret_cast<const float4*>(S + (size_t)x * D) : zero;
+      const float4 b = y < D && owns ? *reinterpret_cast<const float4*>(S + (size_t)y * D) : zero;
+      st[0][v][i] = dr_pack(a.x, b.x); st[1][v][i] = dr_pack(a.y, b.y); st[2][v][i] = dr_pack(a.z, b.z); st[3][v][i] = dr_pack(a.w, b.w);
+    }
+  auto over_lanes = [&](const dr_pair (&sum)[4][2], float (&x)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float a, b, c, d;
+      dr_unpack(sum[e][0], a, b);
+      dr_unpack(sum[e][1], c, d);
+      x[e] = (a + b) + (c + d);
+    }
+#pragma unroll
+    for (int o = 16; o > 2; o >>= 1)
 #pragma unroll
       for (int e = 0; e < 4; ++e) x[e] += __shfl_xor_sync(0xffffffffu, x[e], o);
   };
-  auto two = [&](const float* a, int i) { return dr_pack(a[p + DR_LANES * 2 * i], a[p + DR_LANES * (2 * i + 1)]); };
+  auto two = [&](const float* a, int v, int i) { return dr_pack(a[p + 8 * v + DR_LANES * 2 * i], a[p + 8 * v + DR_LANES * (2 * i + 1)]); };
   for (int t = t0; t < t1; ++t) {
     const float* row = proj + (size_t)t * proj_stride + (size_t)h * D;
     float4 v = zero;
@@ -389,50 +401,45 @@ delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, 
     }
     __syncthreads();
     const float ve[4] = {v.x, v.y, v.z, v.w};
-    dr_pair sum[4] = {0, 0, 0, 0};
+    dr_pair sum[4][2] = {};
 #pragma unroll
-    for (int i = 0; i < P; ++i) {
-      const dr_pair u = two(s_u, i);
+    for (int w = 0; w < 2; ++w)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) sum[e] = dr_fma(u, st[e][i], sum[e]);
-    }
-    float dot[4], o[4];
+      for (int i = 0; i < P; ++i) {
+        const dr_pair u = two(s_u, w, i);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float x, y;
-      dr_unpack(sum[e], x, y);
-      dot[e] = x + y;
-      sum[e] = 0;
-    }
-    over_lanes(dot);
-#pragma unroll
-    for (int i = 0; i < P; ++i) {
-      const dr_pair w = two(s_w, i), au = two(s_au, i), k = two(s_k, i), rr = two(s_r, i);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        st[e][i] = dr_rows2(w, st[e][i], au, dr_pack(-dot[e], -dot[e]), k, dr_pack(ve[e], ve[e]));
-        sum[e] = dr_fma(rr, st[e][i], sum[e]);
+        for (int e = 0; e < 4; ++e) sum[e][w] = dr_fma(u, st[e][w][i], sum[e][w]);
       }
-    }
+    float dot[4], o[4];
+    over_lanes(sum, dot);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float x, y;
-      dr_unpack(sum[e], x, y);
-      o[e] = x + y;
-    }
-    over_lanes(o);
+    for (int e = 0; e < 4; ++e) sum[e][0] = sum[e][1] = 0;
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        const dr_pair w = two(s_w, z, i), au = two(s_au, z, i), k = two(s_k, z, i), rr = two(s_r, z, i);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          st[e][z][i] = dr_rows2(w, st[e][z][i], au, dr_pack(-dot[e], -dot[e]), k, dr_pack(ve[e], ve[e]));
+          sum[e][z] = dr_fma(rr, st[e][z][i], sum[e][z]);
+        }
+      }
+    over_lanes(sum, o);
     if (p == 0 && owns) *reinterpret_cast<float4*>(out + ((size_t)t * H + h) * D + j) = make_float4(o[0], o[1], o[2], o[3]);
     if (t + 1 < t1) __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < P; ++i) {
-    float a[4], b[4];
+  for (int v = 0; v < 2; ++v)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) dr_unpack(st[e][i], a[e], b[e]);
-    const int x = p + DR_LANES * 2 * i, y = x + DR_LANES;
-    if (x < D && owns) *reinterpret_cast<float4*>(S + (size_t)x * D) = make_float4(a[0], a[1], a[2], a[3]);
-    if (y < D && owns) *reinterpret_cast<float4*>(S + (size_t)y * D) = make_float4(b[0], b[1], b[2], b[3]);
-  }
+    for (int i = 0; i < P; ++i) {
+      float a[4], b[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dr_unpack(st[e][v][i], a[e], b[e]);
+      const int x = p + 8 * v + DR_LANES * 2 * i, y = x + DR_LANES;
+      if (x < D && owns) *reinterpret_cast<float4*>(S + (size_t)x * D) = make_float4(a[0], a[1], a[2], a[3]);
+      if (y < D && owns) *reinterpret_cast<float4*>(S + (size_t)y * D) = make_float4(b[0], b[1], b[2], b[3]);
+    }
 }
 
 static int dr_rows(int D) { return D <= 64 ? 4 : D <= 128 ? 8 : 16; }
@@ -456,7 +463,7 @@ extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int 
     while (CB > 16 && (CB / 2 >= D || (long)R * H * ((D + CB - 1) / CB) < 132)) CB /= 2;
     const dim3 single((D + CB - 1) / CB, H, R);
 #define DS_SINGLE(N)                                                                                                                \
-  qb_launch(delta_single_kernel<N>, single, CB * 4, 0, stream, proj, proj_stride, r_off, k_off, v_off, a_off, wpre, a_bias, w_bias, \
+  qb_launch(delta_single_kernel<N>, single, 128, 0, stream, proj, proj_stride, r_off, k_off, v_off, a_off, wpre, a_bias, w_bias, \
             state, out, req_start, req_slot, H, D, CB, decay_scale, unit_eps)
     if (rpt == 4) DS_SINGLE(4);
     else DS_SINGLE(8);
@@ -474,21 +481,23 @@ extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int 
   else DR_PREP(16);
 #undef DR_PREP
   QB_LAUNCH_CHECK();
-  // columns a block: 32 (16 of heads above 64, for their registers), or 16 where that leaves SMs idle
-  const int cols = rpt == 4 && D > 16 && (long)R * H * ((D + 31) / 32) >= 132 ? 32 : 16;
+  // four columns a lane, 32 a block (heads of at most 128, for the registers), or two and 16 where that leaves SMs idle
+  const bool wide = rpt <= 8 && D > 16 && (long)R * H * ((D + 31) / 32) >= 132;
+  const int cols = wide ? 32 : 16;
   const size_t smem = ((size_t)DR_STAGES * DR_STAGE_FLOATS + DR_ARRAYS * dp) * sizeof(float);      // (reads go a token past the end)
   dim3 grid(R, H, (D + cols - 1) / cols);
-#define DR_LAUNCH(N, U, W)                                                                                                     \
+#define DR_LAUNCH(N, C, U)                                                                                                     \
   do {                                                                                                                         \
-    auto kern = delta_rule_kernel<N, U, W>;                                                                                    \
+    auto kern = delta_rule_kernel<N, C, U>;                                                                                    \
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                  \
     if (e != cudaSuccess) return (int)e;                                                                                       \
-    kern<<<grid, 32 * W + 32, smem, stream>>>(proj, proj_stride, v_off, scratch, state, out, req_start, req_slot, T, H, D, status); \
+    kern<<<grid, 160, smem, stream>>>(proj, proj_stride, v_off, scratch, state, out, req_start, req_slot, T, H, D, status);    \
   } while (0)
-  if (rpt == 4 && cols == 32) DR_LAUNCH(4, 8, 8);
-  else if (rpt == 4) DR_LAUNCH(4, 16, 4);
-  else if (rpt == 8) DR_LAUNCH(8, 8, 4);
-  else DR_LAUNCH(16, 4, 4);
+  if (rpt == 4 && wide) DR_LAUNCH(4, 4, 8);
+  else if (rpt == 4) DR_LAUNCH(4, 2, 16);
+  else if (rpt == 8 && wide) DR_LAUNCH(8, 4, 4);
+  else if (rpt == 8) DR_LAUNCH(8, 2, 8);
+  else DR_LAUNCH(16, 2, 4);
 #undef DR_LAUNCH
   QB_LAUNCH_CHECK();
   return 0;
