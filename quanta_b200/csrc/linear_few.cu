@@ -57,16 +57,18 @@ __device__ __forceinline__ void lf_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NT: tiles of 8 input rows.  D, XD: pieces of W and of x a warp holds ahead.
-template <int NT, int D, int XD, int MINB, typename O>
+// NT: tiles of 8 input rows.  D, XD: pieces of W and of x a warp holds ahead.  GLU: W is [gate; up] of N features each, a block takes 8 rows of
+// both, and out = silu(gate) * up of the sums, each rounded to bfloat16 first (what a product and an activation kernel leave).
+template <int NT, int D, int XD, int MINB, bool GLU, typename O>
 __global__ void __launch_bounds__(LF_WARPS * 32, MINB) linear_few_kernel(LinearFew a, int early) {
   static_assert(D % XD == 0, "the ring of x divides the ring of W");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * 16;
+  constexpr int FEATS = GLU ? 8 : 16;
+  const int n0 = blockIdx.x * FEATS;
   const int kbs = (a.K + LF_KB - 1) / LF_KB;
   const __nv_bfloat16* wr[2];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) wr[h] = a.w + (size_t)min(n0 + h * 8 + g, a.N - 1) * a.K + t * 16;
+  for (int h = 0; h < 2; ++h) wr[h] = a.w + (size_t)(GLU ? min(n0 + g, a.N - 1) + h * a.N : min(n0 + h * 8 + g, a.N - 1)) * a.K + t * 16;
   const __nv_bfloat16* xr[NT];
 #pragma unroll
   for (int n = 0; n < NT; ++n) xr[n] = a.x + (size_t)min(n * 8 + g, a.rows - 1) * a.K + t * 16;
@@ -115,21 +117,36 @@ __global__ void __launch_bounds__(LF_WARPS * 32, MINB) linear_few_kernel(LinearF
 #pragma unroll
     for (int i = 0; i < 4; ++i) part[warp][n * 8 + 2 * t + (i & 1)][g + 8 * (i >> 1)] = acc[n][i];
   __syncthreads();
-  for (int v = threadIdx.x; v < TOK * ROWS; v += LF_WARPS * 32) {
-    const int tok = v / ROWS, row = v % ROWS;
-    if (tok >= a.rows || n0 + row >= a.N) continue;
+  auto sum = [&](int tok, int row) {
     float s = part[0][tok][row];
 #pragma unroll
     for (int w = 1; w < LF_WARPS; ++w) s += part[w][tok][row];
+    return s;
+  };
+  for (int v = threadIdx.x; v < TOK * FEATS; v += LF_WARPS * 32) {
+    const int tok = v / FEATS, row = v % FEATS;
+    if (tok >= a.rows || n0 + row >= a.N) continue;
+    float s = sum(tok, row);
+    if (GLU) {
+      const float gate = __bfloat162float(__float2bfloat16_rn(s)), up = __bfloat162float(__float2bfloat16_rn(sum(tok, row + 8)));
+      s = gate / (1.f + expf(-gate)) * up;
+    }
     reinterpret_cast<O*>(a.out)[(size_t)tok * a.N + n0 + row] = qb_from_float<O>(s);
   }
 }
 
 template <int NT, int D, int XD, int MINB>
-static int linear_few_launch(const LinearFew& a, int out_dtype, int early, cudaStream_t stream) {
+static int linear_few_launch(const LinearFew& a, int out_dtype, bool glu, int early, cudaStream_t stream) {
+  if (glu) {
+    const int grid = (a.N + 7) / 8;
+    if (early) qb_launch(linear_few_kernel<NT, D, XD, MINB, true, __nv_bfloat16>, grid, LF_WARPS * 32, 0, stream, a, 1);
+    else linear_few_kernel<NT, D, XD, MINB, true, __nv_bfloat16><<<grid, LF_WARPS * 32, 0, stream>>>(a, 0);
+    QB_LAUNCH_CHECK();
+    return 0;
+  }
   const int grid = (a.N + 15) / 16;
-  if (early) QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(linear_few_kernel<NT, D, XD, MINB, O>, grid, LF_WARPS * 32, 0, stream, a, 1));
-  else QB_DISPATCH_DTYPE(out_dtype, O, (linear_few_kernel<NT, D, XD, MINB, O><<<grid, LF_WARPS * 32, 0, stream>>>(a, 0)));
+  if (early) QB_DISPATCH_DTYPE(out_dtype, O, qb_launch(linear_few_kernel<NT, D, XD, MINB, false, O>, grid, LF_WARPS * 32, 0, stream, a, 1));
+  else QB_DISPATCH_DTYPE(out_dtype, O, (linear_few_kernel<NT, D, XD, MINB, false, O><<<grid, LF_WARPS * 32, 0, stream>>>(a, 0)));
   QB_LAUNCH_CHECK();
   return 0;
 }
@@ -143,14 +160,23 @@ extern "C" int qb_linear_few_takes(int rows, int K, int N) {
 
 // K a multiple of 16; x and w on 32 bytes.  early: W was written two launches before this one at the latest (or by the host), so that
 // its first pieces are read before the launch before this one has ended.
+static int linear_few_any(const LinearFew& a, int out_dtype, bool glu, int early, cudaStream_t stream) {
+  const int rows = a.rows, N = glu ? 2 * a.N : a.N;
+  if (rows <= 0 || N <= 0) return 0;
+  if (a.K <= 0 || a.K % 16 || ((uintptr_t)a.x & 31) || ((uintptr_t)a.w & 31)) return QB_ERR_BAD_ARG;
+  if (rows > 32) return QB_ERR_UNSUPPORTED;
+  if (rows <= 8) return linear_few_launch<1, 4, 4, 2>(a, out_dtype, glu, early, stream);
+  if (rows <= 16) return linear_few_launch<2, 4, 2, 2>(a, out_dtype, glu, early, stream);
+  if ((N + 15) / 16 <= 148) return linear_few_launch<4, 4, 2, 1>(a, out_dtype, glu, early, stream);
+  return linear_few_launch<4, 2, 1, 2>(a, out_dtype, glu, early, stream);
+}
+
 extern "C" int qb_linear_few(const void* x, const void* w, void* out, int out_dtype, int rows, int K, int N, int early,
                              cudaStream_t stream) {
-  if (rows <= 0 || N <= 0) return 0;
-  if (K <= 0 || K % 16 || ((uintptr_t)x & 31) || ((uintptr_t)w & 31)) return QB_ERR_BAD_ARG;
-  if (rows > 32) return QB_ERR_UNSUPPORTED;
-  const LinearFew a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, rows, K, N};
-  if (rows <= 8) return linear_few_launch<1, 4, 4, 2>(a, out_dtype, early, stream);
-  if (rows <= 16) return linear_few_launch<2, 4, 2, 2>(a, out_dtype, early, stream);
-  if ((N + 15) / 16 <= 148) return linear_few_launch<4, 4, 2, 1>(a, out_dtype, early, stream);
-  return linear_few_launch<4, 2, 1, 2>(a, out_dtype, early, stream);
+  return linear_few_any(LinearFew{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, rows, K, N}, out_dtype, false, early, stream);
+}
+
+// out [rows, I] bfloat16 = silu(x W[:I]^T) * (x W[I:]^T), W [2 I, K]
+extern "C" int qb_linear_few_silu(const void* x, const void* w, void* out, int rows, int K, int I, int early, cudaStream_t stream) {
+  return linear_few_any(LinearFew{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, rows, K, I}, QB_BF16, true, early, stream);
 }

@@ -213,16 +213,25 @@ def normed_add_rmsnorm(h: torch.Tensor, y: torch.Tensor | None, y_gain: torch.Te
                        weight: torch.Tensor | None, eps: float, out: torch.Tensor | None,
                        rows: torch.Tensor | None = None, store_h: bool = True, *, y_scale: float = 1.0,
                        y_bias: torch.Tensor | None = None, extra: torch.Tensor | None = None, extra_scale: float = 1.0,
-                       extra_bias: torch.Tensor | None = None) -> None:
+                       extra_bias: torch.Tensor | None = None, conv: tuple | None = None) -> None:
     """``h += y_gain * z * rsqrt(mean(z^2) + y_eps)`` (float32) and ``out = weight * h * rsqrt(mean(h^2) + eps)``: a
     sublayer's output that is normed before it joins the stream, and the norm that follows, in one launch.
     ``z = y_scale * (sum_s y[:, s] + y_bias) + extra_scale * (extra + extra_bias)``: ``y`` float32 ``[T, H]`` or
     ``[T, S, H]`` (slots added in order), ``extra`` float32 ``[T, H]`` or None, the biases ``[H]`` or None.
     ``weight`` None with ``out``: ``out`` is the stream itself (for a sublayer that reads it without a norm);
-    ``y`` None: nothing joins.  ``rows`` / ``store_h`` / ``out`` None as in ``add_rmsnorm``."""
+    ``y`` None: nothing joins.  ``rows`` / ``store_h`` / ``out`` None as in ``add_rmsnorm``.  ``conv`` = (weight ``[H, taps]``, state
+    ``[slots, taps - 1, H]``, request slots ``[T]``), for steps in which every request brings one token and sizes of
+    ``normed_add_conv_supported``: ``out`` is the short convolution of ``short_conv`` (the input added back) over the normed row, which
+    becomes the newest of the request's state rows."""
     _want(h, torch.float32, "h")
     T, H = h.shape
     S = 1
+    if conv is not None:
+        cw, cs, slots = conv
+        _want(cw, torch.float32, "conv weight"); _want(cs, torch.float32, "conv state"); _want(slots, torch.int32, "request slots")
+        if (rows is not None or out is None or weight is None or y is None or slots.numel() != T
+                or cw.shape[0] != H or tuple(cs.shape[1:]) != (cw.shape[1] - 1, H)):
+            raise ValueError("normed_add_rmsnorm: the convolution does not fit")
     if y is not None:
         _want(y, torch.float32, "y"); _want(y_gain, torch.float32, "y_gain")
         S = y.shape[1] if y.dim() == 3 else 1
@@ -249,7 +258,13 @@ def normed_add_rmsnorm(h: torch.Tensor, y: torch.Tensor | None, y_gain: torch.Te
                                        ctypes.c_float(extra_scale), _p(extra_bias), _p(y_gain), ctypes.c_float(y_eps),
                                        _p(weight) if out is not None else ctypes.c_void_p(0), _p(out),
                                        _code(out) if out is not None else F32, _p(rows), n, H, ctypes.c_float(eps),
-                                       int(store_h), _stream()), "normed_add_rmsnorm")
+                                       int(store_h), *((_p(conv[0]), _p(conv[1]), _p(conv[2]), conv[0].shape[1]) if conv is not None else
+                                                       (_p(None), _p(None), _p(None), 0)), _stream()), "normed_add_rmsnorm")
+
+
+def normed_add_conv_supported(H: int, taps: int) -> bool:
+    """Whether ``normed_add_rmsnorm`` takes a convolution over rows of ``H`` numbers."""
+    return bool(lib().qb_normed_add_conv_supported(int(H), int(taps)))
 
 
 def residual_add(h: torch.Tensor, delta: torch.Tensor) -> None:
@@ -605,6 +620,16 @@ def linear_few(x, w, out, early: bool = False) -> None:
     _check(lib().qb_linear_few(_p(x), _p(w), _p(out), _code(out), n, K, w.shape[0], int(early), _stream()), "linear_few")
 
 
+def linear_few_silu(x, w, out, early: bool = False) -> None:
+    """``out [n, I] = silu(x @ w[:I].T) * (x @ w[I:].T)`` in bfloat16, both products rounded to bfloat16 first; as ``linear_few``."""
+    for t, name in ((x, "x"), (w, "w"), (out, "out")):
+        _want(t, torch.bfloat16, name)
+    n, K = x.shape
+    if w.shape[1] != K or w.shape[0] % 2 or tuple(out.shape) != (n, w.shape[0] // 2):
+        raise ValueError("linear_few_silu: shape mismatch")
+    _check(lib().qb_linear_few_silu(_p(x), _p(w), _p(out), n, K, w.shape[0] // 2, int(early), _stream()), "linear_few_silu")
+
+
 EXPERT_ACT_SILU, EXPERT_ACT_CLAMPED = 0, 1
 
 
@@ -869,6 +894,19 @@ def tanh_cols(x, off: int, n: int, out) -> None:
         raise ValueError("tanh_cols: shape mismatch")
     _check(lib().qb_tanh_cols(ctypes.c_void_p(x.data_ptr()), int(x.stride(0)), int(off), _p(out), _code(out), T, n,
                               _stream()), "tanh_cols")
+
+
+TANH_PRODUCT_MAX_ROWS, TANH_PRODUCT_MAX_RANK = 32, 64
+
+
+def tanh_product(x, off: int, w, out) -> None:
+    """``out [T, N] = bfloat16(tanh(x[:, off : off + n])) @ w [N, n].T`` in float32 for at most ``TANH_PRODUCT_MAX_ROWS`` rows and an inner
+    size n of at most ``TANH_PRODUCT_MAX_RANK``: the two factors of a low-rank pair of projections in one launch."""
+    _want(x, torch.float32, "x"); _want(w, torch.bfloat16, "w"); _want(out, torch.float32, "out")
+    T, (N, n) = x.shape[0], w.shape
+    if tuple(out.shape) != (T, N) or off + n > x.shape[1] or x.stride(1) != 1:
+        raise ValueError("tanh_product: shape mismatch")
+    _check(lib().qb_tanh_product(ctypes.c_void_p(x.data_ptr()), int(x.stride(0)), int(off), _p(w), _p(out), T, n, N, _stream()), "tanh_product")
 
 
 LATENT_MAX_RANK = 512

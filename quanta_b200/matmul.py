@@ -100,3 +100,13 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     if out_dtype is not None and out_dtype != x.dtype:
         return torch.mm(x, w.t(), out_dtype=out_dtype)
     return torch.mm(x, w.t())
+
+
+def linear_silu(x: torch.Tensor, w: torch.Tensor, ctx=None) -> torch.Tensor | None:
+    """``silu(x @ w[:I].T) * (x @ w[I:].T)`` of a few bfloat16 rows in one launch, both products rounded to bfloat16 first; None where
+    ``linear`` would not take its kernel for few rows."""
+    if w.dim() != 2 or w.shape[0] % 2 or not _few_bfloat16_rows(x, w, None):
+        return None
+    out = empty_rows(x.shape[0], w.shape[0] // 2, dtype=torch.bfloat16, device=x.device)
+    kernels.linear_few_silu(x, w, out, early=getattr(ctx, "settled", False))
+    return out

@@ -64,9 +64,13 @@ class DeltaRule(Mixer):
     def forward(self, x, ctx, cache, state):
         T, HD = x.shape[0], self.H * self.D
         proj = linear(x, self.w_in, out_dtype=torch.float32, ctx=ctx)
-        inner = empty_rows(T, self.L, dtype=x.dtype, device=x.device)
-        kernels.tanh_cols(proj, 5 * HD, self.L, inner)
-        wpre = linear(inner, self.w_decay, out_dtype=torch.float32, ctx=ctx)
+        if T <= kernels.TANH_PRODUCT_MAX_ROWS and self.L <= kernels.TANH_PRODUCT_MAX_RANK and self.w_decay.dtype == torch.bfloat16:
+            wpre = torch.empty((T, HD), dtype=torch.float32, device=x.device)
+            kernels.tanh_product(proj, 5 * HD, self.w_decay, wpre)
+        else:
+            inner = empty_rows(T, self.L, dtype=x.dtype, device=x.device)
+            kernels.tanh_cols(proj, 5 * HD, self.L, inner)
+            wpre = linear(inner, self.w_decay, out_dtype=torch.float32, ctx=ctx)
         o = torch.empty((T, self.H, self.D), dtype=torch.float32, device=x.device)
         kernels.delta_rule(proj, (0, HD, 2 * HD, 4 * HD), wpre, self.a_bias, self.w_bias, state[self.state_name], o,
                            ctx.req_start, ctx.req_slot, self.H, self.D, self.decay_scale, self.unit_eps, status=ctx.status)

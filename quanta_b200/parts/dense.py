@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 
 from .. import kernels
-from ..matmul import empty_rows, linear
+from ..matmul import empty_rows, linear, linear_silu
 from .base import Addends, FeedForward, TensorSpec, register
 
 
@@ -55,6 +55,10 @@ class GatedDense(FeedForward):
 
     def forward(self, x, ctx):
         T = x.shape[0]
+        if self.activation == "silu" and not self.biases:
+            act = linear_silu(x, self.w_gate_up, ctx)
+            if act is not None:
+                return linear(act, self.w_down, out_dtype=torch.float32, ctx=ctx)
         gate_up = linear(x, self.w_gate_up, ctx=ctx)
         act = empty_rows(T, self.inner, dtype=x.dtype, device=x.device)
         if self.activation == "silu" and not self.biases:

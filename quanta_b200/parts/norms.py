@@ -78,7 +78,7 @@ class RMSNorm(Norm):
 
 
 def normed_add(h, delta: NormedPending, weight, eps: float, out, rows, store_h: bool, groups: int = 1,
-               history=None, n_history: int = 0, history_weights=None) -> None:
+               history=None, n_history: int = 0, history_weights=None, conv=None) -> None:
     """``h += norm(delta)`` and ``out = weight * rms(h)`` (``weight`` None: ``out = h``) in one launch; the addends
     of the sublayer's output (slots, biases, a second branch) are summed there too.  Norms in groups, branches that
     are normed before they are summed, and a stream that becomes a weighted sum of earlier results (``history``)
@@ -94,7 +94,15 @@ def normed_add(h, delta: NormedPending, weight, eps: float, out, rows, store_h: 
         return
     kernels.normed_add_rmsnorm(h, a.y, delta.norm.weight, delta.norm.eps, weight, eps, out, rows=rows, store_h=store_h,
                                y_scale=a.scale, y_bias=a.bias, extra=a.extra, extra_scale=a.extra_scale,
-                               extra_bias=a.extra_bias)
+                               extra_bias=a.extra_bias, conv=conv)
+
+
+def takes_conv(norm, delta, taps: int) -> bool:
+    """Whether ``normed_add`` of ``delta`` with the norm ``norm`` takes a short convolution of so many taps into its launch (of single tokens)."""
+    if not (isinstance(norm, RMSNorm) and norm.groups == 1 and isinstance(delta, NormedPending) and isinstance(delta.norm, RMSNorm)):
+        return False
+    a = delta.addends
+    return delta.norm.groups == 1 and not a.branch_normed and kernels.normed_add_conv_supported(norm.width, taps)
 
 
 def add_sum(h, a: Addends, out, weight=None, groups: int = 1, eps: float = 0.0, rows=None, store_h: bool = True) -> None:

@@ -1,0 +1,93 @@
+"""Launches of a step of few rows that do the work of two: each against the two launches (bit by bit where the operations are the same ones) or
+against float64."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _gen(seed):
+    return torch.Generator(device=DEV).manual_seed(seed)
+
+
+@pytest.mark.parametrize("n,k,inner", [(1, 64, 8), (3, 2048, 5632), (8, 528, 20), (9, 256, 9), (16, 1024, 96), (20, 512, 40), (32, 2048, 1100)])
+def test_gate_up_and_silu(n, k, inner):
+    from quanta_b200 import kernels
+    g = _gen(n + inner)
+    x, w = (torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16) for s in ((n, k), (2 * inner, k)))
+    both, want, out = (torch.empty((n, m), device=DEV, dtype=torch.bfloat16) for m in (2 * inner, inner, inner))
+    kernels.linear_few(x, w, both)
+    kernels.silu_mul(both, want)
+    kernels.linear_few_silu(x, w, out)
+    assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("T,n,N,off,wide", [(1, 1, 5, 0, 4), (2, 16, 300, 3, 20), (32, 16, 128, 0, 16), (7, 17, 129, 2, 64), (9, 64, 2048, 8, 80)])
+def test_tanh_product(T, n, N, off, wide):
+    """One rounding of the result; tanhf may be two units off where its rounding to bfloat16 turns, half a unit of that being 2^-9."""
+    from quanta_b200 import kernels
+    g = _gen(T * n)
+    x, w = torch.randn(T, wide, device=DEV, generator=g), torch.randn(N, n, device=DEV, generator=g).to(torch.bfloat16)
+    out = torch.empty(T, N, device=DEV)
+    kernels.tanh_product(x, off, w, out)
+    inner = torch.empty((T, n), device=DEV, dtype=torch.bfloat16)
+    kernels.tanh_cols(x, off, n, inner)
+    want = inner.double() @ w.double().T
+    assert torch.all((out.double() - want).abs() <= 2.0 ** -24 * want.abs())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,H,taps,slots", [(1, 8, 3, 0), (3, 256, 4, 2), (8, 2048, 3, 0), (5, 4096, 4, 0)])
+def test_norm_and_convolution(T, H, taps, slots, dtype):
+    """Norm, stream, outputs and state as the norm into float32 rows and the convolution's own launch leave them."""
+    from quanta_b200 import kernels
+    g = _gen(T * H)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    h, gy, w, cw = r(T, H), r(H), r(H), r(H, taps)
+    y = r(T, slots, H) if slots else r(T, H)
+    extra = r(T, H) if slots else None
+    state = r(T + 3, taps - 1, H)
+    order = torch.randperm(T + 3, device=DEV, generator=g)[:T].int()
+    h2, state2, normed = h.clone(), state.clone(), torch.empty(T, H, device=DEV)
+    out, want = (torch.empty(T, H, device=DEV, dtype=dtype) for _ in range(2))
+    starts = torch.arange(T + 1, dtype=torch.int32, device=DEV)
+    kernels.normed_add_rmsnorm(h2, y, gy, 1e-6, w, 1e-5, normed, extra=extra, extra_scale=0.5)
+    kernels.short_conv(normed, cw, state2, want, starts[:-1], starts, order)
+    kernels.normed_add_rmsnorm(h, y, gy, 1e-6, w, 1e-5, out, extra=extra, extra_scale=0.5, conv=(cw, state, order))
+    assert torch.equal(h, h2) and torch.equal(state, state2) and torch.equal(out, want)
+    with pytest.raises(ValueError):
+        kernels.normed_add_rmsnorm(h, y, gy, 1e-6, w, 1e-5, out, conv=(cw, state, order[:-1].contiguous()))
+
+
+@pytest.mark.parametrize("lens,ranges", [([1] * 70, 3), ([1] * 31 + [5] + [1] * 40, 1), ([40, 1, 1, 3] * 12, 2), ([1] * 33, 40)])
+def test_latent_attention_of_many_requests(lens, ranges):
+    """Every request's rows are found whatever their number: the same numbers as a request alone."""
+    from quanta_b200 import kernels
+    g, H, C, R, page = _gen(len(lens)), 4, 64, 16, 16
+    T, before = sum(lens), [int(x) for x in torch.randint(0, 150, (len(lens),), generator=torch.Generator().manual_seed(3))]
+    mp = max(b + n for b, n in zip(before, lens)) // page + 1
+    cache = torch.randn(len(lens) * mp, 1, page, C + R, device=DEV, generator=g).to(torch.bfloat16)
+    table = torch.randperm(len(lens) * mp, generator=torch.Generator().manual_seed(1)).int().view(len(lens), mp).to(DEV)
+    q_lat, q_rot = torch.randn(H, T, C, device=DEV, generator=g), torch.randn(T, H, R, device=DEV, generator=g)
+    sink = torch.randn(H, device=DEV, generator=g)
+
+    def run(rows):
+        at = [sum(lens[:r]) for r in rows]
+        pick = torch.tensor([a + i for a, r in zip(at, rows) for i in range(lens[r])], device=DEV)
+        pos = torch.tensor([before[r] + i for r in rows for i in range(lens[r])], dtype=torch.int32, device=DEV)
+        req = torch.tensor([k for k, r in enumerate(rows) for _ in range(lens[r])], dtype=torch.int32, device=DEV)
+        starts = torch.tensor([0, *torch.tensor([lens[r] for r in rows]).cumsum(0).tolist()], dtype=torch.int32, device=DEV)
+        out, st = torch.empty(H, len(pick), C, device=DEV, dtype=torch.bfloat16), kernels.new_status(DEV)
+        kernels.latent_attend(q_lat[:, pick].contiguous(), q_rot[pick].contiguous(), cache, sink, out, pos, req, table[rows].contiguous(),
+                              0.1, ranges, st, req_start=starts)
+        assert st.tolist()[0] == 0
+        return out
+
+    whole, at = run(list(range(len(lens)))), 0
+    assert torch.isfinite(whole.float()).all()
+    for r, n in enumerate(lens):
+        assert torch.equal(run([r]), whole[:, at: at + n]), r
+        at += n
