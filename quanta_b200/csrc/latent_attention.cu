@@ -99,20 +99,37 @@ extern "C" int qb_latent_write(const float* dkv, int dkv_stride, const float* ga
 }
 
 // ---------------------------------------------------------------------------------------------
+// A warp a (token, head), eight a block, pieces of four where they start on 16 bytes (2,048 tokens of 16 heads of 128 + 64: 35 us with a
+// block of 64 threads each and a number at a time, 10 here).
+constexpr int LQ_WARPS = 8;
+
 template <typename A>
-__global__ void latent_query_kernel(const float* __restrict__ q, const float* __restrict__ inv_freq,
-                                    A* __restrict__ q_plain, float* __restrict__ q_rot,
-                                    const int* __restrict__ tok_pos, int T, int H, int D, int R, int rd,
-                                    int interleaved) {
+__global__ void __launch_bounds__(LQ_WARPS * 32)
+latent_query_kernel(const float* __restrict__ q, const float* __restrict__ inv_freq, A* __restrict__ q_plain, float* __restrict__ q_rot,
+                    const int* __restrict__ tok_pos, int T, int H, int D, int R, int rd, int interleaved, int pieces) {
   qb_follow();
-  const int t = blockIdx.x, h = blockIdx.y;
-  const float* row = q + ((size_t)t * H + h) * (D + R);
+  const long unit = (long)blockIdx.x * LQ_WARPS + (threadIdx.x >> 5);
+  if (unit >= (long)T * H) return;
+  const int t = (int)(unit / H), h = (int)(unit % H), lane = threadIdx.x & 31;
+  const float* row = q + unit * (D + R);
   A* qp = q_plain + ((size_t)h * T + t) * D;
-  for (int i = threadIdx.x; i < D; i += blockDim.x) qp[i] = qb_from_float<A>(row[i]);
   const int half = rd / 2;
   const float pos = (float)tok_pos[t];
-  float* qr = q_rot + ((size_t)t * H + h) * R;
-  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+  float* qr = q_rot + unit * R;
+  if (pieces) {
+    for (int i = lane * 4; i < D; i += 128) {
+      const float4 v = *reinterpret_cast<const float4*>(row + i);
+      if constexpr (sizeof(A) == 2) {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+        *reinterpret_cast<uint2*>(qp + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+      } else {
+        *reinterpret_cast<float4*>(qp + i) = v;
+      }
+    }
+  } else {
+    for (int i = lane; i < D; i += 32) qp[i] = qb_from_float<A>(row[i]);
+  }
+  for (int i = lane; i < half; i += 32) {
     float sn, cs;
     sincosf(pos * inv_freq[i], &sn, &cs);
     const int ia = interleaved ? 2 * i : i, ib = interleaved ? ia + 1 : ia + half;
@@ -120,7 +137,7 @@ __global__ void latent_query_kernel(const float* __restrict__ q, const float* __
     qr[ia] = u * cs - v * sn;
     qr[ib] = v * cs + u * sn;
   }
-  for (int i = rd + threadIdx.x; i < R; i += blockDim.x) qr[i] = row[D + i];
+  for (int i = rd + lane; i < R; i += 32) qr[i] = row[D + i];
 }
 
 extern "C" int qb_latent_query(const float* q, const float* inv_freq, void* q_plain, int dtype, float* q_rot,
@@ -128,9 +145,10 @@ extern "C" int qb_latent_query(const float* q, const float* inv_freq, void* q_pl
                                cudaStream_t stream) {
   if (T <= 0) return 0;
   if (rd % 2 || rd < 0 || rd > R) return QB_ERR_BAD_ARG;
-  dim3 grid(T, H);
-  QB_DISPATCH_DTYPE(dtype, A, qb_launch(latent_query_kernel<A>, grid, 64, 0, stream,
-      q, inv_freq, (A*)q_plain, q_rot, tok_pos, T, H, D, R, rd, interleaved));
+  const int pieces = D % 4 == 0 && R % 4 == 0 && (((uintptr_t)q | (uintptr_t)q_plain) & 15) == 0;
+  const long units = (long)T * H;
+  QB_DISPATCH_DTYPE(dtype, A, qb_launch(latent_query_kernel<A>, (unsigned)((units + LQ_WARPS - 1) / LQ_WARPS), LQ_WARPS * 32, 0, stream,
+      q, inv_freq, (A*)q_plain, q_rot, tok_pos, T, H, D, R, rd, interleaved, pieces));
   QB_LAUNCH_CHECK();
   return 0;
 }
@@ -266,11 +284,13 @@ extern "C" int qb_latent_attend(const void* q_lat, int q_lat_dtype, const float*
 // ranges' sums scaled to top; out[h, t, :] = sum of the ranges' vectors scaled to top / denominator, times
 // sigmoid(gate[t, h]) where there is a gate (float32, rows of gate_stride).  The
 // first warp works out the ranges' weights (a lane a range, two for more than 32), then a thread a channel
-// adds the ranges in index order, 16 reads ahead; ranges without a key (maximum minus infinity) are not read.
+// adds the ranges in index order.  Bound by two reads of memory, the channels' and the weights', which run together (8 tokens of 16 heads, 32
+// ranges: 7.1 us with the channels read after the weights, four at a time; 3.8 here).  Ranges without a key (maximum minus infinity)
+// are left out.
 constexpr int LA_MAX_RANGES = 64;
 
-template <typename A>
-__global__ void latent_merge_kernel(const float* __restrict__ part, const float* __restrict__ sink,
+template <typename A, int N>           // N: ranges, at most; a multiple of 16
+__global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restrict__ part, const float* __restrict__ sink,
                                     const float* __restrict__ gate, int gate_stride, A* __restrict__ out, int T, int H,
                                     int C, int n_ranges) {
   qb_follow();
@@ -278,6 +298,13 @@ __global__ void latent_merge_kernel(const float* __restrict__ part, const float*
   __shared__ float s_inv;
   const int t = blockIdx.x / H, h = blockIdx.x % H;
   const float* src = part + ((size_t)t * H + h) * n_ranges * (C + 2);
+  // this thread's channel of every range is asked for before the weights are known (ranges without a key hold anything; not used)
+  float x[N];
+  auto ask = [&](int d) {
+#pragma unroll
+    for (int s = 0; s < N; ++s) x[s] = s < n_ranges && d < C ? src[(size_t)s * (C + 2) + 2 + d] : 0.f;
+  };
+  ask(threadIdx.x);
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     float ms[2], ls[2];
@@ -304,15 +331,11 @@ __global__ void latent_merge_kernel(const float* __restrict__ part, const float*
   const float inv = s_inv;
   A* dst = out + ((size_t)h * T + t) * C;
   for (int d = threadIdx.x; d < C; d += blockDim.x) {
+    if (d != (int)threadIdx.x) ask(d);
     float v = 0.f;
-    for (int s0 = 0; s0 < n_ranges; s0 += 16) {
-      float x[16];
 #pragma unroll
-      for (int s = 0; s < 16; ++s) x[s] = s0 + s < n_ranges && !(s_w[s0 + s] < 0.f) ? src[(size_t)(s0 + s) * (C + 2) + 2 + d] : 0.f;
-#pragma unroll
-      for (int s = 0; s < 16; ++s)
-        if (s0 + s < n_ranges && !(s_w[s0 + s] < 0.f)) v += x[s] * s_w[s0 + s];
-    }
+    for (int s = 0; s < N; ++s)
+      if (s < n_ranges && !(s_w[s] < 0.f)) v += x[s] * s_w[s];
     dst[d] = qb_from_float<A>(v * inv);
   }
 }
@@ -322,8 +345,14 @@ extern "C" int qb_latent_merge(const float* part, const float* sink, const float
   if (T <= 0) return 0;
   if (n_ranges < 1 || n_ranges > LA_MAX_RANGES) return QB_ERR_UNSUPPORTED;
   const int threads = C >= 256 ? 256 : C >= 128 ? 128 : 64;
-  QB_DISPATCH_DTYPE(dtype, A, qb_launch(latent_merge_kernel<A>, T * H, threads, 0, stream, part, sink, gate, gate_stride,
-                                                                                 (A*)out, T, H, C, n_ranges));
+#define LA_MERGE(N) qb_launch(latent_merge_kernel<A, N>, T * H, threads, 0, stream, part, sink, gate, gate_stride, (A*)out, T, H, C, n_ranges)
+  QB_DISPATCH_DTYPE(dtype, A, {
+    if (n_ranges <= 16) LA_MERGE(16);
+    else if (n_ranges <= 32) LA_MERGE(32);
+    else if (n_ranges <= 48) LA_MERGE(48);
+    else LA_MERGE(64);
+  });
+#undef LA_MERGE
   QB_LAUNCH_CHECK();
   return 0;
 }
@@ -396,7 +425,7 @@ latent_attend_mma_kernel(const float* __restrict__ q_lat, const float* __restric
   const int range = blockIdx.y;
   if (warp == 0) {
     // the last rows, which see the most keys, first.  A lane a request, 32 at a time: one thread that walked the requests had a read
-    // of memory in each step (8 requests of one token 13.6 us, MEASURED)
+    // of memory in each step (with 8 requests 13.6 us, 12.6 so and 10.9 with ranges without a key leaving at once and a range a tile)
     int acc = 0, found = 0;
     const int item = (int)gridDim.x - 1 - (int)blockIdx.x;
     for (int r0 = 0; r0 < n_req && !found; r0 += 32) {
@@ -424,6 +453,20 @@ latent_attend_mma_kernel(const float* __restrict__ q_lat, const float* __restric
   const int t0 = req_start[req], n_rows = (req_start[req + 1] - t0) * H;
   const int rows_here = min(LM_ROWS, n_rows - row0);
   const int* bt = block_table + (size_t)req * bt_stride;
+  const int last_pos = tok_pos[t0 + (row0 + rows_here - 1) / H];
+  const int first_pos = tok_pos[t0 + row0 / H];
+  const int first_seen = window > 0 && first_pos >= window ? first_pos - window + 1 : 0;    // by any row of the block
+  const int tile_first = first_seen / LM_KEYS, tile_end = last_pos / LM_KEYS + 1;
+  const int per = (tile_end - tile_first + n_ranges - 1) / n_ranges;
+  const int tile_lo = tile_first + range * per, tile_hi = min(tile_end, tile_lo + per);
+  if (part != nullptr && tile_lo >= tile_hi) {      // a range without a key: the merge reads nothing else of it
+    for (int i = tid; i < rows_here; i += blockDim.x) {
+      float* dst = part + (((size_t)(t0 + (row0 + i) / H) * H + (row0 + i) % H) * n_ranges + range) * (C + 2);
+      dst[0] = -INFINITY;
+      dst[1] = 0.f;
+    }
+    return;
+  }
   // queries: latent part and rotated part side by side, times the score scale, bfloat16; rows past the end zero
   for (int i = warp; i < LM_ROWS; i += (int)(blockDim.x >> 5)) {
     __nv_bfloat16* dst = sQ + (size_t)i * WP;
@@ -448,12 +491,6 @@ latent_attend_mma_kernel(const float* __restrict__ q_lat, const float* __restric
     my_lo[e] = window > 0 && my_pos[e] >= window ? my_pos[e] - window + 1 : 0;
   }
   const bool rg_active = rg * 16 < rows_here;
-  const int last_pos = tok_pos[t0 + (row0 + rows_here - 1) / H];
-  const int first_pos = tok_pos[t0 + row0 / H];
-  const int first_seen = window > 0 && first_pos >= window ? first_pos - window + 1 : 0;    // by any row of the block
-  const int tile_first = first_seen / LM_KEYS, tile_end = last_pos / LM_KEYS + 1;
-  const int per = (tile_end - tile_first + n_ranges - 1) / n_ranges;
-  const int tile_lo = tile_first + range * per, tile_hi = min(tile_end, tile_lo + per);
 
   constexpr float LOG2E = 1.4426950408889634f;    // scores and maxima are kept times log2(e): a weight is one 2^x
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};

@@ -739,6 +739,20 @@ def slot_record(*, position: int = 0, prompt_len: int = 0, drawn: int = 0, last:
     return torch.tensor(rec, dtype=torch.int32)
 
 
+def state_table(tensors: list) -> torch.Tensor | None:
+    """The table of ``zero_state_rows`` for contiguous state tensors ``[slots, ...]``, which it does not keep alive."""
+    if not all(t.is_contiguous() for t in tensors):
+        raise ValueError("state_table: the tensors must be contiguous")
+    rows = [(t.data_ptr(), t[0].numel() * t.element_size()) for t in tensors if t.numel() > 0]
+    return torch.tensor(rows, dtype=torch.int64).to(tensors[0].device) if rows else None
+
+
+def zero_state_rows(table, slot: int) -> None:
+    """Zero row ``slot`` of every tensor of ``state_table`` in one launch."""
+    _want(table, torch.int64, "table")
+    _check(lib().qb_zero_state_rows(_p(table), table.shape[0], int(slot), _stream()), "zero_state_rows")
+
+
 def slots_advance(slots, req_slot, req_start, req_len_after, n_requests: int, status) -> None:
     """Move each request's position in its state slot to what it holds after the step; a slot that is free
     or at another position than the step assumes is recorded in ``status``."""

@@ -90,14 +90,15 @@ class LatentAttention(Mixer):
 
     def _ranges(self, ctx, tensor_cores: bool) -> int:
         """Ranges a token's keys are cut into: one when the step has blocks enough to fill the GPU, else as
-        many as give every SM two blocks, each at least 128 keys long."""
+        many as give every SM two blocks, each at least 128 keys long (the tensor cores' blocks: as many as run at once, a tile of 64
+        keys at least; a request has blocks of its own)."""
+        keys = ctx.max_len_after if self.window is None else min(ctx.max_len_after, self.window + kernels.LATENT_MMA_ROWS)
         if tensor_cores:
-            blocks = -(-ctx.n_tokens * self.H // kernels.LATENT_MMA_ROWS)
+            blocks = max(-(-ctx.n_tokens * self.H // kernels.LATENT_MMA_ROWS), int(ctx.req_start.numel()) - 1)
+            by_work, by_keys = 296 // max(1, blocks), -(-max(1, keys) // 64)
         else:
             blocks = ctx.n_tokens * -(-self.H // 8)
-        by_work = -(-296 // max(1, blocks))
-        keys = ctx.max_len_after if self.window is None else min(ctx.max_len_after, self.window + kernels.LATENT_MMA_ROWS)
-        by_keys = -(-max(1, keys) // 128)
+            by_work, by_keys = -(-296 // max(1, blocks)), -(-max(1, keys) // 128)
         return max(1, min(64, by_work, by_keys))
 
     def forward(self, x, ctx, cache, state):

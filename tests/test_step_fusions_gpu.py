@@ -91,3 +91,13 @@ def test_latent_attention_of_many_requests(lens, ranges):
     for r, n in enumerate(lens):
         assert torch.equal(run([r]), whole[:, at: at + n]), r
         at += n
+
+
+def test_state_rows_are_zeroed_together():
+    """Rows of whole 16-byte pieces, of odd numbers of bytes and of none; the neighbours stay."""
+    from quanta_b200 import kernels
+    state = [torch.ones(shape, dtype=dt, device=DEV) for shape, dt in (((5, 3, 128), torch.float32), ((5, 7), torch.float32), ((5, 3), torch.bfloat16),
+                                                                       ((5,), torch.int64), ((5, 0), torch.float32), ((5, 64, 64, 64), torch.float32))]
+    kernels.zero_state_rows(kernels.state_table(state), 3)
+    for t in state:
+        assert not t[3].any() and all(bool((t[i] == 1).all()) for i in (0, 1, 2, 4))
