@@ -61,16 +61,16 @@ __device__ __forceinline__ float dd_remote(const float* p, int rank) {     // th
 
 struct DecodeArgs {
   const int *dec_tok, *tok_pos, *tok_req, *block_table;
-  int bt_stride, nq, nkv, page_size, page_shift, num_pages, window, chunk, S;
+  int bt_stride, nq, nkv, page_size, page_shift, num_pages, window, chunk, S, early;
   float scale, cap;
   int* status;
 };
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(DD_MAX_WARPS * 32)
-attn_decode_direct_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
+attn_decode_direct_kernel(const __nv_bfloat16* q, const __nv_bfloat16* __restrict__ k_cache,      // q: see qb_follow
                           const __nv_bfloat16* __restrict__ v_cache, __nv_bfloat16* __restrict__ out, const DecodeArgs P) {
-  qb_follow();
+  if (!P.early) qb_follow();
   extern __shared__ __align__(128) unsigned char dd_smem[];
   // rings first; then a warp's sums, a head's 128 numbers in the order 8 e + g | 64 + 8 e + g
   __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(dd_smem);
@@ -87,12 +87,6 @@ attn_decode_direct_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
   constexpr float LOG2E = 1.4426950408889634f;
   const float scale_log2 = P.scale * LOG2E;
   const int* bt = P.block_table + (size_t)P.tok_req[tok] * P.bt_stride;
-
-  uint4 qa[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    qa[i] = g < G ? *reinterpret_cast<const uint4*>(q + ((size_t)tok * P.nq + kvh * G + g) * DD_HD + (t + 4 * i) * 8)
-                  : make_uint4(0, 0, 0, 0);
 
   // rounds of 16 keys: first, first + step, ... up to the group of the last key
   const int step = warps * P.S, last = pos / DD_KEYS;
@@ -119,6 +113,22 @@ attn_decode_direct_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
       dd_copy16(dst + (uint32_t)(DD_KEYS * 256 + i * 256 + ((piece ^ (((i >> 1) & 3) << 1)) << 4)), v_cache + from, row >= 0);
     }
   };
+
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  const int r0 = lo / DD_KEYS + rank * warps + warp;
+  int at = place(r0);
+  const int at1 = place(r0 + step);
+  // the launch before writes the token's own key and value and its queries; the keys of the rounds before its own lie in the cache since
+  // earlier steps and are asked for while that launch ends
+  const bool e0 = P.early && r0 < last, e1 = P.early && r0 + step < last;      // the same for the whole warp
+  if (e0) { ask(at, 0); commit(); }
+  if (e1) { ask(at1, 1); commit(); }
+  if (P.early) qb_follow();
+  uint4 qa[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    qa[i] = g < G ? *reinterpret_cast<const uint4*>(q + ((size_t)tok * P.nq + kvh * G + g) * DD_HD + (t + 4 * i) * 8)
+                  : make_uint4(0, 0, 0, 0);
 
   float m = -INFINITY, l = 0.f;                      // of head g: the maximum of all lanes, this lane's part of the sum
   float o[8][4];                                     // tile e: dims 8 g + e and 64 + 8 g + e of heads 2 t and 2 t + 1
@@ -205,16 +215,10 @@ attn_decode_direct_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
     }
   };
 
-  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
   auto which = [](int at) { return __ballot_sync(0xffffffffu, at >= 0) & 0xffffu; };
-  const int r0 = lo / DD_KEYS + rank * warps + warp;
-  int at = place(r0);
-  const int at1 = place(r0 + step);
   unsigned now = which(at), next = which(at1);       // the keys of the round in use and of the one behind it
-  ask(at, 0);
-  commit();
-  ask(at1, 1);
-  commit();
+  if (!e0) { ask(at, 0); commit(); }
+  if (!e1) { ask(at1, 1); commit(); }
   at = place(r0 + 2 * step);
   int stage = 0;
   for (int r = r0; r <= last; r += step) {           // the same for the whole warp
@@ -338,11 +342,13 @@ extern "C" int qb_attn_decode_direct_wins(int n_dec, int nq, int nkv, int hd, in
   return here <= 13.0 + all * (4 * DD_HD) / 5.0e6 + 0.2 * segments ? 1 : 0;
 }
 
-// dec_tok: the token rows of the n_dec single tokens; longest: keys of the longest request (an upper bound is enough).
+// dec_tok: the token rows of the n_dec single tokens; longest: keys of the longest request (an upper bound is enough).  early: the two
+// launches before this one write no key or value but the tokens' own and neither the tables nor the tokens' places; the kernel then reads
+// these before the launch before it has ended.
 extern "C" int qb_attn_decode_direct(const void* q, const void* k_cache, const void* v_cache, void* out, const int* dec_tok, int n_dec,
                                      const int* tok_pos, const int* tok_req, const int* block_table, int bt_stride, int nq, int nkv,
                                      int hd, int page_size, int num_pages, float scale, int window, int longest, int two_part,
-                                     float cap, int chunk, int* status, cudaStream_t stream) {
+                                     float cap, int chunk, int early, int* status, cudaStream_t stream) {
   if (n_dec <= 0) return 0;
   if (chunk < 0 || (cap > 0.f && !two_part)) return QB_ERR_BAD_ARG;
   if (!qb_attn_decode_direct_supported(nq, nkv, hd) || page_size <= 0) return QB_ERR_UNSUPPORTED;
@@ -358,7 +364,7 @@ extern "C" int qb_attn_decode_direct(const void* q, const void* k_cache, const v
   int warps, S;
   dd_shape(units, dd_keys(longest, window, chunk), warps, S);
   const DecodeArgs P{dec_tok, tok_pos, tok_req, block_table, bt_stride, nq, nkv, page_size, shift, num_pages, window, chunk, S,
-                     scale, cap, status};
+                     early, scale, cap, status};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(units * S));
   cfg.blockDim = dim3((unsigned)(warps * 32));

@@ -45,7 +45,7 @@ __device__ __forceinline__ dr_pair dr_rows2(dr_pair w, dr_pair s, dr_pair au, dr
 __device__ __forceinline__ float dr_decay(float x, float scale) { return expf(-scale * (1.f / (1.f + expf(-x)))); }
 __device__ __forceinline__ float dr_rate(float x) { return 1.f / (1.f + expf(-x)); }
 // 1 / |k| of a head, by one warp: the same additions wherever it is called
-__device__ __forceinline__ float dr_unit(const float* __restrict__ k, int D, int lane, float unit_eps) {
+__device__ __forceinline__ float dr_unit(const float* k, int D, int lane, float unit_eps) {
   float ss = 0.f;
   for (int i = lane; i < D; i += 32) ss = fmaf(k[i], k[i], ss);
   return 1.f / sqrtf(qb_warp_sum(ss) + unit_eps);
@@ -342,19 +342,19 @@ constexpr int DS_MAX_DIM = 128;
 
 template <int RPT>
 __global__ void __launch_bounds__(128, RPT == 4 ? 6 : 3)
-delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, int k_off, int v_off, int a_off,
-                    const float* __restrict__ wpre, const float* __restrict__ a_bias, const float* __restrict__ w_bias,
+delta_single_kernel(const float* proj, int proj_stride, int r_off, int k_off, int v_off, int a_off,
+                    const float* wpre, const float* __restrict__ a_bias, const float* __restrict__ w_bias,
                     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ req_start,
-                    const int* __restrict__ req_slot, int H, int D, int cols, float decay_scale, float unit_eps) {
-  qb_follow();
+                    const int* __restrict__ req_slot, int H, int D, int cols, float decay_scale, float unit_eps, int early) {
+  if (!early) qb_follow();
   constexpr int DP = DR_LANES * RPT;
   __shared__ float s_u[DP], s_w[DP], s_au[DP], s_k[DP], s_r[DP];
   const int tid = threadIdx.x, lane = tid & 31, h = blockIdx.y, r = blockIdx.z;
   const int p = lane >> 2, c = (tid >> 5) * 16 + (lane & 3) * 4, j = blockIdx.x * cols + c;
   const int t0 = req_start[r], t1 = req_start[r + 1];
-  if (t0 >= t1) return;
+  if (!early && t0 >= t1) return;
   float* S = state + ((size_t)req_slot[r] * H + h) * D * D + j;
-  const bool owns = c < cols && j < D;      // other warps help with the preparation
+  const bool owns = c < cols && j < D && t0 < t1;      // other warps help with the preparation
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   // four columns; a lane stands for the lanes p (v = 0) and p + 8 (v = 1) of the kernel for portions, whose parts meet first
   constexpr int P = RPT / 2;
@@ -368,6 +368,9 @@ delta_single_kernel(const float* __restrict__ proj, int proj_stride, int r_off, 
       const float4 b = y < D && owns ? *reinterpret_cast<const float4*>(S + (size_t)y * D) : zero;
       st[0][v][i] = dr_pack(a.x, b.x); st[1][v][i] = dr_pack(a.y, b.y); st[2][v][i] = dr_pack(a.z, b.z); st[3][v][i] = dr_pack(a.w, b.w);
     }
+  // the state is on its way while the launch before ends
+  if (early) qb_follow();
+  if (t0 >= t1) return;
   auto over_lanes = [&](const dr_pair (&sum)[4][2], float (&x)[4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -449,11 +452,12 @@ extern "C" long long qb_delta_rule_scratch(int T, int H, int D) {
   return T <= 0 || H <= 0 || D <= 0 || D > 256 ? 0 : (long long)T * H * DR_ARRAYS * DR_LANES * dr_rows(D);
 }
 
-// scratch: qb_delta_rule_scratch floats, on 16 bytes
+// scratch: qb_delta_rule_scratch floats, on 16 bytes.  early: the two launches before this one write neither the state nor req_start and
+// req_slot (a step of single tokens then reads them before the launch before it has ended).
 extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int k_off, int v_off, int a_off,
                              const float* wpre, const float* a_bias, const float* w_bias, float* state,
                              float* out, float* scratch, const int* req_start, const int* req_slot, int R,
-                             int T, int H, int D, float decay_scale, float unit_eps, int* status, cudaStream_t stream) {
+                             int T, int H, int D, float decay_scale, float unit_eps, int early, int* status, cudaStream_t stream) {
   if (R <= 0 || T <= 0) return 0;
   if (D <= 0 || D > 256 || H <= 0) return QB_ERR_UNSUPPORTED;
   const int rpt = dr_rows(D), dp = rpt * DR_LANES;
@@ -464,7 +468,7 @@ extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int 
     const dim3 single((D + CB - 1) / CB, H, R);
 #define DS_SINGLE(N)                                                                                                                \
   qb_launch(delta_single_kernel<N>, single, 128, 0, stream, proj, proj_stride, r_off, k_off, v_off, a_off, wpre, a_bias, w_bias, \
-            state, out, req_start, req_slot, H, D, CB, decay_scale, unit_eps)
+            state, out, req_start, req_slot, H, D, CB, decay_scale, unit_eps, early)
     if (rpt == 4) DS_SINGLE(4);
     else DS_SINGLE(8);
 #undef DS_SINGLE

@@ -594,12 +594,12 @@ constexpr int RS_FEW = 16;
 
 template <typename TX>
 __global__ void __launch_bounds__(RS_WARPS * 32)
-router_few_kernel(const TX* __restrict__ x, const float* __restrict__ gate, const float* __restrict__ bias,
+router_few_kernel(const TX* x, const float* __restrict__ gate, const float* __restrict__ bias,
                   float* logits, int* idx_out, float* __restrict__ w_out, int T, int E, int K, int k, int renorm,
                   float scale, int select, int* counters, int BM, int* __restrict__ plan,
                   int* __restrict__ sorted_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
-                  int max_tiles, int* status, int tiled) {
-  qb_follow();
+                  int max_tiles, int* status, int tiled, int early) {
+  if (!early) qb_follow();
   constexpr int EPB = RS_WARPS / RS_QUARTERS;
   extern __shared__ __align__(16) unsigned char rs_smem[];      // [RS_TT][K] of TX: the tile's token rows
   __shared__ PlanShared sh;
@@ -623,6 +623,7 @@ router_few_kernel(const TX* __restrict__ x, const float* __restrict__ gate, cons
     }
   };
   fetch(u0 + lane);                                        // into flight before anything else
+  if (early) qb_follow();                                  // (the gate is settled, the token rows are not)
   {
     const int n8 = nt * K * (int)sizeof(TX) / 8;
     const unsigned char* src = reinterpret_cast<const unsigned char*>(x + (size_t)t0 * K);
@@ -676,11 +677,12 @@ extern "C" int qb_router_small_selects(int T, int E, int k) {
 
 // x [T, K] float32 or bfloat16, gate [E, K] float32, logits [T, E] float32 (always written).  select = 1 (see
 // qb_router_small_selects): idx_out / w_out [T, k] and the expert plan as qb_moe_plan lays it down;
-// counters: 1 + ceil(T / 8) int32 that are zero before the call and zero after it.
+// counters: 1 + ceil(T / 8) int32 that are zero before the call and zero after it.  early: the two launches before this
+// one do not write the gate (steps of up to RS_FEW tokens then start to read it before the launch before has ended).
 extern "C" int qb_router_small(const void* x, int x_dtype, const float* gate, const float* bias, float* logits,
                                int* idx_out, float* w_out, int T, int E, int K, int k, int renorm, float scale,
                                int select, int* counters, int BM, int* plan, int* sorted_pair, int* tile_expert,
-                               int* tile_row0, int max_tiles, int* status, int tiled, cudaStream_t stream) {
+                               int* tile_row0, int max_tiles, int* status, int tiled, int early, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (E <= 0 || K <= 0) return QB_ERR_BAD_ARG;
   if (tiled <= 0 || tiled > E) tiled = E;
@@ -701,7 +703,7 @@ extern "C" int qb_router_small(const void* x, int x_dtype, const float* gate, co
     if (err != cudaSuccess) return (int)err;                                                                                      \
     qb_launch(router_few_kernel<TX>, grid, RS_WARPS * 32, smem, stream, (const TX*)x, gate, bias, logits, idx_out, w_out, T, E, K, k,      \
                                                                  renorm, scale, select, counters, BM, plan, sorted_pair,           \
-                                                                 tile_expert, tile_row0, max_tiles, status, tiled);                \
+                                                                 tile_expert, tile_row0, max_tiles, status, tiled, early);         \
   } while (0)
     if (x_dtype == QB_F32) QB_RS_FEW(float);
     else if (x_dtype == QB_BF16) QB_RS_FEW(__nv_bfloat16);

@@ -453,10 +453,12 @@ def attn_decode_direct_wins(n_dec: int, nq: int, nkv: int, hd: int, longest: int
 
 
 def attn_decode_direct(q, k_cache, v_cache, out, dec_tok, n_dec: int, tok_pos, tok_req, block_table, scale: float, window: int,
-                       longest: int, status, *, two_part: bool = False, softcap: float = 0.0, chunk: int = 0) -> None:
+                       longest: int, status, *, two_part: bool = False, softcap: float = 0.0, chunk: int = 0, early: bool = False) -> None:
     """bfloat16 attention of the single tokens ``dec_tok`` in one launch, heads of 128 and at most eight q heads a kv head; ``longest``:
     keys of the longest request (an upper bound is enough).  ``two_part``: the softmax weights enter the sum unrounded, as the three
-    bfloat16 parts of a float32 (two in ``attn_span_split``); ``softcap``, ``chunk`` as in ``window_attention``."""
+    bfloat16 parts of a float32 (two in ``attn_span_split``); ``softcap``, ``chunk`` as in ``window_attention``.  ``early``: the two
+    launches before this one write no key or value but these tokens' own, and neither the table nor the tokens' places (the kernel
+    reads the others before the launch before it has ended)."""
     T, nq, hd = q.shape
     num_pages, nkv, page_size, hd2 = k_cache.shape
     for t, name in ((q, "q"), (k_cache, "k_cache"), (v_cache, "v_cache"), (out, "out")):
@@ -467,7 +469,7 @@ def attn_decode_direct(q, k_cache, v_cache, out, dec_tok, n_dec: int, tok_pos, t
     _check(lib().qb_attn_decode_direct(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(dec_tok), int(n_dec), _p(tok_pos), _p(tok_req),
                                        _p(block_table), block_table.shape[1], nq, nkv, hd, page_size, num_pages,
                                        ctypes.c_float(scale), int(window), int(longest), int(two_part), ctypes.c_float(softcap), int(chunk),
-                                       _p(status), _stream()), "attn_decode_direct")
+                                       int(early), _p(status), _stream()), "attn_decode_direct")
 
 
 def split3_bf16(w: torch.Tensor) -> torch.Tensor:
@@ -529,12 +531,13 @@ def router_small_selects(n_tokens: int, n_experts: int, top_k: int) -> bool:
 
 def router_small(x, gate, bias, logits, idx_out=None, w_out=None, renorm: bool = True, scale: float = 1.0, *,
                  counters=None, bm: int = 0, plan=None, sorted_pair=None, tile_expert=None, tile_row0=None,
-                 status=None, tiled_experts: int = 0) -> None:
+                 status=None, tiled_experts: int = 0, early: bool = False) -> None:
     """Float32 router logits ``logits[T, E] = x[T, K] @ gate[E, K].T`` on the CUDA cores, every logit one sum in
     an order that depends on K alone.  With ``idx_out`` / ``w_out`` / the plan tensors (and
     ``router_small_selects``): the selection (``router_topk``) and the expert plan (``moe_plan``) in the same
     launch; ``counters``: ``1 + ceil(T / 8)`` int32 that are zero before the call and are left zero.
-    ``tiled_experts`` > 0: only the first so many experts get tiles in the plan (the others have no weights)."""
+    ``tiled_experts`` > 0: only the first so many experts get tiles in the plan (the others have no weights).  ``early``: the two
+    launches before this one do not write ``gate`` (a step of few tokens then starts to read it before the launch before it has ended)."""
     _want(gate, torch.float32, "gate"); _want(logits, torch.float32, "logits")
     T, K = x.shape
     E = gate.shape[0]
@@ -556,7 +559,7 @@ def router_small(x, gate, bias, logits, idx_out=None, w_out=None, renorm: bool =
                                  int(renorm), ctypes.c_float(scale), int(select), _p(counters), int(bm), _p(plan),
                                  _p(sorted_pair), _p(tile_expert), _p(tile_row0),
                                  tile_expert.numel() if tile_expert is not None else 0, _p(status), int(tiled_experts),
-                                 _stream()), "router_small")
+                                 int(early), _stream()), "router_small")
 
 
 MOE_SIMT_BM = 32
@@ -826,11 +829,13 @@ DELTA_RULE_MAX_DIM = 256
 
 
 def delta_rule(proj, offsets, wpre, a_bias, w_bias, state, out, req_start, req_slot, n_heads: int, dim: int,
-               decay_scale: float, unit_eps: float, status=None) -> None:
+               decay_scale: float, unit_eps: float, status=None, early: bool = False) -> None:
     """The recurrence ``S <- diag(w) S - (a u)(u^T S) + k v^T``, ``o = S^T r`` per (request, head) over the
     step's tokens, from and into ``state`` ``[slots, heads, dim, dim]`` float32.  ``proj`` float32 ``[T, P]``
     holds r, k, v and the pre-activation of a at the column ``offsets`` (r, k, v, a), heads x dim each;
-    ``wpre`` float32 ``[T, heads*dim]`` the pre-activation of the decay; ``out`` float32 ``[T, heads, dim]``."""
+    ``wpre`` float32 ``[T, heads*dim]`` the pre-activation of the decay; ``out`` float32 ``[T, heads, dim]``.  ``early``: the two
+    launches before this one write neither ``state`` nor the requests' places (a step of single tokens then starts to read them
+    before the launch before it has ended)."""
     for t, n in ((proj, "proj"), (wpre, "wpre"), (a_bias, "a_bias"), (w_bias, "w_bias"), (state, "state"), (out, "out")):
         _want(t, torch.float32, n)
     T = proj.shape[0]
@@ -848,7 +853,7 @@ def delta_rule(proj, offsets, wpre, a_bias, w_bias, state, out, req_start, req_s
     _check(lib().qb_delta_rule(ctypes.c_void_p(proj.data_ptr()), int(proj.stride(0)), r_off, k_off, v_off, a_off,
                                _p(wpre), _p(a_bias), _p(w_bias), _p(state), _p(out), _p(scratch), _p(req_start),
                                _p(req_slot), R, T, n_heads, dim, ctypes.c_float(decay_scale),
-                               ctypes.c_float(unit_eps), _p(status), _stream()), "delta_rule", 1 if T == R and dim % 4 == 0 and dim <= 128 else 2)
+                               ctypes.c_float(unit_eps), int(early), _p(status), _stream()), "delta_rule", 1 if T == R and dim % 4 == 0 and dim <= 128 else 2)
 
 
 def head_norm_gate(o, proj, gate_off: int, gain, out, n_heads: int, dim: int, eps: float, gate: str = "sigmoid") -> None:
@@ -1401,7 +1406,7 @@ def decay_chunks_take(T: int, n_requests: int, longest: int, dim: int, vdim: int
 
 def decay_state(q, k, v, gates: DecayGates, state, out, req_start, req_slot, n_heads: int, n_groups: int, dim: int,
                 vdim: int, *, q_scale: float = 1.0, silu: bool = False, n_state=None, floor=None, den=None,
-                rows16=None, longest: int = 0, segments: bool | None = None) -> None:
+                rows16=None, longest: int = 0, segments: bool | None = None, early: bool = False) -> None:
     """``S <- a S + w k v^T``, ``o = q_scale * S^T q`` per (request, head) over the step's tokens, from and into ``state``
     float32 ``[slots, heads, dim, vdim]``; ``a``, ``w`` from ``gates``.  ``q``, ``k`` ``[T, groups * dim]`` (head h reads
     group ``h // (heads / groups)``) and ``v`` ``[T, heads * vdim]`` are column ranges of rows with one stride, float32 or
@@ -1409,7 +1414,7 @@ def decay_state(q, k, v, gates: DecayGates, state, out, req_start, req_slot, n_h
     and ``den`` float32 ``[T, heads]``: also ``n <- a n + w k`` and ``den = max(|q_scale n . q|, floor) + 1e-6``.
     ``rows16``: the same q, k, v as bfloat16 (activated already, one stride): portions of ``DECAY_CHUNK_MIN`` tokens and
     more then run in chunks on the tensor cores (``decay_chunks_take``); ``longest``: the step's longest portion if known.
-    ``segments`` False keeps them in one pass."""
+    ``segments`` False keeps them in one pass.  ``early`` as in ``delta_rule``."""
     T, H, G, D, E = q.shape[0], int(n_heads), int(n_groups), int(dim), int(vdim)
     _want(state, torch.float32, "state"); _want(out, torch.float32, "out")
     if (H % G or tuple(q.shape) != (T, G * D) or tuple(k.shape) != (T, G * D) or tuple(v.shape) != (T, H * E)
@@ -1447,7 +1452,7 @@ def decay_state(q, k, v, gates: DecayGates, state, out, req_start, req_slot, n_h
         most = DECAY_CHUNK_MIN - 1
     _check(lib().qb_decay_chain(*rows(q, k, v), _code(q), ctypes.c_longlong(q.stride(0)), *g, _p(state), *norm, _p(out),
                                 _p(req_start), _p(req_slot), T, R, H, G, D, E, ctypes.c_float(q_scale), int(silu), most,
-                                _stream()), "decay_chain")
+                                int(early), _stream()), "decay_chain")
 
 
 def decay_out(o, gate, gain, out, n_heads: int, vdim: int, parts: int, eps: float, *, den=None, x=None, skip=None,

@@ -233,7 +233,7 @@ class GQAttention(Mixer):
         longest, total = single_keys(ctx, n_dec)
         if n_dec and kernels.attn_decode_direct_wins(n_dec, self.nq, self.nkv, self.hd, longest, total, window):
             kernels.attn_decode_direct(q, cache.k, cache.v, out, dec_tok, n_dec, ctx.tok_pos, ctx.tok_req, cache.block_table, self.scale,
-                                       window, longest, ctx.status)
+                                       window, longest, ctx.status, early=getattr(ctx, "settled", False))
         elif n_dec:
             n_parts = kernels.attn_decode_parts(self.nkv, max(1, ctx.max_len_after))
             part_o = torch.empty(n_dec * self.nq * n_parts * self.hd, dtype=torch.float32, device=q.device)
@@ -281,7 +281,7 @@ def split_decode(ctx, q, cache_k, cache_v, out, table, scale: float, window: int
     if not kernels.attn_decode_direct_wins(T, nq, cache_k.shape[1], hd, longest, total, window, chunk=chunk, two_part=True):
         return False
     kernels.attn_decode_direct(q, cache_k, cache_v, out, ctx.dec_tok, T, ctx.tok_pos, ctx.tok_req, table, scale, window, longest, ctx.status,
-                               two_part=True, softcap=softcap, chunk=chunk)
+                               two_part=True, softcap=softcap, chunk=chunk, early=getattr(ctx, "settled", False))
     return True
 
 

@@ -202,8 +202,8 @@ class StepContext:
     spans: list | None = None
     token_ids: torch.Tensor | None = None      # int32 [T] the step's token ids (set by the model)
     work: dict = field(default_factory=dict)   # per-step scratch shared by the layers (tile lists and the like)
-    # launches of this step stand between the last write to the weights and the first part (the engine's own: the records' advance,
-    # the embedding), so a kernel may read weights before the launch before it has ended
+    # launches of this step stand between the last write to the weights, the requests' state and the step's integers and the first part
+    # (the engine's own: the records' advance, the embedding), so a kernel may read these before the launch before it has ended
     settled: bool = False
 
 

@@ -80,7 +80,8 @@ class _DecayState(Mixer):
             rows16 = self._columns(act)
         o = torch.empty((T, self.H, self.E), dtype=torch.float32, device=proj.device)
         kernels.decay_state(*self._columns(proj), gates, state[self.state_name], o, ctx.req_start, ctx.req_slot, self.H, self.G,
-                            self.D, self.E, silu=silu, rows16=rows16, longest=ctx.max_new_tokens_per_req, **extra)
+                            self.D, self.E, silu=silu, rows16=rows16, longest=ctx.max_new_tokens_per_req,
+                            early=getattr(ctx, "settled", False), **extra)
         return o
 
 
@@ -179,7 +180,7 @@ class StateSpaceDual(_DecayState):
         o = torch.empty((T, self.H, self.E), dtype=torch.float32, device=x.device)
         gates = kernels.DecayGates.step(proj[:, I + C: I + C + self.H], self.dt_bias, self.A_log)
         kernels.decay_state(queries, keys, values, gates, state[self.state_name], o, ctx.req_start, ctx.req_slot, self.H, self.G,
-                            self.D, self.E, rows16=rows16, longest=ctx.max_new_tokens_per_req)
+                            self.D, self.E, rows16=rows16, longest=ctx.max_new_tokens_per_req, early=getattr(ctx, "settled", False))
         y = empty_rows(T, I, dtype=x.dtype, device=x.device)
         kernels.decay_out(o, proj[:, :I], self.gain, y, self.H, self.E, self.parts, self.eps, x=values, skip=self.skip,
                           gate_first=True)

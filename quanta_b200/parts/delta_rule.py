@@ -73,7 +73,8 @@ class DeltaRule(Mixer):
             wpre = linear(inner, self.w_decay, out_dtype=torch.float32, ctx=ctx)
         o = torch.empty((T, self.H, self.D), dtype=torch.float32, device=x.device)
         kernels.delta_rule(proj, (0, HD, 2 * HD, 4 * HD), wpre, self.a_bias, self.w_bias, state[self.state_name], o,
-                           ctx.req_start, ctx.req_slot, self.H, self.D, self.decay_scale, self.unit_eps, status=ctx.status)
+                           ctx.req_start, ctx.req_slot, self.H, self.D, self.decay_scale, self.unit_eps, status=ctx.status,
+                           early=getattr(ctx, "settled", False))
         y = empty_rows(T, HD, dtype=x.dtype, device=x.device)
         kernels.head_norm_gate(o, proj, 3 * HD, self.gain, y, self.H, self.D, self.norm_eps)
         return linear(y, self.w_o, out_dtype=torch.float32, ctx=ctx)

@@ -159,7 +159,7 @@ class SigmoidTopKExperts(FeedForward):
             kernels.router_small(x, self.gate_w, self.bias, logits, idx, w, self.renorm, self.scaling,
                                  counters=self._plan_counter, bm=bm, plan=plan, sorted_pair=sorted_pair,
                                  tile_expert=tile_expert, tile_row0=tile_row0, status=ctx.status,
-                                 tiled_experts=self.E_w)
+                                 tiled_experts=self.E_w, early=getattr(ctx, "settled", False))
         else:
             kernels.moe_plan(idx, self.E, bm, plan, sorted_pair, tile_expert, tile_row0, ctx.status,
                              tiled_experts=self.E_w)
