@@ -19,7 +19,8 @@
 //   (src/quanta/minimax/moe.py:59-88; rows p sorted by expert, see the plan kernels.)
 //
 // The token rows are read in p order: MODE 1 reads a gathered copy of x (gather kernel below) as one box a
-// stage, or, for steps of few tokens, the rows of x themselves as one box of one row each (gather_k);
+// stage, or, for steps of few rows an expert, the rows of x themselves (gather_k), a box of one row each or
+// four rows an instruction (EG_FOUR_ROWS);
 // MODE 2 reads the act rows MODE 1 wrote.  Rows past the expert's last row compute garbage
 // that the epilogue drops; TMA zero-fills past the end of a tensor, so K need not be a multiple of 64
 // (it must be a multiple of 8: 16-byte rows).  No multicast: every tile comes from this GPU's memory through
@@ -34,6 +35,10 @@
 namespace {
 
 constexpr int EG_M = 128;            // output features per block (UMMA M)
+// Token tiles of more rows than this fetch their rows four an instruction (a box of one row costs the producer warp as much issue as
+// four gathered ones, and from some 64 rows a stage on that is what the tensor cores wait for); smaller tiles, which wait for the weights,
+// took the same time either way and keep the rows past the expert's last out of the copy.
+constexpr int EG_FOUR_ROWS = 32;
 constexpr int EG_BK = 64;            // k elements per stage: 128 bytes, one swizzle row
 constexpr int EG_THREADS = 192;        // producer warp, MMA warp, four epilogue warps
 constexpr int EG_PAIR_THREADS = 320;   // a pair's blocks: eight epilogue warps
@@ -113,6 +118,14 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar), "l"(policy) : "memory");
 }
 
+// four rows of a tensor seen through a map with boxes of one row, one after the other
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, int c0, const int (&row)[4], uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%2, %3, %4, %5, %6}], [%7], %8;"
+      ::"r"(dst), "l"(map), "r"(c0), "r"(row[0]), "r"(row[1]), "r"(row[2]), "r"(row[3]), "r"(bar), "l"(policy) : "memory");
+}
+
 // K-major operand tile in shared memory, rows of 128 bytes, 128-byte swizzle: 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   uint64_t d = 0;
@@ -158,6 +171,13 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
       " [%0], [%1, {%2, %3}], [%4], %5;"
       ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar_cluster), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void tma_gather4_pair(uint32_t dst, const CUtensorMap* map, int c0, const int (&row)[4], uint32_t bar_cluster,
+                                                 uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint"
+      " [%0], [%1, {%2, %3, %4, %5, %6}], [%7], %8;"
+      ::"r"(dst), "l"(map), "r"(c0), "r"(row[0]), "r"(row[1]), "r"(row[2]), "r"(row[3]), "r"(bar_cluster), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -325,6 +345,8 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
     // about the same time and read the same weights, so those stay (measured: 5 % on a 16,384-token step)
     const uint64_t pol_w = PAIR ? l2_policy_evict_last() : l2_policy_evict_first(), pol_x = l2_policy_evict_last();
     const bool by_row = MODE != 2 && gather_k > 0;
+    // tiles of more rows: four rows an instruction (the last valid row again where a group has fewer)
+    const bool by_four = by_row && KS == 1 && NT > EG_FOUR_ROWS;
     // the tile rows this block fetches: all of them, or a pair's half
     const int r_lo = PAIR ? (int)rank * (n_mma / 2) : 0;
     const int r_hi = PAIR ? min(rows, r_lo + n_mma / 2) : rows;
@@ -332,7 +354,10 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
     // Nothing in this loop waits for memory, and it has to come round faster than the tensor cores use a stage (512 cycles for a pair's
     // two matrices): stage and parity are counted, addresses step, and lane 0 runs alone unless rows are fetched one by one.  With a
     // division by the number of stages a turn took 880 cycles, with rows one by one 1,140.
-    const uint32_t x_bytes = by_row ? (uint32_t)rows * BK * 2 : (PAIR ? 2u : 1u) * b_bytes;
+    auto fours = [](int n) { return n > 0 ? (n + 3) & ~3 : 0; };
+    const int first_rows = PAIR ? min(rows, n_mma / 2) : rows;
+    const uint32_t x_bytes = by_four ? (uint32_t)(fours(first_rows) + fours(rows - first_rows)) * BK * 2
+                             : by_row ? (uint32_t)rows * BK * 2 : (PAIR ? 2u : 1u) * b_bytes;
     const uint32_t tx = (PAIR ? 2u : 1u) * NM * a_bytes + x_bytes;
     const uint32_t full0 = smem_u32(&sh.full[0]), empty0 = smem_u32(&sh.empty[0]), ring = smem_u32(tiles);
     // a pair: every copy of either block counts on the first block's barrier, which expects both blocks'
@@ -376,7 +401,14 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
         // boxes of one row: the swizzle follows the shared-memory address, so a row lands where a box of
         // many rows would have put it; the rows past the expert's last keep what the stage held before, and
         // their columns of the product are never read
-        for (int i = r_lo + lane; i < r_hi; i += 32) {
+        if (by_four) {
+          for (int i = r_lo + 4 * lane; i < r_hi; i += 128) {
+            const int row[4] = {s_pair[i], s_pair[min(i + 1, r_hi - 1)], s_pair[min(i + 2, r_hi - 1)], s_pair[min(i + 3, r_hi - 1)]};
+            const uint32_t dst = st + NM * a_bytes + (i - r_lo) * (EG_BK * 2);
+            if (PAIR) tma_gather4_pair(dst, &tm_x, kb * BK, row, bars + 8u * s, pol_x);
+            else tma_gather4(dst, &tm_x, kb * BK, row, bars + 8u * s, pol_x);
+          }
+        } else for (int i = r_lo + lane; i < r_hi; i += 32) {
           const uint32_t dst = st + NM * a_bytes + (i - r_lo) * (EG_BK * 2);
           if (PAIR) tma_load_2d_pair(dst, &tm_x, kb * BK, s_pair[i], bars + 8u * s, pol_x);
           else tma_load_2d(dst, &tm_x, kb * BK, s_pair[i], bars + 8u * s, pol_x);
@@ -626,7 +658,7 @@ extern "C" int qb_gather_rows(const void* x, void* out, const int* sorted_pair, 
 
 // x_rows: bf16 [n_pairs, K] in sorted order (mode 1: the gathered activations; mode 2: the act rows); or,
 // mode 1 with gather_k > 0, the step's activations [n_rows, K] themselves: the kernel fetches the row of
-// token sorted_pair[p] / gather_k for pair p (one TMA box a row: for steps of few tokens).
+// token sorted_pair[p] / gather_k for pair p (for steps of few rows an expert).
 // weights: bf16 [weight_experts, (mode 1 ? 2 : 1) * N_out, K] (weight_experts 0: E; fewer than E when the plan's
 // last experts have no weights and no tiles).  NT: token tile (16..256, a multiple of 16); the plan's
 // tile list must have been made with the same NT.

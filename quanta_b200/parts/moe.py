@@ -93,11 +93,11 @@ class SigmoidTopKExperts(FeedForward):
     # steps of fewer tokens take their logits on the CUDA cores, in one launch with selection and plan (and the
     # float32 path always); measured on a B200 the two ways cost the same at about a hundred tokens
     router_mma_min_tokens = 96
-    # steps with at most this many rows an expert on average fetch the token rows inside the product (one TMA box a
-    # row, the producer warp's lanes sharing them) instead of from a gathered copy; measured on a B200 the box a
-    # row costs more than the copy from some 12 rows an expert on (300 tokens: 701 against 717 us a layer, 512
-    # tokens: 746 against 732 us, 2,048 tokens: 1,358 against 815 us)
-    gather_in_kernel_max_rows = 10
+    # steps with at most this many rows an expert on average fetch the token rows inside the product (tiles of up to 32 rows one TMA box a
+    # row, larger ones four rows an instruction, the producer warp's lanes sharing them) instead of from a gathered copy.  Measured on a
+    # B200, 8 of 256 experts of 3,072 x 1,536, both products, copy / inside: 300 tokens 1,143 / 1,123 us, 536 1,179 / 1,164, 1,024 1,222 / 1,200,
+    # 2,048 1,322 / 1,355, 12,800 3,222 / 4,337 (boxes of one row each were the slower way from some 12 rows an expert on)
+    gather_in_kernel_max_rows = 32
 
     def path_for(self, x) -> str:
         ok16 = kernels.expert_gemm_tc_supported(x, self.H, self.I) and self.w13.dtype == torch.bfloat16
@@ -173,7 +173,7 @@ class SigmoidTopKExperts(FeedForward):
         if path == "tc":
             # bfloat16: TMA-fed tcgen05 products, weights as the 128-row operand, accumulators in TMEM
             if n_pairs <= self.gather_in_kernel_max_rows * self.E:
-                # few tokens: the kernel fetches each pair's token row itself
+                # the kernel fetches the pairs' token rows itself
                 kernels.expert_gemm_tc(self.first_product_mode, x, self.w13, act, sorted_pair, w.view(-1), plan,
                                        tile_expert, tile_row0, self.E, bm, ctx.status, gather_top_k=self.k,
                                        weight_experts=self.E_w, act=ea)

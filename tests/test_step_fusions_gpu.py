@@ -101,3 +101,26 @@ def test_state_rows_are_zeroed_together():
     kernels.zero_state_rows(kernels.state_table(state), 3)
     for t in state:
         assert not t[3].any() and all(bool((t[i] == 1).all()) for i in (0, 1, 2, 4))
+
+
+@pytest.mark.parametrize("T,H,I,E,k,mode", [(3, 64, 40, 8, 2, 1), (40, 72, 72, 4, 2, 1), (100, 200, 136, 8, 2, 3), (300, 136, 264, 4, 1, 1), (700, 64, 72, 8, 2, 1)])
+def test_expert_rows_fetched_inside(T, H, I, E, k, mode):
+    """Token rows fetched inside the first product, one or four at a time, in tiles of every size: the same bits as from a gathered copy."""
+    from quanta_b200 import kernels
+    g = _gen(T + I)
+    x = torch.randn(T, H, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(E, (2 if mode == 1 else 1) * I, H, device=DEV, generator=g) / H ** 0.5).to(torch.bfloat16)
+    idx = torch.stack([torch.randperm(E, device=DEV, generator=g)[:k] for _ in range(T)]).int()
+    idx[: T // 2] = torch.arange(k, device=DEV, dtype=torch.int32)          # some experts have many rows, some few
+    pw, n = torch.rand(T, k, device=DEV, generator=g), T * k
+    for bm in (16, 32, 64, 128, 256):
+        words, tiles = kernels.moe_plan_sizes(n, E, bm)
+        plan, sp, te, tr = (torch.empty(c, device=DEV, dtype=torch.int32) for c in (words, n, tiles, tiles))
+        st = kernels.new_status(DEV)
+        kernels.moe_plan(idx, E, bm, plan, sp, te, tr, st)
+        rows = torch.empty((n, H), device=DEV, dtype=torch.bfloat16)
+        kernels.gather_rows(x, rows, sp, k)
+        a, b = (torch.full((n, I), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(2))
+        kernels.expert_gemm_tc(mode, rows, w, a, sp, pw.view(-1), plan, te, tr, E, bm, st)
+        kernels.expert_gemm_tc(mode, x, w, b, sp, pw.view(-1), plan, te, tr, E, bm, st, gather_top_k=k)
+        assert st.tolist()[0] == 0 and torch.isfinite(a.float()).all() and torch.equal(a, b), bm
