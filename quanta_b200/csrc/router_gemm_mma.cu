@@ -3,7 +3,7 @@
 //
 // The float32 gate is held as THREE bfloat16 matrices hi + mid + lo (each the bfloat16 rounding of what
 // the ones before leave over: 3 x 8 mantissa bits carry the 24 of a float32), so every product
-// x * piece is exact in float32 and the sum runs in the float32 accumulators of mma.m16n8k16.  The inner
+// x * piece is exact in float32 and the sum runs in float32 accumulators.  The inner
 // dimension is taken in chunks of 64: a chunk's sum starts from zero and is then added to the running
 // total, in chunk order, whatever the number of tokens, so a token's logits do not depend on the step.
 // The inner dimension is also cut into ranges of RG_KSPLIT (a constant), one block a range, whose sums
@@ -11,128 +11,177 @@
 // (src/quanta/minimax/moe.py:44, "logits = fp32(x) @ fp32(gate).T".)  Prompt portions use this kernel;
 // steps of few tokens keep the SIMT kernel, which reads the float32 gate once.
 //
-// Block = 128 tokens x 64 experts, eight warps of 32 tokens x 32 experts each (a fragment of the gate serves
-// two fragments of tokens); operands come through shared memory in two stages filled by cp.async.  Needs K % 8 == 0 (16-byte rows).
-#include "common.cuh"
+// A work item is 128 experts x NT tokens of one range: tcgen05.mma with the experts as M and the tokens as N.  One warp copies by TMA, a
+// stage the three pieces' tiles and the tokens'; one issues twelve MMAs a chunk into one of two accumulators; eight add the finished
+// chunk, read from TMEM, to the totals in their registers while the next runs, and write these at an item's end, under the next item's
+// MMAs.  Bound by the operands' way from L2 (every token tile reads its range of the pieces) and the three passes of the tensor cores.
+// 256 experts of 3,072: 300 tokens 28.7 -> 14.4 us, 2,048 45 -> 18.4, 12,800 (60 TFLOP) 210 -> 70; 768 of 6,144, 4,000 tokens 395 -> 111
+// (mma.sync from shared memory before; a block an item without the overlap: 81 us for the 12,800).
+// Needs K % 8 == 0 (16-byte rows).
+#include <climits>
+
+#include "tensor_core.cuh"
 
 namespace {
 
-constexpr int RG_BM = 128, RG_BN = 64, RG_BK = 64, RG_PAD = 8, RG_LD = RG_BK + RG_PAD, RG_THREADS = 256;
-constexpr int RG_KSPLIT = 768;      // inner-dimension range of one block: a multiple of RG_BK
+constexpr int RG_M = 128;           // experts a block
+constexpr int RG_KSPLIT = 768;      // inner-dimension range of one block: a multiple of TC_BK
+constexpr int RG_ADD_WARPS = 8, RG_THREADS = 32 * (RG_ADD_WARPS + 2);
+constexpr uint32_t RG_W_BYTES = RG_M * TC_BK * 2;      // a piece's tile
+constexpr int RG_MAX_STAGES = 4;
+__host__ __device__ constexpr uint32_t rg_stage_bytes(int nt) { return 3 * RG_W_BYTES + (uint32_t)nt * TC_BK * 2; }
+__host__ __device__ constexpr int rg_stages(int nt) { return nt <= 128 ? 3 : 2; }      // 168, 192, 160 KB
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
-  const int n = valid ? 16 : 0;      // 0 source bytes: the 16 destination bytes are zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(n));
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
-}
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
+struct RgShared {
+  uint64_t full[RG_MAX_STAGES], empty[RG_MAX_STAGES], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+  int abort_flag;
+};
 
-// pieces: [3][E][K] bfloat16
-__global__ void __launch_bounds__(RG_THREADS)
-router_gemm_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ pieces,
-                       float* __restrict__ logits, int T, int E, int K) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem_raw);            // [2][RG_BM][RG_LD]
-  __nv_bfloat16* ws = xs + 2 * RG_BM * RG_LD;                                // [2][3][RG_BN][RG_LD]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t0 = blockIdx.y * RG_BM, e0 = blockIdx.x * RG_BN;
-  const int k_begin = blockIdx.z * RG_KSPLIT, k_end = min(K, k_begin + RG_KSPLIT);
-  const int n_stages = (k_end - k_begin + RG_BK - 1) / RG_BK;
-  const int wt = warp & 3, we = warp >> 2;      // this warp's 32 tokens and 32 experts of the block's
-  logits += (size_t)blockIdx.z * T * E;
-
-  auto fetch = [&](int stage, int buf) {
-    const int k0 = k_begin + stage * RG_BK;
-    // 64 rows x 8 chunks of 16 bytes per operand
-    for (int c = tid; c < RG_BM * (RG_BK / 8); c += RG_THREADS) {
-      const int r = c / (RG_BK / 8), kc = (c % (RG_BK / 8)) * 8;
-      const bool ok = t0 + r < T && k0 + kc < K;
-      cp_async16(xs + ((size_t)buf * RG_BM + r) * RG_LD + kc, ok ? x + (size_t)(t0 + r) * K + k0 + kc : x, ok);
-    }
-    for (int c = tid; c < 3 * RG_BN * (RG_BK / 8); c += RG_THREADS) {
-      const int p = c / (RG_BN * (RG_BK / 8)), rem = c % (RG_BN * (RG_BK / 8));
-      const int r = rem / (RG_BK / 8), kc = (rem % (RG_BK / 8)) * 8;
-      const bool ok = e0 + r < E && k0 + kc < K;
-      cp_async16(ws + (((size_t)buf * 3 + p) * RG_BN + r) * RG_LD + kc,
-                 ok ? pieces + ((size_t)p * E + e0 + r) * K + k0 + kc : pieces, ok);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
+// tm_x: x [T, K], boxes [NT][64]; tm_w: the pieces [3][E][K], boxes [1][128][64]
+template <int NT>
+__global__ void __launch_bounds__(RG_THREADS, 1)
+router_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, float* __restrict__ logits,
+                      int T, int E, int K, int tiles, int blocks_e, int items, int* status) {
+  constexpr int STAGES = rg_stages(NT), COLS = NT / 2;      // a warp adds half of the tokens, of 32 experts
+  constexpr uint32_t STAGE = rg_stage_bytes(NT);
+  extern __shared__ unsigned char rg_smem[];
+  __shared__ RgShared sh;
+  const uint32_t ring = (smem_u32(rg_smem) + 1023u) & ~1023u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  volatile int* abort_flag = &sh.abort_flag;
+  // work item -> its first token, expert and k, and its chunks; the items that run at the same time share a range of the pieces
+  auto place = [&](int item, int& t0, int& e0, int& k0) {
+    t0 = item % tiles * NT;
+    e0 = item / tiles % blocks_e * RG_M;
+    k0 = item / tiles / blocks_e * RG_KSPLIT;
+    return (min(K - k0, RG_KSPLIT) + TC_BK - 1) / TC_BK;
   };
-
-  constexpr int NT = RG_BN / 2 / 8;             // accumulator tiles of 8 experts a warp
-  constexpr int MT = 2;                         // fragments of 16 tokens a warp
-  float total[MT][NT][4];
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int i = 0; i < NT; ++i) total[m][i][0] = total[m][i][1] = total[m][i][2] = total[m][i][3] = 0.f;
-
-  fetch(0, 0);
-  for (int s = 0; s < n_stages; ++s) {
-    const int buf = s & 1;
-    if (s + 1 < n_stages) {
-      fetch(s + 1, buf ^ 1);
-      asm volatile("cp.async.wait_group 1;\n" ::);
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(smem_u32(&sh.full[s]), 1);
+      mbar_init(smem_u32(&sh.empty[s]), 1);
     }
-    __syncthreads();
-    float acc[MT][NT][4];
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-      for (int i = 0; i < NT; ++i) acc[m][i][0] = acc[m][i][1] = acc[m][i][2] = acc[m][i][3] = 0.f;
-    const __nv_bfloat16* xa = xs + ((size_t)buf * RG_BM + wt * 16 * MT) * RG_LD;
-#pragma unroll
-    for (int kk = 0; kk < RG_BK / 16; ++kk) {
-      uint32_t a[MT][4];
-#pragma unroll
-      for (int m = 0; m < MT; ++m)
-        ldmatrix_x4(a[m], xa + (size_t)(m * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * RG_LD + kk * 16 + 8 * (lane >> 4));
-#pragma unroll
-      for (int np = 0; np < NT / 2; ++np) {
-#pragma unroll
-        for (int p = 0; p < 3; ++p) {         // hi, then mid, then lo
-          const __nv_bfloat16* wb = ws + (((size_t)buf * 3 + p) * RG_BN + we * (RG_BN / 2) + np * 16) * RG_LD;
-          uint32_t b[4];
-          ldmatrix_x4(b, wb + (size_t)((lane & 7) + 8 * (lane >> 4)) * RG_LD + kk * 16 + 8 * ((lane >> 3) & 1));
-#pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            mma16816(acc[m][2 * np], a[m], b[0], b[1]);
-            mma16816(acc[m][2 * np + 1], a[m], b[2], b[3]);
-          }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&sh.acc_full[b]), 1);
+      mbar_init(smem_u32(&sh.acc_empty[b]), RG_ADD_WARPS);
+    }
+    sh.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == RG_ADD_WARPS) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(smem_u32(&sh.tmem_base)), "r"(2u * NT) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = sh.tmem_base;
+
+  if (warp == RG_ADD_WARPS + 1) {
+    // ---------------- copies ----------------
+    if (lane == 0) {
+      const uint64_t keep = l2_policy_evict_last();
+      int armed = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        int t0, e0, k0;
+        const int chunks = place(item, t0, e0, k0);
+        for (int i = 0; i < chunks; ++i) {
+          const int c = armed, s = c % STAGES;
+          const uint32_t st = ring + (uint32_t)s * STAGE, full = smem_u32(&sh.full[s]);
+          ok = c < STAGES || mbar_wait(smem_u32(&sh.empty[s]), (uint32_t)(c / STAGES - 1) & 1u, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(full, STAGE);
+          tma_load_2d(st + 3 * RG_W_BYTES, &tm_x, k0 + i * TC_BK, t0, full, keep);
+          for (int p = 0; p < 3; ++p) tma_load_3d(st + p * RG_W_BYTES, &tm_w, k0 + i * TC_BK, e0, p, full, keep);
+          armed = c + 1;
+        }
+      }
+      if (*abort_flag) {      // let the copies that were issued land before the shared memory is given away
+        for (int c = max(0, armed - STAGES); c < armed; ++c) {
+          const uint64_t ns = global_ns();
+          for (uint32_t it = 0; it < TC_SPIN_LIMIT && !mbar_try_wait(smem_u32(&sh.full[c % STAGES]), (uint32_t)(c / STAGES) & 1u); ++it)
+            if ((it & 63u) == 63u && global_ns() - ns > TC_WAIT_NS) break;
         }
       }
     }
+  } else if (warp == RG_ADD_WARPS) {
+    // ---------------- MMAs ----------------
+    if (lane == 0) {
+      int c = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        int t0, e0, k0;
+        const int chunks = place(item, t0, e0, k0);
+        const uint32_t idesc = umma_idesc(RG_M, min(NT, (T - t0 + 15) & ~15));
+        for (int i = 0; i < chunks; ++i, ++c) {
+          const int s = c % STAGES, b = c & 1;
+          ok = (c < 2 || mbar_wait(smem_u32(&sh.acc_empty[b]), (uint32_t)(c / 2 - 1) & 1u, abort_flag)) &&
+               mbar_wait(smem_u32(&sh.full[s]), (uint32_t)(c / STAGES) & 1u, abort_flag);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t st = ring + (uint32_t)s * STAGE;
+          const uint64_t xd = umma_desc_sw128(st + 3 * RG_W_BYTES);
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+          for (int k16 = 0; k16 < TC_BK / 16; ++k16)
 #pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        total[m][i][0] += acc[m][i][0]; total[m][i][1] += acc[m][i][1];
-        total[m][i][2] += acc[m][i][2]; total[m][i][3] += acc[m][i][3];
+            for (int p = 0; p < 3; ++p)      // hi, then mid, then lo; 16 k elements: 32 bytes along the swizzled row
+              umma_bf16(tmem + (uint32_t)(b * NT), umma_desc_sw128(st + p * RG_W_BYTES) + (uint64_t)(2 * k16), xd + (uint64_t)(2 * k16),
+                        idesc, k16 + p != 0 ? 1u : 0u);
+          umma_commit(smem_u32(&sh.empty[s]));
+          umma_commit(smem_u32(&sh.acc_full[b]));
+        }
       }
-    __syncthreads();
+    }
+  } else {
+    // ---------------- totals: the chunks' sums in chunk order.  A warp reaches the 32 TMEM lanes of its index modulo 4 ----------------
+    const int quarter = warp & 3, col0 = (warp >> 2) * COLS;
+    const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)col0;
+    int c = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      int t0, e0, k0;
+      const int chunks = place(item, t0, e0, k0);
+      float total[COLS];
+#pragma unroll
+      for (int i = 0; i < COLS; ++i) total[i] = 0.f;
+      for (int i = 0; i < chunks; ++i, ++c) {
+        const int b = c & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.acc_full[b]), (uint32_t)(c / 2) & 1u, abort_flag));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < COLS; j += 32) {
+          uint32_t v0[16], v1[16];
+          tmem_ld16(at + (uint32_t)(b * NT + j), v0);
+          tmem_ld16(at + (uint32_t)(b * NT + j + 16), v1);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int u = 0; u < 16; ++u) {
+            total[j + u] += __uint_as_float(v0[u]);
+            total[j + 16 + u] += __uint_as_float(v1[u]);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sh.acc_empty[b])) : "memory");
+      }
+      const int e = e0 + quarter * 32 + lane, n = T - t0 - col0;      // this warp's tokens (none or fewer than COLS: nothing there)
+      if (ok && e < E) {
+        float* dst = logits + ((size_t)(k0 / RG_KSPLIT) * T + t0 + col0) * E + e;
+#pragma unroll
+        for (int i = 0; i < COLS; ++i)
+          if (i < n) dst[(size_t)i * E] = total[i];
+      }
+    }
   }
-  // accumulator element: row (lane >> 2) + 8 * (i >> 1), column nt * 8 + (lane & 3) * 2 + (i & 1)
-  const int g = lane >> 2, q = lane & 3;
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = t0 + wt * 16 * MT + m * 16 + g + 8 * (i >> 1), e = e0 + we * (RG_BN / 2) + nt * 8 + q * 2 + (i & 1);
-        if (t < T && e < E) logits[(size_t)t * E + e] = total[m][nt][i];
-      }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == RG_ADD_WARPS)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * NT) : "memory");
+  if (threadIdx.x == 0 && sh.abort_flag && status != nullptr) qb_set_status(status, QB_STATUS_WAIT_TIMEOUT, (int)blockIdx.x, 10);
 }
 
 // out[p][i] = the p-th bfloat16 piece of w[i]: hi, mid, lo
@@ -163,19 +212,42 @@ extern "C" int qb_split3_bf16(const float* w, void* out, long long n, cudaStream
 // how many ranges the inner dimension is cut into: the first size of the logits
 extern "C" int qb_router_gemm_mma_parts(int K) { return K <= 0 ? 0 : (K + RG_KSPLIT - 1) / RG_KSPLIT; }
 
-// x bf16 [T, K]; pieces bf16 [3, E, K] (qb_split3_bf16 of the float32 gate); logits float32 [parts, T, E]
-extern "C" int qb_router_gemm_mma(const void* x, const void* pieces, float* logits, int T, int E, int K,
+// x bf16 [T, K]; pieces bf16 [3, E, K] (qb_split3_bf16 of the float32 gate); logits float32 [parts, T, E]; status may be null
+extern "C" int qb_router_gemm_mma(const void* x, const void* pieces, float* logits, int T, int E, int K, int* status,
                                   cudaStream_t stream) {
   if (T <= 0 || E <= 0) return 0;
   if (K <= 0 || K % 8) return QB_ERR_UNSUPPORTED;
   if ((((uintptr_t)x | (uintptr_t)pieces) & 15) != 0) return QB_ERR_UNSUPPORTED;
-  const size_t smem = (size_t)(2 * RG_BM + 2 * 3 * RG_BN) * RG_LD * sizeof(__nv_bfloat16);
-  cudaError_t err = cudaFuncSetAttribute(router_gemm_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err != cudaSuccess) return (int)err;
-  dim3 grid((E + RG_BN - 1) / RG_BN, (T + RG_BM - 1) / RG_BM, (K + RG_KSPLIT - 1) / RG_KSPLIT);
-  if (grid.y > 65535 || grid.z > 65535) return QB_ERR_UNSUPPORTED;
-  router_gemm_mma_kernel<<<grid, RG_THREADS, smem, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)pieces,
-                                                            logits, T, E, K);
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 1;
+  }
+  const int blocks_e = (E + RG_M - 1) / RG_M, parts = (K + RG_KSPLIT - 1) / RG_KSPLIT;
+  // the widest token tile reads the pieces least often; narrower ones where the launch still fits the SMs at once (256 experts of 3,072,
+  // tiles of 64 / 128 / 256: 300 tokens 14.4 / 18.4 / 24.6 us, 2,048 22.5 / 18.5 / 24.6, 4,096 38.9 / 30.6 / 28.7, 12,800 94 / 70 / 70)
+  const auto blocks = [&](int nt) { return (long long)blocks_e * parts * ((T + nt - 1) / nt); };
+  const int nt = blocks(64) <= sms ? 64 : blocks(128) <= sms ? 128 : 256;
+  CUtensorMap tm_x, tm_w;
+  int rc = map_2d(&tm_x, x, (uint64_t)T, (uint64_t)K, (uint32_t)nt);
+  if (rc) return rc;
+  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)E, 3}, strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)E * K * 2};
+  const cuuint32_t box[3] = {TC_BK, RG_M, 1};
+  rc = make_map(&tm_w, pieces, 3, dims, strides, box);
+  if (rc) return rc;
+  if (blocks(nt) > INT_MAX) return QB_ERR_UNSUPPORTED;
+  const int items = (int)blocks(nt), grid = items < sms ? items : sms;
+  const size_t smem = (size_t)rg_stages(nt) * rg_stage_bytes(nt) + 1024;
+#define QB_RG(NT_)                                                                                                              \
+  do {                                                                                                                          \
+    cudaError_t err = cudaFuncSetAttribute(router_gemm_tc_kernel<NT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+    if (err != cudaSuccess) return (int)err;                                                                                    \
+    router_gemm_tc_kernel<NT_><<<grid, RG_THREADS, smem, stream>>>(tm_x, tm_w, logits, T, E, K, (T + nt - 1) / nt, blocks_e, items, status);                       \
+  } while (0)
+  if (nt == 64) QB_RG(64);
+  else if (nt == 128) QB_RG(128);
+  else QB_RG(256);
+#undef QB_RG
   QB_LAUNCH_CHECK();
   return 0;
 }

@@ -26,7 +26,7 @@ _STATUS_TEXT = {1: "token id outside the vocabulary", 2: "page id outside the po
                 7: "a position beyond the table of learned position vectors"}
 _KERNEL_TEXT = {1: "embedding", 2: "rope/cache write", 3: "paged attention", 4: "expert plan",
                 5: "expert product", 6: "decode attention", 7: "prefill attention", 8: "state slots",
-                9: "delta rule"}
+                9: "delta rule", 10: "router"}
 
 
 class KernelError(RuntimeError):
@@ -487,7 +487,7 @@ def router_gemm_mma_parts(K: int) -> int:
     return int(lib().qb_router_gemm_mma_parts(int(K)))
 
 
-def router_gemm_mma(x: torch.Tensor, pieces: torch.Tensor, logits: torch.Tensor) -> None:
+def router_gemm_mma(x: torch.Tensor, pieces: torch.Tensor, logits: torch.Tensor, status=None) -> None:
     """``sum_p logits[p, T, E] = x[T, K] @ (pieces[0] + pieces[1] + pieces[2]).T`` in float32 on the tensor
     cores, ``pieces`` from ``split3_bf16`` of the float32 gate; the inner dimension in fixed chunks of 64,
     and in ``router_gemm_mma_parts(K)`` fixed ranges whose sums ``router_topk`` adds in order."""
@@ -498,7 +498,7 @@ def router_gemm_mma(x: torch.Tensor, pieces: torch.Tensor, logits: torch.Tensor)
     if (pieces.shape[0] != 3 or pieces.shape[2] != K or logits.numel() != parts * T * E
             or not logits.is_contiguous()):
         raise ValueError(f"router_gemm_mma: shape mismatch (logits must be [{parts}, {T}, {E}])")
-    _check(lib().qb_router_gemm_mma(_p(x), _p(pieces), _p(logits), T, E, K, _stream()), "router_gemm_mma")
+    _check(lib().qb_router_gemm_mma(_p(x), _p(pieces), _p(logits), T, E, K, _p(status), _stream()), "router_gemm_mma")
 
 
 ROUTE_SIGMOID_RAW, ROUTE_SIGMOID_RENORM, ROUTE_SOFTMAX_CHOSEN, ROUTE_SOFTMAX_ALL, ROUTE_SIGMOID_SHARE = 0, 1, 2, 3, 4

@@ -106,24 +106,24 @@ class SigmoidTopKExperts(FeedForward):
     def _on_tensor_cores(self, x) -> bool:
         return self.gate_pieces is not None and x.dtype == torch.bfloat16 and x.shape[0] >= self.router_mma_min_tokens
 
-    def router_logits(self, x):
+    def router_logits(self, x, status=None):
         """float32 ``[T, E]``, or ``[chunks, T, E]`` partial sums that the selection adds in index order."""
         T = x.shape[0]
         if self._on_tensor_cores(x):
             # many tokens: float32-accurate logits on the tensor cores (fixed chunks of the inner dimension)
             logits = torch.empty((kernels.router_gemm_mma_parts(self.H), T, self.E), dtype=torch.float32,
                                  device=x.device)
-            kernels.router_gemm_mma(x, self.gate_pieces, logits)
+            kernels.router_gemm_mma(x, self.gate_pieces, logits, status)
         else:
             # a warp a (token, expert) pair: the order of a logit's additions depends on the width alone
             logits = torch.empty((T, self.E), dtype=torch.float32, device=x.device)
             kernels.router_small(x, self.gate_w, self.bias, logits)
         return logits
 
-    def route(self, x):
+    def route(self, x, status=None):
         """Router of this part alone: ``(idx int32 [T,k], weights float32 [T,k])``."""
         T = x.shape[0]
-        logits = self.router_logits(x)
+        logits = self.router_logits(x, status)
         idx = torch.empty((T, self.k), dtype=torch.int32, device=x.device)
         w = torch.empty((T, self.k), dtype=torch.float32, device=x.device)
         kernels.router_topk(logits, self.bias, idx, w, self.renorm, self.scaling)
@@ -134,7 +134,7 @@ class SigmoidTopKExperts(FeedForward):
         if x.is_cuda and not self._on_tensor_cores(x) and kernels.router_small_selects(T, self.E, self.k):
             # logits, selection and the expert plan in one launch
             return self.experts(x, None, None, ctx)
-        idx, w = self.route(x)
+        idx, w = self.route(x, ctx.status)
         return self.experts(x, idx, w, ctx)
 
     def experts(self, x, idx, w, ctx):
