@@ -430,13 +430,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EG_PAIR_THREADS, 1) 
   expert_gemm_tc_body<MODE, 2, true, 1>(QB_EG_ARGS);
 }
 
-// out[p, :] = x[sorted_pair[p] / top_k, :]   (rows of 16-byte chunks)
-__global__ void gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ out,
-                                   const int* __restrict__ sorted_pair, int n_pairs, int top_k, int chunks) {
-  const size_t total = (size_t)n_pairs * chunks;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int p = (int)(i / chunks), c = (int)(i % chunks);
-    out[i] = x[(size_t)(sorted_pair[p] / top_k) * chunks + c];
+// out[p, :] = x[sorted_pair[p] / top_k, :]   (rows of 16-byte chunks).  A warp takes a row, eight chunks a lane on their way; what is
+// written does not stay in L2, so that x, whose rows are read top_k times, does.
+// Bound by the bytes written: 8 rows a token of 3,072, 2,048 tokens 28.7 -> 23.6 us, 12,800 (708 MB) 172 -> 156 (a thread a chunk before).
+constexpr int GR_WARPS = 8, GR_AHEAD = 8;
+__global__ void __launch_bounds__(GR_WARPS * 32) gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ out,
+                                                                    const int* __restrict__ sorted_pair, int n_pairs, int top_k, int chunks) {
+  const int lane = threadIdx.x & 31, p = blockIdx.x * GR_WARPS + (threadIdx.x >> 5);
+  if (p >= n_pairs) return;
+  const uint4* src = x + (size_t)(sorted_pair[p] / top_k) * chunks;
+  uint4* dst = out + (size_t)p * chunks;
+  for (int c0 = lane; c0 < chunks; c0 += 32 * GR_AHEAD) {
+    uint4 v[GR_AHEAD];
+#pragma unroll
+    for (int i = 0; i < GR_AHEAD; ++i)
+      if (c0 + 32 * i < chunks) v[i] = src[c0 + 32 * i];
+#pragma unroll
+    for (int i = 0; i < GR_AHEAD; ++i)
+      if (c0 + 32 * i < chunks) __stcs(dst + c0 + 32 * i, v[i]);
   }
 }
 
@@ -459,9 +470,8 @@ extern "C" int qb_gather_rows(const void* x, void* out, const int* sorted_pair, 
                               cudaStream_t stream) {
   if (n_pairs <= 0) return 0;
   if (K % 8) return QB_ERR_UNSUPPORTED;
-  const size_t total = (size_t)n_pairs * (K / 8);
-  const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-  gather_rows_kernel<<<blocks, 256, 0, stream>>>((const uint4*)x, (uint4*)out, sorted_pair, n_pairs, top_k, K / 8);
+  gather_rows_kernel<<<(n_pairs + GR_WARPS - 1) / GR_WARPS, GR_WARPS * 32, 0, stream>>>((const uint4*)x, (uint4*)out, sorted_pair, n_pairs,
+                                                                                      top_k, K / 8);
   QB_LAUNCH_CHECK();
   return 0;
 }
