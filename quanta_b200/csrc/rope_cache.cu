@@ -254,6 +254,18 @@ struct RopeArgs {
 
 constexpr int ROPE_HD = 128;
 
+// the multiply-adds of both kernels below, written out, so that they round alike
+__device__ __forceinline__ float squares(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.x, v.x, v.y * v.y))); }
+// c x + s o
+__device__ __forceinline__ float4 turned(float4 x, float4 c, float4 o, float4 s) {
+  return make_float4(fmaf(x.x, c.x, o.x * s.x), fmaf(x.y, c.y, o.y * s.y), fmaf(x.z, c.z, o.z * s.z), fmaf(x.w, c.w, o.w * s.w));
+}
+// neighbours (x, y) and (z, w) by two angles
+__device__ __forceinline__ float4 turned_pairs(float4 x, float c, float s, float c2, float s2) {
+  return make_float4(fmaf(x.x, c, -(x.y * s)), fmaf(x.y, c, x.x * s), fmaf(x.z, c2, -(x.w * s2)), fmaf(x.w, c2, x.z * s2));
+}
+__device__ __forceinline__ float4 negated(float4 v) { return make_float4(-v.x, -v.y, -v.z, -v.w); }
+
 template <typename IN, typename A, int HPW>
 __global__ void __launch_bounds__(HPW == 2 ? 1024 : 512, HPW == 2 ? 1 : 2)      // 64 registers: with 85 the 12,800 tokens take 276 us
 qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
@@ -302,7 +314,7 @@ qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* _
   float ss[HPW];
   if (normed) {
 #pragma unroll
-    for (int i = 0; i < HPW; ++i) ss[i] = qb_warp_sum(v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w);
+    for (int i = 0; i < HPW; ++i) ss[i] = qb_warp_sum(squares(v[i]));
     if (a.norm_kind == NORM_PER_LAYER && lane == 0) {
 #pragma unroll
       for (int i = 0; i < HPW; ++i) s_sum[warp + i * warps] = ss[i];
@@ -333,7 +345,7 @@ qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* _
       const int j = upper ? d - half : d;
       c4 = *reinterpret_cast<const float4*>(&s_cos[j]);
       s4 = *reinterpret_cast<const float4*>(&s_sin[j]);
-      if (!upper) s4 = make_float4(-s4.x, -s4.y, -s4.z, -s4.w);
+      if (!upper) s4 = negated(s4);
     }
   }
   const int partner = turns && !a.interleaved ? (upper ? lane - half / 4 : lane + half / 4) : lane;
@@ -370,11 +382,11 @@ qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* _
       }
     }
     if (a.interleaved) {
-      if (turns) x = make_float4(x.x * c4.x - x.y * s4.x, x.y * c4.x + x.x * s4.x, x.z * c4.y - x.w * s4.y, x.w * c4.y + x.z * s4.y);
+      if (turns) x = turned_pairs(x, c4.x, s4.x, c4.y, s4.y);
     } else if (half > 0) {
       const float4 o = make_float4(__shfl_sync(0xffffffffu, x.x, partner), __shfl_sync(0xffffffffu, x.y, partner),
                                    __shfl_sync(0xffffffffu, x.z, partner), __shfl_sync(0xffffffffu, x.w, partner));
-      if (turns) x = make_float4(x.x * c4.x + o.x * s4.x, x.y * c4.y + o.y * s4.y, x.z * c4.z + o.z * s4.z, x.w * c4.w + o.w * s4.w);
+      if (turns) x = turned(x, c4, o, s4);
     }
     if (h < nq) {
       if (a.temp_every > 0 || a.head_scale != nullptr) {
@@ -389,9 +401,187 @@ qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* _
   if (writes && !cache && threadIdx.x == 0) qb_set_status(a.status, QB_STATUS_BAD_PAGE, page, 2);
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same for many tokens, in about half the instructions: a half warp takes a head, a warp PPW pairs of heads, a lane the four elements
+// of two lanes of the kernel above, d .. d + 3 and 64 + d .. 64 + d + 3.  The first of its exchanges is then an addition in the lane and the others
+// leave each lane with one head's sum (the same additions in the same order, so that a token's numbers do not depend on the step);
+// pairs meet by a shuffle among the first 64 elements or, where all 128 turn, in the lane.  Bound by instructions still (the bytes
+// alone: 64 us for the 12,800 tokens below).  48 + 8 + 8 heads in bfloat16, 64 of 128 elements turned, a norm over all heads: 93 tokens 15.4 -> 12.3 us,
+// 2,048 39.9 -> 31.7, 12,800 172 -> 126; 24 + 4 + 4, a norm a head, 12,800 tokens 99 -> 79; 16 + 4 + 4 from float32, neighbours, 59 -> 58.
+// ---------------------------------------------------------------------------------------------
+template <typename IN, typename A, int PPW>
+__global__ void __launch_bounds__(512, 2)
+qknorm_rope_pairs_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
+                         const RopeArgs a) {
+  static_assert(PPW == 2 || PPW == 4, "one or two exchanges that halve a lane's sums");
+  qb_follow();
+  __shared__ __align__(16) float s_cos[ROPE_HD / 2], s_sin[ROPE_HD / 2];
+  __shared__ float s_sum[ROPE_HD];
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, sub = lane & 15, side = lane >> 4;
+  const int nq = a.nq, nk = nq + a.nkv, n = nk + (a.tied_v ? 0 : a.nkv), half = a.rd / 2, d = sub * 4;
+  const bool writes = k_cache != nullptr, normed = a.norm_kind != NORM_NONE, gained = normed && a.q_norm_w != nullptr;
+  const IN* row = qkv + (size_t)t * a.row_stride + d;
+  int pos = 0, page = -1;                // asked for first: a chain of dependent loads
+  if (writes || a.temp_every > 0) pos = a.tok_pos[t];
+  auto head = [&](int i) { return 2 * (warp + i * warps) + side; };
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 v[PPW][2];
+#pragma unroll
+  for (int i = 0; i < PPW; ++i) {
+    const int h = head(i);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) v[i][e] = h < n ? Four<IN>::load(row + h * ROPE_HD + 64 * e) : none;
+  }
+  if (writes) {
+    const int nth = a.page_shift >= 0 ? pos >> a.page_shift : pos / a.page_size;
+    page = a.block_table[(size_t)a.tok_req[t] * a.bt_stride + nth];
+  }
+  for (int j = threadIdx.x; j < half; j += blockDim.x) {
+    const int ax = a.pair_axis ? a.pair_axis[j] : 0;
+    const float ang = (float)a.positions[(size_t)t * a.n_axes + ax] * a.inv_freq[j];
+    sincosf(ang, &s_sin[j], &s_cos[j]);
+  }
+  if (a.bias != nullptr) {
+#pragma unroll
+    for (int i = 0; i < PPW; ++i) {
+      const int h = head(i);
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (h < n) {
+          const float4 b = Four<float>::load(a.bias + h * ROPE_HD + d + 64 * e);
+          v[i][e] = make_float4(v[i][e].x + b.x, v[i][e].y + b.y, v[i][e].z + b.z, v[i][e].w + b.w);
+        }
+    }
+  }
+  float sum = 0.f;                       // of the pair `own` of this warp
+  const int own = PPW == 4 ? (sub >> 2 & 3) : sub >> 3;
+  if (normed) {
+    float s[PPW];
+#pragma unroll
+    for (int i = 0; i < PPW; ++i) s[i] = squares(v[i][0]) + squares(v[i][1]);
+#pragma unroll
+    for (int x = 8, m = PPW; x > 0; x >>= 1) {
+      if (m > 1) {
+        m >>= 1;
+        const bool up = sub & x;
+#pragma unroll
+        for (int i = 0; i < PPW / 2; ++i) {
+          if (i >= m) break;
+          const float give = up ? s[i] : s[i + m], keep = up ? s[i + m] : s[i];
+          s[i] = keep + __shfl_xor_sync(0xffffffffu, give, x);
+        }
+      } else {
+        s[0] += __shfl_xor_sync(0xffffffffu, s[0], x);
+      }
+    }
+    sum = s[0];
+    if (a.norm_kind == NORM_PER_LAYER && sub % (16 / PPW) == 0 && head(own) < n) s_sum[head(own)] = sum;
+  }
+  __syncthreads();
+  float rq = 1.f, rk = 1.f;
+  if (a.norm_kind == NORM_PER_LAYER) {
+    float tq = 0.f, tk = 0.f;
+    for (int h = lane; h < nk; h += 32) {
+      const float s = s_sum[h];
+      tq += h < nq ? s : 0.f;
+      tk += h < nq ? 0.f : s;
+    }
+    rq = rsqrtf(qb_warp_sum(tq) / (float)(nq * ROPE_HD) + a.eps);
+    rk = rsqrtf(qb_warp_sum(tk) / (float)max(a.nkv * ROPE_HD, 1) + a.eps);
+  } else if (normed) {
+    rq = rsqrtf(sum / (float)ROPE_HD + a.eps);      // of the pair `own`
+  }
+  const float temp = a.temp_every > 0 ? 1.f + a.temp_coef * logf((float)((pos + 1) / a.temp_every) + 1.f) : 1.f;
+  // halves: cos and sin of pair j .. j + 3 (the first turns by a c - b s: within 64 elements its lane's sines change sign); neighbours: x, y of
+  // the lane's first four elements, z, w of the others
+  const bool turns = d < a.rd, turns2 = 64 + d < a.rd, upper = d >= half;
+  float4 c4 = make_float4(1.f, 1.f, 1.f, 1.f), s4 = none;
+  if (a.interleaved) {
+    if (turns) { c4.x = s_cos[d / 2]; c4.y = s_cos[d / 2 + 1]; s4.x = s_sin[d / 2]; s4.y = s_sin[d / 2 + 1]; }
+    if (turns2) { c4.z = s_cos[32 + d / 2]; c4.w = s_cos[33 + d / 2]; s4.z = s_sin[32 + d / 2]; s4.w = s_sin[33 + d / 2]; }
+  } else if (turns) {
+    const int j = upper ? d - half : d;
+    c4 = *reinterpret_cast<const float4*>(&s_cos[j]);
+    s4 = *reinterpret_cast<const float4*>(&s_sin[j]);
+    if (!upper) s4 = negated(s4);
+  }
+  const int partner = turns ? (upper ? lane - half / 4 : lane + half / 4) : lane;      // (half at most 32)
+  const bool cache = writes && page >= 0 && page < a.num_pages;
+  const int slot = a.page_shift >= 0 ? pos & (a.page_size - 1) : pos % a.page_size;
+  const size_t at = ((size_t)(cache ? page : 0) * a.nkv * a.page_size + slot) * ROPE_HD + d;      // of kv head 0
+  const int head_step = a.page_size * ROPE_HD;
+  A* q_row = q_out + (size_t)t * nq * ROPE_HD + d;
+#pragma unroll
+  for (int i = 0; i < PPW; ++i) {
+    const int h = head(i), first = h - side;      // first: the same for the whole warp
+    if (first >= n) continue;
+    const int hv = h - (a.tied_v ? nq : nk);
+    if (cache && hv >= 0 && h < n) {         // values go out as they are (blended with an earlier layer's where asked)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float4 x = v[i][e];
+        const size_t mine = ((size_t)t * a.nkv + hv) * ROPE_HD + d + 64 * e;
+        if (a.v_export != nullptr) Four<float>::store(a.v_export + mine, x);
+        if (a.v_first != nullptr) {
+          const float lam = a.v_lambda[0];
+          const float4 f = Four<float>::load(a.v_first + mine);
+          x = make_float4((1.f - lam) * x.x + lam * f.x, (1.f - lam) * x.y + lam * f.y, (1.f - lam) * x.z + lam * f.z,
+                          (1.f - lam) * x.w + lam * f.w);
+        }
+        Four<A>::store(v_cache + at + hv * head_step + 64 * e, x);
+      }
+    }
+    if (first >= nk) continue;
+    float4 x = v[i][0], y = v[i][1];
+    if (normed) {
+      float r = h < nq ? rq : rk;
+      if (a.norm_kind == NORM_PER_HEAD) r = __shfl_sync(0xffffffffu, rq, side * 16 + i * (16 / PPW));
+      x = make_float4(x.x * r, x.y * r, x.z * r, x.w * r);
+      y = make_float4(y.x * r, y.y * r, y.z * r, y.w * r);
+      if (gained && h < nk) {
+        const float* w = (h < nq ? a.q_norm_w : a.k_norm_w) + (a.norm_kind == NORM_PER_LAYER ? (h < nq ? h : h - nq) * ROPE_HD : 0) + d;
+        const float4 g = Four<float>::load(w), g2 = Four<float>::load(w + 64);
+        x = make_float4(g.x * x.x, g.y * x.y, g.z * x.z, g.w * x.w);
+        y = make_float4(g2.x * y.x, g2.y * y.y, g2.z * y.z, g2.w * y.w);
+      }
+    }
+    if (a.interleaved) {
+      if (turns) x = turned_pairs(x, c4.x, s4.x, c4.y, s4.y);
+      if (turns2) y = turned_pairs(y, c4.z, s4.z, c4.w, s4.w);
+    } else if (half == 64) {                   // s4 holds the first halves' signs
+      const float4 o = x;
+      x = turned(x, c4, y, s4);
+      y = turned(y, c4, o, negated(s4));
+    } else if (half > 0) {
+      const float4 o = make_float4(__shfl_sync(0xffffffffu, x.x, partner), __shfl_sync(0xffffffffu, x.y, partner),
+                                   __shfl_sync(0xffffffffu, x.z, partner), __shfl_sync(0xffffffffu, x.w, partner));
+      if (turns) x = turned(x, c4, o, s4);
+    }
+    if (h < nq) {
+      if (a.temp_every > 0 || a.head_scale != nullptr) {
+        const float m = a.head_scale != nullptr ? temp * a.head_scale[h] : temp;
+        x = make_float4(x.x * m, x.y * m, x.z * m, x.w * m);
+        y = make_float4(y.x * m, y.y * m, y.z * m, y.w * m);
+      }
+      Four<A>::store(q_row + h * ROPE_HD, x);
+      Four<A>::store(q_row + h * ROPE_HD + 64, y);
+    } else if (cache && h < nk) {
+      Four<A>::store(k_cache + at + (h - nq) * head_step, x);
+      Four<A>::store(k_cache + at + (h - nq) * head_step + 64, y);
+    }
+  }
+  if (writes && !cache && threadIdx.x == 0) qb_set_status(a.status, QB_STATUS_BAD_PAGE, page, 2);
+}
+
 template <typename IN, typename A>
 static void qknorm_rope_heads(const void* qkv, void* q_out, void* k_cache, void* v_cache, const RopeArgs& a, int T, cudaStream_t stream) {
   const int heads = a.nq + a.nkv * (a.tied_v ? 1 : 2);
+  if (T > 64 && (a.interleaved || a.rd <= 64 || a.rd == ROPE_HD)) {      // (pairs of other widths lie in two lanes' different halves)
+    const int pairs = (heads + 1) / 2, ppw = heads <= 32 ? 2 : 4, threads = (pairs + ppw - 1) / ppw * 32;
+    if (ppw == 2) qb_launch(qknorm_rope_pairs_kernel<IN, A, 2>, T, threads, 0, stream, (const IN*)qkv, (A*)q_out, (A*)k_cache, (A*)v_cache, a);
+    else qb_launch(qknorm_rope_pairs_kernel<IN, A, 4>, T, threads, 0, stream, (const IN*)qkv, (A*)q_out, (A*)k_cache, (A*)v_cache, a);
+    return;
+  }
   // few tokens: two heads a warp, so that a token is one short wait; many: four or eight loads in flight a lane
   const int hpw = T <= 64 && heads <= 64 ? 2 : heads <= 32 ? 4 : 8;
   const int threads = (heads + hpw - 1) / hpw * 32;

@@ -115,3 +115,37 @@ def test_heads_of_128(c):
     kept = q.clone()
     run(bad)
     assert st.tolist()[0] == 2 and torch.equal(q, kept) and torch.equal(kc, before)
+
+
+@pytest.mark.parametrize("c", [c for c in CASES if c["T"] > 64], ids=lambda c: "-".join(str(v).replace("torch.", "") for v in c.values()))
+def test_a_tokens_numbers_do_not_depend_on_the_step(c):
+    """Steps on both sides of 64 tokens (a warp a head, half a warp a head): the same bits."""
+    from quanta_b200 import kernels as k
+    T, nq, nkv, rd, page = c["T"], c["nq"], c["nkv"], c["rd"], c["page"]
+    nk = nkv if c["has_kv"] else 0
+    g = torch.Generator(device=DEV).manual_seed(T + nq)
+    randn = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    n_row = (nq + nk * (1 if c["tied"] else 2)) * HD
+    rows = (randn(T, n_row) * 2).to(c["rows"])
+    layer, gained = c["norm"] == "layer", c["norm"] in ("layer", "head")
+    qw = 1 + 0.2 * randn(nq * HD if layer else HD) if gained else None
+    kw = 1 + 0.2 * randn(nkv * HD if layer else HD) if gained and nk else None
+    kind = {"layer": k.NORM_PER_LAYER, "none": k.NORM_NONE}.get(c["norm"], k.NORM_PER_HEAD)
+    inv = (1e4 ** (-torch.arange(rd // 2, device=DEV) * 2 / max(rd, 1))).float()
+    bias = randn(n_row) if c["bias"] else None
+    pos, req = torch.arange(T, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+    pages = -(-T // page)
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(1)).int().view(1, pages).to(DEV)
+
+    def run(step):
+        q, st = torch.empty(T, nq, HD, device=DEV, dtype=c["dtype"]), k.new_status(DEV)
+        kc, vc = (torch.zeros((pages, nkv, page, HD), device=DEV, dtype=c["dtype"]) for _ in range(2)) if nk else (None, None)
+        for t in range(0, T, step):
+            s = slice(t, min(T, t + step))
+            k.qknorm_rope_write(rows[s], q[s], kc, vc, qw, kw, kind, 1e-5, inv, None, pos[s], pos[s], req[s], table, nq, nkv, HD, rd, page, st,
+                                has_kv=c["has_kv"], bias=bias, interleaved=c["interleaved"], tied_values=c["tied"])
+        assert st.tolist()[0] == 0
+        return [t for t in (q, kc, vc) if t is not None]
+
+    for many, few in zip(run(T), run(33)):
+        assert torch.equal(many, few)
