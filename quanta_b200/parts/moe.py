@@ -90,9 +90,12 @@ class SigmoidTopKExperts(FeedForward):
     # cores) for float32 and for widths that are no multiple of 8.  QUANTA_B200_EXPERT_KERNELS=simt forces
     # the latter for the whole process (a knob for measurements).
     expert_kernels = os.environ.get("QUANTA_B200_EXPERT_KERNELS", "auto")
-    # steps of fewer tokens take their logits on the CUDA cores, in one launch with selection and plan (and the
-    # float32 path always); measured on a B200 the two ways cost the same at about a hundred tokens
-    router_mma_min_tokens = 96
+    # Steps of fewer tokens take their logits on the CUDA cores, in one launch with selection and plan (and the float32 path always).  Their
+    # time grows with tokens x experts x width, that of the tensor cores' launches hardly; measured on a B200 with selection and plan, CUDA /
+    # tensor cores: 256 experts of 3,072, 65 tokens 31 / 27 us, 80 45 / 29 (a pass of 93 tokens 4,725 / 4,665, one of 64 the same),
+    # 8 of 2,112, 65 tokens 25 / 21; 512 of 4,096, 24 tokens 37 / 29, 48 57 / 29.  Up to 16 tokens one launch takes about 10.
+    router_mma_min_tokens = 65
+    router_mma_min_work = (17, 64 * 256 * 3072)      # or this many tokens, and more than this many products
     # steps with at most this many rows an expert on average fetch the token rows inside the product (tiles of up to 32 rows one TMA box a
     # row, larger ones four rows an instruction, the producer warp's lanes sharing them) instead of from a gathered copy.  Measured on a
     # B200, 8 of 256 experts of 3,072 x 1,536, both products, copy / inside: 300 tokens 1,143 / 1,123 us, 536 1,179 / 1,164, 1,024 1,222 / 1,200,
@@ -104,7 +107,9 @@ class SigmoidTopKExperts(FeedForward):
         return "tc" if ok16 and self.expert_kernels != "simt" else "simt"
 
     def _on_tensor_cores(self, x) -> bool:
-        return self.gate_pieces is not None and x.dtype == torch.bfloat16 and x.shape[0] >= self.router_mma_min_tokens
+        T, (few, work) = x.shape[0], self.router_mma_min_work
+        return (self.gate_pieces is not None and x.dtype == torch.bfloat16
+                and (T >= self.router_mma_min_tokens or (T >= few and T * self.E * self.H > work)))
 
     def router_logits(self, x, status=None):
         """float32 ``[T, E]``, or ``[chunks, T, E]`` partial sums that the selection adds in index order."""

@@ -124,3 +124,22 @@ def test_expert_rows_fetched_inside(T, H, I, E, k, mode):
         kernels.expert_gemm_tc(mode, rows, w, a, sp, pw.view(-1), plan, te, tr, E, bm, st)
         kernels.expert_gemm_tc(mode, x, w, b, sp, pw.view(-1), plan, te, tr, E, bm, st, gather_top_k=k)
         assert st.tolist()[0] == 0 and torch.isfinite(a.float()).all() and torch.equal(a, b), bm
+
+
+@pytest.mark.parametrize("T,E,H,tensor_cores", [(64, 40, 264, False), (65, 40, 264, True), (16, 512, 8192, False), (17, 512, 8192, True), (17, 16, 200, False)])
+def test_router_logits_on_both_sides_of_the_line(T, E, H, tensor_cores):
+    """Few products on the CUDA cores, many on the tensor cores: the float64 product to float32 rounding."""
+    from quanta_b200 import kernels
+    from quanta_b200.parts.moe import SigmoidTopKExperts
+    g = _gen(T + E)
+    part = SigmoidTopKExperts.__new__(SigmoidTopKExperts)
+    part.E, part.H, part.bias = E, H, torch.zeros(E, device=DEV)
+    part.gate_w = torch.randn(E, H, device=DEV, generator=g) / H ** 0.5
+    part.gate_pieces = kernels.split3_bf16(part.gate_w)
+    x = torch.randn(T, H, device=DEV, generator=g).to(torch.bfloat16)
+    status = kernels.new_status(DEV)
+    logits = part.router_logits(x, status)
+    assert part._on_tensor_cores(x) == tensor_cores == (logits.dim() == 3) and status.tolist()[0] == 0
+    got = logits.sum(0) if tensor_cores else logits
+    # sums of H products of size 1 / sqrt(H) in float32: no more than a few units of 2^-24 of sqrt(H) such products' absolute sum
+    assert torch.allclose(got.double(), x.double() @ part.gate_w.double().T, atol=2e-5, rtol=1e-5)
