@@ -14,9 +14,10 @@
 // A work item is 128 experts x NT tokens of one range: tcgen05.mma with the experts as M and the tokens as N.  One warp copies by TMA, a
 // stage the three pieces' tiles and the tokens'; one issues twelve MMAs a chunk into one of two accumulators; eight add the finished
 // chunk, read from TMEM, to the totals in their registers while the next runs, and write these at an item's end, under the next item's
-// MMAs.  Bound by the operands' way from L2 (every token tile reads its range of the pieces) and the three passes of the tensor cores.
-// 256 experts of 3,072: 300 tokens 28.7 -> 14.4 us, 2,048 45 -> 18.4, 12,800 (60 TFLOP) 210 -> 70; 768 of 6,144, 4,000 tokens 395 -> 111
-// (mma.sync from shared memory before; a block an item without the overlap: 81 us for the 12,800).
+// MMAs.  Bound by how many bytes of the next chunks can be on their way beside the one in work (three stages of up to 72 KB; with two of 80 the tensor
+// cores were busy 56 % of a block's time, L2 20 %).  256 experts of 3,072: 300 tokens 28.7 -> 14.4 us, 2,048 45 -> 18.4, 12,800 (60 TFLOP)
+// 210 -> 64; 768 of 6,144, 4,000 tokens 395 -> 103 (mma.sync from shared memory before; a block an item without the overlap: 81 us for the
+// 12,800).
 // Needs K % 8 == 0 (16-byte rows).
 #include <climits>
 
@@ -28,12 +29,11 @@ constexpr int RG_M = 128;           // experts a block
 constexpr int RG_KSPLIT = 768;      // inner-dimension range of one block: a multiple of TC_BK
 constexpr int RG_ADD_WARPS = 8, RG_THREADS = 32 * (RG_ADD_WARPS + 2);
 constexpr uint32_t RG_W_BYTES = RG_M * TC_BK * 2;      // a piece's tile
-constexpr int RG_MAX_STAGES = 4;
 __host__ __device__ constexpr uint32_t rg_stage_bytes(int nt) { return 3 * RG_W_BYTES + (uint32_t)nt * TC_BK * 2; }
-__host__ __device__ constexpr int rg_stages(int nt) { return nt <= 128 ? 3 : 2; }      // 168, 192, 160 KB
+constexpr int RG_STAGES = 3;       // 168, 192 or 216 KB
 
 struct RgShared {
-  uint64_t full[RG_MAX_STAGES], empty[RG_MAX_STAGES], acc_full[2], acc_empty[2];
+  uint64_t full[RG_STAGES], empty[RG_STAGES], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -43,8 +43,8 @@ template <int NT>
 __global__ void __launch_bounds__(RG_THREADS, 1)
 router_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, float* __restrict__ logits,
                       int T, int E, int K, int tiles, int blocks_e, int items, int* status) {
-  constexpr int STAGES = rg_stages(NT), COLS = NT / 2;      // a warp adds half of the tokens, of 32 experts
-  constexpr uint32_t STAGE = rg_stage_bytes(NT);
+  constexpr int STAGES = RG_STAGES, COLS = NT / 2;      // a warp adds half of the tokens, of 32 experts
+  constexpr uint32_t STAGE = rg_stage_bytes(NT), TMEM_COLS = NT == 192 ? 512 : 2 * NT;      // (a power of two)
   extern __shared__ unsigned char rg_smem[];
   __shared__ RgShared sh;
   const uint32_t ring = (smem_u32(rg_smem) + 1023u) & ~1023u;
@@ -71,7 +71,7 @@ router_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_con
   }
   if (warp == RG_ADD_WARPS) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(smem_u32(&sh.tmem_base)), "r"(2u * NT) : "memory");
+                 ::"r"(smem_u32(&sh.tmem_base)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -180,7 +180,7 @@ router_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_con
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == RG_ADD_WARPS)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * NT) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   if (threadIdx.x == 0 && sh.abort_flag && status != nullptr) qb_set_status(status, QB_STATUS_WAIT_TIMEOUT, (int)blockIdx.x, 10);
 }
 
@@ -224,10 +224,12 @@ extern "C" int qb_router_gemm_mma(const void* x, const void* pieces, float* logi
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 1;
   }
   const int blocks_e = (E + RG_M - 1) / RG_M, parts = (K + RG_KSPLIT - 1) / RG_KSPLIT;
-  // the widest token tile reads the pieces least often; narrower ones where the launch still fits the SMs at once (256 experts of 3,072,
-  // tiles of 64 / 128 / 256: 300 tokens 14.4 / 18.4 / 24.6 us, 2,048 22.5 / 18.5 / 24.6, 4,096 38.9 / 30.6 / 28.7, 12,800 94 / 70 / 70)
+  // The token tile by the rounds of items over the SMs times an item's time, which goes with the bytes of its stages and its products, 1 + NT / 64
+  // (7, 10.5 and 14 us of 768 k).  256 experts of 3,072, tiles of 64 / 128 / 192: 300 tokens 14.4 / 18.4 / - us, 2,048 22.5 / 18.5 / 22.5, 4,096
+  // 38.9 / 29.7 / 36.9, 12,800 94 / 70 / 64, 16,384 117 / 81 / 78 (256 in a ring of two stages: 28.7, 71 and 87 for the last three).
   const auto blocks = [&](int nt) { return (long long)blocks_e * parts * ((T + nt - 1) / nt); };
-  const int nt = blocks(64) <= sms ? 64 : blocks(128) <= sms ? 128 : 256;
+  const auto cost = [&](int nt) { return ((blocks(nt) + sms - 1) / sms) * (1 + nt / 64); };
+  const int nt = cost(64) <= cost(128) && cost(64) <= cost(192) ? 64 : cost(128) <= cost(192) ? 128 : 192;
   CUtensorMap tm_x, tm_w;
   int rc = map_2d(&tm_x, x, (uint64_t)T, (uint64_t)K, (uint32_t)nt);
   if (rc) return rc;
@@ -237,7 +239,7 @@ extern "C" int qb_router_gemm_mma(const void* x, const void* pieces, float* logi
   if (rc) return rc;
   if (blocks(nt) > INT_MAX) return QB_ERR_UNSUPPORTED;
   const int items = (int)blocks(nt), grid = items < sms ? items : sms;
-  const size_t smem = (size_t)rg_stages(nt) * rg_stage_bytes(nt) + 1024;
+  const size_t smem = (size_t)RG_STAGES * rg_stage_bytes(nt) + 1024;
 #define QB_RG(NT_)                                                                                                              \
   do {                                                                                                                          \
     cudaError_t err = cudaFuncSetAttribute(router_gemm_tc_kernel<NT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
@@ -246,7 +248,7 @@ extern "C" int qb_router_gemm_mma(const void* x, const void* pieces, float* logi
   } while (0)
   if (nt == 64) QB_RG(64);
   else if (nt == 128) QB_RG(128);
-  else QB_RG(256);
+  else QB_RG(192);
 #undef QB_RG
   QB_LAUNCH_CHECK();
   return 0;

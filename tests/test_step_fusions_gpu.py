@@ -143,3 +143,21 @@ def test_router_logits_on_both_sides_of_the_line(T, E, H, tensor_cores):
     got = logits.sum(0) if tensor_cores else logits
     # sums of H products of size 1 / sqrt(H) in float32: no more than a few units of 2^-24 of sqrt(H) such products' absolute sum
     assert torch.allclose(got.double(), x.double() @ part.gate_w.double().T, atol=2e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("T,E,H", [(64, 8, 72), (129, 130, 776), (500, 256, 1536), (4100, 300, 800), (12800, 256, 776), (9000, 129, 1600)])
+def test_router_logits_in_every_token_tile(T, E, H):
+    """Prompts whose router logits take tiles of 64, 128 and 192 tokens, several items a block: a token's logits are the bits it has alone."""
+    from quanta_b200 import kernels
+    g = _gen(T)
+    x = torch.randn(T, H, device=DEV, generator=g).to(torch.bfloat16)
+    gate = torch.randn(E, H, device=DEV, generator=g) / H ** 0.5
+    pieces, parts, status = kernels.split3_bf16(gate), kernels.router_gemm_mma_parts(H), kernels.new_status(DEV)
+    logits = torch.full((parts, T, E), float("nan"), device=DEV)
+    kernels.router_gemm_mma(x, pieces, logits, status)
+    assert status.tolist()[0] == 0
+    assert torch.allclose(logits.double().sum(0), x.double() @ gate.double().T, atol=2e-5, rtol=1e-5)
+    for t in (0, T // 3, T - 1):
+        alone = torch.empty((parts, 1, E), device=DEV)
+        kernels.router_gemm_mma(x[t: t + 1], pieces, alone, status)
+        assert torch.equal(alone[:, 0], logits[:, t])
