@@ -68,8 +68,8 @@ struct DecodeArgs {
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(DD_MAX_WARPS * 32)
-attn_decode_direct_kernel(const __nv_bfloat16* q, const __nv_bfloat16* __restrict__ k_cache,      // q: see qb_follow
-                          const __nv_bfloat16* __restrict__ v_cache, __nv_bfloat16* __restrict__ out, const DecodeArgs P) {
+attn_decode_direct_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k_cache,      // q: see qb_follow
+                          const __nv_bfloat16* v_cache, __nv_bfloat16* __restrict__ out, const DecodeArgs P) {
   if (!P.early) qb_follow();
   extern __shared__ __align__(128) unsigned char dd_smem[];
   // rings first; then a warp's sums, a head's 128 numbers in the order 8 e + g | 64 + 8 e + g

@@ -37,8 +37,10 @@
 // qb_follow(), waits until that launch has ended and its writes are seen, and only then lets the launch after it be placed; so whatever
 // was enqueued two launches before has ended too, and the order on the stream is what it was.  What it saves is the gap between
 // two launches, which a step of few tokens has after each of its launches.  All threads of all blocks call it, whatever they do next.
-// A kernel that reads before it calls qb_follow what no launch in flight writes takes what the launch before does write through
-// pointers without __restrict__ (or by assembly): a read through a const __restrict__ one may be moved in front of the wait.
+// Such a kernel reads through pointers without __restrict__ (or by assembly), whether it reads before it calls qb_follow or only behind it:
+// __restrict__ promises that nobody else writes there while the kernel runs, which the launch before does, and a read through a restricted
+// pointer, const or not, may be moved in front of the wait (it once put old queries into an attention).  What a kernel only writes may be
+// marked, so that reads of later elements pass the stores.
 __device__ __forceinline__ void qb_follow() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -136,11 +136,11 @@ __global__ void memory_gates_kernel(const float* __restrict__ proj, int stride, 
 }
 
 // The same for a step of single tokens: a thread a (request, head), the same numbers without the scan.
-__global__ void memory_gates_single_kernel(const float* __restrict__ proj, int stride, int i_off, int f_off,
-                                           const float* __restrict__ i_bias, const float* __restrict__ f_bias, float cap,
-                                           float* __restrict__ m_state, float* __restrict__ log_decay,
+__global__ void memory_gates_single_kernel(const float* proj, int stride, int i_off, int f_off,
+                                           const float* i_bias, const float* f_bias, float cap,
+                                           float* m_state, float* __restrict__ log_decay,
                                            float* __restrict__ weight, float* __restrict__ floor_out,
-                                           const int* __restrict__ req_slot, int R, int H) {
+                                           const int* req_slot, int R, int H) {
   qb_follow();
   const int at = blockIdx.x * blockDim.x + threadIdx.x;        // token r of request r
   if (at >= R * H) return;
@@ -191,9 +191,9 @@ struct DsShape {
 template <typename U, int VEC, int NR, int TB>
 __global__ void __launch_bounds__(DS_CHAIN_THREADS, TB == 1 && VEC == 4 && NR <= 4 ? 4 : 1)
 ds_chain_kernel(const U* q, const U* k, const U* v, DsShape sh, DsGates gates,
-                float* __restrict__ state, float* __restrict__ n_state, const float* floor_in,
-                float* __restrict__ den, float* __restrict__ out, const int* __restrict__ req_start,
-                const int* __restrict__ req_slot, float q_scale, int silu, int cols, int max_tokens, int early) {
+                float* state, float* n_state, const float* floor_in,
+                float* __restrict__ den, float* __restrict__ out, const int* req_start,
+                const int* req_slot, float q_scale, int silu, int cols, int max_tokens, int early) {
   if (!early) qb_follow();
   extern __shared__ __align__(16) float ds_sm[];
   const int D = sh.D, E = sh.E, H = sh.H;
@@ -933,7 +933,7 @@ extern "C" int qb_decay_chunks(const void* q, const void* k, const void* v, long
 // float32 columns of wider rows -> contiguous rows of the activation dtype, through silu or as they are
 // ---------------------------------------------------------------------------------------------
 template <typename O>
-__global__ void rows_act_kernel(const float* __restrict__ x, long long stride, O* __restrict__ out, int T, int n, int silu,
+__global__ void rows_act_kernel(const float* x, long long stride, O* __restrict__ out, int T, int n, int silu,
                                 int vec) {
   qb_follow();
   if (vec) {
@@ -982,9 +982,9 @@ extern "C" int qb_rows_act(const float* x, long long stride, void* out, int out_
 // ---------------------------------------------------------------------------------------------
 template <typename O, int WARPS, int Q>       // WARPS a part: 1 (four parts a block) or 8; Q 0: shared memory, any sizes
 __global__ void __launch_bounds__(WARPS == 1 ? 128 : 256)
-decay_out_kernel(const float* __restrict__ o, const float* __restrict__ den, const O* __restrict__ x, long long x_stride,
-                 const float* __restrict__ skip, const float* __restrict__ gate, long long gate_stride,
-                 const float* __restrict__ gain, O* __restrict__ out, int T, int H, int E, int parts, float eps,
+decay_out_kernel(const float* o, const float* den, const O* x, long long x_stride,
+                 const float* skip, const float* gate, long long gate_stride,
+                 const float* gain, O* __restrict__ out, int T, int H, int E, int parts, float eps,
                  int gate_first) {
   qb_follow();
   extern __shared__ __align__(16) float s_part[];

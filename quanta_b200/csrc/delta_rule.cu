@@ -343,9 +343,9 @@ constexpr int DS_MAX_DIM = 128;
 template <int RPT>
 __global__ void __launch_bounds__(128, RPT == 4 ? 6 : 3)
 delta_single_kernel(const float* proj, int proj_stride, int r_off, int k_off, int v_off, int a_off,
-                    const float* wpre, const float* __restrict__ a_bias, const float* __restrict__ w_bias,
-                    float* __restrict__ state, float* __restrict__ out, const int* __restrict__ req_start,
-                    const int* __restrict__ req_slot, int H, int D, int cols, float decay_scale, float unit_eps, int early) {
+                    const float* wpre, const float* a_bias, const float* w_bias,
+                    float* state, float* __restrict__ out, const int* req_start,
+                    const int* req_slot, int H, int D, int cols, float decay_scale, float unit_eps, int early) {
   if (!early) qb_follow();
   constexpr int DP = DR_LANES * RPT;
   __shared__ float s_u[DP], s_w[DP], s_au[DP], s_k[DP], s_r[DP];
@@ -510,7 +510,7 @@ extern "C" int qb_delta_rule(const float* proj, int proj_stride, int r_off, int 
 // out[t, c] = tanh(x[t, off + c]) for c < n, in the activation dtype (the inner activation of a
 // low-rank pair of projections whose first product sits inside a wider fused product).
 template <typename O>
-__global__ void tanh_cols_kernel(const float* __restrict__ x, int x_stride, int off, O* __restrict__ out,
+__global__ void tanh_cols_kernel(const float* x, int x_stride, int off, O* __restrict__ out,
                                  int T, int n) {
   qb_follow();
   const size_t total = (size_t)T * n;
@@ -534,7 +534,7 @@ extern "C" int qb_tanh_cols(const float* x, int x_stride, int off, void* out, in
 // outer product, for steps of few rows, whose two launches (4.5 us in a step of 8 requests) this is one of.  The L products of an output
 // are exact in float64 and are added there, so that the result is rounded once.
 template <int L>
-__global__ void __launch_bounds__(128) tanh_product_kernel(const float* __restrict__ x, int x_stride, int off, const __nv_bfloat16* __restrict__ w,
+__global__ void __launch_bounds__(128) tanh_product_kernel(const float* x, int x_stride, int off, const __nv_bfloat16* w,
                                                            float* __restrict__ out, int n, int N) {
   __shared__ float s_in[L];
   const int row = blockIdx.x * 128 + threadIdx.x;

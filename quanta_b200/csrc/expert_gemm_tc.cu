@@ -83,9 +83,8 @@ struct EgShared {
 template <int MODE, int NM, bool PAIR, int KS>
 __device__ __forceinline__ void
 expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
-                    void* __restrict__ out, const int* __restrict__ sorted_pair, const float* __restrict__ pair_w,
-                    const int* __restrict__ plan, const int* __restrict__ tile_expert,
-                    const int* __restrict__ tile_row0, int E, int K, int N_out, int NT, int stages,
+                    void* __restrict__ out, const int* sorted_pair, const float* pair_w, const int* plan,
+                    const int* tile_expert, const int* tile_row0, int E, int K, int N_out, int NT, int stages,
                     int tmem_cols, int gather_k, int* status, EgAct act, int early) {
   if (!early) qb_follow();
   constexpr bool HALF = MODE == 1 && NM == 1;              // 64 gate and 64 up rows in one weight tile
@@ -416,9 +415,8 @@ expert_gemm_tc_body(const CUtensorMap& tm_w, const CUtensorMap& tm_x,
 
 #define QB_EG_PARAMS                                                                                              \
   const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, void* __restrict__ out,     \
-      const int* __restrict__ sorted_pair, const float* __restrict__ pair_w, const int* __restrict__ plan,        \
-      const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, int E, int K, int N_out, int NT,    \
-      int stages, int tmem_cols, int gather_k, int* status, EgAct act, int early
+      const int* sorted_pair, const float* pair_w, const int* plan, const int* tile_expert, const int* tile_row0, \
+      int E, int K, int N_out, int NT, int stages, int tmem_cols, int gather_k, int* status, EgAct act, int early
 #define QB_EG_ARGS tm_w, tm_x, out, sorted_pair, pair_w, plan, tile_expert, tile_row0, E, K, N_out, NT, stages, tmem_cols, gather_k, status, act, early
 
 template <int MODE, int NM, int KS>

@@ -35,12 +35,12 @@ constexpr int LA_MAX_C = 512;      // latent channels (a lane holds C / 32 sums)
 // Block (t, 0): the latent row of token t into the cache.  Block (t, 1): the queries' latent of token t.  dkv and dq are
 // column ranges of rows of row_stride floats.
 template <typename A>
-__global__ void latent_write_kernel(const float* __restrict__ dkv, const float* __restrict__ gain,
-                                    const float* __restrict__ inv_freq, A* __restrict__ cache,
-                                    const float* __restrict__ dq, const float* __restrict__ q_gain,
+__global__ void latent_write_kernel(const float* dkv, const float* gain,
+                                    const float* inv_freq, A* __restrict__ cache,
+                                    const float* dq, const float* q_gain,
                                     A* __restrict__ cq, int q_rank, int dkv_stride, int dq_stride,
-                                    const int* __restrict__ tok_pos, const int* __restrict__ tok_req,
-                                    const int* __restrict__ block_table, int bt_stride, int T, int C, int R,
+                                    const int* tok_pos, const int* tok_req,
+                                    const int* block_table, int bt_stride, int T, int C, int R,
                                     int rd, int interleaved, int page_size, int num_pages, float eps, int* status) {
   qb_follow();
   __shared__ float scratch[32];
@@ -105,8 +105,8 @@ constexpr int LQ_WARPS = 8;
 
 template <typename A>
 __global__ void __launch_bounds__(LQ_WARPS * 32)
-latent_query_kernel(const float* __restrict__ q, const float* __restrict__ inv_freq, A* __restrict__ q_plain, float* __restrict__ q_rot,
-                    const int* __restrict__ tok_pos, int T, int H, int D, int R, int rd, int interleaved, int pieces) {
+latent_query_kernel(const float* q, const float* inv_freq, A* __restrict__ q_plain, float* __restrict__ q_rot,
+                    const int* tok_pos, int T, int H, int D, int R, int rd, int interleaved, int pieces) {
   qb_follow();
   const long unit = (long)blockIdx.x * LQ_WARPS + (threadIdx.x >> 5);
   if (unit >= (long)T * H) return;
@@ -290,8 +290,8 @@ extern "C" int qb_latent_attend(const void* q_lat, int q_lat_dtype, const float*
 constexpr int LA_MAX_RANGES = 64;
 
 template <typename A, int N>           // N: ranges, at most; a multiple of 16
-__global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restrict__ part, const float* __restrict__ sink,
-                                    const float* __restrict__ gate, int gate_stride, A* __restrict__ out, int T, int H,
+__global__ void __launch_bounds__(256) latent_merge_kernel(const float* part, const float* sink,
+                                    const float* gate, int gate_stride, A* __restrict__ out, int T, int H,
                                     int C, int n_ranges) {
   qb_follow();
   __shared__ float s_w[LA_MAX_RANGES];
@@ -400,12 +400,12 @@ __device__ __forceinline__ float lm_exp2(float x) {      // 2^x in one instructi
 
 template <int NT, bool SPLIT>      // NT: n-tiles of 8 channels a warp owns in O, C <= 32 * NT
 __global__ void __launch_bounds__(128 * LM_RG)
-latent_attend_mma_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_rot,
-                         const __nv_bfloat16* __restrict__ cache, float* __restrict__ part,
-                         const int* __restrict__ tok_pos, const int* __restrict__ req_start,
-                         const int* __restrict__ block_table, int bt_stride, int n_req, int T, int H, int C, int R,
+latent_attend_mma_kernel(const float* q_lat, const float* q_rot,
+                         const __nv_bfloat16* cache, float* __restrict__ part,
+                         const int* tok_pos, const int* req_start,
+                         const int* block_table, int bt_stride, int n_req, int T, int H, int C, int R,
                          int page_size, int num_pages, int n_ranges, int window, float scale,
-                         const float* __restrict__ sink, const float* __restrict__ gate, int gate_stride,
+                         const float* sink, const float* gate, int gate_stride,
                          __nv_bfloat16* __restrict__ out, int* status) {
   qb_follow();
   constexpr int CP = 32 * NT;

@@ -359,7 +359,7 @@ __device__ __forceinline__ void plan_small_body(const int* idx, int n_pairs, int
 }
 
 __global__ void __launch_bounds__(1024)
-moe_plan_small_kernel(const int* __restrict__ idx, int n_pairs, int E, int BM, int* __restrict__ plan,
+moe_plan_small_kernel(const int* idx, int n_pairs, int E, int BM, int* __restrict__ plan,
                       int* __restrict__ sorted_pair, int* __restrict__ tile_expert,
                       int* __restrict__ tile_row0, int max_tiles, int* status, int tiled) {
   qb_follow();
@@ -594,7 +594,7 @@ constexpr int RS_FEW = 16;
 
 template <typename TX>
 __global__ void __launch_bounds__(RS_WARPS * 32)
-router_few_kernel(const TX* x, const float* __restrict__ gate, const float* __restrict__ bias,
+router_few_kernel(const TX* x, const float* gate, const float* bias,
                   float* logits, int* idx_out, float* __restrict__ w_out, int T, int E, int K, int k, int renorm,
                   float scale, int select, int* counters, int BM, int* __restrict__ plan,
                   int* __restrict__ sorted_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,

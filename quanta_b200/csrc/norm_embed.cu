@@ -12,9 +12,9 @@
 // none; copies: how many equal residual streams the model keeps (1 for the usual single stream).
 // ---------------------------------------------------------------------------------------------
 template <typename W>
-__global__ void embedding_kernel(float* __restrict__ h, const W* __restrict__ table,
-                                 const int* __restrict__ ids, int T, int H, int V, float scale,
-                                 const W* __restrict__ pos_table, const int* __restrict__ tok_pos, int n_pos,
+__global__ void embedding_kernel(float* __restrict__ h, const W* table,
+                                 const int* ids, int T, int H, int V, float scale,
+                                 const W* pos_table, const int* tok_pos, int n_pos,
                                  int copies, int* status) {
   qb_follow();
   const int t = blockIdx.x;
@@ -167,8 +167,8 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const D* __restrict__ 
 // The same for rows in registers.  Measured on a B200 against the kernel above at 12,800 rows of 3,072: bfloat16 delta 128 -> 75 us
 // (470 MB), eight float32 slots (1.7 GB) 262 -> 233 us; one row of eight slots 3.7 -> 3.1 us.
 template <typename D, typename O>
-__global__ void __launch_bounds__(1024) add_rmsnorm_rows_kernel(float* __restrict__ h, const D* __restrict__ delta, int S, const float* __restrict__ w,
-                                        O* __restrict__ out, const int* __restrict__ rows, int H, float eps, int store_h) {
+__global__ void __launch_bounds__(1024) add_rmsnorm_rows_kernel(float* h, const D* delta, int S, const float* w,
+                                        O* __restrict__ out, const int* rows, int H, float eps, int store_h) {
   qb_follow();
   __shared__ float scratch[32];
   const int r = blockIdx.x, tok = rows ? rows[r] : r, i = threadIdx.x * 8;
@@ -300,10 +300,10 @@ struct NormConv {
 };
 
 template <typename O, int TAPS>
-__global__ void __launch_bounds__(TAPS > 0 ? 512 : 768) normed_add_rmsnorm_rows_kernel(float* __restrict__ h, const float* __restrict__ y, int S, float y_scale,
-                                               const float* __restrict__ y_bias, const float* __restrict__ y2, float y2_scale,
-                                               const float* __restrict__ y2_bias, const float* __restrict__ g, float eps_y,
-                                               const float* __restrict__ w, O* __restrict__ out, const int* __restrict__ rows,
+__global__ void __launch_bounds__(TAPS > 0 ? 512 : 768) normed_add_rmsnorm_rows_kernel(float* h, const float* y, int S, float y_scale,
+                                               const float* y_bias, const float* y2, float y2_scale,
+                                               const float* y2_bias, const float* g, float eps_y,
+                                               const float* w, O* __restrict__ out, const int* rows,
                                                int H, float eps, int store_h, NormConv conv) {
   qb_follow();
   __shared__ float scratch_y[32], scratch[32];
@@ -462,7 +462,7 @@ __global__ void silu_mul_kernel(const A* __restrict__ gu, A* __restrict__ out, i
 // bfloat16 (165 MB) 87 us with one element a thread and a division to find its row, 29 us with this; 8,192 rows of 64 3.4 us, 9.2 with a
 // block a row.
 template <typename A>
-__global__ void silu_mul_rows_kernel(const A* __restrict__ gu, A* __restrict__ out, int n_rows, int I) {
+__global__ void silu_mul_rows_kernel(const A* gu, A* __restrict__ out, int n_rows, int I) {
   qb_follow();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (c >= I) return;
@@ -653,7 +653,7 @@ extern "C" int qb_streams_mix_rmsnorm(float* x, int S, const void* delta, int de
 // out[r, c] = relu(x[r, c])^2     (the activation of an ungated feed-forward; float32 inside)
 // ---------------------------------------------------------------------------------------------
 template <typename A>
-__global__ void relu_squared_kernel(const A* __restrict__ x, A* __restrict__ out, size_t n) {
+__global__ void relu_squared_kernel(const A* x, A* __restrict__ out, size_t n) {
   qb_follow();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const float v = fmaxf(qb_to_float<A>(x[i]), 0.f);
@@ -729,7 +729,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
 // of 64 (42 MB with the bfloat16 result) 24 -> 11.6 us.
 template <typename O>
 __global__ void __launch_bounds__(128)
-head_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_stride, const float* __restrict__ gain,
+head_norm_gate_vec_kernel(const float* o, const float* gate, int gate_stride, const float* gain,
                           O* __restrict__ out, int T, int H, int D, float eps, int gain_shared, int gate_kind) {
   qb_follow();
   const int lanes = D / 4, per = 128 / lanes;            // (token, head) pairs a block

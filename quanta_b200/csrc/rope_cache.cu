@@ -268,7 +268,7 @@ __device__ __forceinline__ float4 negated(float4 v) { return make_float4(-v.x, -
 
 template <typename IN, typename A, int HPW>
 __global__ void __launch_bounds__(HPW == 2 ? 1024 : 512, HPW == 2 ? 1 : 2)      // 64 registers: with 85 the 12,800 tokens take 276 us
-qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
+qknorm_rope_heads_kernel(const IN* qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
                          const RopeArgs a) {
   qb_follow();
   __shared__ __align__(16) float s_cos[ROPE_HD / 2], s_sin[ROPE_HD / 2];
@@ -411,7 +411,7 @@ qknorm_rope_heads_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* _
 // ---------------------------------------------------------------------------------------------
 template <typename IN, typename A, int PPW>
 __global__ void __launch_bounds__(512, 2)
-qknorm_rope_pairs_kernel(const IN* __restrict__ qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
+qknorm_rope_pairs_kernel(const IN* qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
                          const RopeArgs a) {
   static_assert(PPW == 2 || PPW == 4, "one or two exchanges that halve a lane's sums");
   qb_follow();

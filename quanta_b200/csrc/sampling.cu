@@ -301,8 +301,8 @@ extern "C" int qb_apply_penalties(float* logits, int n, int V, const int* prev, 
 // position must be where the step's first token of the request goes; a difference means host and device
 // disagree about a request, which is recorded in the status words (the step's writes then land where
 // the host said; the host raises when it next reads the status).
-__global__ void slots_advance_kernel(int* __restrict__ slots, int n_slots, const int* __restrict__ req_slot,
-                                     const int* __restrict__ req_start, const int* __restrict__ req_len_after, int R,
+__global__ void slots_advance_kernel(int* slots, int n_slots, const int* req_slot,
+                                     const int* req_start, const int* req_len_after, int R,
                                      int* status) {
   qb_follow();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {

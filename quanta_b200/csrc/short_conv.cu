@@ -137,10 +137,10 @@ __global__ void short_conv_state_kernel(const float* __restrict__ x, float* __re
 }
 
 template <typename O>
-__global__ void short_conv_step_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ state,
-                                       O* __restrict__ out, const int* __restrict__ req_start,
-                                       const int* __restrict__ req_slot, int R, int C, int taps, int x_stride,
-                                       const float* __restrict__ bias, int act) {
+__global__ void short_conv_step_kernel(const float* x, const float* w, float* state,
+                                       O* __restrict__ out, const int* req_start,
+                                       const int* req_slot, int R, int C, int taps, int x_stride,
+                                       const float* bias, int act) {
   qb_follow();
   const int r = blockIdx.x;
   if (r >= R) return;
