@@ -139,23 +139,26 @@ __device__ __forceinline__ int dr_first(int p) {
 }
 
 __device__ __forceinline__ unsigned dr_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-// Bounded wait: false when the limit (iterations and 0.2 s) is reached or another warp gave up.
+__device__ __forceinline__ bool dr_done(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// Bounded wait: false when the limit (iterations and 0.2 s) is reached or, where there is a flag, another warp gave up.
 __device__ __forceinline__ bool dr_wait(unsigned bar, unsigned parity, volatile int* abort_flag) {
   unsigned long long t0 = 0;
   for (unsigned it = 0; it < 4000000u; ++it) {
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    if (ok) return true;
+    if (dr_done(bar, parity)) return true;
     if ((it & 63u) == 63u) {
-      if (*abort_flag) return false;
+      if (abort_flag != nullptr && *abort_flag) return false;
       unsigned long long now;
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
       if (t0 == 0) t0 = now;
       else if (now - t0 > 200000000ull) break;
     }
   }
-  *abort_flag = 1;
+  if (abort_flag != nullptr) *abort_flag = 1;
   return false;
 }
 
@@ -192,7 +195,8 @@ delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, co
     const int lane = tid & 31;
     const float* from = scratch + ((size_t)h * T + t0) * PER;
     const float* v_from = proj + (size_t)t0 * proj_stride + v_off + (size_t)h * D + col0;
-    for (int c = 0; c < chunks; ++c) {
+    int c = 0;
+    for (; c < chunks; ++c) {
       const int b = c % DR_STAGES, n = min(CHUNK, n_all - c * CHUNK);
       if (c >= DR_STAGES && !__all_sync(0xffffffffu, dr_wait(dr_smem(&s_empty[b]), (unsigned)(c / DR_STAGES - 1) & 1u, abort_flag))) break;
       const unsigned to = sm0 + 4 * b * DR_STAGE_FLOATS, bar = dr_smem(&s_full[b]);
@@ -210,126 +214,130 @@ delta_rule_kernel(const float* __restrict__ proj, int proj_stride, int v_off, co
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
     }
+    // whichever warp gives up, the copies on their way land before the block leaves its shared memory
     asm volatile("cp.async.wait_all;" ::: "memory");
-    // the copies in flight land before the block leaves: the walking warps wait for every chunk, unless one gave up
-    if (*abort_flag) {
-      if (lane == 0 && status != nullptr) qb_set_status(status, QB_STATUS_WAIT_TIMEOUT, r, 9);
-      __nanosleep(100000);
-    }
-    return;
-  }
-  float* S = state + ((size_t)req_slot[r] * H + h) * D * D + j;
-  auto held = [&](int n, int e) { return j + e < D && p + DR_LANES * n < D; };
-  auto cell = [&](int n, int e) { return held(n, e) ? S[(size_t)(p + DR_LANES * n) * D + e] : 0.f; };
-  dr_pair col[C][P];
+    for (int x = max(0, c - DR_STAGES); x < c; ++x) dr_wait(dr_smem(&s_full[x % DR_STAGES]), (unsigned)(x / DR_STAGES) & 1u, nullptr);
+  } else {
+    float* S = state + ((size_t)req_slot[r] * H + h) * D * D + j;
+    auto held = [&](int n, int e) { return j + e < D && p + DR_LANES * n < D; };
+    auto cell = [&](int n, int e) { return held(n, e) ? S[(size_t)(p + DR_LANES * n) * D + e] : 0.f; };
+    dr_pair col[C][P];
 #pragma unroll
-  for (int e = 0; e < C; ++e)
+    for (int e = 0; e < C; ++e)
 #pragma unroll
-    for (int i = 0; i < P; ++i) col[e][i] = dr_pack(cell(2 * i, e), cell(2 * i + 1, e));
-  struct Token {
-    dr_pair u[P], w[P], au[P], k[P], r[P];
-    float v[C];
-  };
-  // shared-memory reads that stay where they are written, before the exchanges of the token in work (the compiler put them behind: 368 us)
-  auto rows = [&](unsigned a, dr_pair (&x)[P]) {               // this lane's rows of one array
+      for (int i = 0; i < P; ++i) col[e][i] = dr_pack(cell(2 * i, e), cell(2 * i + 1, e));
+    struct Token {
+      dr_pair u[P], w[P], au[P], k[P], r[P];
+      float v[C];
+    };
+    // shared-memory reads that stay where they are written, before the exchanges of the token in work (the compiler put them behind: 368 us)
+    auto rows = [&](unsigned a, dr_pair (&x)[P]) {               // this lane's rows of one array
 #pragma unroll
-    for (int q = 0; q < P / 2; ++q)
-      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x[2 * q]), "=l"(x[2 * q + 1]) : "r"(a + 16 * (q * DR_LANES)));
-  };
-  auto read = [&](unsigned a, unsigned v, Token& t) {
-    rows(a, t.u); rows(a + 8 * DP, t.au); rows(a + 4 * DP, t.w); rows(a + 12 * DP, t.k); rows(a + 16 * DP, t.r);
-    if constexpr (C == 2) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t.v[0]), "=f"(t.v[1]) : "r"(v));
-    else asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.v[0]), "=f"(t.v[1]), "=f"(t.v[2]), "=f"(t.v[3]) : "r"(v));
-  };
-  auto step = [&](const Token& t, float (&o)[C]) {             // this lane's part of the output
-    float dot[C];
-#pragma unroll
-    for (int e = 0; e < C; ++e) {
-      dr_pair sum = 0;
-#pragma unroll
-      for (int i = 0; i < P; ++i) sum = dr_fma(t.u[i], col[e][i], sum);
-      float a, b;
-      dr_unpack(sum, a, b);
-      dot[e] = a + b;
-    }
-#pragma unroll
-    for (int d = DR_LANES / 2; d > 0; d >>= 1)
-#pragma unroll
-      for (int e = 0; e < C; ++e) dot[e] += __shfl_xor_sync(0xffffffffu, dot[e], d);
-#pragma unroll
-    for (int e = 0; e < C; ++e) {
-      const dr_pair minus = dr_pack(-dot[e], -dot[e]), v = dr_pack(t.v[e], t.v[e]);
-      dr_pair sum = 0;
-#pragma unroll
-      for (int i = 0; i < P; ++i) col[e][i] = dr_rows2(t.w[i], col[e][i], t.au[i], minus, t.k[i], v);
-#pragma unroll
-      for (int i = 0; i < P; ++i) sum = dr_fma(t.r[i], col[e][i], sum);
-      float a, b;
-      dr_unpack(sum, a, b);
-      o[e] = a + b;
-    }
-  };
-  float* to = out + ((size_t)t0 * H + h) * D + j;
-  const size_t next = (size_t)H * D;
-  for (int c = 0; c < chunks; ++c) {
-    const int b = c % DR_STAGES;
-    if (!__all_sync(0xffffffffu, dr_wait(dr_smem(&s_full[b]), (unsigned)(c / DR_STAGES) & 1u, abort_flag))) return;
-    unsigned a = sm0 + 4 * b * DR_STAGE_FLOATS, v = a + 4 * (CHUNK * PER + jj);
-    a += 16 * p;
-    const int n = min(CHUNK, n_all - c * CHUNK);
-    Token now;
-    read(a, v, now);
-    int tt = 0;
-#pragma unroll 1
-    for (; tt + U <= n; tt += U) {          // no branch inside: the next token's rows are read during this one's exchanges
-      float o[C][U];
-#pragma unroll
-      for (int x = 0; x < U; ++x) {
-        Token ahead;
-        read(a + 4 * (x + 1) * PER, v + 4 * (x + 1) * COLS, ahead);      // behind the last token: whatever lies there, not used
-        float part[C];
-        step(now, part);
-#pragma unroll
-        for (int e = 0; e < C; ++e) o[e][x] = part[e];
-        now = ahead;
-      }
-      a += 4 * U * PER;
-      v += 4 * U * COLS;
-      const int first = dr_first<U>(p);
+      for (int q = 0; q < P / 2; ++q)
+        asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x[2 * q]), "=l"(x[2 * q + 1]) : "r"(a + 16 * (q * DR_LANES)));
+    };
+    auto read = [&](unsigned a, unsigned v, Token& t) {
+      rows(a, t.u); rows(a + 8 * DP, t.au); rows(a + 4 * DP, t.w); rows(a + 12 * DP, t.k); rows(a + 16 * DP, t.r);
+      if constexpr (C == 2) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t.v[0]), "=f"(t.v[1]) : "r"(v));
+      else asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.v[0]), "=f"(t.v[1]), "=f"(t.v[2]), "=f"(t.v[3]) : "r"(v));
+    };
+    auto step = [&](const Token& t, float (&o)[C]) {             // this lane's part of the output
+      float dot[C];
 #pragma unroll
       for (int e = 0; e < C; ++e) {
-        dr_sum_lanes<U>(o[e], p);
-        if (p % (DR_LANES / U) == 0 && j + e < D) to[(size_t)first * next + e] = o[e][0];
+        dr_pair sum = 0;
+#pragma unroll
+        for (int i = 0; i < P; ++i) sum = dr_fma(t.u[i], col[e][i], sum);
+        float a, b;
+        dr_unpack(sum, a, b);
+        dot[e] = a + b;
       }
-      to += U * next;
-    }
-#pragma unroll 1
-    for (; tt < n; ++tt) {                  // the portion's last tokens
-      float o[C];
+#pragma unroll
+      for (int d = DR_LANES / 2; d > 0; d >>= 1)
+#pragma unroll
+        for (int e = 0; e < C; ++e) dot[e] += __shfl_xor_sync(0xffffffffu, dot[e], d);
+#pragma unroll
+      for (int e = 0; e < C; ++e) {
+        const dr_pair minus = dr_pack(-dot[e], -dot[e]), v = dr_pack(t.v[e], t.v[e]);
+        dr_pair sum = 0;
+#pragma unroll
+        for (int i = 0; i < P; ++i) col[e][i] = dr_rows2(t.w[i], col[e][i], t.au[i], minus, t.k[i], v);
+#pragma unroll
+        for (int i = 0; i < P; ++i) sum = dr_fma(t.r[i], col[e][i], sum);
+        float a, b;
+        dr_unpack(sum, a, b);
+        o[e] = a + b;
+      }
+    };
+    float* to = out + ((size_t)t0 * H + h) * D + j;
+    const size_t next = (size_t)H * D;
+    bool ok = true;
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c % DR_STAGES;
+      ok = __all_sync(0xffffffffu, dr_wait(dr_smem(&s_full[b]), (unsigned)(c / DR_STAGES) & 1u, abort_flag));
+      if (!ok) break;
+      unsigned a = sm0 + 4 * b * DR_STAGE_FLOATS, v = a + 4 * (CHUNK * PER + jj);
+      a += 16 * p;
+      const int n = min(CHUNK, n_all - c * CHUNK);
+      Token now;
       read(a, v, now);
-      a += 4 * PER;
-      v += 4 * COLS;
-      step(now, o);
+      int tt = 0;
+#pragma unroll 1
+      for (; tt + U <= n; tt += U) {          // no branch inside: the next token's rows are read during this one's exchanges
+        float o[C][U];
 #pragma unroll
-      for (int e = 0; e < C; ++e) {
-        float one[1] = {o[e]};
-        dr_sum_lanes<1>(one, p);
-        if (p == 0 && j + e < D) to[e] = one[0];
+        for (int x = 0; x < U; ++x) {
+          Token ahead;
+          read(a + 4 * (x + 1) * PER, v + 4 * (x + 1) * COLS, ahead);      // behind the last token: whatever lies there, not used
+          float part[C];
+          step(now, part);
+#pragma unroll
+          for (int e = 0; e < C; ++e) o[e][x] = part[e];
+          now = ahead;
+        }
+        a += 4 * U * PER;
+        v += 4 * U * COLS;
+        const int first = dr_first<U>(p);
+#pragma unroll
+        for (int e = 0; e < C; ++e) {
+          dr_sum_lanes<U>(o[e], p);
+          if (p % (DR_LANES / U) == 0 && j + e < D) to[(size_t)first * next + e] = o[e][0];
+        }
+        to += U * next;
       }
-      to += next;
+#pragma unroll 1
+      for (; tt < n; ++tt) {                  // the portion's last tokens
+        float o[C];
+        read(a, v, now);
+        a += 4 * PER;
+        v += 4 * COLS;
+        step(now, o);
+#pragma unroll
+        for (int e = 0; e < C; ++e) {
+          float one[1] = {o[e]};
+          dr_sum_lanes<1>(one, p);
+          if (p == 0 && j + e < D) to[e] = one[0];
+        }
+        to += next;
+      }
+      __syncwarp();
+      if ((tid & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dr_smem(&s_empty[b])) : "memory");
     }
-    __syncwarp();
-    if ((tid & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dr_smem(&s_empty[b])) : "memory");
+    if (ok) {
+#pragma unroll
+      for (int e = 0; e < C; ++e)
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          float x, y;
+          dr_unpack(col[e][i], x, y);
+          if (held(2 * i, e)) S[(size_t)(p + DR_LANES * 2 * i) * D + e] = x;
+          if (held(2 * i + 1, e)) S[(size_t)(p + DR_LANES * (2 * i + 1)) * D + e] = y;
+        }
+    }
   }
-#pragma unroll
-  for (int e = 0; e < C; ++e)
-#pragma unroll
-    for (int i = 0; i < P; ++i) {
-      float x, y;
-      dr_unpack(col[e][i], x, y);
-      if (held(2 * i, e)) S[(size_t)(p + DR_LANES * 2 * i) * D + e] = x;
-      if (held(2 * i + 1, e)) S[(size_t)(p + DR_LANES * (2 * i + 1)) * D + e] = y;
-    }
+  // behind the last wait of every warp: whoever gave up, the failure is seen (outputs behind it and the state are not written)
+  __syncthreads();
+  if (tid == 0 && s_abort) qb_set_status(status, QB_STATUS_WAIT_TIMEOUT, r, 9);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1,0 +1,43 @@
+"""Bounded waits between the warps of a block: whichever warp gives up, the block records it.  The status word is written behind a barrier that
+every warp reaches after its last wait; a warp that left before it, or a record that only one role writes, could lose a failure."""
+from __future__ import annotations
+
+import re
+
+import pytest
+
+from quanta_b200.csrc import build
+from tests.test_launch_order import _functions
+
+WAIT = re.compile(r"\w+_wait\([^;]*\babort_flag\)")
+
+
+def _without_lambdas(body: str) -> str:
+    while m := re.search(r"\[[&=\w, ]*\]\s*\([^()]*\)\s*\{", body):
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(body[at], 0)
+            at += 1
+        body = body[: m.start()] + "0" + body[at:]
+    return body
+
+
+def _waiting():
+    for path in sorted(build.SRC_DIR.glob("*.cu")):
+        for name, _, body in _functions(path.read_text()):
+            if WAIT.search(body):
+                yield pytest.param(body, id=f"{path.stem}-{name}")
+
+
+@pytest.mark.parametrize("body", list(_waiting()))
+def test_a_wait_that_ran_out_is_recorded_behind_the_last_barrier(body):
+    body = _without_lambdas(body)
+    first, last = WAIT.search(body).start(), [m.end() for m in WAIT.finditer(body)][-1]
+    barrier = body.rindex("__syncthreads();")
+    records = [m.start() for m in re.finditer("QB_STATUS_WAIT_TIMEOUT", body)]
+    assert last < barrier and records and all(at > barrier for at in records)
+    assert not re.search(r"\breturn;", body[first: barrier])
+
+
+def test_the_waits_are_found():
+    assert len(list(_waiting())) >= 6
