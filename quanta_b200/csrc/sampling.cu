@@ -325,10 +325,16 @@ extern "C" int qb_slots_advance(int* slots, int n_slots, const int* req_slot, co
 }
 
 // A request's rows of every per-request state, zeroed in one launch when it takes its slot (a launch a tensor was 48 for four requests of
-// the model with three recurrences, 100 us before their step).  table: {address, bytes of a row} of each tensor.
-__global__ void __launch_bounds__(256) zero_state_rows_kernel(const long long* __restrict__ table, int slot) {
-  const long long bytes = table[2 * blockIdx.x + 1];
-  unsigned char* row = reinterpret_cast<unsigned char*>(table[2 * blockIdx.x]) + bytes * slot;
+// the model with three recurrences, 100 us before their step).  The rows' places come with the launch, so none is kept from one to the next.
+constexpr int QB_STATE_ROWS = 128;          // a launch: 2 KB of parameters
+struct StateRows {
+  unsigned char* row[QB_STATE_ROWS];
+  long long bytes[QB_STATE_ROWS];
+};
+
+__global__ void __launch_bounds__(256) zero_state_rows_kernel(const __grid_constant__ StateRows rows) {
+  const long long bytes = rows.bytes[blockIdx.x];
+  unsigned char* row = rows.row[blockIdx.x];
   const long long step = (long long)gridDim.y * blockDim.x, first = (long long)blockIdx.y * blockDim.x + threadIdx.x;
   if (((bytes | (long long)(uintptr_t)row) & 15) == 0)
     for (long long i = first; i < bytes / 16; i += step) reinterpret_cast<uint4*>(row)[i] = make_uint4(0, 0, 0, 0);
@@ -336,10 +342,18 @@ __global__ void __launch_bounds__(256) zero_state_rows_kernel(const long long* _
     for (long long i = first; i < bytes; i += step) row[i] = 0;
 }
 
-extern "C" int qb_zero_state_rows(const long long* table, int n, int slot, cudaStream_t stream) {
-  if (n <= 0) return 0;
-  if (slot < 0) return QB_ERR_BAD_ARG;
-  zero_state_rows_kernel<<<dim3(n, 32), 256, 0, stream>>>(table, slot);
-  QB_LAUNCH_CHECK();
+// rows: {address, bytes} of each row, on the host
+extern "C" int qb_zero_state_rows(const long long* rows, int n, cudaStream_t stream) {
+  for (int first = 0; first < n; first += QB_STATE_ROWS) {
+    const int count = n - first < QB_STATE_ROWS ? n - first : QB_STATE_ROWS;
+    StateRows part = {};
+    for (int i = 0; i < count; ++i) {
+      part.row[i] = reinterpret_cast<unsigned char*>(rows[2 * (first + i)]);
+      part.bytes[i] = rows[2 * (first + i) + 1];
+      if (part.row[i] == nullptr || part.bytes[i] < 0) return QB_ERR_BAD_ARG;
+    }
+    zero_state_rows_kernel<<<dim3(count, 32), 256, 0, stream>>>(part);
+    QB_LAUNCH_CHECK();
+  }
   return 0;
 }

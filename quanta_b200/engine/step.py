@@ -94,9 +94,6 @@ class Engine:
         for need in model.state_needs():
             self.state.append({name: torch.zeros((max_requests, *shape), dtype=dt, device=self.device)
                                for name, (shape, dt) in need.items()})
-        # the state tensors live as long as the engine, so their places are laid down once
-        state = [t for per_pos in self.state for t in per_pos.values()]
-        self._state_table = kernels.state_table(state) if state else None
         self.status = kernels.new_status(self.device)
         self.n_axes = max([p.n_axes for p in model.parts() if isinstance(p, PositionEncoding)] or [1])
         self.vocab_size = model.spec.vocab_size
@@ -125,8 +122,7 @@ class Engine:
         was preempted goes on with the next draw number).  ``step`` admits requests it does not know with a
         default record; call this first when the sampler is to read the request's options."""
         slot = self.manager.add_request(rid)
-        if self._state_table is not None:
-            kernels.zero_state_rows(self._state_table, slot)
+        kernels.zero_state_rows([t for per_pos in self.state for t in per_pos.values()], slot)
         opts = {} if params is None else dict(seed=params.seed, temperature=params.temperature, top_k=params.top_k,
                                                 top_p=params.top_p, min_p=params.min_p)
         rec = kernels.slot_record(prompt_len=prompt_len, drawn=drawn, **opts).pin_memory()

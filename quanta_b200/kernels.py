@@ -742,18 +742,24 @@ def slot_record(*, position: int = 0, prompt_len: int = 0, drawn: int = 0, last:
     return torch.tensor(rec, dtype=torch.int32)
 
 
-def state_table(tensors: list) -> torch.Tensor | None:
-    """The table of ``zero_state_rows`` for contiguous state tensors ``[slots, ...]``, which it does not keep alive."""
-    if not all(t.is_contiguous() for t in tensors):
-        raise ValueError("state_table: the tensors must be contiguous")
-    rows = [(t.data_ptr(), t[0].numel() * t.element_size()) for t in tensors if t.numel() > 0]
-    return torch.tensor(rows, dtype=torch.int64).to(tensors[0].device) if rows else None
+STATE_ROWS_A_LAUNCH = 128
 
 
-def zero_state_rows(table, slot: int) -> None:
-    """Zero row ``slot`` of every tensor of ``state_table`` in one launch."""
-    _want(table, torch.int64, "table")
-    _check(lib().qb_zero_state_rows(_p(table), table.shape[0], int(slot), _stream()), "zero_state_rows")
+def zero_state_rows(tensors, slot: int) -> None:
+    """Zero row ``slot`` of every tensor ``[slots, ...]``, together: those that are contiguous on the current device in one launch (of 128
+    each), any other by itself."""
+    rows, slot, here = [], int(slot), torch.cuda.current_device()
+    for t in tensors:
+        if not 0 <= slot < t.shape[0]:
+            raise IndexError(f"zero_state_rows: slot {slot} of a state tensor of {t.shape[0]}")
+        if t.device.index != here or not t.is_contiguous():
+            t[slot].zero_()
+        elif t.numel():
+            size = t.nbytes // t.shape[0]
+            rows += (t.data_ptr() + slot * size, size)
+    if rows:
+        n = len(rows) // 2
+        _check(lib().qb_zero_state_rows((ctypes.c_longlong * len(rows))(*rows), n, _stream()), "zero_state_rows", -(-n // STATE_ROWS_A_LAUNCH))
 
 
 def slots_advance(slots, req_slot, req_start, req_len_after, n_requests: int, status) -> None:

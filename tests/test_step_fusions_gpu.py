@@ -94,13 +94,39 @@ def test_latent_attention_of_many_requests(lens, ranges):
 
 
 def test_state_rows_are_zeroed_together():
-    """Rows of whole 16-byte pieces, of odd numbers of bytes and of none; the neighbours stay."""
+    """Rows of whole 16-byte pieces, of odd numbers of bytes and of none, more of them than one launch takes; the neighbours stay."""
     from quanta_b200 import kernels
     state = [torch.ones(shape, dtype=dt, device=DEV) for shape, dt in (((5, 3, 128), torch.float32), ((5, 7), torch.float32), ((5, 3), torch.bfloat16),
                                                                        ((5,), torch.int64), ((5, 0), torch.float32), ((5, 64, 64, 64), torch.float32))]
-    kernels.zero_state_rows(kernels.state_table(state), 3)
+    state += [torch.ones((5, 1 + i), dtype=torch.uint8, device=DEV) for i in range(130)]
+    state.append(torch.ones((6, 5), device=DEV).t())               # not contiguous
+    kernels.zero_state_rows(state, 3)
     for t in state:
         assert not t[3].any() and all(bool((t[i] == 1).all()) for i in (0, 1, 2, 4))
+    for slot in (-1, 5):
+        with pytest.raises(IndexError):
+            kernels.zero_state_rows(state, slot)
+    assert all(bool((t[4] == 1).all()) for t in state)
+    kernels.zero_state_rows([], 0)
+
+
+def test_admission_zeroes_the_state_that_the_engine_has_now(tmp_path_factory):
+    """A state tensor that was put in the place of another one is zeroed in its stead."""
+    from quanta_b200.engine.model import load_model
+    from quanta_b200.engine.step import Engine
+    from tests import test_guravik_gpu as guravik
+    model, _ = load_model(guravik._folder(tmp_path_factory, "D")[0], dtype="float32")
+    eng = Engine(model, num_pages=8, page_size=16, max_requests=3)
+    old = [dict(per_pos) for per_pos in eng.state]
+    assert any(old)
+    for per_pos in eng.state:
+        for name, t in per_pos.items():
+            t.fill_(2)
+            per_pos[name] = torch.ones_like(t)
+    slot = eng.admit("a")
+    for before, now in zip(old, eng.state):
+        for name, t in now.items():
+            assert not t[slot].any() and t.sum() == t.numel() - t[slot].numel() and bool((before[name] == 2).all())
 
 
 @pytest.mark.parametrize("T,H,I,E,k,mode", [(3, 64, 40, 8, 2, 1), (40, 72, 72, 4, 2, 1), (100, 200, 136, 8, 2, 3), (300, 136, 264, 4, 1, 1), (700, 64, 72, 8, 2, 1)])
