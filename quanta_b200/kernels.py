@@ -262,9 +262,10 @@ def normed_add_rmsnorm(h: torch.Tensor, y: torch.Tensor | None, y_gain: torch.Te
                                                        (_p(None), _p(None), _p(None), 0)), _stream()), "normed_add_rmsnorm")
 
 
-def normed_add_conv_supported(H: int, taps: int) -> bool:
-    """Whether ``normed_add_rmsnorm`` takes a convolution over rows of ``H`` numbers."""
-    return bool(lib().qb_normed_add_conv_supported(int(H), int(taps)))
+def normed_add_conv_supported(H: int, taps: int, *operands) -> bool:
+    """Whether ``normed_add_rmsnorm`` takes a convolution over rows of ``H`` numbers, and these operands (None for those that there are not): it
+    moves them in 16-byte pieces."""
+    return bool(lib().qb_normed_add_conv_supported(int(H), int(taps))) and all(t is None or t.data_ptr() % 16 == 0 for t in operands)
 
 
 def residual_add(h: torch.Tensor, delta: torch.Tensor) -> None:

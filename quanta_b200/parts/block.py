@@ -12,7 +12,6 @@ import torch
 from .. import kernels
 from ..matmul import empty_rows, linear
 from . import norms as _norms
-from .conv import ResidualShortConv
 from .base import (Addends, Block, Embedding, Head, NormedPending, StreamCopy, StreamsPending, TensorSpec, make, register,
                    run_beside)
 
@@ -94,8 +93,8 @@ class SandwichNormBlock(Block):
             pass
         elif self.conv is None:
             self.mixer_norm.forward(h, pending, x)
-        elif (h.dim() == 2 and T > 0 and ctx.n_dec == T and ctx.req_slot.numel() == T and isinstance(self.conv, ResidualShortConv)
-              and _norms.takes_conv(self.mixer_norm, pending, self.conv.taps)):
+        elif (h.dim() == 2 and T > 0 and ctx.n_dec == T and ctx.req_slot.numel() == T
+              and _norms.takes_conv(self.mixer_norm, pending, self.conv, state, h, x)):
             # every request brings one token: norm and convolution in one launch
             _norms.normed_add(h, pending, self.mixer_norm.weight, self.mixer_norm.eps, x, None, True,
                               conv=(self.conv.weight, state[self.conv.state_name], ctx.req_slot))

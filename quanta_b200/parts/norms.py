@@ -6,6 +6,7 @@ import torch
 
 from .. import kernels
 from .base import Addends, Norm, NormedPending, StreamCopy, StreamsPending, TensorSpec, register
+from .conv import ResidualShortConv
 
 
 @register("norm", "rms_norm")
@@ -97,12 +98,15 @@ def normed_add(h, delta: NormedPending, weight, eps: float, out, rows, store_h: 
                                extra_bias=a.extra_bias, conv=conv)
 
 
-def takes_conv(norm, delta, taps: int) -> bool:
-    """Whether ``normed_add`` of ``delta`` with the norm ``norm`` takes a short convolution of so many taps into its launch (of single tokens)."""
-    if not (isinstance(norm, RMSNorm) and norm.groups == 1 and isinstance(delta, NormedPending) and isinstance(delta.norm, RMSNorm)):
+def takes_conv(norm, delta, conv, state: dict, h, out) -> bool:
+    """Whether ``normed_add`` of ``delta`` with the norm ``norm`` takes the convolution ``conv`` into its launch (of single tokens).  Only these
+    very classes: one made from them may have a ``forward`` of its own."""
+    if type(norm) is not RMSNorm or type(conv) is not ResidualShortConv or not isinstance(delta, NormedPending) or not isinstance(delta.norm, RMSNorm):
         return False
     a = delta.addends
-    return delta.norm.groups == 1 and not a.branch_normed and kernels.normed_add_conv_supported(norm.width, taps)
+    return (norm.groups == 1 and delta.norm.groups == 1 and not a.branch_normed
+            and kernels.normed_add_conv_supported(norm.width, conv.taps, h, a.y, a.bias, a.extra, a.extra_bias, delta.norm.weight, norm.weight,
+                                                  out, conv.weight, state[conv.state_name]))
 
 
 def add_sum(h, a: Addends, out, weight=None, groups: int = 1, eps: float = 0.0, rows=None, store_h: bool = True) -> None:
