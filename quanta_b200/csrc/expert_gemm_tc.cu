@@ -493,12 +493,9 @@ extern "C" int qb_expert_gemm_tc(int mode, const void* x_rows, const void* weigh
   if (mode != 1 && mode != 2 && mode != 3) return QB_ERR_BAD_ARG;
   // weight tiles a block: gate and up (mode 1); two blocks of 128 features for the down product of 256-row
   // token tiles (see the kernel)
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 1;
-  }
+  int sms = 0;
+  const int rc_sms = sm_count(sms);
+  if (rc_sms) return rc_sms;
   // the gated first product of so few tiles that blocks of 128 features would leave SMs idle: blocks of 64, gate and up in one weight tile
   // (one token, 8 of 256 experts of 3,072 x 1,536: 96 blocks 33.0 us with one slab a stage, 192 blocks of half the size 28.4)
   const bool half = mode == 1 && NT <= 32 && (size_t)((N_out + EG_M - 1) / EG_M) * (size_t)max_tiles <= (size_t)sms;

@@ -141,13 +141,13 @@ router_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_con
     const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)col0;
     int c = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
       int t0, e0, k0;
       const int chunks = place(item, t0, e0, k0);
       float total[COLS];
 #pragma unroll
       for (int i = 0; i < COLS; ++i) total[i] = 0.f;
-      for (int i = 0; i < chunks; ++i, ++c) {
+      for (int i = 0; i < chunks && ok; ++i, ++c) {
         const int b = c & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.acc_full[b]), (uint32_t)(c / 2) & 1u, abort_flag));
         if (!ok) break;
@@ -168,8 +168,12 @@ router_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_con
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sh.acc_empty[b])) : "memory");
       }
+      if (!ok) {      // a wait ran out: the sums that are missing are no numbers, for callers without status words too
+#pragma unroll
+        for (int i = 0; i < COLS; ++i) total[i] = __int_as_float(0x7fffffff);
+      }
       const int e = e0 + quarter * 32 + lane, n = T - t0 - col0;      // this warp's tokens (none or fewer than COLS: nothing there)
-      if (ok && e < E) {
+      if (e < E) {
         float* dst = logits + ((size_t)(k0 / RG_KSPLIT) * T + t0 + col0) * E + e;
 #pragma unroll
         for (int i = 0; i < COLS; ++i)
@@ -218,11 +222,9 @@ extern "C" int qb_router_gemm_mma(const void* x, const void* pieces, float* logi
   if (T <= 0 || E <= 0) return 0;
   if (K <= 0 || K % 8) return QB_ERR_UNSUPPORTED;
   if ((((uintptr_t)x | (uintptr_t)pieces) & 15) != 0) return QB_ERR_UNSUPPORTED;
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 1;
-  }
+  int sms = 0;
+  int rc = sm_count(sms);
+  if (rc) return rc;
   const int blocks_e = (E + RG_M - 1) / RG_M, parts = (K + RG_KSPLIT - 1) / RG_KSPLIT;
   // The token tile by the rounds of items over the SMs times an item's time, which goes with the bytes of its stages and its products, 1 + NT / 64
   // (7, 10.5 and 14 us of 768 k).  256 experts of 3,072, tiles of 64 / 128 / 192: 300 tokens 14.4 / 18.4 / - us, 2,048 22.5 / 18.5 / 22.5, 4,096
@@ -231,7 +233,7 @@ extern "C" int qb_router_gemm_mma(const void* x, const void* pieces, float* logi
   const auto cost = [&](int nt) { return ((blocks(nt) + sms - 1) / sms) * (1 + nt / 64); };
   const int nt = cost(64) <= cost(128) && cost(64) <= cost(192) ? 64 : cost(128) <= cost(192) ? 128 : 192;
   CUtensorMap tm_x, tm_w;
-  int rc = map_2d(&tm_x, x, (uint64_t)T, (uint64_t)K, (uint32_t)nt);
+  rc = map_2d(&tm_x, x, (uint64_t)T, (uint64_t)K, (uint32_t)nt);
   if (rc) return rc;
   const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)E, 3}, strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)E * K * 2};
   const cuuint32_t box[3] = {TC_BK, RG_M, 1};

@@ -196,4 +196,11 @@ int map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32
   const cuuint32_t box[2] = {TC_BK, box_rows};
   return make_map(map, base, 2, dims, strides, box);
 }
+// SMs of the current device (asked for with every launch: a process may use several devices)
+int sm_count(int& sms) {
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (int)err;
+}
 }  // namespace

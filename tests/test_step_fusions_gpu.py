@@ -187,3 +187,17 @@ def test_router_logits_in_every_token_tile(T, E, H):
         alone = torch.empty((parts, 1, E), device=DEV)
         kernels.router_gemm_mma(x[t: t + 1], pieces, alone, status)
         assert torch.equal(alone[:, 0], logits[:, t])
+
+
+@pytest.mark.parametrize("mode", range(5))
+@pytest.mark.parametrize("T,E,k", [(3, 40, 4), (300, 256, 8)])
+def test_logits_that_are_no_numbers_choose_experts_of_the_table(T, E, k, mode):
+    """A token whose logits a wait kept back (NaN): its experts are inside the table and its weights are no numbers."""
+    from quanta_b200 import kernels
+    logits = torch.randn(2, T, E, device=DEV, generator=_gen(T))
+    logits[0, 1] = torch.full((E,), 0x7FFFFFFF, dtype=torch.int32, device=DEV).view(torch.float32)
+    idx, w = torch.empty((T, k), dtype=torch.int32, device=DEV), torch.empty((T, k), device=DEV)
+    kernels.router_topk(logits, torch.zeros(E, device=DEV), idx, w, mode, 1.0)
+    assert bool(((idx >= 0) & (idx < E)).all()) and bool(torch.isnan(w[1]).all())
+    others = torch.arange(T, device=DEV) != 1
+    assert bool(torch.isfinite(w[others]).all())

@@ -41,3 +41,12 @@ def test_a_wait_that_ran_out_is_recorded_behind_the_last_barrier(body):
 
 def test_the_waits_are_found():
     assert len(list(_waiting())) >= 6
+
+
+def test_router_logits_that_a_wait_kept_back_are_no_numbers():
+    """The router takes no status words from some callers: what it could not sum is NaN there, and the selection passes NaN on (its experts
+    stay inside the table, see the GPU test of the selection)."""
+    (body,) = [b for n, _, b in _functions((build.SRC_DIR / "router_gemm_mma.cu").read_text()) if n == "router_gemm_tc_kernel"]
+    sums = body[body.index("float total[COLS]"):]
+    assert re.search(r"if \(!ok\) \{[^}]*total\[i\] = __int_as_float\(0x7fffffff\);\s*\}", sums)
+    assert "if (ok && e < E)" not in sums and "items && ok" not in body[body.index("const int quarter"):]
