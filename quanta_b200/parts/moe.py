@@ -108,7 +108,7 @@ class SigmoidTopKExperts(FeedForward):
 
     def _on_tensor_cores(self, x) -> bool:
         T, (few, work) = x.shape[0], self.router_mma_min_work
-        return (self.gate_pieces is not None and x.dtype == torch.bfloat16
+        return (self.gate_pieces is not None and x.dtype == torch.bfloat16 and x.data_ptr() % 16 == 0      # (TMA starts on 16 bytes)
                 and (T >= self.router_mma_min_tokens or (T >= few and T * self.E * self.H > work)))
 
     def router_logits(self, x, status=None):
