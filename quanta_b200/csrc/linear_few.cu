@@ -8,7 +8,8 @@
 // for their first pieces before they wait for it, and the products follow the arrival of x.  That pays behind launches that are one
 // short chain of reads (8 requests, a delta rule's model: 637 us for two steps without, 603 with it), not behind those that
 // use the memory or fill the SMs themselves (an attention, the norm over eight experts' slots: the blocks slow them and fall unevenly
-// on the SMs that are left; 8 requests of the M2-family sizes 2,518 us with, 2,474 without).  x is read by every block, out of L1 after the SM's first.  A row's sums are taken in an order that depends on K alone.
+// on the SMs that are left; 8 requests of the M2-family sizes 2,518 us with, 2,474 without).  x is read by every block: out of L1 after the SM's
+// first where its rows fit there (8 rows of 8,192 do), else out of L2.  A row's sums are taken in an order that depends on K alone.
 //
 // Measured on a B200, one product after another in a graph, weights from memory, microseconds (library: at 32 rows, its fastest kernel):
 //   [N, K]            bytes at 6.5 TB/s   library   8 rows   16 rows   32 rows
@@ -18,8 +19,9 @@
 //   2,048 x 5,632            3.5             9.9      6.2       7.5       8.2
 //   2,048 x 2,048            1.3             5.5      2.2       2.8       3.6
 //   3,072 x 768              0.7             4.2      1.8       2.0       2.6
-// Above 16 rows the reads of x outweigh those of W where several blocks follow one another on an SM: there the kernel takes matrices
-// of one block an SM at most (four pieces ahead) and small ones, the library the others; above 32 rows, the library all of them.
+// Whole decode steps (graph, 1,000 keys; library for all / for the larger matrices only / this for all up to 32 rows): four layers of the
+// M2-family sizes, 1 request 398 / 398 / 381 us, 24 2,679 / 2,678 / 2,720, 32 3,144 / 3,112 / 3,142; six layers of width 2,048 with delta rules, 1
+// request 313 / 269 / 233, 16 352 / 315 / 304, 20 362 / 335 / 350, 32 395 / 376 / 398; with three recurrences, 16 589 / 551 / 542, 20 718 / 685 / 721.
 #include "common.cuh"
 
 constexpr int LF_WARPS = 8;
@@ -151,11 +153,14 @@ static int linear_few_launch(const LinearFew& a, int out_dtype, bool glu, int ea
   return 0;
 }
 
-// Whether the kernel is the faster way for `rows` rows of [N, K]: the rule of qb_linear_few.
-static bool linear_few_small(int K, int N) { return (N + 15) / 16 <= 148 || (long long)K * N <= 4 << 20; }
-
+// Whether products of up to 32 rows of [N, K] are this kernel's: by the matrix alone, so that a row's numbers are the same in every step of up
+// to 32 rows (the library's products run at 32 rows up to there).  It is the faster one up to 16 rows, and up to 32 where the matrix has a
+// block an SM at most; in larger ones the mma.sync products of 17 to 32 rows and their reads of x take longer than the weights' bytes, which
+// longer rows make worse.  Library / this, plain launches, microseconds: 3,072 x 8,192 14.5 / 11.3 at 8 rows, 14.6 / 18.8 at 32 (taken); 3,072 x
+// 12,288 19.9 / 15.2 and 19.8 / 27.3, 8,192 x 12,288 36.4 / 33.0 and 36.6 / 53.5 (not); one block an SM: 1,024 x 12,288 20.8 / 10.0 and 20.8 / 16.1
+// (taken), 2,048 x 16,384 20.7 / 16.2 and 21.0 / 23.3 (not).
 extern "C" int qb_linear_few_takes(int rows, int K, int N) {
-  return rows > 0 && rows <= 32 && K >= LF_KB && K % 16 == 0 && N > 0 && (rows <= 16 || linear_few_small(K, N));
+  return rows > 0 && rows <= 32 && K >= LF_KB && K % 16 == 0 && N > 0 && K <= ((N + 15) / 16 <= 148 ? 12288 : 8192);
 }
 
 // K a multiple of 16; x and w on 32 bytes.  early: W was written two launches before this one at the latest (or by the host), so that

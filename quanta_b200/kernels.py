@@ -609,7 +609,8 @@ LINEAR_FEW_MAX = 32
 
 
 def linear_few_takes(rows: int, K: int, N: int) -> bool:
-    """Whether ``linear_few`` is the faster way for ``rows`` bfloat16 rows and a ``[N, K]`` matrix."""
+    """Whether ``linear_few`` takes products of ``rows`` bfloat16 rows and a ``[N, K]`` matrix: the same for every number of rows up to
+    ``LINEAR_FEW_MAX``."""
     return 0 < rows <= LINEAR_FEW_MAX and bool(lib().qb_linear_few_takes(rows, K, N))
 
 

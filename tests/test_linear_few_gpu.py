@@ -55,6 +55,24 @@ def test_linear_takes_few_rows_and_leaves_the_rest(dtype):
         assert out.shape == (x.shape[0], w.shape[0]) and out.dtype == (dtype or torch.bfloat16) and _within(out, x, w)
 
 
+@pytest.mark.parametrize("k,m", [(3072, 8192), (2048, 11264), (2048, 2048), (768, 3072), (5632, 2048), (72, 300), (16384, 2048)])
+def test_a_rows_numbers_do_not_depend_on_the_step(k, m):
+    """Large and small matrices, of this kernel and of the library (rows that are no multiple of 16, long ones): a row has the same bits in every
+    step of up to 32 rows, and in a larger one it is within the same bound."""
+    from quanta_b200.matmul import empty_rows, linear, linear_silu
+    x, w = _operands(33, k, m, k + m)
+    rows = []
+    for n in (1, 7, 8, 9, 16, 17, 31, 32, 33):
+        some = empty_rows(n, k, dtype=torch.bfloat16, device=DEV)
+        some.copy_(x[:n])
+        rows.append((n, linear(some, w, out_dtype=torch.float32), linear_silu(some, w)))
+    for n, out, act in rows:
+        assert _within(out, x[:n], w)
+        if n <= 32:
+            assert torch.equal(out, rows[-2][1][:n]), n
+            assert (act is None) == (rows[0][2] is None) and (act is None or torch.equal(act, rows[-2][2][:n])), n
+
+
 def test_what_hangs_on_the_product_stays_with_torch():
     from quanta_b200.matmul import linear
     x, w = _operands(3, 64, 32, 5)
