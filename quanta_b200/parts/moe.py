@@ -96,11 +96,25 @@ class SigmoidTopKExperts(FeedForward):
     # 8 of 2,112, 65 tokens 25 / 21; 512 of 4,096, 24 tokens 37 / 29, 48 57 / 29.  Up to 16 tokens one launch takes about 10.
     router_mma_min_tokens = 65
     router_mma_min_work = (17, 64 * 256 * 3072)      # or this many tokens, and more than this many products
-    # steps with at most this many rows an expert on average fetch the token rows inside the product (tiles of up to 32 rows one TMA box a
-    # row, larger ones four rows an instruction, the producer warp's lanes sharing them) instead of from a gathered copy.  Measured on a
-    # B200, 8 of 256 experts of 3,072 x 1,536, both products, copy / inside: 300 tokens 1,143 / 1,123 us, 536 1,179 / 1,164, 1,024 1,222 / 1,200,
-    # 2,048 1,322 / 1,355, 12,800 3,222 / 4,337 (boxes of one row each were the slower way from some 12 rows an expert on)
-    gather_in_kernel_max_rows = 32
+    # Steps with at most this many rows an expert on average fetch the token rows inside the product (tiles of up to 32 rows one TMA box a
+    # row, larger ones four rows an instruction, the producer warp's lanes sharing them) instead of from a gathered copy; experts wider
+    # than the second number, whose rows many blocks fetch, up to the third.  Measured on a B200, both products, copy / inside, us:
+    #   experts      width x inner     16 rows        24 rows        32 rows        48 rows
+    #   8 of 256    3,072 x 1,536    1,123 / 1,114  1,141 / 1,139  1,156 / 1,162  1,185 / 1,210
+    #   8 of 128    2,048 x   768      194 /   192    203 /   197    210 /   203    224 /   218
+    #   6 of  64    2,048 x 1,408      179 /   179    182 /   182    187 /   185    198 /   201
+    #   4 of  32    2,880 x 2,880      260 /   259    268 /   266    273 /   270    288 /   283
+    #   8 of  64    4,096 x 6,144    1,454 / 1,442  1,471 / 1,448  1,499 / 1,501  1,530 / 1,541
+    #   4 of  16    6,144 x 8,192      735 /   729    751 /   753    755 /   756    774 /   790
+    #   2 of   8    4,096 x 8,192      262 /   261    268 /   266    270 /   269    272 /   274
+    #   2 of   8    4,096 x 14,336     462 /   470    482 /   487    482 /   497    483 /   502
+    #   2 of   8    2,048 x 14,336     278 /   280    241 /   243    242 /   247    245 /   257
+    # (2 of 8 of 4,096 x 5,632: 204 / 204, 208 / 209, 210 / 214; boxes of one row each were the slower way from some 12 rows an expert on)
+    gather_in_kernel_max_rows, gather_in_kernel_max_inner, gather_in_kernel_wide_rows = 32, 8192, 10
+
+    def gathers_inside(self, n_pairs: int) -> bool:
+        rows = self.gather_in_kernel_max_rows if self.I <= self.gather_in_kernel_max_inner else self.gather_in_kernel_wide_rows
+        return n_pairs <= rows * self.E
 
     def path_for(self, x) -> str:
         ok16 = kernels.expert_gemm_tc_supported(x, self.H, self.I) and self.w13.dtype == torch.bfloat16
@@ -177,7 +191,7 @@ class SigmoidTopKExperts(FeedForward):
         w_down = None if ea[0] == kernels.EXPERT_ACT_CLAMPED else w.view(-1)
         if path == "tc":
             # bfloat16: TMA-fed tcgen05 products, weights as the 128-row operand, accumulators in TMEM
-            if n_pairs <= self.gather_in_kernel_max_rows * self.E:
+            if self.gathers_inside(n_pairs):
                 # the kernel fetches the pairs' token rows itself
                 kernels.expert_gemm_tc(self.first_product_mode, x, self.w13, act, sorted_pair, w.view(-1), plan,
                                        tile_expert, tile_row0, self.E, bm, ctx.status, gather_top_k=self.k,
