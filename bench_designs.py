@@ -294,9 +294,11 @@ def latent_decode(batch: int, context: int, heads: int, C: int, R: int, page: in
     pos = torch.full((batch,), context - 1, dtype=torch.int32, device=dev)
     req = torch.arange(batch, dtype=torch.int32, device=dev)
     st = k.new_status(dev)
-    blocks = -(-batch * heads // k.LATENT_MMA_ROWS) if k.latent_attend_uses_tensor_cores(torch.bfloat16, C, R) else batch * -(-heads // 8)
-    seen = min(context, window + k.LATENT_MMA_ROWS) if window else context
-    n_ranges = max(1, min(64, -(-296 // blocks), -(-seen // 128)))
+    seen = min(context, window + k.LATENT_MMA_ROWS) if window else context        # ranges: as the part cuts them
+    if k.latent_attend_uses_tensor_cores(torch.bfloat16, C, R):
+        n_ranges = max(1, min(64, 296 // max(-(-batch * heads // k.LATENT_MMA_ROWS), batch), -(-seen // 64)))
+    else:
+        n_ranges = max(1, min(64, -(-296 // (batch * -(-heads // 8))), -(-seen // 128)))
     opts = dict(gate=torch.randn(batch, heads, device=dev), float32_weights=True) if lotilix else {}
     starts = torch.arange(batch + 1, dtype=torch.int32, device=dev)
 

@@ -10,8 +10,8 @@
 // A column j of S never meets another column.  Sixteen lanes share one: lane p has its rows p + 16 n.  Its part of u^T S (and of the output)
 // is two sums, over the rows of even and of odd n in the order of n, added up; the sixteen parts meet two by two (lanes 8, 4, 2, 1 apart).
 // Both kernels below do exactly these operations, so a position's numbers depend neither on the cut nor on the batch, not even by rounding.
-// (Portions once ran in chunks of 16 tokens as products, 240 us for the prompt below, whose outputs were 1.7e-7 off float64 against 0.9e-7 here
-// and depended on what shared the step.)
+// (Portions once ran in chunks of 16 tokens as products, 270 us for the prompt below where the chain of that time took 403; their outputs were
+// 1.7e-7 off float64 against 1.1e-7 here, and depended on what shared the step.)
 //
 // The per-head RMS norm with gain and gate that follows is a kernel of the common unit (norm_embed.cu).
 #include "common.cuh"

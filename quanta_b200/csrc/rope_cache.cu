@@ -267,7 +267,7 @@ __device__ __forceinline__ float4 turned_pairs(float4 x, float c, float s, float
 __device__ __forceinline__ float4 negated(float4 v) { return make_float4(-v.x, -v.y, -v.z, -v.w); }
 
 template <typename IN, typename A, int HPW>
-__global__ void __launch_bounds__(HPW == 2 ? 1024 : 512, HPW == 2 ? 1 : 2)      // 64 registers: with 85 the 12,800 tokens take 276 us
+__global__ void __launch_bounds__(HPW == 2 ? 1024 : 512, HPW == 2 ? 1 : 2)
 qknorm_rope_heads_kernel(const IN* qkv, A* __restrict__ q_out, A* __restrict__ k_cache, A* __restrict__ v_cache,
                          const RopeArgs a) {
   qb_follow();

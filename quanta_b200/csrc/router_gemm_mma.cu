@@ -14,8 +14,8 @@
 // A work item is 128 experts x NT tokens of one range: tcgen05.mma with the experts as M and the tokens as N.  One warp copies by TMA, a
 // stage the three pieces' tiles and the tokens'; one issues twelve MMAs a chunk into one of two accumulators; eight add the finished
 // chunk, read from TMEM, to the totals in their registers while the next runs, and write these at an item's end, under the next item's
-// MMAs.  Bound by how many bytes of the next chunks can be on their way beside the one in work (three stages of up to 72 KB; with two of 80 the tensor
-// cores were busy 56 % of a block's time, L2 20 %).  256 experts of 3,072: 300 tokens 28.7 -> 14.4 us, 2,048 45 -> 18.4, 12,800 (60 TFLOP)
+// MMAs.  Bound by how many bytes of the next chunks can be on their way beside the one in work (three stages of up to 72 KB: the tensor
+// cores are busy 55 % of a block's time, L2 22 %).  256 experts of 3,072: 300 tokens 28.7 -> 14.4 us, 2,048 45 -> 18.4, 12,800 (60 GFLOP)
 // 210 -> 64; 768 of 6,144, 4,000 tokens 395 -> 103 (mma.sync from shared memory before; a block an item without the overlap: 81 us for the
 // 12,800).
 // Needs K % 8 == 0 (16-byte rows).

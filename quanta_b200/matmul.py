@@ -1,5 +1,5 @@
-"""Dense projections through the library GEMM (cuBLAS via torch), as the reference does its own
-(``nn.Linear``, src/quanta/minimax/attention.py:166-169).
+"""Dense projections (``nn.Linear`` in the reference, src/quanta/minimax/attention.py:166-169): products of a few rows by the framework's
+own kernels (``csrc/linear_few.cu`` in bfloat16, ``csrc/linear_rows.cu`` in float32), the others by the library's (cuBLAS via torch).
 
 float32 products run as true float32: TF32 and reduced-precision accumulation are switched off
 process-wide when the first engine is built.
@@ -27,8 +27,8 @@ def configure() -> None:
     _configured = True
 
 
-# The library's kernels for products of fewer rows than this are slower than its kernel for this many
-# (measured on B200, weights from HBM: 3072 x 6144 at 8 rows 37 us, at 32 rows 27 us), so activations of
+# The library's kernels for products of fewer rows than this (of matrices that the kernel for few rows does not take) are slower than its
+# kernel for this many (measured on B200, weights from HBM: 3072 x 6144 at 8 rows 37 us, at 32 rows 27 us), so activations of
 # small steps are laid out with spare rows and multiplied as MIN_ROWS rows.  Rows do not mix in a
 # product: what the spare rows hold never reaches a real row.
 MIN_ROWS = 32

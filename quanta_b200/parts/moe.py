@@ -90,10 +90,17 @@ class SigmoidTopKExperts(FeedForward):
     # cores) for float32 and for widths that are no multiple of 8.  QUANTA_B200_EXPERT_KERNELS=simt forces
     # the latter for the whole process (a knob for measurements).
     expert_kernels = os.environ.get("QUANTA_B200_EXPERT_KERNELS", "auto")
-    # Steps of fewer tokens take their logits on the CUDA cores, in one launch with selection and plan (and the float32 path always).  Their
-    # time grows with tokens x experts x width, that of the tensor cores' launches hardly; measured on a B200 with selection and plan, CUDA /
-    # tensor cores: 256 experts of 3,072, 65 tokens 31 / 27 us, 80 45 / 29 (a pass of 93 tokens 4,725 / 4,665, one of 64 the same),
-    # 8 of 2,112, 65 tokens 25 / 21; 512 of 4,096, 24 tokens 37 / 29, 48 57 / 29.  Up to 16 tokens one launch takes about 10.
+    # Steps of fewer tokens take their logits on the CUDA cores, in one launch with selection and plan (and the float32 path always).  Up to 16
+    # tokens that is the faster way; from 17 on the tensor cores' three launches are.  The two differ by float32 rounding, so the line is not
+    # at 17: batches that decode keep one router up to 64 tokens, as long as that costs them no more than some 8 us a layer.  Measured on a
+    # B200 with selection and plan, nothing beside them, CUDA / tensor cores, us:
+    #   tokens            16           17           24           32           40           64           65           95
+    #   256 of 3,072  13.7 / 17.8  22.5 / 18.1  23.1 / 17.9  23.3 / 18.3  25.2 / 18.4  25.5 / 20.3  26.2 / 20.6  40.9 / 20.7
+    #   8 of 2,112     8.7 / 15.4  18.7 / 15.6  18.8 / 15.7  18.3 / 15.5  17.4 / 15.6  17.8 / 15.4  18.5 / 15.1  18.5 / 15.4
+    #   128 of 2,048  10.1 / 16.7  18.6 / 16.8  18.4 / 16.6  18.6 / 17.0  19.1 / 17.0  19.1 / 18.0  19.7 / 18.2  21.7 / 18.1
+    #   512 of 4,096  20.3 / 21.9  28.9 / 22.1  30.2 / 22.3  30.7 / 22.9  47.7 / 23.1  57.2 / 22.9  58.2 / 23.4  74.6 / 23.1
+    #   256 of 7,168  22.7 / 18.9  39.1 / 19.2  40.7 / 19.4  41.1 / 19.2  71.2 / 19.5  72.4 / 19.7  72.7 / 19.8  103  / 19.7
+    # The last two cross the line of work at 25 and 28 tokens.
     router_mma_min_tokens = 65
     router_mma_min_work = (17, 64 * 256 * 3072)      # or this many tokens, and more than this many products
     # Steps with at most this many rows an expert on average fetch the token rows inside the product (tiles of up to 32 rows one TMA box a
